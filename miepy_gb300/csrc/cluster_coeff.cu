@@ -12,12 +12,6 @@
 // p > k r, as the reference's own values do.  A particle at the origin adds its own
 // coefficients.  One CTA per particle writes its contribution; a second kernel sums
 // the particles in index order (deterministic).
-//
-// Far field: E_angular / H_angular (sphere_cluster.py:393-426): the far-field
-// expansion expand_E_far (vsh/expansion.py:45-77) of every particle's p_scat about
-// its own centre, evaluated at points (R, theta, phi) about the origin, summed in
-// Cartesian components and returned as (E_theta, E_phi) at the point.  H uses the
-// swapped coefficients times hfac = -i sqrt(eps_b / mu_b) (expand_H_far, :96-108).
 
 #include <algorithm>
 #include <cstring>
@@ -29,7 +23,6 @@
 namespace {
 
 constexpr int kCCThreads = 256;
-constexpr int kLFF = GB_LMAX_MAX;                // largest order of the far-field kernel
 constexpr int kPMax = 2 * GB_LMAX_MAX + 2;      // orders p <= Lc + Lin + 1
 constexpr int kMUMax = 4 * GB_LMAX_MAX + 1;     // |mu| <= Lc + Lin
 
@@ -186,121 +179,6 @@ __global__ void k_cluster_sum(int N, int n2rc, const double2* __restrict__ contr
     out[e] = s;
 }
 
-// ---------------------------------------------------------------- far field --
-constexpr int kFFThreads = 128;
-
-__device__ double2 emn_cc(int m, int n) {
-    const double mag = sqrt((2.0 * n + 1) * tgamma((double)(n - m) + 1.0) /
-                            ((double)n * (n + 1) * tgamma((double)(n + m) + 1.0)));
-    switch (n & 3) {
-        case 0: return make_double2(mag, 0);
-        case 1: return make_double2(0, mag);
-        case 2: return make_double2(-mag, 0);
-        default: return make_double2(0, -mag);
-    }
-}
-
-__global__ void __launch_bounds__(kFFThreads)
-k_far_field(int N, int L, const double* __restrict__ pos, const double2* __restrict__ p_scat, double k,
-            double ox, double oy, double oz, int Npts, const double* __restrict__ R, const double* __restrict__ th,
-            const double* __restrict__ ph, int magnetic, double2 hfac, double2* __restrict__ out) {
-    const int rmax = L * (L + 2);
-    __shared__ double2 w[kLFF * (kLFF + 2)];       // E_mn (-i)^n
-    __shared__ double negf[kLFF * (kLFF + 2)];
-    for (int r = threadIdx.x; r < rmax; r += blockDim.x) {
-        int n = (int)floor(sqrt((double)r + 1.0));
-        while (n * n > r + 1) n--;
-        while ((n + 1) * (n + 1) <= r + 1) n++;
-        const int m = r + 1 - n * n - n;
-        w[r] = mul_ipow_cc(emn_cc(m, n), 3 * n);   // (-i)^n = i^(3n)
-        const int am = m < 0 ? -m : m;
-        negf[r] = (m < 0) ? (((am & 1) ? -1.0 : 1.0) * tgamma((double)(n - am) + 1.0) / tgamma((double)(n + am) + 1.0)) : 1.0;
-    }
-    __syncthreads();
-    const int pt = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pt >= Npts) return;
-    double st0, ct0, sp0, cp0;
-    sincos(th[pt], &st0, &ct0);
-    sincos(ph[pt], &sp0, &cp0);
-    const double X = ox + R[pt] * st0 * cp0, Y = oy + R[pt] * st0 * sp0, Z = oz + R[pt] * ct0;
-    double2 E[3] = {make_double2(0, 0), make_double2(0, 0), make_double2(0, 0)};
-    for (int i = 0; i < N; i++) {
-        const double dx = X - pos[3 * i], dy = Y - pos[3 * i + 1], dz = Z - pos[3 * i + 2];
-        const double rho2 = dx * dx + dy * dy;
-        const double rad = sqrt(rho2 + dz * dz);
-        const double rho = sqrt(rho2);
-        const double ct = dz / rad, st = rho / rad;
-        const double cph = rho2 > 0 ? dx / rho : 1.0, sph = rho2 > 0 ? dy / rho : 0.0;
-        double s, c;
-        sincos(k * rad, &s, &c);
-        const double2 fac = make_double2(c / (k * rad), s / (k * rad));   // e^{ikr} / (kr)
-        // Legendre P_n^m(ct), m >= 0, n <= L + 1
-        double P[kLFF + 2][kLFF + 2];
-        P[0][0] = 1.0;
-        for (int m = 1; m <= L + 1; m++) P[m][m] = (2 * m - 1) * st * P[m - 1][m - 1];
-        for (int m = 0; m <= L; m++) P[m + 1][m] = ct * (2 * m + 1) * P[m][m];
-        for (int m = 0; m <= L + 1; m++)
-            for (int n = m + 2; n <= L + 1; n++)
-                P[n][m] = ((2 * n - 1) * ct * P[n - 1][m] - (n + m - 1) * P[n - 2][m]) / (double)(n - m);
-        const bool axis = !(st > 0.0);
-        const double2* c0 = p_scat + (long long)i * 2 * rmax + (magnetic ? rmax : 0);
-        const double2* c1 = p_scat + (long long)i * 2 * rmax + (magnetic ? 0 : rmax);
-        double2 Et = make_double2(0, 0), Ep = make_double2(0, 0);
-        for (int n = 1; n <= L; n++) {
-            for (int m = -n; m <= n; m++) {
-                const int am = m < 0 ? -m : m;
-                const int r = n * n + n + m - 1;
-                double pi_v, tau_v;
-                if (axis) {
-                    const bool atpi = ct < 0;
-                    const double sgn = atpi ? (((n + 1) & 1) ? -1.0 : 1.0) : 1.0;
-                    const double sgt = atpi ? ((n & 1) ? -1.0 : 1.0) : 1.0;
-                    if (m == 1) { pi_v = sgn * n * (n + 1) / 2.0; tau_v = sgt * n * (n + 1) / 2.0; }
-                    else if (m == -1) { pi_v = sgn * 0.5; tau_v = -sgt * 0.5; }
-                    else { pi_v = 0.0; tau_v = 0.0; }
-                } else {
-                    pi_v = m / st * negf[r] * P[n][am];
-                    const double pm1 = (am >= 1) ? P[n][am - 1] : -P[n][1] / (double)(n * (n + 1));
-                    const double pp1 = (am + 1 <= n) ? P[n][am + 1] : 0.0;
-                    tau_v = negf[r] * 0.5 * ((n + am) * (n - am + 1) * pm1 - pp1);
-                }
-                // e^{i m phi}
-                double2 e = make_double2(1.0, 0.0), base = make_double2(cph, am == m ? sph : -sph);
-                for (int q = 0; q < am; q++) e = cmul(e, base);
-                const double2 f = cmul(cmul(fac, w[r]), e);
-                const double2 a = c0[r], b = c1[r];
-                const double2 u1 = make_double2(a.x * tau_v + b.x * pi_v, a.y * tau_v + b.y * pi_v);
-                const double2 u2 = make_double2(a.x * pi_v + b.x * tau_v, a.y * pi_v + b.y * tau_v);
-                const double2 t1 = cmul(f, u1);   // E_theta += i f (a tau + b pi)
-                Et.x += -t1.y;
-                Et.y += t1.x;
-                const double2 t2 = cmul(f, u2);   // E_phi -= f (a pi + b tau)
-                Ep.x -= t2.x;
-                Ep.y -= t2.y;
-            }
-        }
-        // (0, E_theta, E_phi) at the particle's angles -> Cartesian
-        const double th_[3] = {ct * cph, ct * sph, -st}, ph_[3] = {-sph, cph, 0.0};
-        for (int d = 0; d < 3; d++) {
-            E[d].x += Et.x * th_[d] + Ep.x * ph_[d];
-            E[d].y += Et.y * th_[d] + Ep.y * ph_[d];
-        }
-    }
-    // Cartesian -> (theta, phi) components at the point
-    const double tt[3] = {ct0 * cp0, ct0 * sp0, -st0}, pp[3] = {-sp0, cp0, 0.0};
-    double2 Eth = make_double2(0, 0), Eph = make_double2(0, 0);
-    for (int d = 0; d < 3; d++) {
-        Eth.x += E[d].x * tt[d]; Eth.y += E[d].y * tt[d];
-        Eph.x += E[d].x * pp[d]; Eph.y += E[d].y * pp[d];
-    }
-    if (magnetic) {
-        Eth = cmul(hfac, Eth);
-        Eph = cmul(hfac, Eph);
-    }
-    out[2LL * pt] = Eth;
-    out[2LL * pt + 1] = Eph;
-}
-
 }   // namespace
 
 extern "C" {
@@ -335,23 +213,6 @@ int gb_cluster_coefficients(int N, int lmax, const double* pos, const double* p_
     const int n2rc = 2 * lmax_to_rmax(lmax_cluster);
     gb::note_launch();
     k_cluster_sum<<<(n2rc + 127) / 128, 128, 0, s>>>(N, n2rc, contrib, reinterpret_cast<double2*>(p_cluster));
-    GB_CUDA_TRY(cudaGetLastError());
-    return GB_OK;
-}
-
-int gb_far_field(int N, int lmax, const double* pos, const double* p_scat, double k, const double* origin, int Npts,
-                 const double* radius, const double* theta, const double* phi, int magnetic, double hfac_re,
-                 double hfac_im, double* out, void* stream) {
-    if (N < 1 || Npts < 0 || !pos || !p_scat || !origin || !out) return gb_set_error(GB_BAD_ARG, "bad far-field arguments");
-    if (lmax < 1 || lmax > kLFF) return gb_set_error(GB_UNSUPPORTED, "far field supports lmax 1..%d", kLFF);
-    if (Npts == 0) return GB_OK;
-    if (!radius || !theta || !phi) return gb_set_error(GB_BAD_ARG, "null point arrays");
-    double o[3];
-    memcpy(o, origin, sizeof(o));
-    gb::note_launch();
-    k_far_field<<<(Npts + kFFThreads - 1) / kFFThreads, kFFThreads, 0, (cudaStream_t)stream>>>(
-        N, lmax, pos, reinterpret_cast<const double2*>(p_scat), k, o[0], o[1], o[2], Npts, radius, theta, phi,
-        magnetic, make_double2(hfac_re, hfac_im), reinterpret_cast<double2*>(out));
     GB_CUDA_TRY(cudaGetLastError());
     return GB_OK;
 }

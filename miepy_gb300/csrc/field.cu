@@ -1,499 +1,532 @@
-// K8: near field of a cluster on a set of points.
+// K8: fields of a cluster on a set of points.
 //
-// Follows sphere_cluster.E_field / H_field (sphere_cluster.py:244-391): outside
-// the spheres the outgoing expansions of p_scat about every particle are summed
-// (expand_E, vsh/expansion.py:13-42, VSH N/M of vsh/vsh_functions.py:40-78 /
-// cpp/src/vsh_functions.cpp:60-98, converted with vec_sph_to_cart); a point
-// inside sphere i instead takes the interior expansion of p_int[i] with
-// j_n(k_int r) (complex argument, the upward recurrence of
-// cpp/src/special.cpp:20-45).  H fields use expand_H: the polarisation-swapped
-// coefficients times -i sqrt(eps/mu).
+// Near field: sphere_cluster.E_field / H_field (sphere_cluster.py:244-391): outside the
+// spheres the outgoing expansions of p_scat about every particle are summed (expand_E,
+// vsh/expansion.py:13-42); a point inside sphere i instead takes the interior expansion
+// of p_int[i] with j_n(k_int r) (complex argument).  H fields use expand_H: the
+// polarisation-swapped coefficients times -i sqrt(eps/mu).  Far field: the far-field form
+// of the expansions (expand_E_far, vsh/expansion.py:45-77) at Cartesian points, or at
+// (R, theta, phi) about the origin in theta and phi components (E_angular / H_angular,
+// sphere_cluster.py:393-426).  The sums per (point, particle) are in expansion.cuh.
 //
-// One thread per point; particles are streamed through shared memory in tiles of
-// 16 with their coefficients; E_mn and the negative-order Legendre factors are
-// tabulated once per CTA.
+// k_field64 (FP64).  Bound by the FP64 pipe (a warp instruction per 64 cycles and SM
+// sub-partition), so a lane takes one point and the particles of a group of 32 points are
+// split over 1 to 8 warps, enough warps to fill every sub-partition evenly; the warps'
+// sums are added in order (deterministic).  The folded coefficients of a tile of
+// particles are formed by the CTA in shared memory.  Against a thread per point with FP64
+// trigonometry and complex divisions per mode: far fields at 7200 directions of 50
+// spheres, lmax 4, 3237 -> 355 us; a whole E_field call on 97 x 100 points around 25
+// spheres, lmax 4, 5.28 -> 1.40 ms (the kernel was 4.17 ms of it).
+//
+// k_field32 (FP32 exterior sums for large maps: a 512 x 512 plane around thousands of
+// spheres is ~5e8 point-particle terms).  Bound by the FP32 pipe; a thread takes two
+// points in packed f32x2 arithmetic and reads every folded coefficient once for both
+// (16-byte broadcast loads of duplicated pairs).  Coordinates are split into two floats so
+// that separations keep FP32 accuracy without FP64 arithmetic; k r is reduced with a
+// two-float k / pi, which the phase of distant spheres needs.  Points inside a sphere are
+// found by the FP32 distance, decided in FP64 and collected, so that their FP64 interior
+// expansions run on full warps.  512 x 512 points, 2000 spheres, lmax 3: 30.7 -> 7.6 ms
+// (526 instructions per 64 terms; with fewer than three warps per sub-partition, the
+// last of its 1.7 waves, the packed FMA pipe is 54 % busy).
 
-#include <vector>
+#include <algorithm>
 
+#include "expansion.cuh"
 #include "gb_common.cuh"
 #include "gb_internal.h"
 
 namespace {
 
-constexpr int kFieldThreads = 128;
+using namespace gbx;
+
+constexpr int kLF = 8;              // largest expansion order of the near-field kernels
+constexpr int kLFF = GB_LMAX_MAX;   // largest order of the angular far field
+constexpr int kTileBytes = 32 * 1024;
+
+struct FieldArgs {
+    int N, Npts, interior, swap;
+    const double* pos;
+    const double* radius;
+    const double2* p_scat;
+    const double2* p_int;
+    double k;
+    const double2* k_int;
+    const double* pts;                        // [Npts][3], or R, theta, phi
+    const double *th, *ph;
+    double ox, oy, oz;
+    double2 pref;                             // 1, or the magnetic prefactor
+    const double2* hfac_int;
+    double2* out;
+    FoldW fold;
+};
 
 __device__ __forceinline__ double2 cdivd(double2 a, double2 b) {
-    const double den = b.x * b.x + b.y * b.y;
-    return make_double2((a.x * b.x + a.y * b.y) / den, (a.y * b.x - a.x * b.y) / den);
-}
-__device__ __forceinline__ double2 cadd2(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 csin(double2 z) {
-    double s, c;
-    sincos(z.x, &s, &c);
-    return make_double2(s * cosh(z.y), c * sinh(z.y));
-}
-__device__ __forceinline__ double2 ccos(double2 z) {
-    double s, c;
-    sincos(z.x, &s, &c);
-    return make_double2(c * cosh(z.y), -s * sinh(z.y));
+    const double den = 1.0 / (b.x * b.x + b.y * b.y);
+    return make_double2((a.x * b.x + a.y * b.y) * den, (a.y * b.x - a.x * b.y) * den);
 }
 
-// E_mn = i^n sqrt((2n+1)(n-m)!/(n(n+1)(n+m)!))  (cpp/src/vsh_functions.cpp:56-58)
-__device__ double2 Emn(int m, int n) {
-    double mag = sqrt((2.0 * n + 1) * tgamma((double)(n - m) + 1.0) / ((double)n * (n + 1) * tgamma((double)(n + m) + 1.0)));
-    switch (n & 3) {
-        case 0: return make_double2(mag, 0);
-        case 1: return make_double2(0, mag);
-        case 2: return make_double2(-mag, 0);
-        default: return make_double2(0, -mag);
+// j_n of complex x, n = 0..L + 1.  The upward recurrence (the reference's,
+// cpp/src/special.cpp:20-45) multiplies its rounding errors by about
+// |y_n / j_n| ~ ((2n-1)!!)^2 / |x|^(2n+1) once n > |x|, so it serves only |x| >= L + 2;
+// below that the values come from Miller's downward recurrence
+// j_{n-1} = (2n+1)/x j_n - j_{n+1}, started at n = L + 26 from (j, j+1) = (1, 0) and
+// normalised by j_0 = sin(x)/x or j_1 = j_0/x - cos(x)/x, whichever is larger in modulus
+// (they have no common zero).
+template <int L>
+__device__ __forceinline__ void bessel_j(double2 x, double2 ix, double2 (&z)[L + 2]) {
+    constexpr int NP = L + 2;
+    double s, c, sh = 0.0, ch = 1.0;
+    sincos(x.x, &s, &c);
+    if (x.y != 0.0) {
+        sh = sinh(x.y);
+        ch = cosh(x.y);
     }
-}
-
-// Adds the expansion of coefficients c [2][rmax] about a particle to E (spherical
-// components, then Cartesian).  outgoing: h_n of real kr, factor i;
-// otherwise j_n of complex kr, factor -i.
-constexpr int kLF = 8;   // largest expansion order of the field kernel
-
-// far: the outgoing expansion's far-field form instead (expand_E_far,
-// vsh/expansion.py:45-77): no radial component, h_n(kr) -> (-i)^n e^{ikr} / (kr) with
-// E_theta = i f E_mn (-i)^n (c0 tau + c1 pi) e^{im phi},
-// E_phi = -f E_mn (-i)^n (c0 pi + c1 tau) e^{im phi}, f = e^{ikr} / (kr).
-__device__ void add_expansion(int L, const double2* __restrict__ c, int rmax, bool outgoing, double2 k, double rad,
-                              double theta, double phi, bool swap, double2 pref, const double2* __restrict__ emn,
-                              const double* __restrict__ negf_tab, double2 E[3], bool far = false) {
-    const int NP = L + 2;
-    // radial functions z_n and derivatives for n = 0..L (the reference's recurrences)
-    double2 z[kLF + 2], zp[kLF + 2];
-    const double2 kr = make_double2(k.x * rad, k.y * rad);
-    double2 ffar = make_double2(0, 0);
-    if (far) {
-        double s, co;
-        sincos(kr.x, &s, &co);
-        ffar = make_double2(co / kr.x, s / kr.x);
-    } else if (outgoing) {
-        const double x = kr.x;
-        double s, co;
-        sincos(x, &s, &co);
-        double j0 = s / x, y0 = -co / x;
-        z[0] = make_double2(j0, y0);
-        double j1 = j0 / x - co / x, y1 = y0 / x - j0;
-        if (NP > 1) z[1] = make_double2(j1, y1);
-        double ja = j0, jb = j1, ya = y0, yb = y1;
-#pragma unroll 1
+    const double2 e0 = cmul(make_double2(s * ch, c * sh), ix);
+    const double2 t1 = cmul(e0, ix), u1 = cmul(make_double2(c * ch, -s * sh), ix);
+    const double2 e1 = make_double2(t1.x - u1.x, t1.y - u1.y);
+    if (x.x * x.x + x.y * x.y >= (double)(NP * NP)) {
+        z[0] = e0;
+        z[1] = e1;
+#pragma unroll
         for (int n = 2; n < NP; n++) {
-            double jn = (2 * n - 1) / x * jb - ja, yn = (2 * n - 1) / x * yb - ya;
-            ja = jb; jb = jn; ya = yb; yb = yn;
-            z[n] = make_double2(jn, yn);
+            const double2 f = make_double2((2 * n - 1) * ix.x, (2 * n - 1) * ix.y);
+            const double2 a = cmul(f, z[n - 1]);
+            z[n] = make_double2(a.x - z[n - 2].x, a.y - z[n - 2].y);
         }
-    } else {
-        // j_n of complex argument.  The upward recurrence (the reference's,
-        // cpp/src/special.cpp:20-45) multiplies its rounding errors by about
-        // |y_n / j_n| ~ ((2n-1)!!)^2 / |kr|^(2n+1) once n > |kr|, so it serves only
-        // |kr| >= NP; below that the values come from Miller's downward recurrence
-        // j_{n-1} = (2n+1)/kr j_n - j_{n+1}, started at n = NP + 24 from (j, j+1) =
-        // (1, 0) and normalised by j_0 = sin(kr)/kr or j_1 = j_0/kr - cos(kr)/kr,
-        // whichever is larger in modulus (they have no common zero).
-        const double2 sz = csin(kr), cz = ccos(kr);
-        const double2 e0 = cdivd(sz, kr);
-        const double2 t1 = cdivd(e0, kr), u1 = cdivd(cz, kr);
-        const double2 e1 = make_double2(t1.x - u1.x, t1.y - u1.y);
-        if (hypot(kr.x, kr.y) >= (double)NP) {
-            z[0] = e0;
-            if (NP > 1) z[1] = e1;
+        return;
+    }
+    double2 hi = make_double2(0.0, 0.0), cur = make_double2(1.0, 0.0);   // j_{n+1}, j_n (unscaled)
+    auto down = [&](int n) {   // j_{n-1}
+        const double2 a = cmul(make_double2((2 * n + 1) * ix.x, (2 * n + 1) * ix.y), cur);
+        const double2 lo = make_double2(a.x - hi.x, a.y - hi.y);
+        hi = cur;
+        cur = lo;
+    };
 #pragma unroll 1
-            for (int n = 2; n < NP; n++) {
-                double2 f = cdivd(make_double2(2.0 * n - 1, 0), kr);
-                double2 a = cmul(f, z[n - 1]);
-                z[n] = make_double2(a.x - z[n - 2].x, a.y - z[n - 2].y);
-            }
-        } else {
-            double2 hi = make_double2(0.0, 0.0), cur = make_double2(1.0, 0.0);   // j_{n+1}, j_n (unscaled)
-#pragma unroll 1
-            for (int n = NP + 24; n >= 1; n--) {
-                const double2 f = cdivd(make_double2(2.0 * n + 1, 0), kr);
-                const double2 a = cmul(f, cur);
-                const double2 lo = make_double2(a.x - hi.x, a.y - hi.y);   // j_{n-1}
-                hi = cur;
-                cur = lo;
-                if (n - 1 < NP) z[n - 1] = lo;
-                if (fabs(cur.x) + fabs(cur.y) > 1e150) {   // keep the unnormalised values finite
-                    hi = make_double2(hi.x * 1e-150, hi.y * 1e-150);
-                    cur = make_double2(cur.x * 1e-150, cur.y * 1e-150);
-#pragma unroll 1
-                    for (int q = n - 1; q < NP; q++) z[q] = make_double2(z[q].x * 1e-150, z[q].y * 1e-150);
-                }
-            }
-            const bool use0 = !(NP > 1) || hypot(e0.x, e0.y) >= hypot(e1.x, e1.y);
-            const double2 s = use0 ? cdivd(e0, z[0]) : cdivd(e1, z[1]);
-#pragma unroll 1
-            for (int n = 0; n < NP; n++) z[n] = cmul(s, z[n]);
+    for (int n = NP + 24; n > NP; n--) {
+        down(n);
+        if (fabs(cur.x) + fabs(cur.y) > 1e150) {   // keep the unnormalised values finite
+            hi = make_double2(hi.x * 1e-150, hi.y * 1e-150);
+            cur = make_double2(cur.x * 1e-150, cur.y * 1e-150);
         }
     }
-    // derivative z_n' = z_{n-1} - (n+1)/kr z_n, n >= 1
-#pragma unroll 1
-    for (int n = 1; n <= L && !far; n++) {
-        double2 f = cdivd(make_double2((double)(n + 1), 0), kr);
-        double2 a = cmul(f, z[n]);
-        zp[n] = make_double2(z[n - 1].x - a.x, z[n - 1].y - a.y);
-    }
-    // Legendre P_n^m (m >= 0, no Condon-Shortley phase) for n <= L+1
-    const double x = cos(theta);
-    const double u = sqrt(fmax(0.0, (1.0 - x) * (1.0 + x)));
-    double P[kLF + 2][kLF + 3];
-#pragma unroll 1
-    for (int a = 0; a < L + 2; a++)
-#pragma unroll 1
-        for (int b = 0; b < L + 3; b++) P[a][b] = 0.0;
-    P[0][0] = 1.0;
-#pragma unroll 1
-    for (int m = 1; m <= L + 1; m++) P[m][m] = (2 * m - 1) * u * P[m - 1][m - 1];
-#pragma unroll 1
-    for (int m = 0; m <= L; m++) P[m + 1][m] = x * (2 * m + 1) * P[m][m];
-#pragma unroll 1
-    for (int m = 0; m <= L + 1; m++)
-#pragma unroll 1
-        for (int n = m + 2; n <= L + 1; n++)
-            P[n][m] = ((2 * n - 1) * x * P[n - 1][m] - (n + m - 1) * P[n - 2][m]) / (double)(n - m);
-    const bool at0 = (theta == 0.0), atpi = (theta == 3.14159265358979323846);
-    const double st = sin(theta), ct = x;
-    double sp, cp;
-    sincos(phi, &sp, &cp);
-    const double2 fac = outgoing ? make_double2(0, 1) : make_double2(0, -1);
-    double2 Es[3] = {make_double2(0, 0), make_double2(0, 0), make_double2(0, 0)};
-#pragma unroll 1
-    for (int n = 1; n <= L; n++) {
-#pragma unroll 1
-        for (int m = -n; m <= n; m++) {
-            const int am = m < 0 ? -m : m;
-            const int r = n * n + n + m - 1;
-            const double negf = negf_tab[r];
-            const double Pnm = negf * P[n][am];
-            double pi_v, tau_v;
-            if (at0 || atpi) {
-                const double sgn = atpi ? (((n + 1) & 1) ? -1.0 : 1.0) : 1.0;    // (-1)^(n+1) at pi
-                const double sgt = atpi ? ((n & 1) ? -1.0 : 1.0) : 1.0;          // (-1)^n at pi
-                if (m == 1) { pi_v = sgn * n * (n + 1) / 2.0; tau_v = sgt * n * (n + 1) / 2.0; }
-                else if (m == -1) { pi_v = sgn * 0.5; tau_v = -sgt * 0.5; }
-                else { pi_v = 0.0; tau_v = 0.0; }
-            } else {
-                pi_v = m / st * Pnm;
-                const double pm1 = (am >= 1) ? P[n][am - 1] : -P[n][1] / (double)(n * (n + 1));
-                const double pp1 = (am + 1 <= n) ? P[n][am + 1] : 0.0;
-                tau_v = negf * 0.5 * ((n + am) * (n - am + 1) * pm1 - pp1);
-            }
-            double sm, cm;
-            sincos((double)m * phi, &sm, &cm);
-            const double2 eph = make_double2(cm, sm);
-            if (far) {
-                const double2 c0 = swap ? c[rmax + r] : c[r];
-                const double2 c1 = swap ? c[r] : c[rmax + r];
-                // i f E_mn (-i)^n e^{im phi}
-                const double2 mi_n = (n & 3) == 0 ? make_double2(1, 0)
-                                   : (n & 3) == 1 ? make_double2(0, -1)
-                                   : (n & 3) == 2 ? make_double2(-1, 0) : make_double2(0, 1);
-                const double2 w = cmul(cmul(make_double2(0, 1), ffar), cmul(cmul(emn[r], mi_n), eph));
-                const double2 a = make_double2(c0.x * tau_v + c1.x * pi_v, c0.y * tau_v + c1.y * pi_v);
-                const double2 b = make_double2(c0.x * pi_v + c1.x * tau_v, c0.y * pi_v + c1.y * tau_v);
-                const double2 t1 = cmul(w, a), t2 = cmul(make_double2(0, 1), cmul(w, b));
-                Es[1].x += t1.x; Es[1].y += t1.y;
-                Es[2].x += t2.x; Es[2].y += t2.y;
-                continue;
-            }
-            const double2 H = z[n], Hp = zp[n];
-            // N: (n(n+1) P H/kr e, (H + kr H') e/kr tau, i (H + kr H') e/kr pi)
-            const double2 hk = cdivd(cmul(H, eph), kr);
-            const double2 g = cdivd(cmul(make_double2(H.x + (kr.x * Hp.x - kr.y * Hp.y), H.y + (kr.x * Hp.y + kr.y * Hp.x)), eph), kr);
-            const double2 N0 = make_double2(n * (n + 1) * Pnm * hk.x, n * (n + 1) * Pnm * hk.y);
-            const double2 N1 = make_double2(g.x * tau_v, g.y * tau_v);
-            const double2 N2 = make_double2(-g.y * pi_v, g.x * pi_v);
-            // M: (0, i pi H e, -tau H e)
-            const double2 he = cmul(H, eph);
-            const double2 M1 = make_double2(-he.y * pi_v, he.x * pi_v);
-            const double2 M2 = make_double2(-he.x * tau_v, -he.y * tau_v);
-            const double2 c0 = swap ? c[rmax + r] : c[r];
-            const double2 c1 = swap ? c[r] : c[rmax + r];
-            const double2 w = cmul(fac, emn[r]);
-            const double2 w0 = cmul(w, c0), w1 = cmul(w, c1);
-            double2 t;
-            t = cmul(w0, N0); Es[0].x += t.x; Es[0].y += t.y;
-            t = cadd2(cmul(w0, N1), cmul(w1, M1)); Es[1].x += t.x; Es[1].y += t.y;
-            t = cadd2(cmul(w0, N2), cmul(w1, M2)); Es[2].x += t.x; Es[2].y += t.y;
+#pragma unroll
+    for (int n = NP; n >= 1; n--) {
+        down(n);
+        z[n - 1] = cur;
+        if (fabs(cur.x) + fabs(cur.y) > 1e150) {
+            hi = make_double2(hi.x * 1e-150, hi.y * 1e-150);
+            cur = make_double2(cur.x * 1e-150, cur.y * 1e-150);
+#pragma unroll
+            for (int q = 0; q < NP; q++)
+                if (q >= n - 1) z[q] = make_double2(z[q].x * 1e-150, z[q].y * 1e-150);
         }
     }
-    // spherical -> Cartesian (vec_sph_to_cart), times the prefactor
-    const double rh[3] = {st * cp, st * sp, ct}, th[3] = {ct * cp, ct * sp, -st}, ph[3] = {-sp, cp, 0.0};
-    for (int d = 0; d < 3; d++) {
-        double2 v = make_double2(Es[0].x * rh[d] + Es[1].x * th[d] + Es[2].x * ph[d],
-                                 Es[0].y * rh[d] + Es[1].y * th[d] + Es[2].y * ph[d]);
-        v = cmul(pref, v);
-        E[d].x += v.x;
-        E[d].y += v.y;
-    }
+    const bool use0 = e0.x * e0.x + e0.y * e0.y >= e1.x * e1.x + e1.y * e1.y;
+    const double2 sc = use0 ? cdivd(e0, z[0]) : cdivd(e1, z[1]);
+#pragma unroll
+    for (int n = 0; n < NP; n++) z[n] = cmul(sc, z[n]);
 }
 
-__global__ void __launch_bounds__(kFieldThreads)
-k_field(int L, int N, const double* __restrict__ pos, const double* __restrict__ radius, const double2* __restrict__ p_scat,
-        const double2* __restrict__ p_int, double k, const double2* __restrict__ k_int, int Npts,
-        const double* __restrict__ pts, int interior, int magnetic, double2 hfac, const double2* __restrict__ hfac_int,
-        double2* __restrict__ out, int far) {
-    const int rmax = L * (L + 2);
-    constexpr int kTile = 16;
-    __shared__ double sp_pos[kTile][3];
-    __shared__ double2 sp_c[kTile * 2 * kLF * (kLF + 2)];
-    __shared__ double2 emn[kLF * (kLF + 2)];
-    __shared__ double negf_tab[kLF * (kLF + 2)];
-    for (int r = threadIdx.x; r < rmax; r += blockDim.x) {
-        int n = (int)floor(sqrt((double)r + 1.0));
-        while (n * n > r + 1) n--;
-        while ((n + 1) * (n + 1) <= r + 1) n++;
-        const int m = r + 1 - n * n - n;
-        emn[r] = Emn(m, n);
-        const int am = m < 0 ? -m : m;
-        negf_tab[r] = (m < 0) ? (((am & 1) ? -1.0 : 1.0) * tgamma((double)(n - am) + 1.0) / tgamma((double)(n + am) + 1.0)) : 1.0;
-    }
-    const int pt = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = pt < Npts;
-    double X = 0, Y = 0, Z = 0;
+// The interior field of sphere i at (X, Y, Z), written to out.
+template <int L>
+__device__ __noinline__ void interior_field(const FieldArgs& a, int i, double X, double Y, double Z, double2* out) {
+    constexpr int rmax = L * (L + 2);
+    const double dx = X - a.pos[3 * i], dy = Y - a.pos[3 * i + 1], dz = Z - a.pos[3 * i + 2];
+    const double rho2 = dx * dx + dy * dy;
+    double inv_r, r;
+    root(rho2 + dz * dz, inv_r, r);
+    Dir<double> d;
+    direction(dx, dy, dz, rho2, inv_r, d);
+    const double2 ki = a.k_int[i];
+    const double2 x = make_double2(ki.x * r, ki.y * r);
+    const double2 ix = cdivd(make_double2(1.0, 0.0), x);
+    double2 z[L + 2];
+    bessel_j<L>(x, ix, z);
+    const double2* ca = a.p_int + (long long)i * 2 * rmax + (a.swap ? rmax : 0);
+    const double2* cb = a.p_int + (long long)i * 2 * rmax + (a.swap ? 0 : rmax);
+    auto radial = [&](int n) {
+        const double2 q = cmul(make_double2(n * ix.x, n * ix.y), z[n]);
+        Rad<double> f;
+        f.zr = z[n].x; f.nzr = -z[n].x; f.zi = z[n].y; f.nzi = -z[n].y;
+        f.dr = z[n - 1].x - q.x; f.di = z[n - 1].y - q.y; f.ndi = -f.di;
+        f.hr = (n + 1) * q.x; f.hi = (n + 1) * q.y; f.nhi = -f.hi;
+        return f;
+    };
+    auto coef = [&](int n, int m, CV<double>(&v)[4]) {
+        double2 w[4];
+        fold_nm(a.fold, REGULAR, n, m, ca, cb, w);
+#pragma unroll
+        for (int q = 0; q < 4; q++) v[q] = CV<double>{w[q].x, w[q].y};
+    };
+    CV<double> Er{0, 0}, Et{0, 0}, Ep{0, 0}, E[3] = {{0, 0}, {0, 0}, {0, 0}};
+    expansion<L, REGULAR, double>(d, radial, coef, Er, Et, Ep);
+    add_cartesian<true, double>(d, Er, Et, Ep, E);
+    const double2 pref = a.hfac_int && a.swap ? a.hfac_int[i] : make_double2(1.0, 0.0);
+    for (int c = 0; c < 3; c++) out[c] = cmul(pref, make_double2(E[c].x, E[c].y));
+}
+
+// Item it of a tile's folding work: particle it / (entries), entry (n, m) in order.
+template <int L>
+__device__ __forceinline__ void fold_item(int e, int& n, int& m) {
+    n = 1;
+    while ((n + 1) * (n + 2) / 2 - 1 <= e) n++;
+    m = e - (n * (n + 1) / 2 - 1);
+}
+__host__ __device__ constexpr int fold_entries(int L) { return L * (L + 3) / 2; }   // (n, m), 1 <= n <= L, 0 <= m <= n
+template <int L>
+__host__ __device__ constexpr int fold_slot(int n, int m) { return m == 0 ? fold_n(n) : fold_n(n) + 3 + 4 * (m - 1); }
+
+// blockDim = 32 PG PS: warp w takes the points of group w / PS and the particles q with
+// q % PS == w % PS of every tile.  ANGULAR: points (R, theta, phi) about the origin, out
+// [Npts][2]; otherwise Cartesian points, out [Npts][3].
+template <int L, int FORM, bool ANGULAR>
+__global__ void __launch_bounds__(256) k_field64(const __grid_constant__ FieldArgs a, int PS) {
+    constexpr int rmax = L * (L + 2), NC = fold_count(L), NE = fold_entries(L);
+    constexpr int kTile = kTileBytes / (NC * 16) < 32 ? kTileBytes / (NC * 16) : 32;
+    static_assert(kTile >= 1, "a particle's coefficients fit in a tile");
+    __shared__ __align__(16) double2 tile[kTileBytes / 16];
+    __shared__ double spos[32][3];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, PG = (blockDim.x >> 5) / PS;
+    const int split = w % PS;
+    const int pt = (blockIdx.x * PG + w / PS) * 32 + lane;
+    const bool valid = pt < a.Npts;
+    double X = 0, Y = 0, Z = 0, st0 = 0, ct0 = 1, sp0 = 0, cp0 = 1;
     if (valid) {
-        X = pts[3LL * pt];
-        Y = pts[3LL * pt + 1];
-        Z = pts[3LL * pt + 2];
-    }
-    // interior test first (the reference overwrites interior points)
-    int inside = -1;
-    if (interior && valid) {
-        for (int i = 0; i < N; i++) {
-            const double dx = X - pos[3 * i], dy = Y - pos[3 * i + 1], dz = Z - pos[3 * i + 2];
-            if (dx * dx + dy * dy + dz * dz < radius[i] * radius[i]) inside = i;   // last match wins, as in the reference loop
+        if (ANGULAR) {
+            sincos(a.th[pt], &st0, &ct0);
+            sincos(a.ph[pt], &sp0, &cp0);
+            const double R = a.pts[pt];
+            X = a.ox + R * st0 * cp0;
+            Y = a.oy + R * st0 * sp0;
+            Z = a.oz + R * ct0;
+        } else {
+            X = a.pts[3LL * pt];
+            Y = a.pts[3LL * pt + 1];
+            Z = a.pts[3LL * pt + 2];
         }
     }
-    double2 E[3] = {make_double2(0, 0), make_double2(0, 0), make_double2(0, 0)};
-    const double2 pref_out = magnetic ? hfac : make_double2(1, 0);
-    for (int t0 = 0; t0 < N; t0 += kTile) {
-        const int cnt = min(kTile, N - t0);
+    const double ik = 1.0 / a.k;
+    int inside = -1;
+    CV<double> E[3] = {{0, 0}, {0, 0}, {0, 0}};
+    const int step = PS * (kTile / PS > 0 ? kTile / PS : 1);
+    for (int t0 = 0; t0 < a.N; t0 += step) {
+        const int cnt = min(step, a.N - t0);
         __syncthreads();
-        for (int e = threadIdx.x; e < cnt * 3; e += blockDim.x) sp_pos[e / 3][e % 3] = pos[3LL * t0 + e];
-        for (int e = threadIdx.x; e < cnt * 2 * rmax; e += blockDim.x)
-            sp_c[e] = p_scat[(long long)t0 * 2 * rmax + e];
+        for (int e = threadIdx.x; e < cnt * 3; e += blockDim.x) spos[e / 3][e % 3] = a.pos[3LL * t0 + e];
+        for (int e = threadIdx.x; e < cnt * NE; e += blockDim.x) {
+            const int q = e / NE;
+            int n, m;
+            fold_item<L>(e - q * NE, n, m);
+            const double2* c = a.p_scat + (long long)(t0 + q) * 2 * rmax;
+            double2 v[4];
+            fold_nm(a.fold, FORM, n, m, c + (a.swap ? rmax : 0), c + (a.swap ? 0 : rmax), v);
+            double2* dst = tile + q * NC + fold_slot<L>(n, m);
+            for (int i = 0; i < (m ? 4 : 3); i++) dst[i] = v[i];
+        }
         __syncthreads();
-        if (!valid || inside >= 0) continue;
-        for (int q = 0; q < cnt; q++) {
-            const double dx = X - sp_pos[q][0], dy = Y - sp_pos[q][1], dz = Z - sp_pos[q][2];
-            const double rad = sqrt(dx * dx + dy * dy + dz * dz);
-            const double theta = acos(dz / rad);
-            const double phi = atan2(dy, dx);
-            add_expansion(L, sp_c + q * 2 * rmax, rmax, true, make_double2(k, 0), rad, theta, phi, magnetic != 0,
-                          pref_out, emn, negf_tab, E, far != 0);
+        if (!valid) continue;
+#pragma unroll 1
+        for (int q = split; q < cnt; q += PS) {
+            const double dx = X - spos[q][0], dy = Y - spos[q][1], dz = Z - spos[q][2];
+            const double rho2 = dx * dx + dy * dy, r2 = rho2 + dz * dz;
+            if (FORM == OUTGOING && a.interior) {
+                const double rs = a.radius[t0 + q];
+                if (r2 < rs * rs) inside = t0 + q;   // the last match wins, as in the reference's loop
+            }
+            double inv_r, r;
+            root(r2, inv_r, r);
+            Dir<double> d;
+            direction(dx, dy, dz, rho2, inv_r, d);
+            double s, c;
+            sincos(a.k * r, &s, &c);
+            const double ix = ik * inv_r;
+            const double2* cf = tile + q * NC;
+            auto coef = [&](int n, int m, CV<double>(&v)[4]) {
+#pragma unroll
+                for (int i = 0; i < (m ? 4 : 3); i++) {
+                    const double2 u = cf[fold_slot<L>(n, m) + i];
+                    v[i] = CV<double>{u.x, u.y};
+                }
+            };
+            Outgoing<double> h;
+            if (FORM == OUTGOING) h.start(s, c, ix);
+            CV<double> Er{0, 0}, Et{0, 0}, Ep{0, 0};
+            expansion<L, FORM, double>(d, h, coef, Er, Et, Ep);
+            if (FORM == FAR) {   // e^{ikr} / (kr)
+                const double fr = c * ix, fi = s * ix;
+                CV<double> t{0, 0}, p{0, 0};
+                caxpy(t, fr, fi, -fi, Et);
+                caxpy(p, fr, fi, -fi, Ep);
+                Et = t;
+                Ep = p;
+            }
+            add_cartesian<FORM == OUTGOING, double>(d, Er, Et, Ep, E);
+        }
+    }
+    // the splits' sums, added in order by the group's first warp
+    if (PS > 1) {
+        __syncthreads();
+        double* red = reinterpret_cast<double*>(tile);           // [warps][6][32]
+        int* rin = reinterpret_cast<int*>(red + 8 * 6 * 32);     // [warps][32]
+        if (split) {
+            for (int c = 0; c < 3; c++) {
+                red[(w * 6 + 2 * c) * 32 + lane] = E[c].x;
+                red[(w * 6 + 2 * c + 1) * 32 + lane] = E[c].y;
+            }
+            rin[w * 32 + lane] = inside;
+        }
+        __syncthreads();
+        if (split) return;
+        for (int q = 1; q < PS; q++) {
+            for (int c = 0; c < 3; c++) {
+                E[c].x += red[((w + q) * 6 + 2 * c) * 32 + lane];
+                E[c].y += red[((w + q) * 6 + 2 * c + 1) * 32 + lane];
+            }
+            inside = max(inside, rin[(w + q) * 32 + lane]);
         }
     }
     if (!valid) return;
-    if (inside >= 0) {
-        const int i = inside;
-        const double dx = X - pos[3 * i], dy = Y - pos[3 * i + 1], dz = Z - pos[3 * i + 2];
-        const double rad = sqrt(dx * dx + dy * dy + dz * dz);
-        const double theta = acos(dz / rad);
-        const double phi = atan2(dy, dx);
-        const double2 pref = magnetic ? hfac_int[i] : make_double2(1, 0);
-        add_expansion(L, p_int + (long long)i * 2 * rmax, rmax, false, k_int[i], rad, theta, phi, magnetic != 0, pref,
-                      emn, negf_tab, E);
+    if (ANGULAR) {   // Cartesian -> (theta, phi) components at the point
+        const double tt[3] = {ct0 * cp0, ct0 * sp0, -st0}, pp[3] = {-sp0, cp0, 0.0};
+        double2 Eth = make_double2(0, 0), Eph = make_double2(0, 0);
+        for (int c = 0; c < 3; c++) {
+            Eth.x += E[c].x * tt[c]; Eth.y += E[c].y * tt[c];
+            Eph.x += E[c].x * pp[c]; Eph.y += E[c].y * pp[c];
+        }
+        a.out[2LL * pt] = cmul(a.pref, Eth);
+        a.out[2LL * pt + 1] = cmul(a.pref, Eph);
+        return;
     }
-    for (int d = 0; d < 3; d++) out[3LL * pt + d] = E[d];
+    if (FORM == OUTGOING && inside >= 0) {
+        if constexpr (FORM == OUTGOING) interior_field<L>(a, inside, X, Y, Z, a.out + 3LL * pt);
+        return;
+    }
+    for (int c = 0; c < 3; c++) a.out[3LL * pt + c] = cmul(a.pref, make_double2(E[c].x, E[c].y));
 }
 
 // ------------------------------------------------------------ FP32 field --
-// The same exterior sum in FP32 for large maps (a 512 x 512 plane around
-// thousands of spheres is ~1e9 point-particle terms): no trigonometry per term
-// beyond one sincosf of k r; angles enter through r-hat components, e^{i m phi}
-// by powering (x + i y)/rho.  Coefficients are pre-multiplied by i E_mn in shared
-// memory (tiles of 32 particles); separations are formed in FP64.  Points inside a
-// sphere take the FP64 interior expansion, as in k_field.
-constexpr int kTile32 = 32;
+constexpr int kThreads32 = 128;
+constexpr int kPoints32 = 2 * kThreads32;
 
-template <int LT>
-__global__ void __launch_bounds__(kFieldThreads)
-k_field32(int Lrun, int N, const double* __restrict__ pos, const double* __restrict__ radius,
-          const double2* __restrict__ p_scat, const double2* __restrict__ p_int, double k,
-          const double2* __restrict__ k_int, int Npts, const double* __restrict__ pts, int interior, int magnetic,
-          double2 hfac, const double2* __restrict__ hfac_int, double2* __restrict__ out) {
-    // LT > 0: lmax known at compile time, every per-term loop unrolled (arrays in
-    // registers); LT == 0: any lmax up to kLF
-    const int L = LT > 0 ? LT : Lrun;
-    const int rmax = L * (L + 2);
-    __shared__ double sp_pos[kTile32][3];
-    __shared__ float2 sw0[kTile32 * kLF * (kLF + 2)];
-    __shared__ float2 sw1[kTile32 * kLF * (kLF + 2)];
-    __shared__ double2 emn[kLF * (kLF + 2)];
-    __shared__ double negf_tab[kLF * (kLF + 2)];
-    __shared__ float negf32[kLF * (kLF + 2)];
-    for (int r = threadIdx.x; r < rmax; r += blockDim.x) {
-        int n = (int)floor(sqrt((double)r + 1.0));
-        while (n * n > r + 1) n--;
-        while ((n + 1) * (n + 1) <= r + 1) n++;
-        const int m = r + 1 - n * n - n;
-        emn[r] = Emn(m, n);
-        const int am = m < 0 ? -m : m;
-        negf_tab[r] = (m < 0) ? (((am & 1) ? -1.0 : 1.0) * tgamma((double)(n - am) + 1.0) / tgamma((double)(n + am) + 1.0)) : 1.0;
-        negf32[r] = (float)negf_tab[r];
+__device__ __forceinline__ float rsqrt_approx(float v) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+__device__ __forceinline__ float2 bc(float v) { return make_float2(v, v); }
+
+template <int L>
+__global__ void __launch_bounds__(kThreads32, L <= 4 ? 4 : 2)
+k_field32(const __grid_constant__ FieldArgs a, float kpi_h, float kpi_l, float ik) {
+    constexpr int rmax = L * (L + 2), NC = fold_count(L), NE = fold_entries(L);
+    constexpr int kTile = kTileBytes / (NC * 16) < 32 ? kTileBytes / (NC * 16) : 32;
+    __shared__ __align__(16) float4 tile[kTile * NC];   // (re, re, im, im)
+    __shared__ float4 spos[kTile][2];                   // x.h, y.h, z.h, test radius^2; x.l, y.l, z.l
+    __shared__ int n_in, list[kPoints32];
+    const int tid = threadIdx.x;
+    const long long p0 = (long long)blockIdx.x * kPoints32 + tid, p1 = p0 + kThreads32;
+    float2 Xh[3], Xl[3];
+    for (int c = 0; c < 3; c++) {
+        const double u = p0 < a.Npts ? a.pts[3 * p0 + c] : 0.0, v = p1 < a.Npts ? a.pts[3 * p1 + c] : 0.0;
+        Xh[c] = make_float2((float)u, (float)v);
+        Xl[c] = make_float2((float)(u - (double)Xh[c].x), (float)(v - (double)Xh[c].y));
     }
-    const int pt = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = pt < Npts;
-    double X = 0, Y = 0, Z = 0;
-    if (valid) {
-        X = pts[3LL * pt];
-        Y = pts[3LL * pt + 1];
-        Z = pts[3LL * pt + 2];
-    }
-    int inside = -1;
-    if (interior && valid) {
-        for (int i = 0; i < N; i++) {
-            const double dx = X - pos[3 * i], dy = Y - pos[3 * i + 1], dz = Z - pos[3 * i + 2];
-            if (dx * dx + dy * dy + dz * dz < radius[i] * radius[i]) inside = i;
-        }
-    }
-    const float kf = (float)k;
-    float Ex[2] = {0.f, 0.f}, Ey[2] = {0.f, 0.f}, Ez[2] = {0.f, 0.f};
-    for (int t0 = 0; t0 < N; t0 += kTile32) {
-        const int cnt = min(kTile32, N - t0);
+    if (tid == 0) n_in = 0;
+    int in0 = -1, in1 = -1;
+    const float2 zero = make_float2(0.f, 0.f);
+    CV<float2> E[3] = {{zero, zero}, {zero, zero}, {zero, zero}};
+    for (int t0 = 0; t0 < a.N; t0 += kTile) {
+        const int cnt = min(kTile, a.N - t0);
         __syncthreads();
-        for (int e = threadIdx.x; e < cnt * 3; e += blockDim.x) sp_pos[e / 3][e % 3] = pos[3LL * t0 + e];
-        for (int e = threadIdx.x; e < cnt * rmax; e += blockDim.x) {
-            const int q = e / rmax, r = e % rmax;
-            const double2* c = p_scat + (long long)(t0 + q) * 2 * rmax;
-            const double2 c0 = magnetic ? c[rmax + r] : c[r];
-            const double2 c1 = magnetic ? c[r] : c[rmax + r];
-            const double2 w = cmul(make_double2(0, 1), emn[r]);   // outgoing: factor i
-            const double2 a = cmul(w, c0), b = cmul(w, c1);
-            sw0[e] = make_float2((float)a.x, (float)a.y);
-            sw1[e] = make_float2((float)b.x, (float)b.y);
+        for (int q = tid; q < cnt; q += kThreads32) {
+            float h[3], l[3];
+            for (int c = 0; c < 3; c++) {
+                const double v = a.pos[3LL * (t0 + q) + c];
+                h[c] = (float)v;
+                l[c] = (float)(v - (double)h[c]);
+            }
+            // points nearer than this are decided in FP64
+            const double rs = a.interior ? a.radius[t0 + q] : 0.0;
+            spos[q][0] = make_float4(h[0], h[1], h[2], a.interior ? (float)(rs * rs * 1.0001) : -1.f);
+            spos[q][1] = make_float4(l[0], l[1], l[2], 0.f);
+        }
+        for (int e = tid; e < cnt * NE; e += kThreads32) {
+            const int q = e / NE;
+            int n, m;
+            fold_item<L>(e - q * NE, n, m);
+            const double2* c = a.p_scat + (long long)(t0 + q) * 2 * rmax;
+            double2 v[4];
+            fold_nm(a.fold, OUTGOING, n, m, c + (a.swap ? rmax : 0), c + (a.swap ? 0 : rmax), v);
+            float4* dst = tile + q * NC + fold_slot<L>(n, m);
+            for (int i = 0; i < (m ? 4 : 3); i++) {
+                const float x = (float)v[i].x, y = (float)v[i].y;
+                dst[i] = make_float4(x, x, y, y);
+            }
         }
         __syncthreads();
-        if (!valid || inside >= 0) continue;
+#pragma unroll 1
         for (int q = 0; q < cnt; q++) {
-            const float dx = (float)(X - sp_pos[q][0]), dy = (float)(Y - sp_pos[q][1]), dz = (float)(Z - sp_pos[q][2]);
-            const float rho2 = dx * dx + dy * dy;
-            const float r = sqrtf(rho2 + dz * dz);
-            const float inv_r = 1.f / r;
-            const float rho = sqrtf(rho2);
-            const float ct = dz * inv_r, st = rho * inv_r;
-            float cphi = 1.f, sphi = 0.f;
-            if (rho > 0.f) {
-                const float ir = 1.f / rho;
-                cphi = dx * ir;
-                sphi = dy * ir;
+            const float4 ph = spos[q][0], pl = spos[q][1];
+            // (Xh - ph) exactly by TwoSum, its error added to the low parts: the separation
+            // rounded once, as an FP64 difference rounded to FP32 would be
+            auto diff = [](float2 xh, float2 xl, float p_h, float p_l) {
+                const float2 p = bc(p_h), t = vsub(xh, p), bb = vsub(t, xh);
+                const float2 e = vsub(vsub(xh, vsub(t, bb)), vadd(p, bb));
+                return vadd(t, vadd(e, vsub(xl, bc(p_l))));
+            };
+            const float2 dx = diff(Xh[0], Xl[0], ph.x, pl.x), dy = diff(Xh[1], Xl[1], ph.y, pl.y),
+                         dz = diff(Xh[2], Xl[2], ph.z, pl.z);
+            const float2 rho2 = vfma(dx, dx, vmul(dy, dy));
+            const float2 r2 = vfma(dz, dz, rho2);
+            if (fminf(r2.x, r2.y) < ph.w) {   // perhaps inside: the last match wins
+                const double* pp = a.pos + 3LL * (t0 + q);
+                const double rs = a.radius[t0 + q];
+                auto test = [&](long long pt, int& in) {
+                    if (pt >= a.Npts) return;
+                    const double x = a.pts[3 * pt] - pp[0], y = a.pts[3 * pt + 1] - pp[1], z = a.pts[3 * pt + 2] - pp[2];
+                    if (x * x + y * y + z * z < rs * rs) in = t0 + q;
+                };
+                test(p0, in0);
+                test(p1, in1);
             }
-            // h_n(x) = j_n + i y_n, n = 0..L, by the upward recurrences
-            const float x = kf * r, ix = 1.f / x;
-            float sx, cx;
-            sincosf(x, &sx, &cx);
-            float hr[kLF + 1], hi[kLF + 1];
-            hr[0] = sx * ix;
-            hi[0] = -cx * ix;
-            hr[1] = hr[0] * ix - cx * ix;
-            hi[1] = hi[0] * ix - hr[0];
+            // r and 1/r, each corrected by a Newton step; likewise 1/rho
+            float2 ir = make_float2(rsqrt_approx(r2.x), rsqrt_approx(r2.y));
+            float2 r = vmul(r2, ir);
+            r = vfma(vfma(vneg(r), r, r2), vmul(bc(0.5f), ir), r);
+            ir = vfma(vfma(vneg(r), ir, bc(1.f)), ir, ir);
+            const bool ax0 = !(rho2.x > 1e-36f), ax1 = !(rho2.y > 1e-36f);   // phi = 0 on the z axis
+            float2 ih = make_float2(rsqrt_approx(rho2.x), rsqrt_approx(rho2.y));
+            float2 rho = vmul(rho2, ih);
+            rho = vfma(vfma(vneg(rho), rho, rho2), vmul(bc(0.5f), ih), rho);
+            ih = vfma(vfma(vneg(rho), ih, bc(1.f)), ih, ih);
+            Dir<float2> d;
+            d.ct = vmul(dz, ir);
+            d.st = vmul(rho, ir);
+            d.cp = vmul(dx, ih);
+            d.sp = vmul(dy, ih);
+            if (ax0) { d.st.x = 0.f; d.cp.x = 1.f; d.sp.x = 0.f; }
+            if (ax1) { d.st.y = 0.f; d.cp.y = 1.f; d.sp.y = 0.f; }
+            // k r = pi (2 j + f): f from the two-float k / pi
+            const float2 u = vmul(r, bc(kpi_h));
+            const float2 j = make_float2(2.f * rintf(0.5f * u.x), 2.f * rintf(0.5f * u.y));
+            const float2 f = vfma(r, bc(kpi_l), vfma(r, bc(kpi_h), vneg(j)));
+            float2 s, c;
+            sincospif(f.x, &s.x, &c.x);
+            sincospif(f.y, &s.y, &c.y);
+            Outgoing<float2> h;
+            h.start(s, c, vmul(ir, bc(ik)));
+            const float4* cf = tile + q * NC;
+            auto coef = [&](int n, int m, CV<float2>(&v)[4]) {
 #pragma unroll
-            for (int n = 2; n <= L; n++) {
-                const float f = (2 * n - 1) * ix;
-                hr[n] = f * hr[n - 1] - hr[n - 2];
-                hi[n] = f * hi[n - 1] - hi[n - 2];
-            }
-            // Legendre P_n^m(ct), m >= 0, no Condon-Shortley phase
-            float P[kLF + 1][kLF + 2];
-            P[0][0] = 1.f;
-#pragma unroll
-            for (int m = 1; m <= L; m++) P[m][m] = (2 * m - 1) * st * P[m - 1][m - 1];
-#pragma unroll
-            for (int m = 0; m < L; m++) P[m + 1][m] = ct * (2 * m + 1) * P[m][m];
-#pragma unroll
-            for (int m = 0; m <= L; m++)
-#pragma unroll
-                for (int n = m + 2; n <= L; n++)
-                    P[n][m] = ((2 * n - 1) * ct * P[n - 1][m] - (n + m - 1) * P[n - 2][m]) / (float)(n - m);
-            const bool axis = !(st > 0.f);
-            const float2* w0 = sw0 + q * rmax;
-            const float2* w1 = sw1 + q * rmax;
-            float Er[2] = {0.f, 0.f}, Et[2] = {0.f, 0.f}, Ep[2] = {0.f, 0.f};
-#pragma unroll
-            for (int n = 1; n <= L; n++) {
-                // radial parts: h_n / x and (x h_n)'/x = h_{n-1} - n h_n / x
-                const float hx_r = hr[n] * ix, hx_i = hi[n] * ix;
-                const float dr = hr[n - 1] - n * hx_r, di = hi[n - 1] - n * hx_i;
-                // e^{i m phi} for m = -n: conj((cphi + i sphi)^n)
-                float er = 1.f, ei = 0.f;
-                #pragma unroll
-                for (int s = 0; s < n; s++) {
-                    const float t = er * cphi + ei * sphi;   // multiply by e^{-i phi}
-                    ei = ei * cphi - er * sphi;
-                    er = t;
+                for (int i = 0; i < (m ? 4 : 3); i++) {
+                    const float4 w = cf[fold_slot<L>(n, m) + i];
+                    v[i] = CV<float2>{make_float2(w.x, w.y), make_float2(w.z, w.w)};
                 }
-#pragma unroll
-                for (int m = -n; m <= n; m++) {
-                    const int am = m < 0 ? -m : m;
-                    const int rr = n * n + n + m - 1;
-                    const float nf = negf32[rr];
-                    const float Pnm = nf * P[n][am];
-                    float pi_v, tau_v;
-                    if (axis) {
-                        const bool atpi = ct < 0.f;
-                        const float sgn = atpi ? (((n + 1) & 1) ? -1.f : 1.f) : 1.f;
-                        const float sgt = atpi ? ((n & 1) ? -1.f : 1.f) : 1.f;
-                        if (m == 1) { pi_v = sgn * n * (n + 1) * 0.5f; tau_v = sgt * n * (n + 1) * 0.5f; }
-                        else if (m == -1) { pi_v = sgn * 0.5f; tau_v = -sgt * 0.5f; }
-                        else { pi_v = 0.f; tau_v = 0.f; }
-                    } else {
-                        pi_v = m / st * Pnm;
-                        const float pm1 = (am >= 1) ? P[n][am - 1] : -P[n][1] / (float)(n * (n + 1));
-                        const float pp1 = (am + 1 <= n) ? P[n][am + 1] : 0.f;
-                        tau_v = nf * 0.5f * ((n + am) * (n - am + 1) * pm1 - pp1);
-                    }
-                    const float2 a = w0[rr], b = w1[rr];
-                    // u = a e, v = b e
-                    const float ur = a.x * er - a.y * ei, ui = a.x * ei + a.y * er;
-                    const float vr = b.x * er - b.y * ei, vi = b.x * ei + b.y * er;
-                    // N = (n(n+1) P h/x, d tau, i d pi) e ;  M = (0, i pi h, -tau h) e
-                    const float c0 = n * (n + 1) * Pnm;
-                    Er[0] += c0 * (ur * hx_r - ui * hx_i);
-                    Er[1] += c0 * (ur * hx_i + ui * hx_r);
-                    const float udr = ur * dr - ui * di, udi = ur * di + ui * dr;   // u d
-                    const float vhr = vr * hr[n] - vi * hi[n], vhi = vr * hi[n] + vi * hr[n];   // v h
-                    Et[0] += tau_v * udr - pi_v * vhi;
-                    Et[1] += tau_v * udi + pi_v * vhr;
-                    Ep[0] += -pi_v * udi - tau_v * vhr;
-                    Ep[1] += pi_v * udr - tau_v * vhi;
-                    const float t = er * cphi - ei * sphi;   // e <- e e^{i phi}
-                    ei = er * sphi + ei * cphi;
-                    er = t;
-                }
-            }
-            // spherical -> Cartesian
-            const float rh0 = st * cphi, rh1 = st * sphi, rh2 = ct;
-            const float th0 = ct * cphi, th1 = ct * sphi, th2 = -st;
-            const float ph0 = -sphi, ph1 = cphi;
-            for (int c = 0; c < 2; c++) {
-                Ex[c] += Er[c] * rh0 + Et[c] * th0 + Ep[c] * ph0;
-                Ey[c] += Er[c] * rh1 + Et[c] * th1 + Ep[c] * ph1;
-                Ez[c] += Er[c] * rh2 + Et[c] * th2;
-            }
+            };
+            CV<float2> Er{zero, zero}, Et{zero, zero}, Ep{zero, zero};
+            expansion<L, OUTGOING, float2>(d, h, coef, Er, Et, Ep);
+            add_cartesian<true, float2>(d, Er, Et, Ep, E);
         }
     }
-    if (!valid) return;
-    double2 E[3];
-    if (inside >= 0) {
-        E[0] = E[1] = E[2] = make_double2(0, 0);
-        const int i = inside;
-        const double dx = X - pos[3 * i], dy = Y - pos[3 * i + 1], dz = Z - pos[3 * i + 2];
-        const double rad = sqrt(dx * dx + dy * dy + dz * dz);
-        const double theta = acos(dz / rad);
-        const double phi = atan2(dy, dx);
-        const double2 pref = magnetic ? hfac_int[i] : make_double2(1, 0);
-        add_expansion(L, p_int + (long long)i * 2 * rmax, rmax, false, k_int[i], rad, theta, phi, magnetic != 0, pref,
-                      emn, negf_tab, E);
-    } else {
-        const double2 pref = magnetic ? hfac : make_double2(1, 0);
-        E[0] = cmul(pref, make_double2(Ex[0], Ex[1]));
-        E[1] = cmul(pref, make_double2(Ey[0], Ey[1]));
-        E[2] = cmul(pref, make_double2(Ez[0], Ez[1]));
+    auto store = [&](long long pt, int in, bool second) {
+        if (pt >= a.Npts) return;
+        if (in >= 0) {
+            list[atomicAdd(&n_in, 1)] = tid + (second ? kThreads32 : 0);
+            // the sphere's index waits in the point's own output (read back below)
+            a.out[3 * pt] = make_double2((double)in, 0.0);
+            return;
+        }
+        for (int c = 0; c < 3; c++)
+            a.out[3 * pt + c] = cmul(a.pref, second ? make_double2(E[c].x.y, E[c].y.y) : make_double2(E[c].x.x, E[c].y.x));
+    };
+    store(p0, in0, false);
+    store(p1, in1, true);
+    __syncthreads();
+    for (int e = tid; e < n_in; e += kThreads32) {
+        const long long pt = (long long)blockIdx.x * kPoints32 + list[e];
+        const int i = (int)a.out[3 * pt].x;
+        interior_field<L>(a, i, a.pts[3 * pt], a.pts[3 * pt + 1], a.pts[3 * pt + 2], a.out + 3 * pt);
     }
-    for (int d = 0; d < 3; d++) out[3LL * pt + d] = E[d];
+}
+
+template <int L, int FORM, bool ANGULAR>
+int launch64(const FieldArgs& a, cudaStream_t s) {
+    // splits of the particles: enough warps for three per SM sub-partition
+    const long long groups = ((long long)a.Npts + 31) / 32, want = 12LL * gb::sm_count();
+    int PS = 1;
+    while (PS < 8 && 2 * PS <= a.N && groups * PS < want) PS *= 2;
+    const int PG = groups * PS >= want && PS < 4 ? 4 / PS : 1;
+    const unsigned grid = (unsigned)((groups + PG - 1) / PG);
+    gb::note_launch();
+    k_field64<L, FORM, ANGULAR><<<grid, 32 * PG * PS, 0, s>>>(a, PS);
+    GB_CUDA_TRY(cudaGetLastError());
+    return GB_OK;
+}
+
+template <int L>
+int launch32(const FieldArgs& a, cudaStream_t s) {
+    const double kpi = a.k / 3.14159265358979323846;
+    const float h = (float)kpi, l = (float)(kpi - (double)h);
+    gb::note_launch();
+    k_field32<L><<<(unsigned)((a.Npts + (long long)kPoints32 - 1) / kPoints32), kThreads32, 0, s>>>(a, h, l,
+                                                                                                    (float)(1.0 / a.k));
+    GB_CUDA_TRY(cudaGetLastError());
+    return GB_OK;
+}
+
+FieldArgs field_args(int N, const double* pos, const double* p_scat, double k, int Npts, const double* pts, int magnetic,
+                     double hfac_re, double hfac_im, double* out) {
+    FieldArgs a{};
+    a.N = N;
+    a.Npts = Npts;
+    a.swap = magnetic != 0;
+    a.pos = pos;
+    a.p_scat = reinterpret_cast<const double2*>(p_scat);
+    a.k = k;
+    a.pts = pts;
+    a.pref = magnetic ? make_double2(hfac_re, hfac_im) : make_double2(1.0, 0.0);
+    a.out = reinterpret_cast<double2*>(out);
+    static const FoldW w = fold_weights();
+    a.fold = w;
+    return a;
+}
+
+// one instance per order
+#define GB_BY_LMAX8(CALL)                                            \
+    switch (lmax) {                                                  \
+        case 1: return CALL(1);                                      \
+        case 2: return CALL(2);                                      \
+        case 3: return CALL(3);                                      \
+        case 4: return CALL(4);                                      \
+        case 5: return CALL(5);                                      \
+        case 6: return CALL(6);                                      \
+        case 7: return CALL(7);                                      \
+        default: return CALL(8);                                     \
+    }
+
+int near_field(bool fp32, int N, int lmax, const double* pos, const double* radius, const double* p_scat,
+               const double* p_int, double k, const double* k_int, int Npts, const double* pts, int interior,
+               int magnetic, double hfac_re, double hfac_im, const double* hfac_int, double* out, void* stream) {
+    if (N < 1 || Npts < 0 || !pos || !p_scat || !pts || !out) return gb_set_error(GB_BAD_ARG, "bad field arguments");
+    if (interior && (!radius || !p_int || !k_int)) return gb_set_error(GB_BAD_ARG, "interior fields need radius, p_int, k_int");
+    if (magnetic && interior && !hfac_int) return gb_set_error(GB_BAD_ARG, "interior H fields need hfac_int");
+    if (Npts == 0) return GB_OK;
+    if (lmax < 1 || lmax > kLF) return gb_set_error(GB_UNSUPPORTED, "near field supports lmax 1..%d (got %d)", kLF, lmax);
+    FieldArgs a = field_args(N, pos, p_scat, k, Npts, pts, magnetic, hfac_re, hfac_im, out);
+    a.interior = interior != 0;
+    a.radius = radius;
+    a.p_int = reinterpret_cast<const double2*>(p_int);
+    a.k_int = reinterpret_cast<const double2*>(k_int);
+    a.hfac_int = reinterpret_cast<const double2*>(hfac_int);
+    const cudaStream_t s = (cudaStream_t)stream;
+#define GB_F32(Lv) launch32<Lv>(a, s)
+#define GB_F64(Lv) launch64<Lv, OUTGOING, false>(a, s)
+    if (fp32) GB_BY_LMAX8(GB_F32)
+    GB_BY_LMAX8(GB_F64)
+#undef GB_F32
+#undef GB_F64
 }
 
 }   // namespace
@@ -502,24 +535,17 @@ extern "C" int gb_near_field(int N, int lmax, const double* pos, const double* r
                              const double* p_int, double k, const double* k_int, int Npts, const double* pts,
                              int interior, int magnetic, double hfac_re, double hfac_im, const double* hfac_int,
                              double* out, void* stream) {
-    if (N < 1 || Npts < 0 || !pos || !p_scat || !pts || !out) return gb_set_error(GB_BAD_ARG, "bad field arguments");
-    if (interior && (!radius || !p_int || !k_int)) return gb_set_error(GB_BAD_ARG, "interior fields need radius, p_int, k_int");
-    if (magnetic && interior && !hfac_int) return gb_set_error(GB_BAD_ARG, "interior H fields need hfac_int");
-    if (Npts == 0) return GB_OK;
-    cudaStream_t s = (cudaStream_t)stream;
-    const unsigned grid = (unsigned)((Npts + kFieldThreads - 1) / kFieldThreads);
-    const double2 hf = make_double2(hfac_re, hfac_im);
-    const double2* pi2 = reinterpret_cast<const double2*>(p_int);
-    const double2* ps2 = reinterpret_cast<const double2*>(p_scat);
-    const double2* ki2 = reinterpret_cast<const double2*>(k_int);
-    const double2* hi2 = reinterpret_cast<const double2*>(hfac_int);
-    double2* o2 = reinterpret_cast<double2*>(out);
-    if (lmax < 1 || lmax > kLF) return gb_set_error(GB_UNSUPPORTED, "near field supports lmax 1..%d (got %d)", kLF, lmax);
-    gb::note_launch();
-    k_field<<<grid, kFieldThreads, 0, s>>>(lmax, N, pos, radius, ps2, pi2, k, ki2, Npts, pts, interior, magnetic, hf,
-                                           hi2, o2, 0);
-    GB_CUDA_TRY(cudaGetLastError());
-    return GB_OK;
+    return near_field(false, N, lmax, pos, radius, p_scat, p_int, k, k_int, Npts, pts, interior, magnetic, hfac_re,
+                      hfac_im, hfac_int, out, stream);
+}
+
+// Same arguments and result as gb_near_field, with the exterior sums in FP32.
+extern "C" int gb_near_field32(int N, int lmax, const double* pos, const double* radius, const double* p_scat,
+                               const double* p_int, double k, const double* k_int, int Npts, const double* pts,
+                               int interior, int magnetic, double hfac_re, double hfac_im, const double* hfac_int,
+                               double* out, void* stream) {
+    return near_field(true, N, lmax, pos, radius, p_scat, p_int, k, k_int, Npts, pts, interior, magnetic, hfac_re,
+                      hfac_im, hfac_int, out, stream);
 }
 
 // The far-field form of every particle's outgoing expansion, summed at the points
@@ -532,34 +558,30 @@ extern "C" int gb_far_field_expansions(int N, int lmax, const double* pos, const
     if (N < 1 || Npts < 0 || !pos || !p_scat || !pts || !out) return gb_set_error(GB_BAD_ARG, "bad field arguments");
     if (lmax < 1 || lmax > kLF) return gb_set_error(GB_UNSUPPORTED, "far field supports lmax 1..%d (got %d)", kLF, lmax);
     if (Npts == 0) return GB_OK;
-    cudaStream_t s = (cudaStream_t)stream;
-    const unsigned grid = (unsigned)((Npts + kFieldThreads - 1) / kFieldThreads);
-    gb::note_launch();
-    k_field<<<grid, kFieldThreads, 0, s>>>(lmax, N, pos, nullptr, reinterpret_cast<const double2*>(p_scat), nullptr, k,
-                                           nullptr, Npts, pts, 0, magnetic, make_double2(hfac_re, hfac_im), nullptr,
-                                           reinterpret_cast<double2*>(out), 1);
-    GB_CUDA_TRY(cudaGetLastError());
-    return GB_OK;
+    const FieldArgs a = field_args(N, pos, p_scat, k, Npts, pts, magnetic, hfac_re, hfac_im, out);
+    const cudaStream_t s = (cudaStream_t)stream;
+#define GB_FAR(Lv) launch64<Lv, FAR, false>(a, s)
+    GB_BY_LMAX8(GB_FAR)
+#undef GB_FAR
 }
 
-// Same arguments and result as gb_near_field, with the exterior sums in FP32.
-extern "C" int gb_near_field32(int N, int lmax, const double* pos, const double* radius, const double* p_scat,
-                               const double* p_int, double k, const double* k_int, int Npts, const double* pts,
-                               int interior, int magnetic, double hfac_re, double hfac_im, const double* hfac_int,
-                               double* out, void* stream) {
-    if (N < 1 || Npts < 0 || !pos || !p_scat || !pts || !out) return gb_set_error(GB_BAD_ARG, "bad field arguments");
-    if (interior && (!radius || !p_int || !k_int)) return gb_set_error(GB_BAD_ARG, "interior fields need radius, p_int, k_int");
-    if (magnetic && interior && !hfac_int) return gb_set_error(GB_BAD_ARG, "interior H fields need hfac_int");
+extern "C" int gb_far_field(int N, int lmax, const double* pos, const double* p_scat, double k, const double* origin,
+                            int Npts, const double* radius, const double* theta, const double* phi, int magnetic,
+                            double hfac_re, double hfac_im, double* out, void* stream) {
+    if (N < 1 || Npts < 0 || !pos || !p_scat || !origin || !out) return gb_set_error(GB_BAD_ARG, "bad far-field arguments");
+    if (lmax < 1 || lmax > kLFF) return gb_set_error(GB_UNSUPPORTED, "far field supports lmax 1..%d", kLFF);
     if (Npts == 0) return GB_OK;
-    if (lmax < 1 || lmax > kLF) return gb_set_error(GB_UNSUPPORTED, "near field supports lmax 1..%d (got %d)", kLF, lmax);
-    const unsigned grid = (unsigned)((Npts + kFieldThreads - 1) / kFieldThreads);
-    auto kfn = lmax == 1 ? k_field32<1> : lmax == 2 ? k_field32<2> : lmax == 3 ? k_field32<3>
-             : lmax == 4 ? k_field32<4> : k_field32<0>;
-    gb::note_launch();
-    kfn<<<grid, kFieldThreads, 0, (cudaStream_t)stream>>>(
-        lmax, N, pos, radius, reinterpret_cast<const double2*>(p_scat), reinterpret_cast<const double2*>(p_int), k,
-        reinterpret_cast<const double2*>(k_int), Npts, pts, interior, magnetic, make_double2(hfac_re, hfac_im),
-        reinterpret_cast<const double2*>(hfac_int), reinterpret_cast<double2*>(out));
-    GB_CUDA_TRY(cudaGetLastError());
-    return GB_OK;
+    if (!radius || !theta || !phi) return gb_set_error(GB_BAD_ARG, "null point arrays");
+    FieldArgs a = field_args(N, pos, p_scat, k, Npts, radius, magnetic, hfac_re, hfac_im, out);
+    a.th = theta;
+    a.ph = phi;
+    a.ox = origin[0];   // host array
+    a.oy = origin[1];
+    a.oz = origin[2];
+    const cudaStream_t s = (cudaStream_t)stream;
+#define GB_ANG(Lv) launch64<Lv, FAR, true>(a, s)
+    if (lmax == 9) return GB_ANG(9);
+    if (lmax == 10) return GB_ANG(10);
+    GB_BY_LMAX8(GB_ANG)
+#undef GB_ANG
 }
