@@ -54,6 +54,7 @@
 #include "gb_common.cuh"
 #include "gb_internal.h"
 #include "solve_plan.cuh"
+#include "solve_team.h"
 
 namespace {
 
@@ -2399,6 +2400,25 @@ __global__ void k_scale_t(const double2* __restrict__ t, const double2* __restri
         out[e] = cmul(t[e], d[e]);
 }
 
+// The single-launch solve (solve_team.cu) in the solver's workspace: states at off_state,
+// the error flag and barrier counters in the refinement states' place, the operand
+// vectors and partial dots in the vectors' place; one readback at the end.
+int team_route(const gb::TeamPlan& tp, const Plan& P, const gb::SysDev* dsys, int dense_D, const double2* mat,
+               const double2* tvec, const double* b, double* x, double tol, int maxiter, unsigned char* base, const WS& w,
+               int* status, int* iters, double* resid, cudaStream_t stream) {
+    KState* st = reinterpret_cast<KState*>(base + w.off_state);
+    DevPlan D{};
+    D.err = reinterpret_cast<int*>(base + w.off_ostate);
+    int e = gb::team_solve(tp, P.nsys, dsys, dense_D, P.R, mat, tvec, reinterpret_cast<const double2*>(b),
+                           reinterpret_cast<double2*>(x), st, D.err, reinterpret_cast<double2*>(base + w.off_vec),
+                           P.total_vec, tol, maxiter, stream);
+    if (e) return e;
+    std::vector<KState> h;
+    e = read_state(D, st, P.nsys * P.R, h, stream);
+    if (e) return e;
+    return finish_status(h.data(), P.nsys * P.R, status, iters, resid);
+}
+
 // pdiag (optional): the diagonal right preconditioner of run_bicgstab for every
 // BiCGSTAB of the solve (the mixed method's refinement residuals stay unpreconditioned).
 // mat_tc (optional, R = 4 or 8): the bf16 tiles of the tensor-core pass, used for
@@ -2411,6 +2431,23 @@ int solve_impl(const Plan& P, int prec, double tol, int maxiter, double inner_to
                cudaStream_t stream, const void* mat_tc = nullptr, const double* pdiag = nullptr) {
     const int pol32 = mat_tc ? 3 : 1;
     const void* m32 = mat_tc ? mat_tc : static_cast<const void*>(mat64);
+    // small FP64 systems in one launch
+    if (prec == GB_PREC_FP64 && !pdiag && !P.tmat) {
+        int Dmax = 0;
+        for (const gb::SysDev& d : P.sd) Dmax = std::max(Dmax, d.D);
+        const gb::TeamPlan tp = gb::team_plan(P.nsys, Dmax, R, true);
+        if (tp.ok) {
+            void* dsys = nullptr;
+            int slot = 0;
+            int e = gb::stage_acquire(P.sd.data(), sizeof(gb::SysDev) * P.nsys, stream, &dsys, &slot);
+            if (e) return e;
+            const double2* t2 = reinterpret_cast<const double2*>(tvec);
+            e = team_route(tp, P, static_cast<const gb::SysDev*>(dsys), 0, reinterpret_cast<const double2*>(mat128), t2, b,
+                           x, tol, maxiter, base, w, status, iters, resid, stream);
+            const int e2 = gb::stage_release(slot, stream);   // the solve has synchronised (or failed)
+            return e ? e : e2;
+        }
+    }
     DevPlan D;
     int e = upload_plan(P, base, w, stream, D);
     if (e) return e;
@@ -2916,6 +2953,10 @@ int gb_solve_dense(int D, int R, const double* T, const double* b, double* x, do
     WS w = ws_layout(P, GB_PREC_FP64, true);
     if (ws_bytes < w.total) return gb_set_error(GB_OVER_BUDGET, "workspace %zu B < required %zu B", ws_bytes, w.total);
     unsigned char* base = static_cast<unsigned char*>(workspace);
+    const gb::TeamPlan tp = gb::team_plan(1, D, R, false);
+    if (tp.ok)
+        return team_route(tp, P, nullptr, D, reinterpret_cast<const double2*>(T), nullptr, b, x, tol, maxiter, base, w,
+                          status, iters, resid, s);
     DevPlan Dp;
     int e = upload_plan(P, base, w, s, Dp);
     if (e) return e;
@@ -2957,6 +2998,10 @@ int gb_solve_dense_noalloc(int D, int R, const double* T, const double* b, doubl
     unsigned char* base = nullptr;
     int e = noalloc_scratch(&base);
     if (e) return e;
+    const gb::TeamPlan tp = gb::team_plan(1, D, R, false);
+    if (tp.ok)
+        return team_route(tp, P, nullptr, D, reinterpret_cast<const double2*>(T), nullptr, b, x, tol, maxiter, base, w,
+                          status, iters, resid, s);
     DevPlan Dp;
     e = upload_plan_pageable(P, base, w, s, Dp);
     if (e) return e;
