@@ -14,10 +14,24 @@
 //   y_w[r] = eps(r) sig(r) t_i[rho(r)] x_i[rho(r)]      (for block row j)
 // and (A_ij z_j)[r] = eps(r) c_u[rho(r)],  (S A_ij S z_i)[r] = sig(r) eps(r) c_w[rho(r)].
 // Column sums let a warp stream a block row by row with every lane owning fixed
-// columns: 128-bit coalesced loads, per-lane accumulators, no per-row cross-lane
-// reduction.  A lane owns NS "slots" (row offset, column group) so that RPS rows
-// are covered per step by all 32 lanes; slot sums of one column are combined in
-// shared memory once per block.
+// columns: per-lane accumulators, no per-row cross-lane reduction.
+//
+// Half a block.  A block is [[P, Q], [Q, P]] over the two polarisations (translation
+// mixes them symmetrically), so its first rmax rows hold all of it, and in the sums and
+// differences of the polarisations it is diagonal: with y+- = (y[r] +- y[rmax + r]) / 2,
+//   c+- [s] = sum_{r < rmax} (P +- Q)[r][s] y+-[r],
+//   c[s] = c+[s] + c-[s],  c[rmax + s] = c+[s] - c-[s].
+// The products therefore read the upper half of every block and take half the
+// multiplications; a column index 2 s + (0: +, 1: -) has a fixed sign per lane.  Blocks of
+// up to kWholeB columns (lmax <= 3) read the upper half too, but run through all rows of
+// the block, taking the lower ones from the upper ones' other half: their passes are bound
+// by the copies and the work per block rather than by the multiplications, and the sums
+// stay those of the block itself, to the last bit, so that quantities that cancel (the
+// torque on a lossless sphere) keep their residues.
+// Per pass, before and after: complex64 N = 200, lmax 4, R = 2 66 -> 51 us; N = 97, lmax 8
+// 131 -> 73 us; N = 2000, lmax 3 2.26 -> 1.86 ms; double-float N = 200, lmax 4, R = 2 292
+// -> 172 us, one pair of eight right-hand sides 404 -> 172 us (its own y plane: two CTAs
+// per SM instead of one); complex128 N = 61, lmax 5 155 -> 97 us.
 //
 // Three arithmetic policies share the kernel:
 //   Pol64  complex128 matrix, FP64 FMAs (the plain method);
@@ -120,6 +134,10 @@ __device__ __forceinline__ float2 shfl_xor(float2 a, int o) {
     return make_float2(__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o));
 }
 template <typename C> __device__ __forceinline__ C czero() { C z; z.x = 0; z.y = 0; return z; }
+__device__ __forceinline__ double2 half(double2 a) { return make_double2(0.5 * a.x, 0.5 * a.y); }
+__device__ __forceinline__ float2 half(float2 a) { return make_float2(0.5f * a.x, 0.5f * a.y); }
+
+constexpr int kWholeB = 30;   // largest block that is summed row by row, not in +- combinations
 
 // ---------------------------------------------- programmatic dependent launch --
 // The kernels of a BiCGSTAB iteration are launched with programmatic stream
@@ -179,13 +197,14 @@ GB_KS_CFIELD(beta)
 
 enum { ST_RUNNING = -1 };
 
+__device__ __forceinline__ float2 bc(float v) { return make_float2(v, v); }
+
 // --------------------------------------------------------------- policies --
 // Arithmetic of the GEMV.  A lane multiplies one matrix element m by the y
 // values of its row; complex products use packed f32x2 FMAs where the policy is
 // FP32-based: with m = (re, im) as loaded,
 //   a += m * y.re,  b += m * y.im,  and m y = (a.x - b.y, a.y + b.x),
 // so no shuffling of m is needed and each complex multiply-add is two FFMA2.
-__device__ __forceinline__ float2 bc(float v) { return make_float2(v, v); }
 __device__ __forceinline__ float2 neg2(float2 v) { return make_float2(-v.x, -v.y); }
 
 // (h, l) += p exactly (TwoSum on both components), error into l
@@ -217,6 +236,12 @@ struct Pol64 {                 // complex128 matrix, FP64 FMAs
     __device__ static M load(const unsigned char* hi, const unsigned char*, unsigned off) {
         return M{*reinterpret_cast<const double2*>(hi + off)};
     }
+    // P + sign Q of the elements at offP and offQ
+    __device__ static M load(const unsigned char* hi, const unsigned char*, unsigned offP, unsigned offQ, float sign) {
+        const double2 p = *reinterpret_cast<const double2*>(hi + offP), q = *reinterpret_cast<const double2*>(hi + offQ);
+        const unsigned neg = sign < 0.f ? 1u : 0u;
+        return M{make_double2(p.x + flipd(q.x, neg), p.y + flipd(q.y, neg))};
+    }
     __device__ static void zero(Acc& a) { a = make_double2(0, 0); }
     __device__ static void prep(M&) {}
     __device__ static void mac(Acc& a, const M& m, const YT& y) { cfma(a, m.h, y); }
@@ -237,6 +262,10 @@ struct Pol32 {                 // complex64 matrix, packed FP32 FMAs
     struct M { float2 h; };
     __device__ static M load(const unsigned char* hi, const unsigned char*, unsigned off) {
         return M{*reinterpret_cast<const float2*>(hi + off)};
+    }
+    __device__ static M load(const unsigned char* hi, const unsigned char*, unsigned offP, unsigned offQ, float sign) {
+        return M{__ffma2_rn(bc(sign), *reinterpret_cast<const float2*>(hi + offQ),
+                            *reinterpret_cast<const float2*>(hi + offP))};
     }
     __device__ static void zero(Acc& s) { s.a = s.b = make_float2(0, 0); }
     __device__ static void prep(M&) {}
@@ -269,6 +298,18 @@ struct PolDF {
         M m;
         m.h = *reinterpret_cast<const float2*>(hi + off);
         m.l = *reinterpret_cast<const float2*>(lo + off);
+        return m;
+    }
+    // P + sign Q as a double-float: the high words by TwoSum, its error with the low words
+    __device__ static M load(const unsigned char* hi, const unsigned char* lo, unsigned offP, unsigned offQ, float sign) {
+        const float2 sg = bc(sign);
+        const float2 ph = *reinterpret_cast<const float2*>(hi + offP), pl = *reinterpret_cast<const float2*>(lo + offP);
+        const float2 qh = __fmul2_rn(sg, *reinterpret_cast<const float2*>(hi + offQ));
+        M m;
+        m.h = __fadd2_rn(ph, qh);
+        const float2 bb = fsub2(m.h, ph);
+        m.l = __fadd2_rn(fsub2(ph, fsub2(m.h, bb)), fsub2(qh, bb));
+        m.l = __fadd2_rn(m.l, __ffma2_rn(sg, *reinterpret_cast<const float2*>(lo + offQ), pl));
         return m;
     }
     __device__ static void zero(Acc& s) { s.ha = s.la = s.hb = s.lb = make_float2(0, 0); }
@@ -340,12 +381,55 @@ template <> __device__ __forceinline__ float4 make_y<2>(double2 z) {
     return make_float4(hx, hy, __double2float_rn(z.x - (double)hx), __double2float_rn(z.y - (double)hy));
 }
 
-// Layout: [D][R] interleaved (element (row, rr) at vec_off + row*R + rr).
+// z's +- combinations over the polarisations (see the top of the file): the row (k, 2 r +
+// sigma) of a y vector holds (z[r] +- z[rmax + r]) / 2, sigma 0 for +.  sig(rmax + r) =
+// -sig(r), so Yw's are sig(r) times Yu's of the other sign.  Planes of pl (1 or 2)
+// right-hand sides, each [D][pl], follow each other within the cluster's segment, so that
+// a matrix pass copies only its own right-hand sides.  Small blocks (kWholeB) keep z
+// itself in their planes; YK 3 (the tensor-core pass): z as [D][R].
+template <int YK, typename C>
+__device__ __forceinline__ void store_y(const gb::SysDev& S, int part, int r, int rr, int R, int pl, C z0, C z1,
+                                        unsigned sneg, typename YType<YK>::t* __restrict__ Yu,
+                                        typename YType<YK>::t* __restrict__ Yw) {
+    if constexpr (YK == 3) {
+        const long long o = S.vec_off + ((long long)part * S.B + r) * R + rr, o1 = o + (long long)S.rmax * R;
+        Yu[o] = make_y<YK>(z0);
+        Yu[o1] = make_y<YK>(z1);
+        Yw[o] = make_y<YK>(cflip(z0, sneg));
+        Yw[o1] = make_y<YK>(cflip(z1, sneg ^ 1u));
+    } else if (S.B <= kWholeB) {
+        const long long o = S.vec_off + (long long)(rr / pl) * pl * S.D + ((long long)part * S.B + r) * pl + rr % pl;
+        const long long o1 = o + (long long)S.rmax * pl;
+        Yu[o] = make_y<YK>(z0);
+        Yu[o1] = make_y<YK>(z1);
+        Yw[o] = make_y<YK>(cflip(z0, sneg));
+        Yw[o1] = make_y<YK>(cflip(z1, sneg ^ 1u));
+    } else {
+        const long long o = S.vec_off + (long long)(rr / pl) * pl * S.D + ((long long)part * S.B + 2 * r) * pl + rr % pl;
+        const C yp = half(cadd(z0, z1)), ym = half(csub(z0, z1));
+        Yu[o] = make_y<YK>(yp);
+        Yu[o + pl] = make_y<YK>(ym);
+        Yw[o] = make_y<YK>(cflip(ym, sneg));
+        Yw[o + pl] = make_y<YK>(cflip(yp, sneg));
+    }
+}
+
+// t x with its rounding fixed (which of the two products is fused is otherwise the
+// compiler's choice in each kernel)
+template <typename C> __device__ __forceinline__ C tmul(C t, C x) {
+    C z;
+    z.x = fma(t.x, x.x, -(t.y * x.y));
+    z.y = fma(t.x, x.y, t.y * x.x);
+    return z;
+}
+
+// One thread per (row of the first polarisation, rhs), for the rows of both; x is [D][R]
+// interleaved (element (row, rr) at vec_off + row*R + rr).  blockDim = kVRows / 2 * R.
 template <int YK, typename VT, int R>
-__global__ void __launch_bounds__(kVRows)
+__global__ void __launch_bounds__(kVRows / 2 * R)
 k_yprep(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items, int nitems, const KState* __restrict__ st,
         int mask_mode, const double2* __restrict__ tvec, const VT* __restrict__ x, typename YType<YK>::t* __restrict__ Yu,
-        typename YType<YK>::t* __restrict__ Yw, YUpd<VT> up) {
+        typename YType<YK>::t* __restrict__ Yw, YUpd<VT> up, int pl) {
     const int it = blockIdx.x;
     if (it >= nitems) {
         pdl_wait();
@@ -354,49 +438,42 @@ k_yprep(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items, int 
     // prologue on plan data and the Mie vector (constant during a solve)
     const Item I = items[it];
     const gb::SysDev S = sys[I.sys];
-    const int lr = threadIdx.x;
-    const bool row_ok = lr < I.nr;
-    const int row = I.r0 + (row_ok ? lr : 0);
-    const int part = row / S.B, Rr = row % S.B;
-    const int info = __ldg(S.rowinfo + Rr);
+    const int hr = threadIdx.x / R, rr = threadIdx.x - hr * R;
+    const bool row_ok = 2 * hr < I.nr;
+    const int h = I.r0 / 2 + (row_ok ? hr : 0);
+    const int part = h / S.rmax, r = h - part * S.rmax;
+    const int info = __ldg(S.rowinfo + r);   // of (0, r); the other polarisation's signs are opposite
     const int rho = info & ((1 << 29) - 1);
     const unsigned eneg = (info >> 29) & 1, sneg = (info >> 30) & 1;
-    const long long src = (long long)part * S.B + rho;
     using C = typename Arith<VT>::C;
     using T = typename Arith<VT>::T;
     const T tg{};
-    const C t = to_c<C>(tvec[S.t_off + src]);
+    const long long src = (long long)part * S.B + rho;
+    const C t0 = to_c<C>(tvec[S.t_off + src]), t1 = to_c<C>(tvec[S.t_off + src + S.rmax]);
     pdl_wait();
     pdl_trigger();
     if (!row_ok || !any_active<R>(st, I.sys, mask_mode)) return;
-#pragma unroll
-    for (int rr = 0; rr < R; rr++) {
-        const long long es = S.vec_off + src * R + rr;
-        C xv;
-        if (up.kind != 0 && active_rhs<R>(st, I.sys, rr, 0)) {
-            // the BiCGSTAB vector update this product's input needs, on the source row
-            // this thread alone reads: p = r + beta (p - omega v) or s = r - alpha v
-            const KState& k = st[I.sys * R + rr];
-            const C rv = to_c<C>(up.r[es]), vv = to_c<C>(up.v[es]);
-            C nv;
-            if (up.kind == 1) {
-                const C pv = to_c<C>(up.out[es]);
-                nv = cadd(rv, cmul(ks_beta(k, tg), csub(pv, cmul(ks_omega(k, tg), vv))));
-            } else {
-                nv = csub(rv, cmul(ks_alpha(k, tg), vv));
-            }
-            const VT q = from_c<VT>(nv);
-            up.out[es] = q;
-            xv = to_c<C>(q);
+    const bool update = up.kind != 0 && active_rhs<R>(st, I.sys, rr, 0);
+    auto source = [&](long long es) -> C {
+        if (!update) return to_c<C>(x[es]);
+        // the BiCGSTAB vector update this product's input needs, on the source row
+        // this thread alone reads: p = r + beta (p - omega v) or s = r - alpha v
+        const KState& k = st[I.sys * R + rr];
+        const C rv = to_c<C>(up.r[es]), vv = to_c<C>(up.v[es]);
+        C nv;
+        if (up.kind == 1) {
+            const C pv = to_c<C>(up.out[es]);
+            nv = cadd(rv, cmul(ks_beta(k, tg), csub(pv, cmul(ks_omega(k, tg), vv))));
         } else {
-            xv = to_c<C>(x[es]);
+            nv = csub(rv, cmul(ks_alpha(k, tg), vv));
         }
-        const C yu = cflip(cmul(t, xv), eneg);
-        const C yw = cflip(yu, sneg);
-        const long long o = S.vec_off + (long long)row * R + rr;
-        Yu[o] = make_y<YK>(yu);
-        Yw[o] = make_y<YK>(yw);
-    }
+        const VT q = from_c<VT>(nv);
+        up.out[es] = q;
+        return to_c<C>(q);
+    };
+    const long long es = S.vec_off + src * R + rr;
+    const C z0 = cflip(tmul(t0, source(es)), eneg), z1 = cflip(tmul(t1, source(es + (long long)S.rmax * R)), eneg ^ 1u);
+    store_y<YK>(S, part, r, rr, R, pl, z0, z1, sneg, Yu, Yw);
 }
 
 // y vectors of clusters of general particles (the T-matrix overload of the
@@ -404,13 +481,13 @@ k_yprep(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items, int 
 // (I + T_agg) x = x + A (T x) with the packed translation blocks A).  One CTA per
 // particle (an item of the reduce plan): it applies the BiCGSTAB vector update of
 // the particle's rows, keeps the updated vector in shared memory, then forms
-// z = eps(r) (T x)[rho(r)] for every row r with the particle's T-matrix: complex64
+// z = eps(r) (T x)[rho(r)] for every row r with the particle's T-matrix, complex64
 // in FP32 arithmetic for the FP32 solver, complex128 in FP64 otherwise.
 template <int YK, typename VT, int R>
 __global__ void __launch_bounds__(kRBThreads)
 k_yprep_tmat(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items, int nitems,
              const KState* __restrict__ st, int mask_mode, const VT* __restrict__ x,
-             typename YType<YK>::t* __restrict__ Yu, typename YType<YK>::t* __restrict__ Yw, YUpd<VT> up) {
+             typename YType<YK>::t* __restrict__ Yu, typename YType<YK>::t* __restrict__ Yw, YUpd<VT> up, int pl) {
     const int it = blockIdx.x;
     if (it >= nitems) {
         pdl_wait();
@@ -422,7 +499,7 @@ k_yprep_tmat(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items,
     using T = typename Arith<VT>::T;
     const T tg{};
     const int B = S.B, part = I.r0 / B, tid = threadIdx.x;
-    __shared__ C xs[kRBThreads];   // [B][R], B R <= kRBThreads
+    __shared__ C xs[kRBThreads], zs[kRBThreads];   // [B][R], B R <= kRBThreads
     pdl_wait();
     pdl_trigger();
     if (!any_active<R>(st, I.sys, mask_mode)) return;   // the same for the whole CTA
@@ -453,7 +530,7 @@ k_yprep_tmat(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items,
         const int r = tid / R, rr = tid - r * R;
         const int info = __ldg(S.rowinfo + r);
         const int rho = info & ((1 << 29) - 1);
-        const unsigned eneg = (info >> 29) & 1, sneg = (info >> 30) & 1;
+        const unsigned eneg = (info >> 29) & 1;
         C z = czero<C>();
         if constexpr (std::is_same<C, float2>::value) {
             const float2* Tr = S.tmat64 + ((long long)part * B + rho) * B;
@@ -462,11 +539,14 @@ k_yprep_tmat(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items,
             const double2* Tr = S.tmat128 + ((long long)part * B + rho) * B;
             for (int c = 0; c < B; c++) cfma(z, __ldg(Tr + c), xs[c * R + rr]);
         }
-        const C yu = cflip(z, eneg);
-        const C yw = cflip(yu, sneg);
-        const long long o = S.vec_off + ((long long)part * B + r) * R + rr;
-        Yu[o] = make_y<YK>(yu);
-        Yw[o] = make_y<YK>(yw);
+        zs[tid] = cflip(z, eneg);
+    }
+    __syncthreads();
+    const int HR = S.rmax * R;
+    if (tid < HR) {
+        const int r = tid / R, rr = tid - r * R;
+        const unsigned sneg = ((unsigned)__ldg(S.rowinfo + r) >> 30) & 1u;
+        store_y<YK>(S, part, r, rr, R, pl, zs[tid], zs[HR + tid], sneg, Yu, Yw);
     }
 }
 
@@ -544,13 +624,13 @@ struct GemvLayout {
 // producer runs S-1 chunks ahead of the consumer, so with cpb chunks per block the
 // y_u of at most 1 + ceil((S-1)/cpb) blocks are live: the first chunk of block
 // b + nys is issued only once every chunk of block b has been consumed.  (All
-// blocks of one launch have the block size Bmax.)
-__host__ __device__ inline GemvLayout gemv_layout(int Bmax, int rows_per_chunk, int RT, int S, int mat_bytes, bool df,
+// blocks of one launch have the block size Bmax; a pass reads Bmax / 2 rows of each.)
+__host__ __device__ inline GemvLayout gemv_layout(int Bmax, int rows_per_chunk, int RR, int S, int mat_bytes, bool df,
                                                   int y_bytes) {
     GemvLayout g;
     g.chunk_cap = ((rows_per_chunk * Bmax * mat_bytes) + 127) & ~127;
-    g.y_bytes = (Bmax * RT * y_bytes + 127) & ~127;
-    const int cpb = (Bmax + rows_per_chunk - 1) / rows_per_chunk;
+    g.y_bytes = (Bmax * RR * y_bytes + 127) & ~127;
+    const int cpb = (Bmax / 2 + rows_per_chunk - 1) / rows_per_chunk;
     const int live = 1 + (S - 1 + cpb - 1) / cpb;
     g.nys = live < S ? live : S;
     // + 256 B of padding (kGemvPad): lanes whose columns lie past the block's end
@@ -560,12 +640,13 @@ __host__ __device__ inline GemvLayout gemv_layout(int Bmax, int rows_per_chunk, 
 }
 
 // Row-lane mapping: LPR lanes share a matrix row, RPW = 32/LPR rows per step;
-// lane (ro, cl) owns the columns cl + LPR*k (k < CPL) of its row, so one y load
-// serves CPL elements and the smem reads of a row are contiguous across lanes.
+// lane (ro, cl) owns the +- columns cl + LPR*k (k < CPL) of its row, all of one sign
+// (LPR is even: column 2 s + sigma, sigma = cl & 1), so one y load serves CPL elements;
+// a +- pair of lanes reads the same two matrix elements.
 // Column sums of the RPW rows are combined by shuffles once per block.  A chunk
 // is G steps (G*RPW rows, the last chunk of a block may be shorter).
-// RR right-hand sides per launch (rr0 .. rr0+RR-1), RT the row stride of y and
-// of the partials.
+// RR right-hand sides per launch (rr0 .. rr0+RR-1: plane rr0 / RR of the y vectors), RT
+// the row stride of the partials.
 template <class Pol, int RR, int RT, int LPR, int CPL, int G, int S>
 __global__ void __launch_bounds__(kGemvThreads)
 k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, long long sbeg, long long send,
@@ -579,12 +660,15 @@ k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, lo
     constexpr int MB = Pol::MB;
     constexpr bool DF = Pol::DF;
     constexpr int RPW = 32 / LPR;
-    constexpr int RC = G * RPW;   // rows per full chunk
+    // the +- columns, or a small block's own rows: then a chunk is a block's upper half
+    constexpr bool PM = LPR * CPL > kWholeB + 2;
+    const int RC = PM ? G * RPW : Bmax / 2;   // rows per full chunk
     const int rr0 = (RR == RT) ? 0 : rr0_rt;
     extern __shared__ __align__(128) unsigned char gemv_smem[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int ro = lane / LPR, cl = lane % LPR;
-    const GemvLayout lay = gemv_layout(Bmax, RC, RT, S, MB, DF, sizeof(YT));
+    const GemvLayout lay = gemv_layout(Bmax, RC, RR, S, MB, DF, sizeof(YT));
+    const float sign = (cl & 1) ? -1.f : 1.f;
     unsigned char* wbase = gemv_smem + (size_t)wid * lay.warp_bytes;
     uint64_t* bars = reinterpret_cast<uint64_t*>(wbase);
     unsigned char* yring = wbase + 128;
@@ -616,12 +700,12 @@ k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, lo
         for (int q = 0; q < RR; q++) act |= active_rhs<RT>(st, sp.sys, rr0 + q, mask_mode);
         if (!act) continue;
         const gb::SysDev& Sd = sys[sp.sys];
-        const int B = Sd.B;
-        const long long vec_off = Sd.vec_off;
+        const int B = Sd.B, H = Sd.rmax;              // the pass reads rows 0 .. H - 1 of a block
+        const long long vec_off = Sd.vec_off + (long long)rr0 * Sd.D;   // of the plane
         const SysPlan& pl = plan[sp.sys];
-        const int cpb = (B + RC - 1) / RC;            // chunks per block
+        const int cpb = (H + RC - 1) / RC;            // chunks per block
         const int total = sp.nb * cpb;
-        const unsigned ybytes = (unsigned)(B * RT * sizeof(YT));
+        const unsigned ybytes = (unsigned)(B * RR * sizeof(YT));
         const unsigned row_bytes = (unsigned)(B * MB);
         // first block of the strip: pair p0 = (i, j0), j0 = i + 1 + (p0 - pair_start(i))
         const int j0 = sp.i + 1 + (int)(sp.p0 - pair_start(sp.i, Sd.N));
@@ -630,7 +714,7 @@ k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, lo
         int pb = 0, pc = 0;                           // producer cursor: block, chunk within block
         auto issue = [&]() {                          // lane 0: next chunk (+ its block's y_u with the first)
             const int r0 = pc * RC;
-            const int nrows = min(RC, B - r0);
+            const int nrows = min(RC, H - r0);
             const unsigned bytes = (unsigned)nrows * row_bytes;
             uint64_t* bar = bars + pstage;
             unsigned char* dst = stages + (size_t)pstage * stage_stride;
@@ -639,14 +723,14 @@ k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, lo
             tma_1d_hint(dst, mstrip_h + src, bytes, bar, stream_pol);
             if (DF) tma_1d_hint(dst + lay.chunk_cap, mstrip_l + src, bytes, bar, stream_pol);
             if (pc == 0)
-                tma_1d(yring + (size_t)(pb % lay.nys) * lay.y_bytes, Yu + vec_off + (long long)(j0 + pb) * B * RT,
+                tma_1d(yring + (size_t)(pb % lay.nys) * lay.y_bytes, Yu + vec_off + (long long)(j0 + pb) * B * RR,
                        ybytes, bar);
             pstage = (pstage + 1 == S) ? 0 : pstage + 1;
             if (++pc == cpb) { pc = 0; ++pb; }
         };
         {   // y_w of particle i: the same for every block of the strip
-            const YT* src = Yw + vec_off + (long long)sp.i * B * RT;
-            for (int e = lane; e < B * RT; e += 32) syw[e] = src[e];
+            const YT* src = Yw + vec_off + (long long)sp.i * B * RR;
+            for (int e = lane; e < B * RR; e += 32) syw[e] = src[e];
         }
         Acc cu[CPL][RR], cw[CPL][RR];
 #pragma unroll
@@ -680,22 +764,33 @@ k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, lo
                 }
                 const unsigned char* stg = stages + (size_t)cstage * stage_stride;
                 const int row0 = c * RC;
-                const int nrows = min(RC, B - row0);
-                // One step: rows lr of the chunk.  Columns cl + LPR*k >= B (when LPR*CPL
-                // exceeds the block size) accumulate whatever follows the row in shared
-                // memory; those sums are never stored.
+                const int nrows = min(RC, H - row0);
+                // One step: row lr of the chunk (of the block, small blocks).  Columns
+                // cl + LPR*k >= B (when LPR*CPL exceeds the block size) accumulate whatever
+                // follows the row in shared memory; those sums are never stored.
                 auto step = [&](int lr) {
-                    const int row = row0 + lr;
+                    const int yrow = (PM ? 2 * (row0 + lr) + (cl & 1) : lr) * RR;
                     YT yu[RR], yw[RR];
 #pragma unroll
                     for (int q = 0; q < RR; q++) {
-                        yu[q] = syu[row * RT + rr0 + q];
-                        yw[q] = syw[row * RT + rr0 + q];
+                        yu[q] = syu[yrow + q];
+                        yw[q] = syw[yrow + q];
                     }
-                    const unsigned rbase = (unsigned)lr * row_bytes + (unsigned)cl * MB;
+                    const unsigned qoff = row_bytes / 2;
+                    const bool lower = !PM && lr >= H;   // row r + rmax is row r with its halves exchanged
+                    const unsigned rbase = (unsigned)(lower ? lr - H : lr) * row_bytes +
+                                           (unsigned)(PM ? cl >> 1 : cl) * MB;
 #pragma unroll
                     for (int k = 0; k < CPL; k++) {
-                        typename Pol::M m = Pol::load(stg, stg + lay.chunk_cap, rbase + LPR * k * MB);
+                        typename Pol::M m;
+                        if constexpr (PM) {
+                            const unsigned off = rbase + LPR / 2 * k * MB;
+                            m = Pol::load(stg, stg + lay.chunk_cap, off, off + qoff, sign);
+                        } else {
+                            const unsigned off = rbase + LPR * k * MB;
+                            m = Pol::load(stg, stg + lay.chunk_cap,
+                                          lower ? (cl + LPR * k < H ? off + qoff : off - qoff) : off);
+                        }
                         Pol::prep(m);
 #pragma unroll
                         for (int q = 0; q < RR; q++) {
@@ -704,7 +799,10 @@ k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, lo
                         }
                     }
                 };
-                if (nrows == RC) {   // full chunk: every lane has a row in every step
+                if constexpr (!PM) {
+#pragma unroll 4
+                    for (int r = ro; r < B; r += RPW) step(r);
+                } else if (nrows == RC) {   // full chunk: every lane has a row in every step
 #pragma unroll
                     for (int g = 0; g < G; g++) step(g * RPW + ro);
                 } else {
@@ -1155,15 +1253,15 @@ __device__ __forceinline__ void sum_terms(const OutT* __restrict__ p, long long 
 // threads form G = kRBThreads / W groups that split the terms, thread (g, w) streaming
 // word w of its terms, so every term is one coalesced read.  The groups are combined
 // in order (deterministic),
-// then thread (row, rhs) applies the sign/permutation of its row, adds the identity
-// term, stores y and contributes to the CTA's partial dot products (modes as k_reduce).
+// then thread (row, rhs) recombines the +- columns (pm; the tensor-core pass's columns are
+// the block's own), applies the sign/permutation of its row, adds the identity term, stores y and contributes to the CTA's partial dot products (modes as k_reduce).
 template <typename OutT, typename VT, int R>
 __global__ void __launch_bounds__(kRBThreads)
 k_reduce_blk(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items, int nitems,
              const SysPlan* __restrict__ plan, const long long* __restrict__ row_strip, const KState* __restrict__ st,
              int mask_mode, const OutT* __restrict__ CU, const OutT* __restrict__ CW, const VT* __restrict__ x,
              VT* __restrict__ y, int mode, const VT* __restrict__ aux, const double2* __restrict__ b128,
-             double2* __restrict__ dots, ScalarFuse fz, const double2* __restrict__ xscale) {
+             double2* __restrict__ dots, ScalarFuse fz, const double2* __restrict__ xscale, int pm) {
     const int it = blockIdx.x;
     if (it >= nitems) {
         pdl_wait();
@@ -1222,6 +1320,16 @@ k_reduce_blk(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items,
         }
     }
     __syncthreads();
+    if (tid < BR) {   // the groups' sums of every column, in order
+        C a = partU[tid], c = partW[tid];
+        for (int q = 1; q < G; q++) {
+            a = cadd(a, partU[q * BR + tid]);
+            c = cadd(c, partW[q * BR + tid]);
+        }
+        partU[tid] = a;
+        partW[tid] = c;
+    }
+    __syncthreads();
     DotAcc<T> d0, d1;
     d0.zero();
     d1.zero();
@@ -1230,10 +1338,15 @@ k_reduce_blk(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items,
         const int info = info_p;
         const int rho = info & ((1 << 29) - 1);
         const unsigned eneg = (info >> 29) & 1, sneg = (info >> 30) & 1;
-        C a = czero<C>(), c = czero<C>();
-        for (int q = 0; q < G; q++) {
-            a = cadd(a, partU[q * BR + rho * R + rr]);
-            c = cadd(c, partW[q * BR + rho * R + rr]);
+        C a, c;
+        if (pm && S.B > kWholeB) {   // c[s] = c+ + c-, c[rmax + s] = c+ - c- from the columns 2 s + (0, 1)
+            const unsigned second = rho >= S.rmax ? 1u : 0u;
+            const int at = 2 * (rho - (second ? S.rmax : 0)) * R + rr;
+            a = cadd(partU[at], cflip(partU[at + R], second));
+            c = cadd(partW[at], cflip(partW[at + R], second));
+        } else {
+            a = partU[rho * R + rr];
+            c = partW[rho * R + rr];
         }
         const C tx = cadd(cflip(a, eneg), cflip(c, eneg ^ sneg));
         if (active_rhs<R>(st, I.sys, rr, mask_mode)) {
@@ -1833,7 +1946,9 @@ Shape pick_shape(int Bmax) {
 // 10 elements of 16 B).
 constexpr int kGemvPad = 256;
 inline bool shape_fits(const Shape& c, int B, int elem_bytes) {
-    return c.lpr * c.cpl >= B && (c.lpr * c.cpl - B) * elem_bytes <= kGemvPad;
+    // (small blocks and the others have shapes of their own)
+    return c.lpr * c.cpl >= B && (c.lpr * c.cpl - B) * elem_bytes <= kGemvPad &&
+           (c.lpr * c.cpl <= kWholeB + 2) == (B <= kWholeB);
 }
 
 // Shapes measured by gb_autotune_gemv, per (block size, policy, RR, RT); the model
@@ -1875,7 +1990,8 @@ int launch_pgemv_group(const Plan& P, const DevPlan& D, const StripGroup& grp, c
                             Bmax);
     const int rpw = 32 / sh.lpr;
     const int G = gemv_steps(sh.lpr, sh.cpl, Pol::MB * (Pol::DF ? 2 : 1));
-    const GemvLayout g = gemv_layout(Bmax, G * rpw, RT, S, Pol::MB, Pol::DF, sizeof(YT));
+    const bool whole = sh.lpr * sh.cpl <= kWholeB + 2;
+    const GemvLayout g = gemv_layout(Bmax, whole ? Bmax / 2 : G * rpw, RR, S, Pol::MB, Pol::DF, sizeof(YT));
     const size_t smem = (size_t)kGemvWarps * g.warp_bytes;
     if (smem > 227 * 1024) return gb_set_error(GB_UNSUPPORTED, "GEMV needs %zu B of shared memory", smem);
     const long long n = grp.end - grp.beg;
@@ -1936,6 +2052,12 @@ int launch_pgemv_all(const Plan& P, const DevPlan& D, const KState* st, int mask
     }
 }
 
+inline bool df_wide(const Plan& P) {
+    bool wide = false;
+    for (const StripGroup& grp : P.groups) wide |= pick_shape(grp.B).cpl >= 5;
+    return wide;
+}
+
 // Double-float pass for R right-hand sides: one launch for both of R = 2, or one per
 // right-hand side where the wide shapes (5 columns per lane) would not keep two
 // sets of double-float accumulators in registers, and one per pair or per
@@ -1946,9 +2068,7 @@ int launch_df(const Plan& P, const DevPlan& D, const KState* st, int mask, const
     if constexpr (R == 1) {
         return launch_pgemv<PolDF, 1, 1>(P, D, st, mask, hi, lo, Yu, Yw, CU, CW, 0, D.err, stream);
     } else {
-        bool wide = false;
-        for (const StripGroup& grp : P.groups) wide |= pick_shape(grp.B).cpl >= 5;
-        if (!wide) {
+        if (!df_wide(P)) {
             if constexpr (R == 2)
                 return launch_pgemv<PolDF, 2, 2>(P, D, st, mask, hi, lo, Yu, Yw, CU, CW, 0, D.err, stream);
             for (int rr = 0; rr < R; rr += 2) {
@@ -1992,68 +2112,54 @@ int launch_apply(const Plan& P, const DevPlan& D, const WS& w, unsigned char* ba
     void* CW = base + w.off_cw;
     const unsigned vb = (unsigned)P.nv;
     int e = GB_OK;
+    auto yprep = [&](auto yk, int pl) -> int {   // y vectors in planes of pl right-hand sides
+        constexpr int YK = decltype(yk)::value;
+        using YT = typename YType<YK>::t;
+        gb::note_launch();
+        if constexpr (YK != 3) {
+            if (P.tmat) {
+                GB_CUDA_TRY(launch_pdl(k_yprep_tmat<YK, VT, R>, dim3((unsigned)P.nr), dim3(kRBThreads), 0, stream, D.sys,
+                                       D.ritems, P.nr, st, mask, xin, reinterpret_cast<YT*>(Yu),
+                                       reinterpret_cast<YT*>(Yw), up, pl));
+                return GB_OK;
+            }
+        }
+        GB_CUDA_TRY(launch_pdl(k_yprep<YK, VT, R>, dim3(vb), dim3(kVRows / 2 * R), 0, stream, D.sys, D.vitems, P.nv, st,
+                               mask, tvec, xin, reinterpret_cast<YT*>(Yu), reinterpret_cast<YT*>(Yw), up, pl));
+        return GB_OK;
+    };
+    auto reduce = [&](auto out, int pm) -> int {
+        using OutT = decltype(out);
+        gb::note_launch();
+        GB_CUDA_TRY(launch_pdl(k_reduce_blk<OutT, VT, R>, dim3((unsigned)P.nr), dim3(kRBThreads), 0, stream, D.sys,
+                               D.ritems, P.nr, D.sp, D.row_strip, st, mask, reinterpret_cast<const OutT*>(CU),
+                               reinterpret_cast<const OutT*>(CW), xin, yout, mode, aux, b128, dots, fz, xscale, pm));
+        return GB_OK;
+    };
+    constexpr int PL = R < 2 ? R : 2;
     if (pol == 0) {
-        gb::note_launch();
-        if (P.tmat)
-            GB_CUDA_TRY(launch_pdl(k_yprep_tmat<0, VT, R>, dim3((unsigned)P.nr), dim3(kRBThreads), 0, stream, D.sys,
-                                   D.ritems, P.nr, st, mask, xin, reinterpret_cast<double2*>(Yu),
-                                   reinterpret_cast<double2*>(Yw), up));
-        else
-            GB_CUDA_TRY(launch_pdl(k_yprep<0, VT, R>, dim3(vb), dim3(kVRows), 0, stream, D.sys, D.vitems, P.nv, st,
-                                   mask, tvec, xin, reinterpret_cast<double2*>(Yu), reinterpret_cast<double2*>(Yw), up));
-        if (P.nstrips) e = launch_pgemv_all<Pol64, R>(P, D, st, mask, mat_hi, Yu, Yw, CU, CW, stream);
-        if (e) return e;
-        gb::note_launch();
-        GB_CUDA_TRY(launch_pdl(k_reduce_blk<double2, VT, R>, dim3((unsigned)P.nr), dim3(kRBThreads), 0, stream, D.sys,
-                               D.ritems, P.nr, D.sp, D.row_strip, st, mask, reinterpret_cast<const double2*>(CU),
-                               reinterpret_cast<const double2*>(CW), xin, yout, mode, aux, b128, dots, fz, xscale));
+        e = yprep(std::integral_constant<int, 0>(), PL);
+        if (!e && P.nstrips) e = launch_pgemv_all<Pol64, R>(P, D, st, mask, mat_hi, Yu, Yw, CU, CW, stream);
+        if (!e) e = reduce(double2(), 1);
     } else if (pol == 1) {
-        gb::note_launch();
-        if (P.tmat)
-            GB_CUDA_TRY(launch_pdl(k_yprep_tmat<1, VT, R>, dim3((unsigned)P.nr), dim3(kRBThreads), 0, stream, D.sys,
-                                   D.ritems, P.nr, st, mask, xin, reinterpret_cast<float4*>(Yu),
-                                   reinterpret_cast<float4*>(Yw), up));
-        else
-            GB_CUDA_TRY(launch_pdl(k_yprep<1, VT, R>, dim3(vb), dim3(kVRows), 0, stream, D.sys, D.vitems, P.nv, st,
-                                   mask, tvec, xin, reinterpret_cast<float4*>(Yu), reinterpret_cast<float4*>(Yw), up));
-        if (P.nstrips) e = launch_pgemv_all<Pol32, R>(P, D, st, mask, mat_hi, Yu, Yw, CU, CW, stream);
-        if (e) return e;
-        gb::note_launch();
-        GB_CUDA_TRY(launch_pdl(k_reduce_blk<float2, VT, R>, dim3((unsigned)P.nr), dim3(kRBThreads), 0, stream, D.sys,
-                               D.ritems, P.nr, D.sp, D.row_strip, st, mask, reinterpret_cast<const float2*>(CU),
-                               reinterpret_cast<const float2*>(CW), xin, yout, mode, aux, b128, dots, fz, xscale));
+        e = yprep(std::integral_constant<int, 1>(), PL);
+        if (!e && P.nstrips) e = launch_pgemv_all<Pol32, R>(P, D, st, mask, mat_hi, Yu, Yw, CU, CW, stream);
+        if (!e) e = reduce(float2(), 1);
     } else if (pol == 3) {   // tensor-core pass on the bf16 tiles (mat_hi): float2 y vectors and partials
         if constexpr (R == 4 || R == 8) {
             if (P.tmat) return gb_set_error(GB_UNSUPPORTED, "the tensor-core pass serves sphere clusters");
-            gb::note_launch();
-            GB_CUDA_TRY(launch_pdl(k_yprep<3, VT, R>, dim3(vb), dim3(kVRows), 0, stream, D.sys, D.vitems, P.nv, st,
-                                   mask, tvec, xin, reinterpret_cast<float2*>(Yu), reinterpret_cast<float2*>(Yw), up));
-            if (P.nstrips) e = launch_pgemv_tcore(P, D, R, st, mask, mat_hi, Yu, Yw, CU, CW, stream);
-            if (e) return e;
-            gb::note_launch();
-            GB_CUDA_TRY(launch_pdl(k_reduce_blk<float2, VT, R>, dim3((unsigned)P.nr), dim3(kRBThreads), 0, stream,
-                                   D.sys, D.ritems, P.nr, D.sp, D.row_strip, st, mask,
-                                   reinterpret_cast<const float2*>(CU), reinterpret_cast<const float2*>(CW), xin, yout,
-                                   mode, aux, b128, dots, fz, xscale));
+            e = yprep(std::integral_constant<int, 3>(), R);
+            if (!e && P.nstrips) e = launch_pgemv_tcore(P, D, R, st, mask, mat_hi, Yu, Yw, CU, CW, stream);
+            if (!e) e = reduce(float2(), 0);
         } else {
             return gb_set_error(GB_UNSUPPORTED, "the tensor-core pass needs R = 4 or 8 (got %d)", R);
         }
     } else {
-        gb::note_launch();
-        if (P.tmat)
-            GB_CUDA_TRY(launch_pdl(k_yprep_tmat<2, VT, R>, dim3((unsigned)P.nr), dim3(kRBThreads), 0, stream, D.sys,
-                                   D.ritems, P.nr, st, mask, xin, reinterpret_cast<float4*>(Yu),
-                                   reinterpret_cast<float4*>(Yw), up));
-        else
-            GB_CUDA_TRY(launch_pdl(k_yprep<2, VT, R>, dim3(vb), dim3(kVRows), 0, stream, D.sys, D.vitems, P.nv, st,
-                                   mask, tvec, xin, reinterpret_cast<float4*>(Yu), reinterpret_cast<float4*>(Yw), up));
-        if (P.nstrips) e = launch_df<R>(P, D, st, mask, mat_hi, mat_lo, Yu, Yw, CU, CW, stream);
-        if (e) return e;
-        gb::note_launch();
-        GB_CUDA_TRY(launch_pdl(k_reduce_blk<float4, VT, R>, dim3((unsigned)P.nr), dim3(kRBThreads), 0, stream, D.sys,
-                               D.ritems, P.nr, D.sp, D.row_strip, st, mask, reinterpret_cast<const float4*>(CU),
-                               reinterpret_cast<const float4*>(CW), xin, yout, mode, aux, b128, dots, fz, xscale));
+        e = yprep(std::integral_constant<int, 2>(), df_wide(P) ? 1 : PL);
+        if (!e && P.nstrips) e = launch_df<R>(P, D, st, mask, mat_hi, mat_lo, Yu, Yw, CU, CW, stream);
+        if (!e) e = reduce(float4(), 1);
     }
+    if (e) return e;
     GB_CUDA_TRY(cudaGetLastError());
     return GB_OK;
 }
