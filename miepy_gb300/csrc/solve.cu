@@ -711,22 +711,30 @@ k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, lo
         const int j0 = sp.i + 1 + (int)(sp.p0 - pair_start(sp.i, Sd.N));
         const unsigned char* mstrip_h = mh + (Sd.mat_off + sp.p0 * (long long)B * B) * MB;
         const unsigned char* mstrip_l = DF ? ml + (Sd.mat_off + sp.p0 * (long long)B * B) * MB : nullptr;
-        int pb = 0, pc = 0;                           // producer cursor: block, chunk within block
+        // producer cursor: first row of the next chunk, its place in the strip, its block's
+        // y vector and y slot
+        int pr = 0, py = 0;
+        size_t psrc = 0;
+        const YT* ysrc = Yu + vec_off + (long long)j0 * B * RR;
         auto issue = [&]() {                          // lane 0: next chunk (+ its block's y_u with the first)
-            const int r0 = pc * RC;
-            const int nrows = min(RC, H - r0);
-            const unsigned bytes = (unsigned)nrows * row_bytes;
+            const unsigned bytes = (unsigned)min(RC, H - pr) * row_bytes;
             uint64_t* bar = bars + pstage;
-            unsigned char* dst = stages + (size_t)pstage * stage_stride;
-            const long long src = (long long)pb * B * row_bytes + (long long)r0 * row_bytes;
-            mbar_expect_tx(bar, bytes * (DF ? 2u : 1u) + (pc == 0 ? ybytes : 0u));
-            tma_1d_hint(dst, mstrip_h + src, bytes, bar, stream_pol);
-            if (DF) tma_1d_hint(dst + lay.chunk_cap, mstrip_l + src, bytes, bar, stream_pol);
-            if (pc == 0)
-                tma_1d(yring + (size_t)(pb % lay.nys) * lay.y_bytes, Yu + vec_off + (long long)(j0 + pb) * B * RR,
-                       ybytes, bar);
+            unsigned char* dst = stages + pstage * stage_stride;
+            mbar_expect_tx(bar, bytes * (DF ? 2u : 1u) + (pr == 0 ? ybytes : 0u));
+            tma_1d_hint(dst, mstrip_h + psrc, bytes, bar, stream_pol);
+            if (DF) tma_1d_hint(dst + lay.chunk_cap, mstrip_l + psrc, bytes, bar, stream_pol);
+            if (pr == 0) {
+                tma_1d(yring + py * lay.y_bytes, ysrc, ybytes, bar);
+                ysrc += B * RR;
+                py = (py + 1 == lay.nys) ? 0 : py + 1;
+            }
             pstage = (pstage + 1 == S) ? 0 : pstage + 1;
-            if (++pc == cpb) { pc = 0; ++pb; }
+            pr += RC;
+            psrc += bytes;
+            if (pr >= H) {   // past the lower half, which is not read
+                pr = 0;
+                psrc += (size_t)(B - H) * row_bytes;
+            }
         };
         {   // y_w of particle i: the same for every block of the strip
             const YT* src = Yw + vec_off + (long long)sp.i * B * RR;
@@ -743,13 +751,14 @@ k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, lo
         if (lane == 0)
             for (int t = 0; t < npre; t++) issue();
         in_flight = npre;
-        int issued = npre;
+        int issued = npre, cy = 0;
         for (int b = 0; b < sp.nb && !failed; b++) {
 #pragma unroll
             for (int k = 0; k < CPL; k++)
 #pragma unroll
                 for (int q = 0; q < RR; q++) Pol::zero(cw[k][q]);
-            const YT* syu = reinterpret_cast<const YT*>(yring + (size_t)(b % lay.nys) * lay.y_bytes);
+            const YT* syu = reinterpret_cast<const YT*>(yring + cy * lay.y_bytes);
+            cy = (cy + 1 == lay.nys) ? 0 : cy + 1;
             for (int c = 0; c < cpb; c++) {
                 if (issued < total) {   // into the stage freed by the previous chunk
                     if (lane == 0) issue();
@@ -765,32 +774,19 @@ k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, lo
                 const unsigned char* stg = stages + (size_t)cstage * stage_stride;
                 const int row0 = c * RC;
                 const int nrows = min(RC, H - row0);
-                // One step: row lr of the chunk (of the block, small blocks).  Columns
+                // One step: a row of the chunk with the row's y values.  Columns
                 // cl + LPR*k >= B (when LPR*CPL exceeds the block size) accumulate whatever
                 // follows the row in shared memory; those sums are never stored.
-                auto step = [&](int lr) {
-                    const int yrow = (PM ? 2 * (row0 + lr) + (cl & 1) : lr) * RR;
+                auto step = [&](int yrow, auto load) {
                     YT yu[RR], yw[RR];
 #pragma unroll
                     for (int q = 0; q < RR; q++) {
-                        yu[q] = syu[yrow + q];
-                        yw[q] = syw[yrow + q];
+                        yu[q] = syu[yrow * RR + q];
+                        yw[q] = syw[yrow * RR + q];
                     }
-                    const unsigned qoff = row_bytes / 2;
-                    const bool lower = !PM && lr >= H;   // row r + rmax is row r with its halves exchanged
-                    const unsigned rbase = (unsigned)(lower ? lr - H : lr) * row_bytes +
-                                           (unsigned)(PM ? cl >> 1 : cl) * MB;
 #pragma unroll
                     for (int k = 0; k < CPL; k++) {
-                        typename Pol::M m;
-                        if constexpr (PM) {
-                            const unsigned off = rbase + LPR / 2 * k * MB;
-                            m = Pol::load(stg, stg + lay.chunk_cap, off, off + qoff, sign);
-                        } else {
-                            const unsigned off = rbase + LPR * k * MB;
-                            m = Pol::load(stg, stg + lay.chunk_cap,
-                                          lower ? (cl + LPR * k < H ? off + qoff : off - qoff) : off);
-                        }
+                        typename Pol::M m = load(k);
                         Pol::prep(m);
 #pragma unroll
                         for (int q = 0; q < RR; q++) {
@@ -799,16 +795,47 @@ k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, lo
                         }
                     }
                 };
-                if constexpr (!PM) {
-#pragma unroll 4
-                    for (int r = ro; r < B; r += RPW) step(r);
-                } else if (nrows == RC) {   // full chunk: every lane has a row in every step
+                const unsigned qoff = row_bytes / 2;
+                if constexpr (PM) {
+                    const unsigned char* col = stg + (cl >> 1) * MB;
+                    auto pm_step = [&](int lr) {
+                        const unsigned char* row = col + lr * row_bytes;
+                        step(2 * (row0 + lr) + (cl & 1), [&](int k) {
+                            return Pol::load(row, row + lay.chunk_cap, LPR / 2 * k * MB, LPR / 2 * k * MB + qoff, sign);
+                        });
+                    };
+                    if (nrows == RC) {   // full chunk: every lane has a row in every step
 #pragma unroll
-                    for (int g = 0; g < G; g++) step(g * RPW + ro);
-                } else {
+                        for (int g = 0; g < G; g++) pm_step(g * RPW + ro);
+                    } else {
 #pragma unroll
-                    for (int g = 0; g < G; g++)
-                        if (g * RPW + ro < nrows) step(g * RPW + ro);
+                        for (int g = 0; g < G; g++)
+                            if (g * RPW + ro < nrows) pm_step(g * RPW + ro);
+                    }
+                } else {   // the block's rows: the upper ones, then row r + rmax as row r with its halves exchanged
+                    constexpr int NS = (kWholeB / 2 + RPW - 1) / RPW;   // steps over the rows of one half
+                    const unsigned char* col = stg + cl * MB;
+#pragma unroll
+                    for (int g = 0; g < NS; g++) {
+                        const int r = ro + g * RPW;
+                        if (r < H) {
+                            const unsigned char* row = col + r * row_bytes;
+                            step(r, [&](int k) { return Pol::load(row, row + lay.chunk_cap, LPR * k * MB); });
+                        }
+                    }
+                    const int low = (H - ro + RPW - 1) / RPW * RPW + ro - H;   // the lane's first lower row, less H
+                    int swap[CPL];                                             // the other half's column
+#pragma unroll
+                    for (int k = 0; k < CPL; k++)
+                        swap[k] = LPR * k * MB + (cl + LPR * k < H ? (int)qoff : -(int)qoff);
+#pragma unroll
+                    for (int g = 0; g < NS; g++) {
+                        const int r = low + g * RPW;
+                        if (r < H) {
+                            const unsigned char* row = col + r * row_bytes;
+                            step(H + r, [&](int k) { return Pol::load(row + swap[k], row + lay.chunk_cap + swap[k], 0u); });
+                        }
+                    }
                 }
                 __syncwarp();   // every lane is done with this stage (and, at the block's end, its y slot)
                 if (lane == 0) asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -1962,15 +1989,17 @@ Shape tuned_shape(int B, int pol, int RR, int RT) {
     return f != g_tuned.end() ? f->second : pick_shape(B);
 }
 
-// Steps per chunk for a shape: chunks of about 6 KB of matrix for the block size
-// the shape is made for (LPR*CPL columns); with three stages and two y slots per
-// warp, two 4-warp CTAs share an SM.  (3 KB chunks with three CTAs per SM, and a
-// fourth stage, measured no faster for the complex64 pass and 7 % slower for the
-// compute-bound double-float pass, whose longer unrolled steps help.)
-constexpr int gemv_steps(int lpr, int cpl, int elem_bytes) {
-    return (6144 / ((32 / lpr) * lpr * cpl * elem_bytes)) < 1 ? 1
-           : (6144 / ((32 / lpr) * lpr * cpl * elem_bytes)) > 8 ? 8
-                                                                : 6144 / ((32 / lpr) * lpr * cpl * elem_bytes);
+// Steps per chunk of bytes of matrix for a shape (LPR*CPL columns), with three stages and
+// two y slots per warp.  6 KB chunks (two 4-warp CTAs per SM) where the pass is
+// compute-bound (double-float, complex128) or has no more strips than those CTAs have
+// warps, so that the bytes in flight per warp count; else 3 KB (three or four CTAs): the
+// complex64 pass of N = 200, lmax 4 takes 33.9 us against 41.7 (R = 1), 38.9 against 44.8
+// (R = 2), N = 97, lmax 8, R = 2 89.6 against 108.5, but N = 20, lmax 6 8.1 against 6.0.
+// (Small blocks: a chunk is a block's upper half.)
+constexpr int gemv_steps(int lpr, int cpl, int elem_bytes, int bytes = 6144) {
+    return (bytes / ((32 / lpr) * lpr * cpl * elem_bytes)) < 1 ? 1
+           : (bytes / ((32 / lpr) * lpr * cpl * elem_bytes)) > 8 ? 8
+                                                                : bytes / ((32 / lpr) * lpr * cpl * elem_bytes);
 }
 
 template <class Pol, int RR, int RT>
@@ -1989,8 +2018,9 @@ int launch_pgemv_group(const Plan& P, const DevPlan& D, const StripGroup& grp, c
         return gb_set_error(GB_UNSUPPORTED, "GEMV shape %dx%d overruns the %d-column block's padding", sh.lpr, sh.cpl,
                             Bmax);
     const int rpw = 32 / sh.lpr;
-    const int G = gemv_steps(sh.lpr, sh.cpl, Pol::MB * (Pol::DF ? 2 : 1));
     const bool whole = sh.lpr * sh.cpl <= kWholeB + 2;
+    const bool fine = Pol::ID == 1 && !whole && grp.end - grp.beg > 8LL * gb::sm_count();
+    const int G = gemv_steps(sh.lpr, sh.cpl, Pol::MB * (Pol::DF ? 2 : 1), fine ? 3072 : 6144);
     const GemvLayout g = gemv_layout(Bmax, whole ? Bmax / 2 : G * rpw, RR, S, Pol::MB, Pol::DF, sizeof(YT));
     const size_t smem = (size_t)kGemvWarps * g.warp_bytes;
     if (smem > 227 * 1024) return gb_set_error(GB_UNSUPPORTED, "GEMV needs %zu B of shared memory", smem);
@@ -2001,8 +2031,9 @@ int launch_pgemv_group(const Plan& P, const DevPlan& D, const StripGroup& grp, c
                                                                       0x7fffffffLL));
 #define GB_PG(LPRV, CPLV)                                                                                        \
     if (sh.lpr == LPRV && sh.cpl == CPLV) {                                                                      \
-        constexpr int GV = gemv_steps(LPRV, CPLV, Pol::MB * (Pol::DF ? 2 : 1));                                  \
-        auto kfn = k_pgemv<Pol, RR, RT, LPRV, CPLV, GV, S>;                                                      \
+        constexpr int EB = Pol::MB * (Pol::DF ? 2 : 1);                                                          \
+        constexpr int GV = gemv_steps(LPRV, CPLV, EB), GF = Pol::ID == 1 ? gemv_steps(LPRV, CPLV, EB, 3072) : GV; \
+        auto kfn = fine ? k_pgemv<Pol, RR, RT, LPRV, CPLV, GF, S> : k_pgemv<Pol, RR, RT, LPRV, CPLV, GV, S>;     \
         if (smem > 48 * 1024)                                                                                    \
             GB_CUDA_TRY(gb::ensure_dynamic_smem(reinterpret_cast<const void*>(kfn), smem));      \
         gb::note_launch();                                                                                       \
