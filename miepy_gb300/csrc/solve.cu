@@ -684,8 +684,8 @@ k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, lo
     // ring position: chunk number gc of this warp lives in stage gc % S, phase gc / S
     unsigned cstage = 0, cphase = 0;      // consumer
     unsigned pstage = 0;                  // producer (lane 0)
-    const long long warp = ((long long)blockIdx.x * kGemvThreads + threadIdx.x) >> 5;
-    const long long nwarps = ((long long)gridDim.x * kGemvThreads) >> 5;
+    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
     bool failed = false;
     int in_flight = 0;                    // chunks issued and not yet consumed
     const uint64_t stream_pol = l2_evict_first_policy();
@@ -2022,13 +2022,16 @@ int launch_pgemv_group(const Plan& P, const DevPlan& D, const StripGroup& grp, c
     const bool fine = Pol::ID == 1 && !whole && grp.end - grp.beg > 8LL * gb::sm_count();
     const int G = gemv_steps(sh.lpr, sh.cpl, Pol::MB * (Pol::DF ? 2 : 1), fine ? 3072 : 6144);
     const GemvLayout g = gemv_layout(Bmax, whole ? Bmax / 2 : G * rpw, RR, S, Pol::MB, Pol::DF, sizeof(YT));
-    const size_t smem = (size_t)kGemvWarps * g.warp_bytes;
+    // complex128 passes of few strips per SM: one warp per CTA, so that the strips, all of
+    // the time there, spread over the sub-partitions (N = 61, lmax 5: 120 us against 124,
+    // R = 2 205 against 216; no gain for the other passes)
+    const int warps = Pol::ID == 0 && grp.end - grp.beg <= 32LL * gb::sm_count() ? 1 : kGemvWarps, threads = 32 * warps;
+    const size_t smem = (size_t)warps * g.warp_bytes;
     if (smem > 227 * 1024) return gb_set_error(GB_UNSUPPORTED, "GEMV needs %zu B of shared memory", smem);
     const long long n = grp.end - grp.beg;
     // one strip per warp (no persistent loop): CTAs retire after their strips, so
     // kernels of higher-priority streams are dispatched between them
-    const long long grid = std::max<long long>(1, std::min<long long>((n * 32 + kGemvThreads - 1) / kGemvThreads,
-                                                                      0x7fffffffLL));
+    const long long grid = std::max<long long>(1, std::min<long long>((n + warps - 1) / warps, 0x7fffffffLL));
 #define GB_PG(LPRV, CPLV)                                                                                        \
     if (sh.lpr == LPRV && sh.cpl == CPLV) {                                                                      \
         constexpr int EB = Pol::MB * (Pol::DF ? 2 : 1);                                                          \
@@ -2037,7 +2040,7 @@ int launch_pgemv_group(const Plan& P, const DevPlan& D, const StripGroup& grp, c
         if (smem > 48 * 1024)                                                                                    \
             GB_CUDA_TRY(gb::ensure_dynamic_smem(reinterpret_cast<const void*>(kfn), smem));      \
         gb::note_launch();                                                                                       \
-        GB_CUDA_TRY(launch_pdl(kfn, dim3((unsigned)grid), dim3(kGemvThreads), smem, stream, D.sys, D.strips,    \
+        GB_CUDA_TRY(launch_pdl(kfn, dim3((unsigned)grid), dim3(threads), smem, stream, D.sys, D.strips,         \
                                grp.beg, grp.end, st, mask, mat_hi, mat_lo, reinterpret_cast<const YT*>(Yu),        \
                                reinterpret_cast<const YT*>(Yw), reinterpret_cast<OutT*>(CU),                      \
                                reinterpret_cast<OutT*>(CW), D.sp, rr0, Bmax, err));                               \
