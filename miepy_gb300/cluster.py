@@ -278,13 +278,7 @@ class sphere_cluster:
         return cross_sections(*[np.sum(A) for A in C])
 
     def cross_sections(self):
-        Cs = Ca = Ce = 0
-        for i in range(self.Nparticles):
-            C = self.cross_sections_of_particle(i)
-            Cs += C.scattering
-            Ca += C.absorption
-            Ce += C.extinction
-        return cross_sections(Cs, Ca, Ce)
+        return cross_sections(*self._xs.sum(axis=(0, 2, 3)))
 
     # ------------------------------------------------- cluster coefficients --
     def solve_cluster_coefficients(self, lmax=None):
@@ -317,10 +311,10 @@ class sphere_cluster:
         f = 4 * np.pi / k ** 2
         Cs = np.zeros((2, lmax))
         Ce = np.zeros((2, lmax))
-        for r in range(lmax_to_rmax(lmax)):
-            n = int(np.floor(np.sqrt(r + 1)))
-            Cs[:, n - 1] += f * np.abs(pc[:, r]) ** 2
-            Ce[:, n - 1] += f * np.real(np.conj(p0[:, r]) * pc[:, r])
+        sca, ext = f * np.abs(pc) ** 2, f * np.real(np.conj(p0) * pc)
+        for n in range(1, lmax + 1):   # modes n^2 - 1 .. n^2 + 2 n - 1
+            Cs[:, n - 1] = sca[:, n * n - 1: n * (n + 2)].sum(axis=1)
+            Ce[:, n - 1] = ext[:, n * n - 1: n * (n + 2)].sum(axis=1)
         return cross_sections(Cs, Ce - Cs, Ce)
 
     def _angular(self, theta, phi, radius, source, magnetic):

@@ -121,7 +121,9 @@ class material_struct:
         self.mu_b = self.medium.mu(value)
         self.n_b = (self.eps_b * self.mu_b) ** 0.5
         self.k_b = 2 * np.pi * self.n_b / value
+        seen = {}   # particles of one material object: evaluated once
         for i, m in enumerate(self.materials):
-            self.eps[i] = m.eps(value)
-            self.mu[i] = m.mu(value)
+            if id(m) not in seen:
+                seen[id(m)] = m.eps(value), m.mu(value)
+            self.eps[i], self.mu[i] = seen[id(m)]
         self.n[...] = (self.eps * self.mu) ** 0.5

@@ -11,7 +11,7 @@ from __future__ import annotations
 import numpy as np
 
 from .modes import lmax_to_rmax, mode_indices
-from .special import Emn, pi_func, tau_func
+from .special import pi_tau_emn
 
 
 def sph_basis_vectors(theta, phi):
@@ -100,15 +100,8 @@ class plane_wave:
         """p_src [N, 2, rmax] (sources/plane_waves.py:126-156)."""
         position = np.asarray(position, dtype=float).reshape(-1, 3)
         rmax = lmax_to_rmax(lmax)
-        pi_vals = np.empty(rmax)
-        tau_vals = np.empty(rmax)
-        emn_vals = np.empty(rmax)
-        m_vals = np.empty(rmax, dtype=int)
-        for r, n, m in mode_indices(lmax):
-            pi_vals[r] = pi_func(n, m, self.theta)
-            tau_vals[r] = tau_func(n, m, self.theta)
-            emn_vals[r] = np.abs(Emn(m, n))
-            m_vals[r] = m
+        pi_vals, tau_vals, emn_vals = pi_tau_emn(lmax, self.theta)
+        m_vals = np.array([m for _, _, m in mode_indices(lmax)])
         phases = k * (position @ self.k_hat) + self.phase
         f = self.amplitude * np.exp(1j * (phases[:, None] - m_vals * self.phi)) * emn_vals
         p_src = np.empty([position.shape[0], 2, rmax], dtype=complex)

@@ -8,6 +8,7 @@ pi_func / tau_func with their exact limits at theta = 0 and pi
 
 from __future__ import annotations
 
+from functools import lru_cache
 from math import factorial
 
 import numpy as np
@@ -78,3 +79,42 @@ def tau_func(n, m, theta):
 
 def Emn(m, n):
     return (1j) ** n * np.sqrt((2 * n + 1) * factorial(n - m) / (n * (n + 1) * factorial(n + m)))
+
+
+@lru_cache(maxsize=16)
+def _mode_constants(lmax):
+    """n, |m|, m, the negative-order Legendre factor and |E_mn| of every mode."""
+    nm = [(n, m) for n in range(1, lmax + 1) for m in range(-n, n + 1)]
+    n, m = (np.array(v) for v in zip(*nm))
+    neg = np.array([_neg_factor(*v) if v[1] < 0 else 1.0 for v in nm])
+    emn = np.array([np.sqrt((2 * a + 1) * factorial(a - b) / (a * (a + 1) * factorial(a + b))) for a, b in nm])
+    return n, np.abs(m), m, neg, emn
+
+
+def pi_tau_emn(lmax, theta):
+    """pi_func, tau_func and |Emn| of every mode (in mode order) at one angle, from one
+    Legendre table: the values of the functions above, in the same arithmetic."""
+    n, am, m, neg, emn = _mode_constants(int(lmax))
+    theta = float(theta)
+    if theta == 0 or theta == np.pi:
+        half = n * (n + 1) / 2.0   # the exact limits, of |m| = 1 only
+        pi = np.where(m == 1, half, np.where(m == -1, 0.5, 0.0))
+        tau = np.where(m == 1, half, np.where(m == -1, -0.5, 0.0))
+        return (pi, tau, emn) if theta == 0 else ((-1.0) ** (n + 1) * pi, (-1.0) ** n * tau, emn)
+    x = float(np.cos(theta))
+    u = float(np.sqrt(max(0.0, (1.0 - x) * (1.0 + x))))
+    top = int(lmax) + 1
+    P = [[0.0] * (top + 1) for _ in range(top + 1)]
+    P[0][0] = 1.0
+    for k in range(1, top + 1):
+        P[k][k] = (2 * k - 1) * u * P[k - 1][k - 1]
+    for k in range(top):
+        P[k + 1][k] = x * (2 * k + 1) * P[k][k]
+    for k in range(top + 1):
+        for a in range(k + 2, top + 1):
+            P[a][k] = ((2 * a - 1) * x * P[a - 1][k] - (a + k - 1) * P[a - 2][k]) / (a - k)
+    P = np.array(P)
+    pp1 = np.where(am + 1 <= n, P[n, am + 1], 0.0)
+    pm1 = np.where(am >= 1, P[n, np.maximum(am - 1, 0)], -P[n, 1] / (n * (n + 1)))
+    d = 0.5 * ((n + am) * (n - am + 1) * pm1 - pp1)
+    return m / np.sin(theta) * (P[n, am] * neg), d * neg, emn
