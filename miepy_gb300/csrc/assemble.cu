@@ -27,6 +27,7 @@
 
 #include "gb_common.cuh"
 #include "gb_internal.h"
+#include "lattice.h"
 
 namespace {
 
@@ -45,11 +46,11 @@ __constant__ double c_inv_int[2 * GB_LMAX_MAX + 4] = {
 // they fit, one at large lmax, where two would cost occupancy.
 struct AsmSmem {
     int PM, MU, M, PB, NB;
-    size_t off_geo, off_h, off_P, off_e, off_G, off_Gs, off_T, off_Tf, off_Tl, total;
+    size_t off_geo, off_h, off_P, off_e, off_G, off_T, off_Tf, off_Tl, total;
 };
 
 __host__ __device__ inline AsmSmem asm_layout(int L, int M, int PB, bool fp64_sums, bool want64, int NB,
-                                               bool split = false, bool gsum = false) {
+                                               bool split = false, bool latt = false) {
     AsmSmem s;
     s.PM = 2 * L + 2;
     s.MU = 4 * L + 1;
@@ -58,14 +59,14 @@ __host__ __device__ inline AsmSmem asm_layout(int L, int M, int PB, bool fp64_su
     s.NB = NB;
     size_t o = 0;
     auto take = [&](size_t bytes) { size_t r = o; o += (bytes + 15) & ~size_t(15); return r; };
-    // the double-float path reads its G tables (k_asm_gtab) and needs no special functions
-    const size_t sf = fp64_sums ? 1 : 0;
+    // the double-float path and the lattice sums read their G tables (k_asm_gtab, lattice.cu)
+    // and need no special functions
+    const size_t sf = fp64_sums && !latt ? 1 : 0;
     s.off_geo = take(sf * sizeof(double) * 8 * PB);
     s.off_h = take(sf * sizeof(double2) * s.PM * PB);
     s.off_e = take(sf * sizeof(double2) * s.MU * PB);
     s.off_P = take(sf * sizeof(double) * s.PM * s.PM * PB);
     s.off_G = take(16 * (size_t)s.PM * s.MU * PB);          // double2 (FP64 sums) or float4 (double-float)
-    s.off_Gs = take(gsum ? sizeof(double2) * s.PM * s.MU : 0);   // lattice sums: the group's running G sum
     const size_t kinds = split ? 1 : 2;   // (A, B) per tuple, or one of them at a time
     s.off_T = take(fp64_sums ? sizeof(double2) * kinds * NB * M : 0);   // NB buffers of tuple values
     s.off_Tf = take(want64 ? sizeof(float2) * kinds * NB * M : 0);
@@ -179,24 +180,17 @@ struct Refl {
     double2 r0 = {0, 0};
 };
 
-// Periodic lattice (sphere_aggregate_tmatrix_periodic, interactions.py:153-186):
-// block (i, j) gains sum_c e^{-i k khat.c} A(pos_i - pos_j - c) mie_j over the
-// lattice cells c (cells [ncell][3], device).  Groups hold PB cells of one ordered
-// pair (gpp groups per pair); each group sums its phase-weighted tuple values in
-// shared memory and adds its block to the dense output with one atomic add per
-// entry.
+// Periodic lattice (sphere_aggregate_tmatrix_periodic, interactions.py:153-186): one CTA
+// per ordered pair (i, j), whose summed G table (lattice.cu) it reads from the pair's block
+// of the output, in tables parts, before it writes the block.
 struct Latt {
-    const double* cells = nullptr;
-    int ncell = 0;
-    int gpp = 1;   // groups per ordered pair, each over cpg consecutive cells in chunks of PB
-    int cpg = 1;
-    double kx = 0, ky = 0, kz = 0;
+    int tables = 1;
 };
 
 // FP64_SUMS: tuple sums in FP64 (complex128 or dense output); otherwise in
 // double-float on the FP32 pipes, straight to the complex64 hi / lo outputs.
-// MODE 0: the aggregate T-matrix; 1: the dense reflection matrix (Refl); 2: the
-// lattice sums of a periodic cluster, added to a dense output (Latt).
+// MODE 0: the aggregate T-matrix; 1: the dense reflection matrix (Refl); 2: the blocks
+// of a periodic cluster from their lattice sums (Latt).
 // Occupancy: the double-float (mixed) path fits five CTAs per SM in 48 registers
 // without spills; the FP64 paths keep three (at five they spill).
 // TS: whole-group phases on the packed double-float path (lmax <= 5, one tuple-value
@@ -229,7 +223,6 @@ k_assemble(const gb::SysDev* __restrict__ sys, int nsys, const long long* __rest
     double2* eph = reinterpret_cast<double2*>(smem + lay.off_e);        // [PB][MU]
     double* Pl = reinterpret_cast<double*>(smem + lay.off_P);           // [PB][PM][PM]
     double2* G64 = reinterpret_cast<double2*>(smem + lay.off_G);        // [PB][PM][MU]
-    double2* Gs = reinterpret_cast<double2*>(smem + lay.off_Gs);        // [PM][MU] (lattice sums)
     float4* G32 = reinterpret_cast<float4*>(smem + lay.off_G);
     double2* Tv = reinterpret_cast<double2*>(smem + lay.off_T);
     float2* Tf = reinterpret_cast<float2*>(smem + lay.off_Tf);
@@ -242,40 +235,18 @@ k_assemble(const gb::SysDev* __restrict__ sys, int nsys, const long long* __rest
         const int PM = 2 * L + 2, MU = 4 * L + 1;
         const long long gl = g - grp_base[s];
         const long long p_first = gl * (long long)PB;
-        long long lat_pair = 0;   // lattice: the ordered pair (i, j) = (lat_pair / N, lat_pair % N) ...
-        int lat_c0 = 0;           // ... the first cell of the chunk ...
-        int lat_end = 0;          // ... and the end of the group's cells
-        int np;
-        if constexpr (LATT) {
-            lat_pair = gl / latt.gpp;
-            lat_c0 = (int)(gl - lat_pair * latt.gpp) * latt.cpg;
-            lat_end = min(lat_c0 + latt.cpg, latt.ncell);
-            np = min(PB, lat_end - lat_c0);
-        } else {
-            const long long Ptot = REFL ? (long long)N * N : S.P;   // all ordered pairs for the reflection
-            np = (int)min((long long)PB, Ptot - p_first);
-        }
+        // all ordered pairs for the reflection and the lattice
+        const long long Ptot = REFL || LATT ? (long long)N * N : S.P;
+        const int np = (int)min((long long)PB, Ptot - p_first);
 
-        // lattice sums: phases 1a-1c for every chunk of PB cells of the group, each
-        // chunk's phase-weighted G tables added to the running sum Gs; other modes run
-        // them once
-        for (bool first = true;; first = false) {
         // ---- phase 1a (FP64 paths; the double-float path reads the G tables of
         // k_asm_gtab): one thread per pair: geometry, then h_p(kr) by the upward
         // j/y recurrence of spherical_hn_recursion (cpp/src/special.cpp:90-111).  The
         // angles enter only through cos/sin of theta and phi, straight from the
         // separation vector (the reference goes through acos/atan2 and back).
-        if (FP64_SUMS && tid < np) {
+        if (FP64_SUMS && !LATT && tid < np) {
             int i, j;
-            double lx = 0.0, ly = 0.0, lz = 0.0;   // lattice: the cell that holds the image of particle j
-            if (LATT) {
-                i = (int)(lat_pair / N);
-                j = (int)(lat_pair % N);
-                const double* c = latt.cells + 3 * (long long)(lat_c0 + tid);
-                lx = c[0];
-                ly = c[1];
-                lz = c[2];
-            } else if (REFL) {
+            if (REFL) {
                 i = (int)((p_first + tid) / N);
                 j = (int)((p_first + tid) % N);
             } else {
@@ -284,7 +255,7 @@ k_assemble(const gb::SysDev* __restrict__ sys, int nsys, const long long* __rest
             const double* pi_ = pos + S.pos_off + 3 * (long long)i;
             const double* pj_ = pos + S.pos_off + 3 * (long long)j;
             const double zi = REFL ? 2.0 * refl.z - pi_[2] : pi_[2];   // mirror image of particle i
-            const double dx = pi_[0] - (pj_[0] + lx), dy = pi_[1] - (pj_[1] + ly), dz = zi - (pj_[2] + lz);
+            const double dx = pi_[0] - pj_[0], dy = pi_[1] - pj_[1], dz = zi - pj_[2];
             const double rho2 = dx * dx + dy * dy;
             const double rad = sqrt(rho2 + dz * dz);
             const double inv_r = 1.0 / rad;
@@ -300,12 +271,6 @@ k_assemble(const gb::SysDev* __restrict__ sys, int nsys, const long long* __rest
             ge[1] = rho * inv_r;                            // sin(theta) >= 0
             ge[2] = cphi;
             ge[3] = sphi;
-            if (LATT) {   // the Bloch phase e^{-i k khat.c} of the cell
-                double sp, cp;
-                sincos(-S.k * (latt.kx * lx + latt.ky * ly + latt.kz * lz), &sp, &cp);
-                ge[4] = cp;
-                ge[5] = sp;
-            }
             const double z = S.k * rad;
             const double inv_z = 1.0 / z;
             double sz, cz;
@@ -323,11 +288,25 @@ k_assemble(const gb::SysDev* __restrict__ sys, int nsys, const long long* __rest
                 h[q] = make_double2(jn, yn);
             }
         }
-        if constexpr (FP64_SUMS) __syncthreads();
+        if constexpr (FP64_SUMS && !LATT) __syncthreads();
         // ---- phase 1b: P_q^mu(cos theta) (no Condon-Shortley phase), one thread per
         // (pair, mu); e^{i mu phi} by binary powering, one thread per (pair, mu >= 0).
-        // The double-float path instead loads the group's G tables.
-        if constexpr (FP64_SUMS) {
+        // The double-float path and the lattice sums instead load their G tables.
+        if constexpr (LATT) {
+            const long long i = p_first / N, j = p_first % N;   // one pair per group
+            for (int it = tid; it < PM * MU; it += NT) {
+                const int q = it / MU, mi = it - q * MU, mu = mi - 2 * L;
+                double2 g = make_double2(0.0, 0.0);
+                if ((mu < 0 ? -mu : mu) <= q)
+                    for (int c = 0; c < latt.tables; c++) {
+                        const int at = c * (PM * PM) + q * q + q + mu;
+                        const double2 v = out128[(i * B + at / B) * dense_ld + j * B + at % B];
+                        g.x += v.x;
+                        g.y += v.y;
+                    }
+                G64[(size_t)q * MUs + mi] = g;
+            }
+        } else if constexpr (FP64_SUMS) {
             for (int it = tid; it < np * PM; it += NT) {
                 const int pp = it / PM, mu = it % PM;
                 const double x = geo[8 * pp], u = geo[8 * pp + 1];
@@ -380,7 +359,7 @@ k_assemble(const gb::SysDev* __restrict__ sys, int nsys, const long long* __rest
         __syncthreads();
         // ---- phase 1c (FP64 paths): G[p][mu] = P_p^mu h_p e^{i mu phi} (negative mu
         // through the (-1)^mu (p-mu)!/(p+mu)! ratio)
-        if constexpr (FP64_SUMS) {
+        if constexpr (FP64_SUMS && !LATT) {
             for (int it = tid; it < np * PM * MU; it += NT) {
                 const int pp = it / (PM * MU), rem = it % (PM * MU);
                 const int q = rem / MU, mi = rem % MU, mu = mi - 2 * L, am = mu < 0 ? -mu : mu;
@@ -396,30 +375,6 @@ k_assemble(const gb::SysDev* __restrict__ sys, int nsys, const long long* __rest
             }
             __syncthreads();
         }
-        if constexpr (LATT) {
-            // the chunk's cells into the running sum, G = sum_c e^{-i k khat.c} G_c (the
-            // tuple sums are linear in G), each thread its own entries
-            for (int qm = tid; qm < PM * MU; qm += NT) {
-                const int q = qm / MU, mi = qm - q * MU;
-                double2 acc = first ? make_double2(0.0, 0.0) : Gs[(size_t)q * MUs + mi];
-                for (int pp = 0; pp < np; pp++) {
-                    const double2 ph = make_double2(geo[8 * pp + 4], geo[8 * pp + 5]);
-                    const double2 gv = cmul(ph, G64[(size_t)PMs * MUs * pp + (size_t)q * MUs + mi]);
-                    acc.x += gv.x;
-                    acc.y += gv.y;
-                }
-                Gs[(size_t)q * MUs + mi] = acc;
-            }
-            __syncthreads();   // before the next chunk rewrites the cells' tables
-            lat_c0 += PB;
-            if (lat_c0 >= lat_end) break;
-            np = min(PB, lat_end - lat_c0);
-        } else {
-            (void)first;
-            break;
-        }
-        }
-
         // ---- phases 2 and 3, software-pipelined over the group's pairs: each thread
         // writes pair pp's block (phase 3) and then forms the tuple values of pair
         // pp + 1 (phase 2) into the other buffer, one barrier per pair.
@@ -435,21 +390,11 @@ k_assemble(const gb::SysDev* __restrict__ sys, int nsys, const long long* __rest
             const bool wantA = kind != 1, wantB = kind != 0;
             const int Q = L + 1;
             for (int it = tid; it < S.M; it += NT) {
-                int t, mi, nv;
-                int2 qq;
-                if constexpr (FP64_SUMS) {
-                    t = it;
-                    const int4 e = S.nmvu[t];
-                    qq = S.qab[t];
-                    mi = (e.w - e.y) + 2 * L;
-                    nv = e.x + e.z;
-                } else {   // sorted order: the lanes of a warp run sums of equal length
-                    const int4 f = S.tinfo[it];
-                    t = f.x;
-                    nv = f.y;
-                    mi = f.z + 2 * L;
-                    qq = make_int2(f.w & 255, f.w >> 8);
-                }
+                // sorted order: the lanes of a warp run sums of equal length (packed FP64,
+                // N = 200, lmax 4: 593 -> 498 us; N = 97, lmax 8: 1976 -> 1612 us)
+                const int4 f = S.tinfo[it];
+                const int t = f.x, nv = f.y, mi = f.z + 2 * L;
+                const int2 qq = make_int2(f.w & 255, f.w >> 8);
                 if constexpr (FP64_SUMS) {
                     const double* ca = S.cA + (size_t)t * Q;
                     const double* cb = S.cB + (size_t)t * Q;
@@ -563,6 +508,17 @@ k_assemble(const gb::SysDev* __restrict__ sys, int nsys, const long long* __rest
                         out64lo[base + e] = make_float2(flipf(v.x, neg), flipf(v.y, neg));
                     }
                 }
+            } else if (LATT) {   // block (i, j), times mie(j, b, v)
+                const int i = (int)(p / N), j = (int)(p % N);
+                const double2* mj_ = mie + (long long)j * 2 * L;
+                for (int e = tid; e < BB; e += NT) {
+                    const int R = e / B, C = e % B;
+                    const int code = __ldg(S.elem_map + e);
+                    const unsigned neg = code & 1;
+                    double2 v = tv[code >> 1];
+                    v = make_double2(flipd(v.x, neg), flipd(v.y, neg));
+                    out128[((long long)i * B + R) * dense_ld + (long long)j * B + C] = cmul(v, mj_[__ldg(S.miecol + C)]);
+                }
             } else if (REFL) {
                 // block (i, j) only: -r0 (-1)^(m+n+a+1) transfer mie(j, b, v)
                 const int i = (int)(p / N), j = (int)(p % N);
@@ -605,33 +561,6 @@ k_assemble(const gb::SysDev* __restrict__ sys, int nsys, const long long* __rest
                 }
             }
         };
-        if constexpr (LATT) {
-            // the tuple values once from the group's summed G table (into the first
-            // cell's slot), then the group's share of block (i, j), times mie(j, b, v),
-            // added to the dense output
-            for (int qm = tid; qm < PM * MU; qm += NT) {
-                const int q = qm / MU, mi = qm - q * MU;
-                G64[(size_t)q * MUs + mi] = Gs[(size_t)q * MUs + mi];
-            }
-            __syncthreads();
-            tuples(0, 0, 2);
-            __syncthreads();
-            const int i = (int)(lat_pair / N), j = (int)(lat_pair % N);
-            const double2* mj_ = mie + (long long)j * 2 * L;
-            for (int e = tid; e < B * B; e += NT) {
-                const int R = e / B, C = e % B;
-                const int code = __ldg(S.elem_map + e);
-                const unsigned neg = code & 1;
-                double2 v = Tv[code >> 1];
-                v = make_double2(flipd(v.x, neg), flipd(v.y, neg));
-                const double2 w = cmul(v, mj_[__ldg(S.miecol + C)]);
-                double* o = reinterpret_cast<double*>(out128 + ((long long)i * B + R) * dense_ld + (long long)j * B + C);
-                atomicAdd(o, w.x);
-                atomicAdd(o + 1, w.y);
-            }
-            __syncthreads();   // the next group rewrites the tables and the sums
-            continue;
-        }
         if constexpr (TS) {
             // the group's (tuple, pair) sums spread evenly over the threads: item it is
             // tuple it % M of pair it / M
@@ -1155,6 +1084,15 @@ int launch_assemble(int nsys, const gb_system* sys, const double* pos, const dou
                 PB = NB = pb;
             }
         }
+        // few pairs: no more of them per group than fill every SM's CTAs (three with FP64
+        // sums, five otherwise) once, so that the groups run beside each other rather than
+        // their pairs one after another (dense, N = 30, lmax 3: 121 -> 44 us; packed FP64,
+        // N = 20, lmax 6: 131 -> 66 us; the blocks' bits do not depend on it)
+        const long long slots = (fp64_sums ? 3LL : 5LL) * gb::sm_count();
+        const int fill = (int)std::min<long long>(32, std::max<long long>(1, (total_pairs + slots - 1) / slots));
+        PB = std::min(PB, fill);
+        if (ts) NB = PB;
+        if (latt) PB = NB = 1;
         // one pair's A and B tuple values together beyond a CTA's shared memory (lmax 10):
         // the split kernel forms and writes them one kind at a time
         const bool split = !ts && !refl && !latt && asm_layout(L, Mmax, PB, fp64_sums, want64, NB).total > 227 * 1024;
@@ -1162,30 +1100,19 @@ int launch_assemble(int nsys, const gb_system* sys, const double* pos, const dou
         const AsmSmem lay = asm_layout(L, Mmax, PB, fp64_sums, want64, NB, split, latt != nullptr);
         const size_t smem = lay.total;
         if (smem > 227 * 1024) return gb_set_error(GB_UNSUPPORTED, "assembler needs %zu B of shared memory", smem);
-        Latt lt = latt ? *latt : Latt();
-        if (latt) {
-            if (lt.ncell < 1) return GB_OK;
-            // each group sums a range of whole chunks of PB cells (its tuple sums and
-            // block additions once per range); enough groups to fill the SMs about
-            // twice, at least one per ordered pair
-            long long pairs = 0;
-            for (const gb::SysDev& d : sd) pairs += (long long)d.N * d.N;
-            const long long chunks = (lt.ncell + PB - 1) / PB;
-            const long long want = 6LL * gb::sm_count();
-            const long long g = std::min<long long>(chunks, std::max<long long>(1, (want + pairs - 1) / pairs));
-            lt.cpg = (int)(((chunks + g - 1) / g) * PB);
-            lt.gpp = (lt.ncell + lt.cpg - 1) / lt.cpg;
-        }
         std::vector<long long> gbase(ns + 1, 0);
         for (int s = 0; s < ns; s++) {
-            const long long np_s = refl ? (long long)sd[s].N * sd[s].N : sd[s].P;
-            gbase[s + 1] = gbase[s] + (latt ? (long long)sd[s].N * sd[s].N * lt.gpp : (np_s + PB - 1) / PB);
+            const long long np_s = refl || latt ? (long long)sd[s].N * sd[s].N : sd[s].P;
+            gbase[s + 1] = gbase[s] + (np_s + PB - 1) / PB;
         }
         const long long ngroups = gbase[ns];
         // the double-float path's G-table pass: PG pairs per CTA (the most, up to 32,
         // whose special functions fit in 48 KB of shared memory)
         int PG = 32;
         while (PG > 1 && gtab_layout(L, PG).total > 48 * 1024) PG >>= 1;
+        // (few pairs: fewer per CTA, at least four, until two CTAs per SM are filled)
+        const long long spread = (total_pairs + 2LL * gb::sm_count() - 1) / (2LL * gb::sm_count());
+        PG = std::min(PG, (int)std::max<long long>(4, std::min<long long>(32, spread)));
         std::vector<long long> gbase2(ns + 1, 0);
         for (int s = 0; s < ns; s++) gbase2[s + 1] = gbase2[s] + (fp64_sums ? 0 : (sd[s].P + PG - 1) / PG);
         // one staging upload: descriptors, then the group prefix sums of both passes
@@ -1247,7 +1174,7 @@ int launch_assemble(int nsys, const gb_system* sys, const double* pos, const dou
         kfn<<<(unsigned)std::min<long long>(ngroups, 0x7fffffffLL), nt, smem, stream>>>(
             dsys, ns, dbase, ngroups, L, Mmax, PB, NB, pos, reinterpret_cast<const double2*>(mie),
             reinterpret_cast<double2*>(out128), reinterpret_cast<float2*>(out64), reinterpret_cast<float2*>(out64lo),
-            dense_ld, refl ? *refl : Refl(), lt);
+            dense_ld, refl ? *refl : Refl(), latt ? *latt : Latt());
         GB_CUDA_TRY(cudaGetLastError());
         st = gb::stage_release(slot, stream);
         if (st) return st;
@@ -1288,20 +1215,24 @@ int gb_aggregate_periodic_dense(int N, int lmax, const double* pos, const double
     if (!pos || !mie || !out || (ncell > 0 && !cells)) return gb_set_error(GB_BAD_ARG, "null pointer");
     if (N < 1 || lmax < 1 || lmax > GB_LMAX_MAX || ncell < 0)
         return gb_set_error(GB_BAD_ARG, "N=%d lmax=%d ncell=%d invalid", N, lmax, ncell);
+    if (!(k > 0.0)) return gb_set_error(GB_BAD_ARG, "cluster 0: wavenumber must be positive");
+    cudaStream_t st = (cudaStream_t)stream;
     const long long D = 2LL * lmax_to_rmax(lmax) * N;
-    GB_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(double2) * D * D, (cudaStream_t)stream));
     gb_system s{N, lmax, k, 0, 0, 0, 0};
-    if (N > 1) {
-        const int e = launch_assemble(1, &s, pos, mie, out, nullptr, nullptr, D, true, (cudaStream_t)stream);
-        if (e) return e;
+    if (lmax > 9) {   // the lattice blocks' tuple values exceed a CTA's shared memory (as the assembler reports)
+        if (ncell > 0) return gb_set_error(GB_UNSUPPORTED, "lattice sums support lmax 1..9 (got %d)", lmax);
+        return gb_assemble_sphere_dense(N, lmax, pos, mie, k, out, stream);
     }
+    const gb::Tables* T = nullptr;
+    int e = gb::get_tables(lmax, st, &T);
+    if (e) return e;
+    // the summed tables into the output's own blocks, then the blocks from them
+    e = gb::launch_lattice_sums(N, lmax, pos, k, cells, ncell, kx, ky, kz, T->neg_ratio, reinterpret_cast<double2*>(out), D,
+                                st);
+    if (e) return e;
     Latt lt;
-    lt.cells = cells;
-    lt.ncell = ncell;
-    lt.kx = kx;
-    lt.ky = ky;
-    lt.kz = kz;
-    return launch_assemble(1, &s, pos, mie, out, nullptr, nullptr, D, true, (cudaStream_t)stream, nullptr, &lt);
+    lt.tables = gb::lattice_chunks(N, lmax, ncell);
+    return launch_assemble(1, &s, pos, mie, out, nullptr, nullptr, D, true, st, nullptr, &lt);
 }
 
 int gb_assemble_sphere_packed(int N, int lmax, const double* pos, double k, double* out128, float* out64,
