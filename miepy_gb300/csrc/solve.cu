@@ -1146,8 +1146,9 @@ struct ScalarFuse {
 
 // Called by every thread of a CTA of cluster sys once its partial dots are
 // written and fenced.  The last CTA of the cluster sums the cluster's partials
-// with all its NT threads (strided per thread, then warp butterflies, then the
-// warps in order: a fixed order, deterministic) and updates the scalars.
+// (R <= 2: strided over its NT threads, then butterflies of the warps that hold
+// partials, then the warps in order; R > 2: a warp per sum: a fixed order,
+// deterministic) and updates the scalars.
 template <int R, int NT, typename T>
 __device__ void fused_scalar_cta(const ScalarFuse& fz, const SysPlan* __restrict__ plan,
                                  const double2* __restrict__ dots_raw, int sys, int nitems_sys) {
@@ -1170,24 +1171,38 @@ __device__ void fused_scalar_cta(const ScalarFuse& fz, const SysPlan* __restrict
     const bool vec = (fz.phase == 0 || fz.phase == 3);
     const int b0 = vec ? pl.vbeg : pl.rbeg, b1 = vec ? pl.vend : pl.rend;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int nact = R > 2 ? 1 : min(NT / 32, (b1 - b0 + 31) / 32);
+    if constexpr (R > 2) {
+        for (int q = wid; q < 2 * R; q += NT / 32) {
+            DotAcc<T> d, t;
+            d.zero();
+            for (int it = b0 + lane; it < b1; it += 32) {
+                t.load_cg(dots + ((long long)it * R + (q >> 1)) * 2 + (q & 1));
+                d.add(t);
+            }
+            for (int o = 16; o > 0; o >>= 1) d.add(d.shuffled(o));
+            if (lane == 0) s_red[0][q >> 1][q & 1] = d;
+        }
+    } else if (wid < nact) {
 #pragma unroll
-    for (int rr = 0; rr < R; rr++) {
-        DotAcc<T> d0, d1, t;
-        d0.zero();
-        d1.zero();
-        for (int it = b0 + (int)threadIdx.x; it < b1; it += NT) {
-            t.load_cg(dots + ((long long)it * R + rr) * 2 + 0);   // written by other CTAs
-            d0.add(t);
-            t.load_cg(dots + ((long long)it * R + rr) * 2 + 1);
-            d1.add(t);
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            d0.add(d0.shuffled(o));
-            d1.add(d1.shuffled(o));
-        }
-        if (lane == 0) {
-            s_red[wid][rr][0] = d0;
-            s_red[wid][rr][1] = d1;
+        for (int rr = 0; rr < R; rr++) {
+            DotAcc<T> d0, d1, t;
+            d0.zero();
+            d1.zero();
+            for (int it = b0 + (int)threadIdx.x; it < b1; it += NT) {
+                t.load_cg(dots + ((long long)it * R + rr) * 2 + 0);   // written by other CTAs
+                d0.add(t);
+                t.load_cg(dots + ((long long)it * R + rr) * 2 + 1);
+                d1.add(t);
+            }
+            for (int o = 16; o > 0; o >>= 1) {
+                d0.add(d0.shuffled(o));
+                d1.add(d1.shuffled(o));
+            }
+            if (lane == 0) {
+                s_red[wid][rr][0] = d0;
+                s_red[wid][rr][1] = d1;
+            }
         }
     }
     __syncthreads();
@@ -1198,7 +1213,7 @@ __device__ void fused_scalar_cta(const ScalarFuse& fz, const SysPlan* __restrict
         DotAcc<T> d0, d1;
         d0.zero();
         d1.zero();
-        for (int w = 0; w < NT / 32; w++) {
+        for (int w = 0; w < nact; w++) {
             d0.add(s_red[w][rr][0]);
             d1.add(s_red[w][rr][1]);
         }
@@ -1400,10 +1415,12 @@ k_reduce_blk(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items,
     // lanes of equal rhs leave each warp's sums in lanes 0..R-1; the warps holding
     // rows are then added in order (a fixed tree: deterministic)
     const int lane = tid & 31, wid = tid >> 5, nw = (BR + 31) / 32;
+    if (wid < nw) {
 #pragma unroll
-    for (int o = 16; o >= R; o >>= 1) {
-        d0.add(d0.shuffled(o));
-        d1.add(d1.shuffled(o));
+        for (int o = 16; o >= R; o >>= 1) {
+            d0.add(d0.shuffled(o));
+            if (mode == 2) d1.add(d1.shuffled(o));   // zero otherwise
+        }
     }
     if (lane < R && wid < nw) {
         red[wid][lane][0] = d0;
@@ -1487,8 +1504,11 @@ k_reduce_dense(const gb::SysDev* __restrict__ sys, const Item* __restrict__ item
 // kind 2: s-update  s = r - alpha v
 // kind 3: x/r       x += alpha p + omega s (times pdiag, when given); r = s - omega t;  dots: |r|^2, <r0, r>
 // kind 4: restart   r0 = r (r already b - A x)
+// Threads of the vector updates: more than two right-hand sides have them side by side.
+__host__ __device__ constexpr int vec_threads(int R) { return R > 2 ? 2 * kVRows : kVRows; }
+
 template <typename VT, int R>
-__global__ void __launch_bounds__(kVRows)
+__global__ void __launch_bounds__(vec_threads(R))
 k_vec(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items, int nitems, const KState* __restrict__ st,
       int kind, const double2* __restrict__ b, VT* __restrict__ bx, VT* __restrict__ x, VT* __restrict__ r,
       VT* __restrict__ r0, VT* __restrict__ p, VT* __restrict__ v, VT* __restrict__ s, const VT* __restrict__ t,
@@ -1508,20 +1528,24 @@ k_vec(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items, int ni
     using C = typename Arith<VT>::C;
     using T = typename Arith<VT>::T;
     const T tg{};
-    __shared__ DotAcc<T> red[kVRows / 32][R][2];
-    const int lr = threadIdx.x;
-    DotAcc<T> d0[R], d1[R];
+    // a thread per row with the row's right-hand sides (R <= 2), or NT threads over the
+    // item's elements, each always on one right-hand side
+    constexpr bool SPREAD = R > 2;
+    constexpr int NT = vec_threads(R), ND = SPREAD ? 1 : R;
+    __shared__ DotAcc<T> red[NT / 32][R][2];
+    DotAcc<T> d0[ND], d1[ND];
 #pragma unroll
-    for (int rr = 0; rr < R; rr++) {
+    for (int rr = 0; rr < ND; rr++) {
         d0[rr].zero();
         d1[rr].zero();
     }
-    if (lr < I.nr) {
-        const long long vo = S.vec_off + (long long)(I.r0 + lr) * R;
+    {
 #pragma unroll
-        for (int rr = 0; rr < R; rr++) {
-            if (!active_rhs<R>(st, I.sys, rr, mask)) continue;
-            const long long e = vo + rr;
+        for (int q = 0; q < (SPREAD ? R * kVRows / NT : R); q++) {
+            const int el = SPREAD ? (int)threadIdx.x + q * NT : (int)threadIdx.x * R + q;
+            const int lr = SPREAD ? el / R : (int)threadIdx.x, rr = SPREAD ? el % R : q, dq = SPREAD ? 0 : q;
+            if (lr >= I.nr || !active_rhs<R>(st, I.sys, rr, mask)) continue;
+            const long long e = S.vec_off + (long long)(I.r0 + lr) * R + rr;
             const KState& k = st[I.sys * R + rr];
             if (kind == 0) {
                 const VT bq = b ? from_d2<VT>(b[e]) : bx[e];
@@ -1529,7 +1553,7 @@ k_vec(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items, int ni
                 x[e] = z; p[e] = z; v[e] = z;
                 r[e] = bq; r0[e] = bq;
                 if (bx && b) bx[e] = bq;
-                d0[rr].add_norm2(to_c<C>(bq));
+                d0[dq].add_norm2(to_c<C>(bq));
             } else if (kind == 1) {
                 const C rv = to_c<C>(r[e]), pv = to_c<C>(p[e]), vv = to_c<C>(v[e]);
                 const C bt = cmul(ks_beta(k, tg), csub(pv, cmul(ks_omega(k, tg), vv)));
@@ -1546,38 +1570,39 @@ k_vec(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items, int ni
                 const VT rq = from_c<VT>(csub(sv, wt));
                 r[e] = rq;
                 const C rd = to_c<C>(rq), r0v = to_c<C>(r0[e]);
-                d0[rr].add_norm2(rd);
-                d1[rr].fma_conj(r0v, rd);
+                d0[dq].add_norm2(rd);
+                d1[dq].fma_conj(r0v, rd);
             } else if (kind == 4) {
                 r0[e] = r[e];
             }
         }
     }
     if (kind == 1 || kind == 2 || kind == 4) return;
-    const int lane = lr & 31, wid = lr >> 5;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
-    for (int rr = 0; rr < R; rr++) {
-        for (int o = 16; o > 0; o >>= 1) {
+    for (int rr = 0; rr < ND; rr++) {
+        for (int o = 16; o >= (SPREAD ? R : 1); o >>= 1) {
             d0[rr].add(d0[rr].shuffled(o));
             d1[rr].add(d1[rr].shuffled(o));
         }
-        if (lane == 0) {
-            red[wid][rr][0] = d0[rr];
-            red[wid][rr][1] = d1[rr];
+        if (lane < (SPREAD ? R : 1)) {
+            red[wid][rr + lane][0] = d0[rr];
+            red[wid][rr + lane][1] = d1[rr];
         }
     }
     __syncthreads();
+    const int lr = threadIdx.x;
     if (lr < R * 2) {
         const int rr = lr >> 1, which = lr & 1;
         DotAcc<T> sm;
         sm.zero();
-        for (int w = 0; w < kVRows / 32; w++) sm.add(red[w][rr][which]);
+        for (int w = 0; w < NT / 32; w++) sm.add(red[w][rr][which]);
         sm.store(dots + ((long long)it * R + rr) * 2 + which);
     }
     if (fz.st) {
         if (lr < R * 2) __threadfence();   // this thread's partial before the arrival count
         const SysPlan pl = plan[I.sys];
-        fused_scalar_cta<R, kVRows, T>(fz, plan, dots, I.sys, pl.vend - pl.vbeg);
+        fused_scalar_cta<R, NT, T>(fz, plan, dots, I.sys, pl.vend - pl.vbeg);
     }
 }
 
@@ -2329,12 +2354,12 @@ int run_bicgstab(const Plan& P, const DevPlan& D, const WS& w, unsigned char* ba
         int e;
         if (DENSE) {
             gb::note_launch();
-            k_vec<VT, R><<<vb, kVRows, 0, sm>>>(D.sys, D.vitems, P.nv, st, 1, nullptr, nullptr, x, r, r0, p, v, s, t,
+            k_vec<VT, R><<<vb, vec_threads(R), 0, sm>>>(D.sys, D.vitems, P.nv, st, 1, nullptr, nullptr, x, r, r0, p, v, s, t,
                                                 dots);
             e = apply(p, v, 1, r0, 0, nullptr, sm, fuse(1));
             if (e) return e;
             gb::note_launch();
-            k_vec<VT, R><<<vb, kVRows, 0, sm>>>(D.sys, D.vitems, P.nv, st, 2, nullptr, nullptr, x, r, r0, p, v, s, t,
+            k_vec<VT, R><<<vb, vec_threads(R), 0, sm>>>(D.sys, D.vitems, P.nv, st, 2, nullptr, nullptr, x, r, r0, p, v, s, t,
                                                 dots);
             e = apply(s, t, 2, s, 0, nullptr, sm, fuse(2));
             if (e) return e;
@@ -2349,7 +2374,7 @@ int run_bicgstab(const Plan& P, const DevPlan& D, const WS& w, unsigned char* ba
             if (e) return e;
         }
         gb::note_launch();
-        GB_CUDA_TRY(launch_pdl(k_vec<VT, R>, dim3(vb), dim3(kVRows), 0, sm, D.sys, D.vitems, P.nv, st, 3, nullptr,
+        GB_CUDA_TRY(launch_pdl(k_vec<VT, R>, dim3(vb), dim3(vec_threads(R)), 0, sm, D.sys, D.vitems, P.nv, st, 3, nullptr,
                                nullptr, x, r, r0, p, v, s, t, dots, D.sp, fuse(3), pdiag));
         GB_CUDA_TRY(cudaGetLastError());
         return GB_OK;
@@ -2357,7 +2382,7 @@ int run_bicgstab(const Plan& P, const DevPlan& D, const WS& w, unsigned char* ba
 
     // init: x = 0, r = r0 = b, scalars
     gb::note_launch();
-    k_vec<VT, R><<<vb, kVRows, 0, stream>>>(D.sys, D.vitems, P.nv, st, 0, b128, bvt ? bvt : bx, x, r, r0, p, v, s, t,
+    k_vec<VT, R><<<vb, vec_threads(R), 0, stream>>>(D.sys, D.vitems, P.nv, st, 0, b128, bvt ? bvt : bx, x, r, r0, p, v, s, t,
                                             dots, D.sp, fuse(0));
     GB_CUDA_TRY(cudaGetLastError());
     const VT* bsrc_vt = bvt ? bvt : bx;
@@ -2484,7 +2509,7 @@ int run_bicgstab(const Plan& P, const DevPlan& D, const WS& w, unsigned char* ba
             int e = apply(x, r, 3, bsrc_vt, 1, b128, stream);
             if (e) return e;
             gb::note_launch();
-            k_vec<VT, R><<<vb, kVRows, 0, stream>>>(D.sys, D.vitems, P.nv, st, 4, nullptr, nullptr, x, r, r0, p, v, s,
+            k_vec<VT, R><<<vb, vec_threads(R), 0, stream>>>(D.sys, D.vitems, P.nv, st, 4, nullptr, nullptr, x, r, r0, p, v, s,
                                                     t, dots);
             gb::note_launch();
             k_scalar<R, typename Arith<VT>::T><<<sblocks, 128, 0, stream>>>(D.sp, P.nsys, st, 4, dots, tol, maxiter);
