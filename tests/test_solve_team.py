@@ -102,3 +102,33 @@ def test_packed_ragged_batches(R):
             for q in range(R):
                 d = (want - got)[..., q].norm() / want[..., q].norm()
                 assert d < 2e-11, (shapes[s], q, float(d))
+
+
+@pytest.mark.parametrize("R", [1, 2])
+@pytest.mark.parametrize("shapes", [[(2, 1)], [(5, 2)], [(3, 7)], [(26, 3)], [(14, 6)], [(15, 6)], [(5, 2), (7, 1), (2, 4)],
+                                    [(5, 2)] * 152, [(5, 2)] * 153])
+def test_small_mixed_solves(shapes, R):
+    """The mixed method's small systems and batches, at and past the limits of the
+    single-launch solve: the true residual (double-float product) meets the tolerance."""
+    from miepy_gb300.engine import ClusterBatch
+    rng = np.random.default_rng(11)
+    specs = []
+    for N, L in shapes:
+        pos = np.array([(i % 4, i // 4 % 4, i // 16) for i in range(N)], float) * 3e-7 + rng.uniform(-2e-8, 2e-8, (N, 3))
+        mie = (rng.normal(size=(N, 2, L)) + 1j * rng.normal(size=(N, 2, L))) * 0.1 ** np.arange(1, L + 1)
+        p = rng.normal(size=(N, 2, L * (L + 2), R)) + 1j * rng.normal(size=(N, 2, L * (L + 2), R))
+        specs.append(dict(position=pos, mie_scat=mie, k=1.05e7, p_src=p))
+    b = ClusterBatch(specs, R=R, precision="mixed").assemble()
+    b.solve(tol=1e-10, inner_tol=1e-4)
+    assert np.all(b.status == 0) and np.all(b.resid <= 1e-10) and np.all(b.iters >= 1)
+    d = b.b - b.apply(b.x, "mixed")
+    for s in range(len(shapes)):
+        for q in range(R):
+            rel = b.cluster_view(s, d)[..., q].norm() / b.cluster_view(s, b.b)[..., q].norm()
+            assert float(rel) < 2e-10
+    # a right-hand side that cannot be solved ends as the refinement reports it
+    specs[0]["p_src"] = specs[0]["p_src"].copy()
+    specs[0]["p_src"][0, 0, 0, 0] = np.inf
+    b.load(specs).assemble()
+    b.solve(tol=1e-10, inner_tol=1e-4)
+    assert b.status[0] == nat.GB_NAN and np.all(b.status[R:] == 0)
