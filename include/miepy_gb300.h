@@ -214,11 +214,12 @@ int gb_sphere_preconditioner(long long n, const double* tvec, double* pdiag, voi
 int gb_dense_precondition_matrix(int D, int bs, const double* T, const double* Minv, double* Tp, void* stream);
 int gb_block_diag_apply(int D, int R, int bs, const double* Minv, const double* u, double* x, void* stream);
 
-/* Bytes of the bf16 tile arena for a batch: per pair block 2 planes of Bp x Kp bf16
- * (Bp = B rounded up to 8, Kp = 2B rounded up to 16), clusters in batch order. */
+/* Bytes of the bf16 tile arena for a batch: per pair block [[P, Q], [Q, P]] (over the
+ * polarisations) the hi and lo planes of P + Q and of P - Q, each Hp x Kp bf16 (Hp = B / 2
+ * rounded up to 8, at least 16, Kp = B rounded up to 16), clusters in batch order. */
 size_t gb_tc_matrix_bytes(int nsys, const gb_system* sys);
 /* mat_tc = the bf16 hi/lo tiles of the packed complex64 matrix mat64 (hi = bf16(a),
- * lo = bf16(a - hi) per real component), in the core-matrix layout the tensor-core
+ * lo = bf16(a - hi) per real component of a = P + Q and P - Q), in the core-matrix layout the tensor-core
  * pass streams into shared memory; one launch, to be repeated after every
  * assembly.  Both pointers 16-byte aligned. */
 int gb_tc_matrix_build(int nsys, const gb_system* sys, const float* mat64, void* mat_tc, void* stream);

@@ -886,7 +886,7 @@ int sm_count() {
 
 int make_sysdev(int nsys, const gb_system* sys, cudaStream_t stream, std::vector<SysDev>& out) {
     out.resize(nsys);
-    long long tc_off = 0;
+    long long tc_off = 0, ty_off = 0;
     for (int s = 0; s < nsys; s++) {
         const gb_system& a = sys[s];
         if (a.N < 1 || a.lmax < 1 || a.lmax > GB_LMAX_MAX)
@@ -924,6 +924,8 @@ int make_sysdev(int nsys, const gb_system* sys, cudaStream_t stream, std::vector
         d.miecol = T->miecol;
         d.tc_off = tc_off;
         tc_off += d.P * tc_block_bytes(d.B);
+        d.ty_off = ty_off;
+        ty_off += a.N * tc_y_bytes(d.B, 1);
     }
     return GB_OK;
 }

@@ -87,18 +87,24 @@ struct SysDev {
     // byte offset of this cluster's blocks in the bf16 tile arena of the tensor-core
     // matrix pass (tc_block_bytes(B) per pair, clusters in batch order)
     long long tc_off = 0;
+    // byte offset per right-hand side of its particles' operands of that pass
+    long long ty_off = 0;
 };
 
-// bf16 tiles of one B x B complex64 block for the tensor-core matrix pass: the hi
-// and lo planes (hi = bf16(a), lo = bf16(a - hi), per real component), each
-// Bp x Kp bf16 (Bp = B rounded up to 8 rows, Kp = 2B real columns rounded up to 16)
-// in the K-major core-matrix layout of tcgen05 operands: element (m, k) at
-// (m / 8) * (Kp * 16) + (k / 8) * 128 + (m % 8) * 16 + (k % 8) * 2 bytes; padding
-// rows and columns hold zeros.
-__host__ __device__ inline int tc_rows(int B) { return (B + 7) & ~7; }
-__host__ __device__ inline int tc_cols(int B) { return (2 * B + 15) & ~15; }
+// bf16 tiles of one B x B complex64 block [[P, Q], [Q, P]] for the tensor-core matrix
+// pass: the hi and lo planes (hi = bf16(a), lo = bf16(a - hi), per real component) of
+// P + Q, then of P - Q, each Hp x Kp bf16 (Hp = B / 2 rounded up to 8 rows, at least 16, Kp = B real
+// columns rounded up to 16) in the K-major core-matrix layout of tcgen05 operands: element
+// (m, k) at (m / 8) * (Kp * 16) + (k / 8) * 128 + (m % 8) * 16 + (k % 8) * 2 bytes;
+// padding rows and columns hold zeros.
+__host__ __device__ inline int tc_rows(int B) { return B <= 30 ? 16 : (B / 2 + 7) & ~7; }
+__host__ __device__ inline int tc_cols(int B) { return (B + 15) & ~15; }
 __host__ __device__ inline long long tc_plane_bytes(int B) { return 2LL * tc_rows(B) * tc_cols(B); }
-__host__ __device__ inline long long tc_block_bytes(int B) { return 2 * tc_plane_bytes(B); }
+__host__ __device__ inline long long tc_block_bytes(int B) { return 4 * tc_plane_bytes(B); }
+// one particle's operand of that pass, U or W, for R right-hand sides: pieces of 2R rows
+// (row 2 q: re, 2 q + 1: im of right-hand side q) x Kp columns in the layout above, hi
+// of sign + and of sign -, then lo
+__host__ __device__ inline long long tc_y_bytes(int B, int R) { return 16LL * tc_cols(B) * R; }
 
 // Pinned staging ring for per-call descriptor uploads (assemble.cu).
 int stage_acquire(const void* src, size_t bytes, cudaStream_t stream, void** dev_out, int* slot_out);

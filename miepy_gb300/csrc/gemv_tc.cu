@@ -15,31 +15,41 @@
 // mixed method's FP32 inner solves (to 1e-4) use it; its refinement residuals keep
 // the CUDA-core complex64 and double-float passes.
 //
-// A complex block product as one real GEMM: A is [B rows][2B real columns] (re, im
-// interleaved along K); a complex vector z becomes two real B-operand rows,
-// (re z, -im z) giving re(A z) and (im z, re z) giving im(A z).  One MMA per K-step
-// multiplies A_hi by N = 8R rows [U_h | W_h | U_l | W_l] and a second A_lo by the
-// first 4R, into one accumulator of N FP32 columns:
+// Half of a block is read: with P, Q its upper quadrants (block = [[P, Q], [Q, P]] over
+// the polarisations) the tiles hold P + Q and P - Q, which act on (z1 +- z2) / 2, z1 and z2
+// the two polarisations of a vector z.  A complex product as a real GEMM: a tile is
+// [B/2 rows][B real columns] (re, im interleaved along K); a complex vector becomes two
+// real B-operand rows, (re z, -im z) giving re(A z) and (im z, re z) giving im(A z).  For
+// both signs one MMA per K-step multiplies A_hi by N = 16R rows [U_h+ W_h+ U_h- W_h- | U_l+
+// W_l+ U_l- W_l-] and a second A_lo by the first 8R, into an accumulator of N FP32 columns;
+// of the tile's planes (+ hi, + lo, - hi, - lo, their rows one after the other) the first
+// MMA's 128 rows hold + hi and, from row 2 Hp on, - hi, the second's + lo and - lo at the
+// same rows, and only the columns of a row's own sign are read out:
 //   U = A z_j (row product of block (i, j), summed along the strip),
 //   W = A w_i (column product, one partial per block), w_i = S z_i,
-// with z[s] = eps(s) y[rho(s)] formed from the solver's y vectors, and the results
-// stored as the CUDA-core pass stores its column sums, C[rho(r)] = eps(r) (A z)[r],
-// so the block reduce that follows is shared.
+// with z[s] = eps(s) y[rho(s)] of the solver's y vectors.  k_yprep_tc writes each particle's
+// rows of U and of W once per product as bf16 pieces in the operand's layout, so that a
+// block's operand arrives by copies.  The results C[rho(r)] = eps(r) (A z)[r] are stored
+// by sign as the CUDA-core pass stores its +- column sums: C[s] = c+ + c-, C[rmax + s] =
+// c+ - c- with c+ = eps (the sum of sign -) and c- = eps (that of sign +), as eps of the
+// two polarisations are opposite; element (column, right-hand side q) of a term lies at 16-byte
+// word (q / 2) B + sign rmax + column, so that a warp's stores are contiguous.
 //
-// Pipeline per CTA (160 threads, two CTAs per SM, persistent over strips): a
-// producer warp walks the CTA's strips ahead of the others and, per block, writes a
-// job record and streams the block's two planes with its y_w (and the strip's y_u
-// with its first block) by bulk copies (TMA) into a ring of 3 stages, reusing a stage
-// once the MMAs that read it have committed to its empty barrier; the 4 consumer
-// warps build the block's B operand (bf16, core-matrix layout) in one of two buffers;
-// thread 0 issues the block's MMAs (M = 128: the block's rows, padding rows read and
-// discarded) into one of two TMEM accumulators and commits them to mbarriers;
-// meanwhile the consumer warps read the previous block's accumulator rows
-// (tcgen05.ld), write its column partials and keep the strip's row sums.  Every wait
-// is bounded; an expired wait sets the error flag, the consumers decide to stop
-// together through a reduction barrier, and the CTA waits (again bounded) for its
+// Pipeline per CTA (6 warps, two CTAs per SM where their stages fit, persistent over
+// strips), each role running ahead of the next one as far as the rings let it: a producer
+// warp copies, per block, the tile and the operand's pieces (TMA bulk copies) into a ring
+// of stages, with a job record; one thread issues the block's MMAs (M = 128: the rows past
+// the tile's read what follows it and are discarded) into one of two accumulators; the
+// warps of the tile's rows read the accumulator (tcgen05.ld), write its column partials and
+// keep the strip's row sums.  Every wait is bounded; an expired wait sets the error flag and the
+// abort flag, which ends the other roles' waits, and the CTA waits (again bounded) for its
 // copies and MMAs in flight before it frees its TMEM and exits.
-
+//
+// Bound: per block, the issue of 9 copies (270 cycles) and of the MMAs, two CTAs per SM, next
+// to the tiles' 27 us at the measured copy rate.  N = 200, lmax 4: 45 us at R = 8, 33 at
+// R = 4; with whole blocks, their operand built by each CTA, 102 and 89.  (Issued from
+// divergent code, copies and MMAs took 83 to 160 cycles each: 71 and 57 us; a sign at a
+// time, with twice the MMAs, each bound by its 128 rows: 49 and 36.)
 #include <cuda_bf16.h>
 
 #include "gb_common.cuh"
@@ -48,8 +58,8 @@
 
 namespace {
 
-constexpr int kTcThreads = 160;   // 4 consumer warps + 1 producer warp
-constexpr int kTcStages = 3;
+constexpr int kTcThreads = 192;   // warps 0-3: accumulator rows out; 4: copies in; 5: MMAs
+constexpr int kTcMaxStages = 5;
 constexpr long long kTcWaitCycles = 400000000LL;   // about 0.2 s of SM clock
 
 __device__ __forceinline__ unsigned su32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -72,12 +82,23 @@ __device__ __forceinline__ bool bar_try(uint64_t* b, unsigned parity) {
         : "memory");
     return ok != 0;
 }
-__device__ __forceinline__ bool bar_wait(uint64_t* b, unsigned parity) {
+// bounded; given a flag, it also ends (false) once the flag is set
+__device__ __forceinline__ bool bar_wait(uint64_t* b, unsigned parity, const volatile int* stop = nullptr) {
     if (bar_try(b, parity)) return true;
     const long long t0 = clock64();
     while (!bar_try(b, parity))
-        if (clock64() - t0 > kTcWaitCycles) return false;
+        if ((stop && *stop) || clock64() - t0 > kTcWaitCycles) return false;
     return true;
+}
+// one lane of the warp (the same one each time); warp-uniform code around it keeps the
+// operands of the copies and MMAs in uniform registers
+__device__ __forceinline__ bool elect_one() {
+    unsigned p;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ void bar_arrive(uint64_t* b) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(su32(b)) : "memory");
 }
 __device__ __forceinline__ void bulk_copy(void* dst, const void* src, unsigned bytes, uint64_t* b) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
@@ -137,385 +158,362 @@ __host__ __device__ constexpr unsigned idesc_bf16(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(N >> 3) << 17) | ((unsigned)(M >> 4) << 24);
 }
 
-__device__ __forceinline__ unsigned bf2(float lo_half, float hi_half) {   // (first, second) in memory order
-    __nv_bfloat162 v = __floats2bfloat162_rn(lo_half, hi_half);
-    return *reinterpret_cast<unsigned*>(&v);
-}
-__device__ __forceinline__ float bf_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
-
 // ------------------------------------------------------------ shared layout --
-// Header: S full barriers, 2 MMA barriers, the TMEM address, the abort flag, then S
-// job records; the row map at off_row; the two B-operand buffers; S stages, each
-// the block's two bf16 planes, its y_u (particle j) and y_w (particle i).
+// Header: the barriers, the TMEM address, the abort flag, the consumed count, the job
+// records of the stages and of the two accumulators; then the stages, each a block's tile
+// (hi, lo of P + Q, then of P - Q) and the operand's pieces (8, 2R rows each).
 struct TcJob {
-    long long cw;    // element offset of the block's column partials in CW
+    long long cw;    // element offset of the block's column partials in CW; -1: no more blocks for this CTA
     long long cu;    // element offset of the strip's row partials in CU (last block of a strip), else -1
-    int valid;       // 0: no more blocks for this CTA
-    int pad;
+};
+// Block k's record lies in slot k % kTcJobs.  It is read by the MMA thread and by the warps
+// that read the accumulator out, which are at most kTcMaxStages + 1 blocks behind.
+constexpr int kTcJobs = 8;
+static_assert(kTcJobs >= kTcMaxStages + 2, "job records");
+struct TcHeader {
+    uint64_t full[kTcMaxStages], empty[kTcMaxStages];   // a stage's copies landed; its MMAs done
+    uint64_t mdone[2], job[2], free[2];                 // an accumulator's MMAs done, job known, read out
+    long long consumed;                                 // jobs the MMA thread has taken
+    TcJob jobs[kTcJobs];
+    unsigned tmem;
+    int abort;
 };
 struct TcLayout {
-    unsigned sbo, plane, tile, ybytes, stage, bbytes;
-    unsigned off_jobs, off_row, off_b, off_stage, total;
+    unsigned sbo, plane, tile, piece, stage, total;
 };
-__host__ __device__ inline TcLayout tc_layout(int B, int R) {
+constexpr unsigned kTcStageOff = 512;
+static_assert(sizeof(TcHeader) <= kTcStageOff, "header");
+__host__ __device__ inline TcLayout tc_layout(int B, int R, int S) {
     TcLayout L;
-    const int Kp = gb::tc_cols(B), Bp = gb::tc_rows(B);
-    L.sbo = (unsigned)Kp * 16u;
-    L.plane = (unsigned)(Bp / 8) * L.sbo;
-    L.tile = 2u * L.plane;
-    L.ybytes = (unsigned)(B * R * 8);
-    L.stage = (L.tile + 2u * L.ybytes + 127u) & ~127u;
-    L.bbytes = (unsigned)(8 * R) * (unsigned)Kp * 2u;
-    L.off_jobs = 128;   // after 2S + 2 barriers, the TMEM slot, the abort flag, the consumed count
-    L.off_row = 256;
-    L.off_b = 1024;
-    L.off_stage = L.off_b + 2u * L.bbytes;
-    unsigned end = L.off_stage + (unsigned)kTcStages * L.stage;
-    // an M = 128 MMA reads 16 row groups of each plane: the lo plane of the last
-    // stage reads up to plane + 16 sbo past that stage's start
-    const unsigned reach = L.off_stage + (unsigned)(kTcStages - 1) * L.stage + L.plane + 16u * L.sbo;
+    L.sbo = (unsigned)gb::tc_cols(B) * 16u;
+    L.plane = (unsigned)(gb::tc_rows(B) / 8) * L.sbo;
+    L.tile = 4u * L.plane;
+    L.piece = (unsigned)(R / 4) * L.sbo;   // 2R rows
+    L.stage = L.tile + 8u * L.piece;
+    const unsigned end = kTcStageOff + (unsigned)S * L.stage;
+    // an M = 128 MMA reads 16 row groups from the first and second plane on
+    const unsigned reach = kTcStageOff + (unsigned)(S - 1) * L.stage + L.plane + 16u * L.sbo;
     L.total = end > reach ? end : reach;
     return L;
 }
 
 // ------------------------------------------------------------- tile builder --
-// mat64 [pairs][B][B] complex64 (the assembler's hi plane) -> bf16 hi/lo tiles.
-// blockIdx.y = cluster; CTAs stride over its pairs; one thread per (row, 4 complex
-// columns): two 16-byte loads, a 16-byte store into each plane.
+// mat64 [pairs][B][B] complex64 (the assembler's hi plane; its upper half is read) ->
+// bf16 hi/lo tiles of P + Q and P - Q.  blockIdx.y = cluster; CTAs stride over its pairs;
+// one thread per (row, 4 complex columns): a 16-byte store into each plane.  Bound by its
+// reads and writes: N = 200, lmax 4 59 us (6.2 TB/s), 119 us with whole blocks.
 __global__ void __launch_bounds__(256)
 k_tc_tiles(const gb::SysDev* __restrict__ sys, const float2* __restrict__ mat64, unsigned char* __restrict__ out) {
     const gb::SysDev S = sys[blockIdx.y];
-    const int B = S.B, Bp = gb::tc_rows(B), Kp = gb::tc_cols(B), KG = Kp / 8;
+    const int B = S.B, H = B / 2, KG = gb::tc_cols(B) / 8;
     const long long plane = gb::tc_plane_bytes(B), blk = gb::tc_block_bytes(B);
-    const unsigned sbo = (unsigned)Kp * 16u;
-    const int items = Bp * KG;
+    const unsigned sbo = (unsigned)gb::tc_cols(B) * 16u;
+    const int items = gb::tc_rows(B) * KG;
     for (long long p = blockIdx.x; p < S.P; p += gridDim.x) {
         const float2* src = mat64 + S.mat_off + p * (long long)B * B;
         unsigned char* dst = out + S.tc_off + p * blk;
         for (int it = threadIdx.x; it < items; it += blockDim.x) {
             const int m8 = it & 7, rest = it >> 3, g = rest % KG, m = (rest / KG) * 8 + m8;
-            float2 a[4];
-            if (m < B && 4 * g + 3 < B) {
-                const float4* q = reinterpret_cast<const float4*>(src + (long long)m * B + 4 * g);
-                const float4 u = __ldg(q), v = __ldg(q + 1);
-                a[0] = make_float2(u.x, u.y);
-                a[1] = make_float2(u.z, u.w);
-                a[2] = make_float2(v.x, v.y);
-                a[3] = make_float2(v.z, v.w);
+            const float2* row = src + (long long)m * B + 4 * g;
+            float2 P[4], Q[4];
+            if (m < H && 4 * g + 3 < H && H % 2 == 0) {   // 16-byte aligned: B and H are even
+                const float4* pv = reinterpret_cast<const float4*>(row);
+                const float4* qv = reinterpret_cast<const float4*>(row + H);
+                const float4 a = __ldg(pv), b = __ldg(pv + 1), c = __ldg(qv), d = __ldg(qv + 1);
+                P[0] = make_float2(a.x, a.y), P[1] = make_float2(a.z, a.w);
+                P[2] = make_float2(b.x, b.y), P[3] = make_float2(b.z, b.w);
+                Q[0] = make_float2(c.x, c.y), Q[1] = make_float2(c.z, c.w);
+                Q[2] = make_float2(d.x, d.y), Q[3] = make_float2(d.z, d.w);
             } else {
 #pragma unroll
                 for (int e = 0; e < 4; e++) {
-                    const int c = 4 * g + e;
-                    a[e] = (m < B && c < B) ? __ldg(src + (long long)m * B + c) : make_float2(0.f, 0.f);
+                    const bool in = m < H && 4 * g + e < H;
+                    P[e] = in ? __ldg(row + e) : make_float2(0.f, 0.f);
+                    Q[e] = in ? __ldg(row + H + e) : make_float2(0.f, 0.f);
                 }
             }
-            uint4 h, l;
-            unsigned* hp = &h.x;
-            unsigned* lp = &l.x;
+            unsigned char* at = dst + (size_t)(m >> 3) * sbo + (size_t)g * 128 + (size_t)m8 * 16;
 #pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const float hr = bf_round(a[e].x), hi = bf_round(a[e].y);
-                hp[e] = bf2(hr, hi);
-                lp[e] = bf2(a[e].x - hr, a[e].y - hi);
+            for (int s = 0; s < 2; s++) {
+                uint4 h, l;
+                unsigned* hp = &h.x;
+                unsigned* lp = &l.x;
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const float ax = s ? P[e].x - Q[e].x : P[e].x + Q[e].x, ay = s ? P[e].y - Q[e].y : P[e].y + Q[e].y;
+                    const float hr = gb::bf_round(ax), hi = gb::bf_round(ay);
+                    hp[e] = gb::bf2(hr, hi);
+                    lp[e] = gb::bf2(ax - hr, ay - hi);
+                }
+                *reinterpret_cast<uint4*>(at + 2 * s * plane) = h;
+                *reinterpret_cast<uint4*>(at + (2 * s + 1) * plane) = l;
             }
-            const size_t off = (size_t)(m >> 3) * sbo + (size_t)g * 128 + (size_t)m8 * 16;
-            *reinterpret_cast<uint4*>(dst + off) = h;
-            *reinterpret_cast<uint4*>(dst + plane + off) = l;
         }
     }
 }
 
 // ------------------------------------------------------------- matrix pass --
-// NC consecutive TMEM columns (NC = 32 or 64) of the warp's 32 lanes, loaded in
-// x16 pieces and waited for once, in one statement.
-template <int NC> __device__ __forceinline__ void tmem_ld_cols(unsigned taddr, float* v);
-template <> __device__ __forceinline__ void tmem_ld_cols<32>(unsigned taddr, float* v) {
-    unsigned r[32];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n"
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n"
-        "tcgen05.wait::ld.sync.aligned;\n"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr), "r"(taddr + 16u)
-        : "memory");
+// The warp's 32 TMEM lanes of columns a0 .. a0 + NC - 1 and a1 .. a1 + NC - 1 (NC = 16 or
+// 32), in x16 pieces, each pair waited for in the statement that loads it.
+template <int NC> __device__ __forceinline__ void tmem_ld2(unsigned a0, unsigned a1, float* v0, float* v1) {
 #pragma unroll
-    for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
-}
-template <> __device__ __forceinline__ void tmem_ld_cols<64>(unsigned taddr, float* v) {
-    tmem_ld_cols<32>(taddr, v);
-    tmem_ld_cols<32>(taddr + 32u, v + 32);
+    for (int c = 0; c < NC; c += 16) {
+        unsigned r[32];
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n"
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n"
+            "tcgen05.wait::ld.sync.aligned;\n"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+              "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+              "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+            : "r"(a0 + (unsigned)c), "r"(a1 + (unsigned)c)
+            : "memory");
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            v0[c + i] = __uint_as_float(r[i]);
+            v1[c + i] = __uint_as_float(r[16 + i]);
+        }
+    }
 }
 
-// The pass over strips [sbeg, send) of one block size B.  Warps 0-3 consume, warp 4
-// produces.  The producer (its lane 0) walks this CTA's strips (every gridDim.x-th,
-// skipping clusters with no active right-hand side); for each block it waits until
-// the block that last used the stage has finished its MMAs (the stage's empty
-// barrier, committed with them), writes the block's job record (its partials'
-// offsets) into the stage's slot and streams the block's bf16 planes, y_u of
-// particle j and y_w of particle i into the stage; after the last block it arrives
-// on the next stage's full barrier with an invalid job.  The consumers build each
-// block's B operand, meet at a named barrier, and thread 0 issues the MMAs,
-// committing them to the accumulator's barrier and the stage's empty barrier; then
-// every consumer reads the previous block's accumulator rows.  Each consumer keeps
-// the jobs of the block it builds and of the block it reads out in registers.
-constexpr int kTcConsumers = 128;   // warps 0-3
+// The pass over strips [sbeg, send) of one block size B with S stages.
 template <int R>
-__global__ void __launch_bounds__(kTcThreads, 1)
+__global__ void __launch_bounds__(kTcThreads)
 k_pgemv_tc(const gb::SysDev* __restrict__ sys, const gb::Strip* __restrict__ strips, long long sbeg, long long send,
            const gb::KState* __restrict__ st, int mask, const unsigned char* __restrict__ mat_tc,
-           const float2* __restrict__ Yu, const float2* __restrict__ Yw, float2* __restrict__ CU,
-           float2* __restrict__ CW, const gb::SysPlan* __restrict__ plan, int B, int* __restrict__ err) {
-    constexpr int N = 8 * R;             // B-operand rows: [U_h | W_h | U_l | W_l], 2R each
-    constexpr int S = kTcStages;
-    constexpr unsigned NCOL = 2 * N;     // two accumulators of N FP32 columns (64 or 128: a power of 2 >= 32)
+           const unsigned char* __restrict__ Yu, const unsigned char* __restrict__ Yw, float2* __restrict__ CU,
+           float2* __restrict__ CW, const gb::SysPlan* __restrict__ plan, int B, int S, int* __restrict__ err) {
+    constexpr int N = 16 * R;             // columns of an accumulator
+    constexpr unsigned NCOL = 2 * N;      // two accumulators (128 or 256: a power of 2 >= 32)
     constexpr unsigned IDESC_FULL = idesc_bf16(128, N);
     constexpr unsigned IDESC_HALF = idesc_bf16(128, N / 2);
-    const TcLayout L = tc_layout(B, R);
-    const int Kp = gb::tc_cols(B);
+    const TcLayout L = tc_layout(B, R, S);
+    const int H = B / 2, minus = 2 * gb::tc_rows(B);   // TMEM lane (MMA row) of sign -'s first row
     extern __shared__ __align__(1024) unsigned char sm[];
-    uint64_t* full = reinterpret_cast<uint64_t*>(sm);
-    uint64_t* empty = full + S;
-    uint64_t* mdone = empty + S;
-    unsigned* tslot = reinterpret_cast<unsigned*>(mdone + 2);
-    volatile int* sabort = reinterpret_cast<volatile int*>(tslot + 1);
-    long long* sconsumed = reinterpret_cast<long long*>(tslot + 2);
-    TcJob* jobs = reinterpret_cast<TcJob*>(sm + L.off_jobs);
-    int* srow = reinterpret_cast<int*>(sm + L.off_row);
-    unsigned char* bbuf = sm + L.off_b;
-    unsigned char* stages = sm + L.off_stage;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const long long G = gridDim.x;
+    TcHeader& hd = *reinterpret_cast<TcHeader*>(sm);
+    unsigned char* stages = sm + kTcStageOff;
+    volatile int* stop = &hd.abort;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
 
     if (tid == 0) {
         for (int q = 0; q < S; q++) {
-            bar_init(full + q, 1);
-            bar_init(empty + q, 1);
+            bar_init(hd.full + q, 1);
+            bar_init(hd.empty + q, 1);
         }
-        bar_init(mdone, 1);
-        bar_init(mdone + 1, 1);
-        *sabort = 0;
-        *sconsumed = 0;
+        for (int x = 0; x < 2; x++) {
+            bar_init(hd.mdone + x, 1);
+            bar_init(hd.job + x, 1);
+            bar_init(hd.free + x, (H + 31) / 32 + (minus + H + 31) / 32 - minus / 32);   // the warps that hold rows
+        }
+        hd.abort = 0;
+        hd.consumed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
-    {   // both B-operand buffers start at zero: their K padding is never written again
-        uint4* z = reinterpret_cast<uint4*>(bbuf);
-        for (unsigned e = tid; e < 2u * L.bbytes / 16u; e += kTcThreads) z[e] = make_uint4(0, 0, 0, 0);
-    }
-    const int* rowinfo = sys[strips[sbeg].sys].rowinfo;   // every cluster of the launch has block size B
-    for (int r = tid; r < B; r += kTcThreads) srow[r] = __ldg(rowinfo + r);
     if (warp == 0) {
-        tmem_alloc(tslot, NCOL);
+        tmem_alloc(&hd.tmem, NCOL);
         tmem_relinquish();
     }
     proxy_fence();
     tc_before_sync();
     __syncthreads();
     tc_after_sync();
-    const unsigned tmem = *tslot;
-    pdl_wait_tc();   // y vectors and solver state come from the preceding kernels
+    const unsigned tmem = hd.tmem;
+    pdl_wait_tc();   // operands and solver state come from the preceding kernels
     pdl_trigger_tc();
+    auto give_up = [&]() {
+        *stop = 1;
+        atomicExch(err, 1);
+    };
 
-    if (warp == kTcConsumers / 32) {
+    long long k = 0;   // producer: jobs written
+    if (warp == 4) {
         // ------------------------------------------------------------ producer
-        long long k = 0;   // stages written (blocks and the final invalid job)
-        if (lane == 0) {
-            long long pw = sbeg + blockIdx.x;
-            int pb = 0;
-            const uint64_t pol = evict_first_policy();
-            auto seek = [&]() {
-                while (pw < send && !gb::any_active<R>(st, strips[pw].sys, mask)) pw += G;
-            };
-            seek();
-            for (;; k++) {
-                const int s = (int)(k % S);
-                if (k >= S && !bar_wait(empty + s, (unsigned)((k / S - 1) & 1))) {   // the stage's last MMAs
-                    *sabort = 1;
-                    atomicExch(err, 1);
-                    break;
+        // Walks this CTA's strips (every gridDim.x-th, skipping clusters with no active
+        // right-hand side), the records of 32 of them loaded at once.
+        const long long G = gridDim.x;
+        const uint64_t pol = evict_first_policy();
+        long long pw = sbeg + blockIdx.x;
+        gb::Strip mine{};
+        int at = 32;   // strip of the 32 loaded
+        int cur = -1, NP = 0, s = 0;
+        unsigned phase = 1;   // of the stage's empty barrier: passes at once the first time round
+        bool act = false;
+        long long t_off = 0, y_off = 0, cw0 = 0, cu0 = 0, sb0 = 0;
+        bool run = true;
+        for (; run && pw < send; pw += G) {
+            if (at == 32) {
+                at = 0;
+                if (pw + lane * G < send) mine = strips[pw + lane * G];
+            }
+            const int sysi = __shfl_sync(0xffffffffu, mine.sys, at), i = __shfl_sync(0xffffffffu, mine.i, at),
+                      nb = __shfl_sync(0xffffffffu, mine.nb, at);
+            const long long p0 = __shfl_sync(0xffffffffu, mine.p0, at);
+            at++;
+            if (sysi != cur) {
+                cur = sysi;
+                act = gb::any_active<R>(st, cur, mask);
+                const gb::SysDev& Sd = sys[cur];
+                const gb::SysPlan& pl = plan[cur];
+                NP = Sd.N;
+                t_off = Sd.tc_off;
+                y_off = Sd.ty_off * R;
+                cw0 = pl.cw_off;
+                cu0 = pl.cu_off;
+                sb0 = pl.strip_base;
+            }
+            if (!act) continue;
+            const int j0 = i + 1 + (int)(p0 - pair_start(i, NP));
+            const unsigned char* wsrc = Yw + y_off + (long long)i * (4LL * L.piece);
+            const unsigned char* usrc = Yu + y_off + (long long)j0 * (4LL * L.piece);
+            const unsigned char* tsrc = mat_tc + t_off + p0 * (long long)L.tile;
+            for (int pb = 0; pb < nb; pb++, k++) {
+                run = __all_sync(0xffffffffu, bar_wait(hd.empty + s, phase, stop));
+                if (!run) break;
+                if (elect_one()) {
+                    const long long j = j0 + pb;
+                    TcJob J;
+                    J.cw = cw0 + (j * (j - 1) / 2 + i) * (long long)B * R;
+                    J.cu = (pb == nb - 1) ? cu0 + (pw - sb0) * (long long)B * R : -1;
+                    hd.jobs[k % kTcJobs] = J;
+                    bar_expect_tx(hd.full + s, L.stage);   // arrive (release): the job record goes with it
+                    unsigned char* dst = stages + (size_t)s * L.stage;
+                    bulk_copy_hint(dst, tsrc, L.tile, hd.full + s, pol);
+#pragma unroll
+                    for (int c = 0; c < 8; c++)   // (hi / lo, sign, U / W)
+                        bulk_copy(dst + L.tile + c * L.piece, ((c & 1) ? wsrc : usrc) + (c >> 1) * L.piece, L.piece,
+                                  hd.full + s);
                 }
-                if (*sabort) break;
-                if (pw >= send) {   // the end: an invalid job, with a plain arrive
-                    jobs[s].valid = 0;
-                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(su32(full + s)) : "memory");
-                    k++;
-                    break;
-                }
-                const gb::Strip sp = strips[pw];
-                const gb::SysDev& Sd = sys[sp.sys];
-                const gb::SysPlan& pl = plan[sp.sys];
-                const int j = sp.i + 1 + (int)(sp.p0 - pair_start(sp.i, Sd.N)) + pb;
-                TcJob J;
-                J.cw = pl.cw_off + ((long long)j * (j - 1) / 2 + sp.i) * (long long)B * R;
-                J.cu = (pb == sp.nb - 1) ? pl.cu_off + (pw - pl.strip_base) * (long long)B * R : -1;
-                J.valid = 1;
-                J.pad = 0;
-                jobs[s] = J;
-                unsigned char* dst = stages + (size_t)s * L.stage;
-                bar_expect_tx(full + s, L.tile + 2u * L.ybytes);   // arrive (release): the job record goes with it
-                bulk_copy_hint(dst, mat_tc + Sd.tc_off + (sp.p0 + pb) * (long long)L.tile, L.tile, full + s, pol);
-                bulk_copy(dst + L.tile, Yu + Sd.vec_off + (long long)j * B * R, L.ybytes, full + s);
-                bulk_copy(dst + L.tile + L.ybytes, Yw + Sd.vec_off + (long long)sp.i * B * R, L.ybytes, full + s);
-                if (++pb >= sp.nb) {
-                    pb = 0;
-                    pw += G;
-                    seek();
+                __syncwarp();
+                tsrc += L.tile;
+                usrc += 4u * L.piece;
+                if (++s == S) {
+                    s = 0;
+                    phase ^= 1u;
                 }
             }
         }
-        __syncthreads();   // every thread of the CTA meets here once the consumers are done
-        if (lane == 0)     // drain: every stage written and not consumed (bounded waits)
-            for (long long q = *sconsumed; q < k; q++) (void)bar_wait(full + (q % S), (unsigned)((q / S) & 1));
-    } else {
-        // ------------------------------------------------------------ consumers
+        if (!run && lane == 0) give_up();
+        if (run && lane == 0) {   // the end: an invalid job, with a plain arrive
+            if (bar_wait(hd.empty + s, phase, stop)) {
+                hd.jobs[k % kTcJobs].cw = -1;
+                bar_arrive(hd.full + s);
+                k++;
+            } else {
+                give_up();
+            }
+        }
+    } else if (warp == 5) {
+        // --------------------------------------------------------- MMA issuer
+        const int KS = gb::tc_cols(B) / 16;   // <= 5
+        long long g = 0;                      // blocks whose MMAs were issued
+        int s = 0;
+        unsigned phase = 0;
+        bool ok = true;
+        while (true) {
+            const int x = (int)(g & 1);
+            // the accumulator read out (block g - 2), the stage's copies landed
+            ok = bar_wait(hd.free + x, (unsigned)((g >> 1) & 1) ^ 1u, stop) && bar_wait(hd.full + s, phase, stop);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            const bool valid = __all_sync(0xffffffffu, hd.jobs[g % kTcJobs].cw >= 0);
+            if (elect_one()) bar_arrive(hd.job + x);
+            __syncwarp();
+            if (!valid) break;
+            tc_after_sync();
+            const unsigned a = su32(stages) + (unsigned)s * L.stage, b = a + L.tile;
+            const unsigned d = tmem + (unsigned)(x * N);
+            const uint64_t da = smem_desc(a, 128, L.sbo), db = smem_desc(b, 128, L.sbo);   // + 16 per 256 bytes
+            if (elect_one()) {
+#pragma unroll
+                for (int ks = 0; ks < 5; ks++) {
+                    if (ks < KS) {
+                        mma_bf16(d, da + 16u * ks, db + 16u * ks, IDESC_FULL, ks > 0);
+                        mma_bf16(d, da + 16u * ks + (L.plane >> 4), db + 16u * ks, IDESC_HALF, 1);
+                    }
+                }
+                mma_commit(hd.mdone + x);
+                mma_commit(hd.empty + s);   // the stage is free once these MMAs have read it
+            }
+            __syncwarp();
+            g++;
+            if (++s == S) {
+                s = 0;
+                phase ^= 1u;
+            }
+        }
+        if (lane == 0) hd.consumed = ok ? g + 1 : g;
+        if (!ok && lane == 0) {
+            give_up();
+            for (long long e = (g >= 2 ? g - 2 : 0); e < g; e++)   // bounded waits for the MMAs still in flight
+                (void)bar_wait(hd.mdone + (e & 1), (unsigned)((e >> 1) & 1));
+        }
+    } else if (warp * 32 < H || (warp * 32 + 31 >= minus && warp * 32 < minus + H)) {
+        // ---------------------------------------------------- accumulators out
+        const int sig = warp * 32 < H ? 0 : 1, m = tid - sig * minus;   // sign (of all the warp's rows), row
+        const bool row = m >= 0 && m < H;
+        int at = 0;          // its 16-byte word in a term: column rho(m) of the other sign
+        unsigned eneg = 0;
+        if (row) {
+            const int info = __ldg(sys[strips[sbeg].sys].rowinfo + m);   // every cluster of the launch has block size B
+            at = (sig ^ 1) * H + (info & ((1 << 29) - 1));
+            eneg = (info >> 29) & 1;
+        }
+        const unsigned taddr = tmem + ((unsigned)(warp * 32) << 16) + (unsigned)(sig * 4 * R);
         float u[2 * R];
 #pragma unroll
         for (int q = 0; q < 2 * R; q++) u[q] = 0.f;
-        const int m = warp * 32 + lane;   // accumulator row (TMEM lane) of this thread
-        const bool warp_rows = warp * 32 < B;
-        int rho_m = 0;
-        unsigned eneg_m = 0;
-        if (m < B) {
-            rho_m = srow[m] & ((1 << 29) - 1);
-            eneg_m = (srow[m] >> 29) & 1;
-        }
-        // block e's accumulator: its column partials out, its row partial into u; at the
-        // strip's end the row partials out
-        auto epilogue = [&](long long e, const TcJob& J) -> bool {
+        for (long long e = 0;; e++) {
             const int x = (int)(e & 1);
-            bool ok = bar_wait(mdone + x, (unsigned)((e >> 1) & 1));
+            const unsigned phase = (unsigned)((e >> 1) & 1);
+            bool ok = bar_wait(hd.job + x, phase, stop);
             ok = __all_sync(0xffffffffu, ok);
+            if (!ok) {
+                if (lane == 0) give_up();
+                break;
+            }
+            const TcJob J = hd.jobs[e % kTcJobs];
+            if (J.cw < 0) break;   // the same record for every lane
+            ok = bar_wait(hd.mdone + x, phase, stop);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) {
+                if (lane == 0) give_up();
+                break;
+            }
             tc_after_sync();
-            if (ok && warp_rows) {
-                float v[N];
-                tmem_ld_cols<N>(tmem + ((unsigned)(warp * 32) << 16) + (unsigned)(x * N), v);
-                if (m < B) {
-                    float2 w[R];
+            float h[4 * R], l[4 * R];   // of z_h and of z_l: U, then W
+            tmem_ld2<4 * R>(taddr + (unsigned)(x * N), taddr + (unsigned)(x * N + 8 * R), h, l);
+            tc_before_sync();
+            __syncwarp();
+            if (lane == 0) bar_arrive(hd.free + x);
+            if (row) {
+                float4* cwp = reinterpret_cast<float4*>(CW + J.cw) + at;
 #pragma unroll
-                    for (int q = 0; q < R; q++) {
-                        u[2 * q] += v[2 * q] + v[4 * R + 2 * q];
-                        u[2 * q + 1] += v[2 * q + 1] + v[4 * R + 2 * q + 1];
-                        w[q] = make_float2(flipf(v[2 * R + 2 * q] + v[6 * R + 2 * q], eneg_m),
-                                           flipf(v[2 * R + 2 * q + 1] + v[6 * R + 2 * q + 1], eneg_m));
-                    }
-                    float4* cwp = reinterpret_cast<float4*>(CW + J.cw + (long long)rho_m * R);
+                for (int q = 0; q < 2 * R; q += 4) {
 #pragma unroll
-                    for (int q = 0; q < R; q += 2) cwp[q / 2] = make_float4(w[q].x, w[q].y, w[q + 1].x, w[q + 1].y);
+                    for (int c = q; c < q + 4; c++) u[c] += h[c] + l[c];
+                    const int w = 2 * R + q;
+                    cwp[q / 4 * B] = make_float4(flipf(h[w] + l[w], eneg), flipf(h[w + 1] + l[w + 1], eneg),
+                                                 flipf(h[w + 2] + l[w + 2], eneg), flipf(h[w + 3] + l[w + 3], eneg));
                 }
             }
-            tc_before_sync();
-            if (!ok && lane == 0) {
-                *sabort = 1;
-                atomicExch(err, 1);
-            }
             if (J.cu >= 0) {   // the strip's row partial
-                if (ok && m < B) {
-                    float4* cup = reinterpret_cast<float4*>(CU + J.cu + (long long)rho_m * R);
+                if (row) {
+                    float4* cup = reinterpret_cast<float4*>(CU + J.cu) + at;
 #pragma unroll
-                    for (int q = 0; q < R; q += 2)
-                        cup[q / 2] = make_float4(flipf(u[2 * q], eneg_m), flipf(u[2 * q + 1], eneg_m),
-                                                 flipf(u[2 * q + 2], eneg_m), flipf(u[2 * q + 3], eneg_m));
+                    for (int q = 0; q < 2 * R; q += 4)
+                        cup[q / 4 * B] = make_float4(flipf(u[q], eneg), flipf(u[q + 1], eneg), flipf(u[q + 2], eneg),
+                                                     flipf(u[q + 3], eneg));
                 }
 #pragma unroll
                 for (int q = 0; q < 2 * R; q++) u[q] = 0.f;
             }
-            return ok;
-        };
-
-        long long g = 0;   // blocks whose MMAs were issued
-        bool aborted = false;
-        TcJob prev;
-        prev.valid = 0;
-        while (true) {
-            const int s = (int)(g % S), x = (int)(g & 1);
-            unsigned char* stg = stages + (size_t)s * L.stage;
-            bool ok = false;
-            TcJob J;
-            J.valid = 0;
-            if (!*sabort) {
-                ok = bar_wait(full + s, (unsigned)((g / S) & 1));
-                if (!ok) {
-                    *sabort = 1;
-                    atomicExch(err, 1);
-                } else {
-                    J = jobs[s];
-                }
-            }
-            // B operand of block g into buffer x (last read by the MMAs of block g - 2,
-            // which completed before this thread's epilogue of g - 2)
-            if (ok && J.valid) {
-                const float2* yu = reinterpret_cast<const float2*>(stg + L.tile);
-                const float2* yw = reinterpret_cast<const float2*>(stg + L.tile + L.ybytes);
-                unsigned char* bb = bbuf + (size_t)x * L.bbytes;
-                for (int it = tid; it < B * R; it += kTcConsumers) {
-                    const int sc = it / R, q = it - sc * R;
-                    const int info = srow[sc];
-                    const int rs = info & ((1 << 29) - 1);
-                    const unsigned en = (info >> 29) & 1;
-                    const float2 zu = yu[rs * R + q], zw = yw[rs * R + q];
-                    const float zr[2] = {flipf(zu.x, en), flipf(zw.x, en)};
-                    const float zi[2] = {flipf(zu.y, en), flipf(zw.y, en)};
-                    const unsigned col = (unsigned)(sc >> 2) * 128u + (unsigned)(sc & 3) * 4u;
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {   // h 0: U rows (z_j), 1: W rows (w_i)
-                        const float hr = bf_round(zr[h]), hi = bf_round(zi[h]);
-                        const float lr = zr[h] - hr, li = zi[h] - hi;
-                        const int n0 = h * 2 * R + 2 * q, n1 = n0 + 4 * R;   // hi rows, lo rows (n0 even)
-                        unsigned char* r0 = bb + (n0 >> 3) * L.sbo + col + (n0 & 7) * 16;
-                        unsigned char* r1 = bb + (n1 >> 3) * L.sbo + col + (n1 & 7) * 16;
-                        *reinterpret_cast<unsigned*>(r0) = bf2(hr, -hi);        // row n0:     re(A z)
-                        *reinterpret_cast<unsigned*>(r0 + 16) = bf2(hi, hr);    // row n0 + 1: im(A z)
-                        *reinterpret_cast<unsigned*>(r1) = bf2(lr, -li);
-                        *reinterpret_cast<unsigned*>(r1 + 16) = bf2(li, lr);
-                    }
-                }
-            }
-            proxy_fence();   // generic writes of the B operand -> the tensor core's reads
-            tc_before_sync();
-            // the consumer warps' barrier, with the OR of every consumer's view of the
-            // abort flag (the producer may set it at any time): one decision for all
-            unsigned stop = (!ok || *sabort) ? 1u : 0u;
-            asm volatile(
-                "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.or.pred q, 1, %2, p;\n"
-                " selp.u32 %0, 1, 0, q;\n}\n"
-                : "=r"(stop)
-                : "r"(stop), "n"(kTcConsumers)
-                : "memory");
-            tc_after_sync();
-            if (stop) {
-                aborted = true;
-                break;
-            }
-            if (!J.valid) break;   // the same record for every consumer: the end of this CTA's blocks
-            if (tid == 0) {
-                const unsigned a_hi = su32(stg), a_lo = a_hi + L.plane, bsm = su32(bbuf + (size_t)x * L.bbytes);
-                const unsigned d = tmem + (unsigned)(x * N);
-                for (int ks = 0; ks < Kp / 16; ks++) {
-                    const uint64_t bd = smem_desc(bsm + ks * 256, 128, L.sbo);
-                    mma_bf16(d, smem_desc(a_hi + ks * 256, 128, L.sbo), bd, IDESC_FULL, ks > 0);
-                    mma_bf16(d, smem_desc(a_lo + ks * 256, 128, L.sbo), bd, IDESC_HALF, 1);
-                }
-                mma_commit(mdone + x);
-                mma_commit(empty + s);   // the stage is free once these MMAs have read it
-            }
-            g++;
-            if (g >= 2) epilogue(g - 2, prev);   // the previous block's accumulator out
-            prev = J;
         }
-        if (!aborted && g >= 1 && !epilogue(g - 1, prev)) aborted = true;
-        if (tid == 0) {
-            *sconsumed = g;
-            if (aborted)   // bounded waits for the MMAs still in flight
-                for (long long e = (g >= 2 ? g - 2 : 0); e < g; e++)
-                    (void)bar_wait(mdone + (e & 1), (unsigned)((e >> 1) & 1));
-        }
-        tc_before_sync();
-        __syncthreads();
     }
-    // every thread has passed the CTA barrier above (the producer then drained its copies)
     tc_before_sync();
+    __syncthreads();
+    if (warp == 4 && lane == 0)   // drain: copies of jobs written and not taken (bounded waits)
+        for (long long q = hd.consumed; q < k; q++) (void)bar_wait(hd.full + (q % S), (unsigned)((q / S) & 1));
     __syncthreads();
     if (warp == 0) {
         tc_after_sync();
@@ -532,18 +530,18 @@ int launch_pgemv_tc(int R, const SysDev* sys, const Strip* strips, long long sbe
                     const SysPlan* plan, int B, int* err, cudaStream_t stream) {
     if (send <= sbeg) return GB_OK;
     if (R != 4 && R != 8) return gb_set_error(GB_UNSUPPORTED, "tensor-core pass: R must be 4 or 8 (got %d)", R);
-    if (tc_rows(B) > 128) return gb_set_error(GB_UNSUPPORTED, "tensor-core pass: block size %d > 128 rows", B);
-    if ((reinterpret_cast<uintptr_t>(mat_tc) | reinterpret_cast<uintptr_t>(Yu)) & 15)
+    if (B > 70) return gb_set_error(GB_UNSUPPORTED, "tensor-core pass: block size %d > 70 (lmax 5)", B);
+    if ((reinterpret_cast<uintptr_t>(mat_tc) | reinterpret_cast<uintptr_t>(Yu) | reinterpret_cast<uintptr_t>(Yw)) & 15)
         return gb_set_error(GB_BAD_ARG, "tensor-core pass: matrix and y vectors must be 16-byte aligned");
-    const TcLayout L = tc_layout(B, R);
-    if (L.total > 227u * 1024u)
-        return gb_set_error(GB_UNSUPPORTED, "tensor-core pass: block size %d needs %u B of shared memory", B, L.total);
+    // as many stages as let two CTAs share an SM (228 KB, 1 KB of them reserved per CTA): 3 at
+    // B = 70, 5 up to B = 48
+    int S = kTcMaxStages;
+    while (S > 3 && 2u * (tc_layout(B, R, S).total + 1024u) > 228u * 1024u) S--;
+    const TcLayout L = tc_layout(B, R, S);
     const void* kfn = R == 4 ? reinterpret_cast<const void*>(k_pgemv_tc<4>) : reinterpret_cast<const void*>(k_pgemv_tc<8>);
     GB_CUDA_TRY(ensure_dynamic_smem(kfn, L.total));
-    // two CTAs per SM where their shared memory fits (228 KB per SM, 1 KB reserved per CTA)
-    const int per_sm = 2u * (L.total + 1024u) <= 228u * 1024u ? 2 : 1;
     const long long n = send - sbeg;
-    const long long grid = n < (long long)sm_count() * per_sm ? n : (long long)sm_count() * per_sm;
+    const long long grid = n < 2LL * sm_count() ? n : 2LL * sm_count();
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -556,16 +554,16 @@ int launch_pgemv_tc(int R, const SysDev* sys, const Strip* strips, long long sbe
     cfg.numAttrs = 1;
     note_launch();
     const unsigned char* m = static_cast<const unsigned char*>(mat_tc);
-    const float2* yu = static_cast<const float2*>(Yu);
-    const float2* yw = static_cast<const float2*>(Yw);
+    const unsigned char* yu = static_cast<const unsigned char*>(Yu);
+    const unsigned char* yw = static_cast<const unsigned char*>(Yw);
     float2* cu = static_cast<float2*>(CU);
     float2* cw = static_cast<float2*>(CW);
     if (R == 4)
         GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_pgemv_tc<4>, sys, strips, sbeg, send, st, mask, m, yu, yw, cu, cw, plan, B,
-                                       err));
+                                       S, err));
     else
         GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_pgemv_tc<8>, sys, strips, sbeg, send, st, mask, m, yu, yw, cu, cw, plan, B,
-                                       err));
+                                       S, err));
     return GB_OK;
 }
 

@@ -365,7 +365,6 @@ template <int YK> struct YType;
 template <> struct YType<0> { using t = double2; };
 template <> struct YType<1> { using t = float4; };   // (re, re, im, im): broadcast pairs for f32x2 FMAs
 template <> struct YType<2> { using t = float4; };
-template <> struct YType<3> { using t = float2; };   // (re, im): the tensor-core pass builds its own operands
 
 template <int YK> __device__ __forceinline__ typename YType<YK>::t make_y(double2 z);
 template <int YK> __device__ __forceinline__ typename YType<YK>::t make_y(float2 z);
@@ -374,8 +373,6 @@ template <> __device__ __forceinline__ double2 make_y<0>(float2 z) { return to_d
 template <> __device__ __forceinline__ float4 make_y<1>(float2 z) { return make_float4(z.x, z.x, z.y, z.y); }
 template <> __device__ __forceinline__ float4 make_y<1>(double2 z) { return make_y<1>(from_d2<float2>(z)); }
 template <> __device__ __forceinline__ float4 make_y<2>(float2 z) { return make_float4(z.x, z.y, 0.f, 0.f); }
-template <> __device__ __forceinline__ float2 make_y<3>(float2 z) { return z; }
-template <> __device__ __forceinline__ float2 make_y<3>(double2 z) { return from_d2<float2>(z); }
 template <> __device__ __forceinline__ float4 make_y<2>(double2 z) {
     const float hx = __double2float_rn(z.x), hy = __double2float_rn(z.y);
     return make_float4(hx, hy, __double2float_rn(z.x - (double)hx), __double2float_rn(z.y - (double)hy));
@@ -386,18 +383,12 @@ template <> __device__ __forceinline__ float4 make_y<2>(double2 z) {
 // -sig(r), so Yw's are sig(r) times Yu's of the other sign.  Planes of pl (1 or 2)
 // right-hand sides, each [D][pl], follow each other within the cluster's segment, so that
 // a matrix pass copies only its own right-hand sides.  Small blocks (kWholeB) keep z
-// itself in their planes; YK 3 (the tensor-core pass): z as [D][R].
+// itself in their planes.
 template <int YK, typename C>
 __device__ __forceinline__ void store_y(const gb::SysDev& S, int part, int r, int rr, int R, int pl, C z0, C z1,
                                         unsigned sneg, typename YType<YK>::t* __restrict__ Yu,
                                         typename YType<YK>::t* __restrict__ Yw) {
-    if constexpr (YK == 3) {
-        const long long o = S.vec_off + ((long long)part * S.B + r) * R + rr, o1 = o + (long long)S.rmax * R;
-        Yu[o] = make_y<YK>(z0);
-        Yu[o1] = make_y<YK>(z1);
-        Yw[o] = make_y<YK>(cflip(z0, sneg));
-        Yw[o1] = make_y<YK>(cflip(z1, sneg ^ 1u));
-    } else if (S.B <= kWholeB) {
+    if (S.B <= kWholeB) {
         const long long o = S.vec_off + (long long)(rr / pl) * pl * S.D + ((long long)part * S.B + r) * pl + rr % pl;
         const long long o1 = o + (long long)S.rmax * pl;
         Yu[o] = make_y<YK>(z0);
@@ -421,6 +412,28 @@ template <typename C> __device__ __forceinline__ C tmul(C t, C x) {
     z.x = fma(t.x, x.x, -(t.y * x.y));
     z.y = fma(t.x, x.y, t.y * x.x);
     return z;
+}
+
+// Element es of a product's input: x, or (update) the BiCGSTAB vector update the input
+// needs, p = r + beta (p - omega v) or s = r - alpha v, stored too; each element is one
+// thread's alone.
+template <typename C, typename T, typename VT>
+__device__ __forceinline__ C updated_x(const YUpd<VT>& up, bool update, const KState* st, int ks, const VT* x,
+                                       long long es) {
+    if (!update) return to_c<C>(x[es]);
+    const T tg{};
+    const KState& k = st[ks];
+    const C rv = to_c<C>(up.r[es]), vv = to_c<C>(up.v[es]);
+    C nv;
+    if (up.kind == 1) {
+        const C pv = to_c<C>(up.out[es]);
+        nv = cadd(rv, cmul(ks_beta(k, tg), csub(pv, cmul(ks_omega(k, tg), vv))));
+    } else {
+        nv = csub(rv, cmul(ks_alpha(k, tg), vv));
+    }
+    const VT q = from_c<VT>(nv);
+    up.out[es] = q;
+    return to_c<C>(q);
 }
 
 // One thread per (row of the first polarisation, rhs), for the rows of both; x is [D][R]
@@ -447,33 +460,90 @@ k_yprep(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items, int 
     const unsigned eneg = (info >> 29) & 1, sneg = (info >> 30) & 1;
     using C = typename Arith<VT>::C;
     using T = typename Arith<VT>::T;
-    const T tg{};
     const long long src = (long long)part * S.B + rho;
     const C t0 = to_c<C>(tvec[S.t_off + src]), t1 = to_c<C>(tvec[S.t_off + src + S.rmax]);
     pdl_wait();
     pdl_trigger();
     if (!row_ok || !any_active<R>(st, I.sys, mask_mode)) return;
     const bool update = up.kind != 0 && active_rhs<R>(st, I.sys, rr, 0);
-    auto source = [&](long long es) -> C {
-        if (!update) return to_c<C>(x[es]);
-        // the BiCGSTAB vector update this product's input needs, on the source row
-        // this thread alone reads: p = r + beta (p - omega v) or s = r - alpha v
-        const KState& k = st[I.sys * R + rr];
-        const C rv = to_c<C>(up.r[es]), vv = to_c<C>(up.v[es]);
-        C nv;
-        if (up.kind == 1) {
-            const C pv = to_c<C>(up.out[es]);
-            nv = cadd(rv, cmul(ks_beta(k, tg), csub(pv, cmul(ks_omega(k, tg), vv))));
-        } else {
-            nv = csub(rv, cmul(ks_alpha(k, tg), vv));
-        }
-        const VT q = from_c<VT>(nv);
-        up.out[es] = q;
-        return to_c<C>(q);
-    };
+    auto source = [&](long long es) -> C { return updated_x<C, T>(up, update, st, I.sys * R + rr, x, es); };
     const long long es = S.vec_off + src * R + rr;
     const C z0 = cflip(tmul(t0, source(es)), eneg), z1 = cflip(tmul(t1, source(es + (long long)S.rmax * R)), eneg ^ 1u);
     store_y<YK>(S, part, r, rr, R, pl, z0, z1, sneg, Yu, Yw);
+}
+
+// The operands of the tensor-core pass (gb_internal.h): one CTA per particle, one thread
+// per (4 columns, rhs), which writes its 16 bytes of every row: column c holds z[c] =
+// eps(c) y[rho(c)] = eps(c) eps(rho(c)) (t x)[c], so x is read in order.  The columns past
+// rmax are zeros.  (With 4-byte stores by one thread per column a product took 6 us longer at
+// N = 30, lmax 1 and 1.5 us at N = 200, lmax 4, both R = 8.)
+constexpr int kTcYThreads = 64;   // >= Kp / 8 * R: 48 for R = 8 (B <= 48), 40 for R = 4 (B <= 70)
+template <typename VT, int R>
+__global__ void __launch_bounds__(kTcYThreads)
+k_yprep_tc(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items, const KState* __restrict__ st, int mask_mode,
+           const double2* __restrict__ tvec, const VT* __restrict__ x, unsigned char* __restrict__ Yu,
+           unsigned char* __restrict__ Yw, YUpd<VT> up) {
+    const Item I = items[blockIdx.x];   // prologue on plan data and the Mie vector
+    const gb::SysDev S = sys[I.sys];
+    const int H = S.rmax, Kp = gb::tc_cols(S.B), part = I.r0 / S.B;
+    const int g = threadIdx.x / R, rr = threadIdx.x - g * R;
+    using C = typename Arith<VT>::C;
+    using T = typename Arith<VT>::T;
+    C t0[4], t1[4];
+    unsigned flip[4], sneg[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        const int c = 4 * g + e;
+        if (c >= H) continue;
+        const int info = __ldg(S.rowinfo + c), rinfo = __ldg(S.rowinfo + (info & ((1 << 29) - 1)));
+        flip[e] = ((unsigned)(info ^ rinfo) >> 29) & 1u;   // the same for both polarisations
+        sneg[e] = ((unsigned)rinfo >> 30) & 1u;
+        t0[e] = to_c<C>(tvec[S.t_off + I.r0 + c]);
+        t1[e] = to_c<C>(tvec[S.t_off + I.r0 + c + H]);
+    }
+    pdl_wait();
+    pdl_trigger();
+    if (8 * g >= Kp || !any_active<R>(st, I.sys, mask_mode)) return;
+    const bool update = up.kind != 0 && active_rhs<R>(st, I.sys, rr, 0);
+    float2 yp[4], ym[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        const int c = 4 * g + e;
+        yp[e] = ym[e] = make_float2(0.f, 0.f);
+        if (c >= H) continue;
+        const long long es = S.vec_off + (long long)(I.r0 + c) * R + rr;
+        const C z0 = cflip(tmul(t0[e], updated_x<C, T>(up, update, st, I.sys * R + rr, x, es)), flip[e]);
+        const C z1 = cflip(tmul(t1[e], updated_x<C, T>(up, update, st, I.sys * R + rr, x, es + (long long)H * R)), flip[e]);
+        yp[e] = to_c<float2>(half(cadd(z0, z1)));
+        ym[e] = to_c<float2>(half(csub(z0, z1)));
+    }
+    const size_t piece = 4 * (size_t)R * Kp;
+    const size_t o = S.ty_off * R + part * gb::tc_y_bytes(S.B, R) + (size_t)(rr >> 2) * Kp * 16 + (size_t)g * 128 +
+                     (2 * rr & 7) * 16;
+    uint4* u = reinterpret_cast<uint4*>(Yu + o);
+    uint4* w = reinterpret_cast<uint4*>(Yw + o);
+    const size_t step = piece / 16;
+#pragma unroll
+    for (int s = 0; s < 2; s++) {   // sign; W of sign + is sig y-, of sign - sig y+
+        unsigned v[4][4];           // hi re, hi im, lo re, lo im
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const float2 y = s ? ym[e] : yp[e];
+            const float hr = gb::bf_round(y.x), hi = gb::bf_round(y.y), lr = y.x - hr, li = y.y - hi;
+            v[0][e] = gb::bf2(hr, -hi);
+            v[1][e] = gb::bf2(hi, hr);
+            v[2][e] = gb::bf2(lr, -li);
+            v[3][e] = gb::bf2(li, lr);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            u[(2 * (q >> 1) + s) * step + (q & 1)] = make_uint4(v[q][0], v[q][1], v[q][2], v[q][3]);
+            unsigned f[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) f[e] = v[q][e] ^ (4 * g + e < H && sneg[e] ? 0x80008000u : 0u);
+            w[(2 * (q >> 1) + 1 - s) * step + (q & 1)] = make_uint4(f[0], f[1], f[2], f[3]);
+        }
+    }
 }
 
 // y vectors of clusters of general particles (the T-matrix overload of the
@@ -1295,8 +1365,8 @@ __device__ __forceinline__ void sum_terms(const OutT* __restrict__ p, long long 
 // threads form G = kRBThreads / W groups that split the terms, thread (g, w) streaming
 // word w of its terms, so every term is one coalesced read.  The groups are combined
 // in order (deterministic),
-// then thread (row, rhs) recombines the +- columns (pm; the tensor-core pass's columns are
-// the block's own), applies the sign/permutation of its row, adds the identity term, stores y and contributes to the CTA's partial dot products (modes as k_reduce).
+// then thread (row, rhs) recombines the +- columns (pm 1: of blocks above kWholeB, 2: in
+// the tensor-core pass's order), applies the sign/permutation of its row, adds the identity term, stores y and contributes to the CTA's partial dot products (modes as k_reduce).
 template <typename OutT, typename VT, int R>
 __global__ void __launch_bounds__(kRBThreads)
 k_reduce_blk(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items, int nitems,
@@ -1381,11 +1451,12 @@ k_reduce_blk(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items,
         const int rho = info & ((1 << 29) - 1);
         const unsigned eneg = (info >> 29) & 1, sneg = (info >> 30) & 1;
         C a, c;
-        if (pm && S.B > kWholeB) {   // c[s] = c+ + c-, c[rmax + s] = c+ - c- from the columns 2 s + (0, 1)
+        if (pm == 2 || S.B > kWholeB) {   // c[s] = c+ + c-, c[rmax + s] = c+ - c- from the columns 2 s + (0, 1)
             const unsigned second = rho >= S.rmax ? 1u : 0u;
-            const int at = 2 * (rho - (second ? S.rmax : 0)) * R + rr;
-            a = cadd(partU[at], cflip(partU[at + R], second));
-            c = cadd(partW[at], cflip(partW[at + R], second));
+            const int s = rho - (second ? S.rmax : 0);
+            const int at = pm == 2 ? 2 * ((rr >> 1) * B + s) + (rr & 1) : 2 * s * R + rr, m = pm == 2 ? B : R;
+            a = cadd(partU[at], cflip(partU[at + m], second));
+            c = cadd(partW[at], cflip(partW[at + m], second));
         } else {
             a = partU[rho * R + rr];
             c = partW[rho * R + rr];
@@ -1761,7 +1832,7 @@ struct StripGroup {     // strips [beg, end) of clusters with block size B (one 
 
 struct Plan {
     int nsys = 0, R = 1, nv = 0, nr = 0;
-    long long nstrips = 0, total_pairs = 0, total_vec = 0, total_t = 0, max_B = 0, cw_elems = 0, cu_elems = 0;
+    long long nstrips = 0, total_pairs = 0, total_vec = 0, total_t = 0, total_ty = 0, max_B = 0, cw_elems = 0, cu_elems = 0;
     bool tmat = false;   // general particles: y vectors from per-particle T-matrices (k_yprep_tmat)
     std::vector<StripGroup> groups;
     std::vector<gb::SysDev> sd;
@@ -1831,6 +1902,7 @@ int build_plan(int nsys, const gb_system* sys, int R, cudaStream_t stream, Plan&
         add_items(P.ritems, s, d.D, d.B, pl.rbeg, pl.rend);   // one item per particle block
         P.total_vec = std::max<long long>(P.total_vec, d.vec_off + (long long)d.D * R);
         P.total_t = std::max<long long>(P.total_t, d.t_off + (long long)d.D);
+        P.total_ty = std::max<long long>(P.total_ty, d.ty_off + d.N * gb::tc_y_bytes(d.B, 1));
         P.max_B = std::max<long long>(P.max_B, d.B);
     }
     P.nstrips = (long long)P.strips.size();
@@ -1878,8 +1950,11 @@ WS ws_layout(const Plan& P, int prec, bool dense) {
     if (!dense) {
         w.off_cu = take(sizeof(double2) * (size_t)std::max<long long>(P.cu_elems, 1));
         w.off_cw = take(sizeof(double2) * (size_t)std::max<long long>(P.cw_elems, 1));
-        w.off_yu = take(16 * (size_t)P.total_vec);
-        w.off_yw = take(16 * (size_t)P.total_vec);
+        // (the tensor-core pass pads its operands' columns to 16)
+        const size_t yb = std::max<size_t>(16 * (size_t)P.total_vec,
+                                           R >= 4 && prec != GB_PREC_FP64 ? (size_t)P.total_ty * R : 0);
+        w.off_yu = take(yb);
+        w.off_yw = take(yb);
         w.off_tx = take(0);
     } else {
         w.off_cu = w.off_cw = w.off_yu = w.off_yw = take(0);
@@ -2175,13 +2250,11 @@ int launch_apply(const Plan& P, const DevPlan& D, const WS& w, unsigned char* ba
         constexpr int YK = decltype(yk)::value;
         using YT = typename YType<YK>::t;
         gb::note_launch();
-        if constexpr (YK != 3) {
-            if (P.tmat) {
-                GB_CUDA_TRY(launch_pdl(k_yprep_tmat<YK, VT, R>, dim3((unsigned)P.nr), dim3(kRBThreads), 0, stream, D.sys,
-                                       D.ritems, P.nr, st, mask, xin, reinterpret_cast<YT*>(Yu),
-                                       reinterpret_cast<YT*>(Yw), up, pl));
-                return GB_OK;
-            }
+        if (P.tmat) {
+            GB_CUDA_TRY(launch_pdl(k_yprep_tmat<YK, VT, R>, dim3((unsigned)P.nr), dim3(kRBThreads), 0, stream, D.sys,
+                                   D.ritems, P.nr, st, mask, xin, reinterpret_cast<YT*>(Yu),
+                                   reinterpret_cast<YT*>(Yw), up, pl));
+            return GB_OK;
         }
         GB_CUDA_TRY(launch_pdl(k_yprep<YK, VT, R>, dim3(vb), dim3(kVRows / 2 * R), 0, stream, D.sys, D.vitems, P.nv, st,
                                mask, tvec, xin, reinterpret_cast<YT*>(Yu), reinterpret_cast<YT*>(Yw), up, pl));
@@ -2204,12 +2277,17 @@ int launch_apply(const Plan& P, const DevPlan& D, const WS& w, unsigned char* ba
         e = yprep(std::integral_constant<int, 1>(), PL);
         if (!e && P.nstrips) e = launch_pgemv_all<Pol32, R>(P, D, st, mask, mat_hi, Yu, Yw, CU, CW, stream);
         if (!e) e = reduce(float2(), 1);
-    } else if (pol == 3) {   // tensor-core pass on the bf16 tiles (mat_hi): float2 y vectors and partials
+    } else if (pol == 3) {   // tensor-core pass on the bf16 tiles (mat_hi): float2 partials
         if constexpr (R == 4 || R == 8) {
             if (P.tmat) return gb_set_error(GB_UNSUPPORTED, "the tensor-core pass serves sphere clusters");
-            e = yprep(std::integral_constant<int, 3>(), R);
-            if (!e && P.nstrips) e = launch_pgemv_tcore(P, D, R, st, mask, mat_hi, Yu, Yw, CU, CW, stream);
-            if (!e) e = reduce(float2(), 0);
+            if (P.max_B > 70)
+                return gb_set_error(GB_UNSUPPORTED, "tensor-core pass: block size %lld > 70 (lmax 5)", P.max_B);
+            gb::note_launch();
+            GB_CUDA_TRY(launch_pdl(k_yprep_tc<VT, R>, dim3((unsigned)P.nr), dim3(kTcYThreads), 0, stream, D.sys, D.ritems,
+                                   st, mask, tvec, xin, static_cast<unsigned char*>(Yu), static_cast<unsigned char*>(Yw),
+                                   up));
+            if (P.nstrips) e = launch_pgemv_tcore(P, D, R, st, mask, mat_hi, Yu, Yw, CU, CW, stream);
+            if (!e) e = reduce(float2(), 2);
         } else {
             return gb_set_error(GB_UNSUPPORTED, "the tensor-core pass needs R = 4 or 8 (got %d)", R);
         }

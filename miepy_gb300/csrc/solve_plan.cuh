@@ -2,6 +2,7 @@
 // CUDA-core matrix pass (solve.cu) and the tensor-core matrix pass (gemv_tc.cu).
 #pragma once
 
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include "gb_internal.h"
@@ -48,11 +49,19 @@ __device__ __forceinline__ bool any_active(const KState* st, int sys, int mask_m
     return a;
 }
 
+// two bf16 in memory order; a float rounded to bf16
+__device__ __forceinline__ unsigned bf2(float first, float second) {
+    __nv_bfloat162 v = __floats2bfloat162_rn(first, second);
+    return *reinterpret_cast<unsigned*>(&v);
+}
+__device__ __forceinline__ float bf_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
+
 // Tensor-core matrix pass (gemv_tc.cu) over strips [sbeg, send) of one block size
 // B: the same column partials (CW, per pair by destination block row) and row
 // partials (CU, per strip) as the CUDA-core pass with complex64 arithmetic, as
 // float2 [B][R] per term, from the bf16 hi/lo tiles of the matrix (mat_tc) and the
-// y vectors Yu, Yw (float2 [D][R]).  R is 4 or 8.
+// operands Yu, Yw of the particles (tc_y_bytes(B, R) each, k_yprep_tc), as +- column sums.
+// R is 4 or 8.
 int launch_pgemv_tc(int R, const SysDev* sys, const Strip* strips, long long sbeg, long long send, const KState* st,
                     int mask, const void* mat_tc, const void* Yu, const void* Yw, void* CU, void* CW,
                     const SysPlan* plan, int B, int* err, cudaStream_t stream);
