@@ -25,8 +25,8 @@
 // of the tile's planes (+ hi, + lo, - hi, - lo, their rows one after the other) the first
 // MMA's 128 rows hold + hi and, from row 2 Hp on, - hi, the second's + lo and - lo at the
 // same rows, and only the columns of a row's own sign are read out:
-//   U = A z_j (row product of block (i, j), summed along the strip),
-//   W = A w_i (column product, one partial per block), w_i = S z_i,
+//   U = A z_j (row product of block (i, j)),
+//   W = A w_i (column product), w_i = S z_i,
 // with z[s] = eps(s) y[rho(s)] of the solver's y vectors.  k_yprep_tc writes each particle's
 // rows of U and of W once per product as bf16 pieces in the operand's layout, so that a
 // block's operand arrives by copies.  The results C[rho(r)] = eps(r) (A z)[r] are stored
@@ -35,21 +35,27 @@
 // two polarisations are opposite; element (column, right-hand side q) of a term lies at 16-byte
 // word (q / 2) B + sign rmax + column, so that a warp's stores are contiguous.
 //
+// Work unit: a rectangle of up to 4 rows x several columns of blocks, column by column, its
+// row sums (of all its columns) and the column's sums kept in registers: the partials of a
+// block by itself are a third of its tile's bytes at R = 8, B = 48, and went through HBM both
+// in this pass and in the reduce (N = 200, lmax 4, R = 8: 92 MB a product; with rectangles
+// 25 MB, the product 56 us against 79).
+//
 // Pipeline per CTA (6 warps, two CTAs per SM where their stages fit, persistent over
-// strips), each role running ahead of the next one as far as the rings let it: a producer
+// units), each role running ahead of the next one as far as the rings let it: a producer
 // warp copies, per block, the tile and the operand's pieces (TMA bulk copies) into a ring
 // of stages, with a job record; one thread issues the block's MMAs (M = 128: the rows past
 // the tile's read what follows it and are discarded) into one of two accumulators; the
-// warps of the tile's rows read the accumulator (tcgen05.ld), write its column partials and
-// keep the strip's row sums.  Every wait is bounded; an expired wait sets the error flag and the
+// warps of the tile's rows read the accumulator (tcgen05.ld) and add it to the sums.  Every wait is bounded; an expired wait sets the error flag and the
 // abort flag, which ends the other roles' waits, and the CTA waits (again bounded) for its
 // copies and MMAs in flight before it frees its TMEM and exits.
 //
-// Bound: per block, the issue of 9 copies (270 cycles) and of the MMAs, two CTAs per SM, next
-// to the tiles' 27 us at the measured copy rate.  N = 200, lmax 4: 45 us at R = 8, 33 at
-// R = 4; with whole blocks, their operand built by each CTA, 102 and 89.  (Issued from
-// divergent code, copies and MMAs took 83 to 160 cycles each: 71 and 57 us; a sign at a
-// time, with twice the MMAs, each bound by its 128 rows: 49 and 36.)
+// Bound: per block, the issue of 9 copies (270 cycles) and of the MMAs and the copies' bytes
+// from L2 (the operand's 12 KB with the tile's 9 KB at R = 8, B = 48), next to the tiles' 27
+// us at the measured copy rate.  N = 200, lmax 4: 42 us at R = 8, 35 at R = 4; with whole
+// blocks, their operand built by each CTA, 102 and 89.  (Issued from divergent code, copies
+// and MMAs took 83 to 160 cycles each: 71 and 57 us; a sign at a time, with twice the MMAs,
+// each bound by its 128 rows: 49 and 36.)
 #include <cuda_bf16.h>
 
 #include "gb_common.cuh"
@@ -163,8 +169,12 @@ __host__ __device__ constexpr unsigned idesc_bf16(int M, int N) {
 // records of the stages and of the two accumulators; then the stages, each a block's tile
 // (hi, lo of P + Q, then of P - Q) and the operand's pieces (8, 2R rows each).
 struct TcJob {
-    long long cw;    // element offset of the block's column partials in CW; -1: no more blocks for this CTA
-    long long cu;    // element offset of the strip's row partials in CU (last block of a strip), else -1
+    long long cw;    // first element of the column's partial in CW; -1: no more blocks for this CTA
+    long long cu;    // of the unit's first row's partial in CU
+    int row;         // the block's row of the unit
+    int rows;        // the unit's rows, at its last block, else 0
+    int stride;      // elements between the rows' partials
+    int last;        // the column's last block
 };
 // Block k's record lies in slot k % kTcJobs.  It is read by the MMA thread and by the warps
 // that read the accumulator out, which are at most kTcMaxStages + 1 blocks behind.
@@ -253,37 +263,45 @@ k_tc_tiles(const gb::SysDev* __restrict__ sys, const float2* __restrict__ mat64,
 }
 
 // ------------------------------------------------------------- matrix pass --
-// The warp's 32 TMEM lanes of columns a0 .. a0 + NC - 1 and a1 .. a1 + NC - 1 (NC = 16 or
-// 32), in x16 pieces, each pair waited for in the statement that loads it.
-template <int NC> __device__ __forceinline__ void tmem_ld2(unsigned a0, unsigned a1, float* v0, float* v1) {
+// The warp's 32 TMEM lanes of columns a0 .. a0 + NC - 1 and a1 .. a1 + NC - 1 (NC = 8 or
+// 16), waited for in the statement that loads them.
+template <int NC> __device__ __forceinline__ void tmem_ld_pair(unsigned a0, unsigned a1, unsigned* r);
+template <> __device__ __forceinline__ void tmem_ld_pair<8>(unsigned a0, unsigned a1, unsigned* r) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%16];\n"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%17];\n"
+        "tcgen05.wait::ld.sync.aligned;\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(a0), "r"(a1)
+        : "memory");
+}
+template <> __device__ __forceinline__ void tmem_ld_pair<16>(unsigned a0, unsigned a1, unsigned* r) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n"
+        "tcgen05.wait::ld.sync.aligned;\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(a0), "r"(a1)
+        : "memory");
+}
+template <int NC> __device__ __forceinline__ void tmem_ld2(unsigned a0, unsigned a1, float (&v0)[NC], float (&v1)[NC]) {
+    unsigned r[2 * NC];
+    tmem_ld_pair<NC>(a0, a1, r);
 #pragma unroll
-    for (int c = 0; c < NC; c += 16) {
-        unsigned r[32];
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n"
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n"
-            "tcgen05.wait::ld.sync.aligned;\n"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-              "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-              "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-            : "r"(a0 + (unsigned)c), "r"(a1 + (unsigned)c)
-            : "memory");
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            v0[c + i] = __uint_as_float(r[i]);
-            v1[c + i] = __uint_as_float(r[16 + i]);
-        }
+    for (int i = 0; i < NC; i++) {
+        v0[i] = __uint_as_float(r[i]);
+        v1[i] = __uint_as_float(r[NC + i]);
     }
 }
 
-// The pass over strips [sbeg, send) of one block size B with S stages.
+// The pass over units [ubeg, uend) of one block size B with S stages.
 template <int R>
-__global__ void __launch_bounds__(kTcThreads)
-k_pgemv_tc(const gb::SysDev* __restrict__ sys, const gb::Strip* __restrict__ strips, long long sbeg, long long send,
+__global__ void __launch_bounds__(kTcThreads, 2)
+k_pgemv_tc(const gb::SysDev* __restrict__ sys, const gb::TcUnit* __restrict__ units, long long ubeg, long long uend, int I,
            const gb::KState* __restrict__ st, int mask, const unsigned char* __restrict__ mat_tc,
            const unsigned char* __restrict__ Yu, const unsigned char* __restrict__ Yw, float2* __restrict__ CU,
-           float2* __restrict__ CW, const gb::SysPlan* __restrict__ plan, int B, int S, int* __restrict__ err) {
+           float2* __restrict__ CW, const gb::SysPlan* __restrict__ plan, const long long* __restrict__ tc_rows, int B, int S,
+           int* __restrict__ err) {
     constexpr int N = 16 * R;             // columns of an accumulator
     constexpr unsigned NCOL = 2 * N;      // two accumulators (128 or 256: a power of 2 >= 32)
     constexpr unsigned IDESC_FULL = idesc_bf16(128, N);
@@ -329,26 +347,27 @@ k_pgemv_tc(const gb::SysDev* __restrict__ sys, const gb::Strip* __restrict__ str
     long long k = 0;   // producer: jobs written
     if (warp == 4) {
         // ------------------------------------------------------------ producer
-        // Walks this CTA's strips (every gridDim.x-th, skipping clusters with no active
+        // Walks this CTA's units (every gridDim.x-th, skipping clusters with no active
         // right-hand side), the records of 32 of them loaded at once.
         const long long G = gridDim.x;
         const uint64_t pol = evict_first_policy();
-        long long pw = sbeg + blockIdx.x;
-        gb::Strip mine{};
-        int at = 32;   // strip of the 32 loaded
+        const unsigned pbytes = 4u * L.piece;   // of a particle's operand
+        const int BR = B * R;
+        gb::TcUnit mine{};
+        int at = 32;   // unit of the 32 loaded
         int cur = -1, NP = 0, s = 0;
         unsigned phase = 1;   // of the stage's empty barrier: passes at once the first time round
         bool act = false;
-        long long t_off = 0, y_off = 0, cw0 = 0, cu0 = 0, sb0 = 0;
+        long long t_off = 0, y_off = 0, cw0 = 0, cu0 = 0, rows0 = 0;
         bool run = true;
-        for (; run && pw < send; pw += G) {
+        for (long long pw = ubeg + blockIdx.x; run && pw < uend; pw += G) {
             if (at == 32) {
                 at = 0;
-                if (pw + lane * G < send) mine = strips[pw + lane * G];
+                if (pw + lane * G < uend) mine = units[pw + lane * G];
             }
-            const int sysi = __shfl_sync(0xffffffffu, mine.sys, at), i = __shfl_sync(0xffffffffu, mine.i, at),
-                      nb = __shfl_sync(0xffffffffu, mine.nb, at);
-            const long long p0 = __shfl_sync(0xffffffffu, mine.p0, at);
+            const int sysi = __shfl_sync(0xffffffffu, mine.sys, at), i0 = __shfl_sync(0xffffffffu, mine.i0, at),
+                      j0 = __shfl_sync(0xffffffffu, mine.j0, at), nj = __shfl_sync(0xffffffffu, mine.nj, at),
+                      c = __shfl_sync(0xffffffffu, mine.c, at), C = __shfl_sync(0xffffffffu, mine.C, at);
             at++;
             if (sysi != cur) {
                 cur = sysi;
@@ -358,39 +377,53 @@ k_pgemv_tc(const gb::SysDev* __restrict__ sys, const gb::Strip* __restrict__ str
                 NP = Sd.N;
                 t_off = Sd.tc_off;
                 y_off = Sd.ty_off * R;
-                cw0 = pl.cw_off;
-                cu0 = pl.cu_off;
-                sb0 = pl.strip_base;
+                cw0 = pl.tc_cw;
+                cu0 = pl.tc_cu;
+                rows0 = pl.tc_base;
             }
             if (!act) continue;
-            const int j0 = i + 1 + (int)(p0 - pair_start(i, NP));
-            const unsigned char* wsrc = Yw + y_off + (long long)i * (4LL * L.piece);
-            const unsigned char* usrc = Yu + y_off + (long long)j0 * (4LL * L.piece);
-            const unsigned char* tsrc = mat_tc + t_off + p0 * (long long)L.tile;
-            for (int pb = 0; pb < nb; pb++, k++) {
-                run = __all_sync(0xffffffffu, bar_wait(hd.empty + s, phase, stop));
-                if (!run) break;
-                if (elect_one()) {
-                    const long long j = j0 + pb;
-                    TcJob J;
-                    J.cw = cw0 + (j * (j - 1) / 2 + i) * (long long)B * R;
-                    J.cu = (pb == nb - 1) ? cu0 + (pw - sb0) * (long long)B * R : -1;
-                    hd.jobs[k % kTcJobs] = J;
-                    bar_expect_tx(hd.full + s, L.stage);   // arrive (release): the job record goes with it
-                    unsigned char* dst = stages + (size_t)s * L.stage;
-                    bulk_copy_hint(dst, tsrc, L.tile, hd.full + s, pol);
+            const int rows = min(I, NP - i0), stride = C * BR;
+            const long long cu = cu0 + (tc_rows[rows0 + i0] + c) * BR;
+            long long term = tc_rows[rows0 + NP + 1 + j0] + i0 / I;   // the column's partial of this row group
+            const unsigned char* usrc = Yu + y_off + (long long)j0 * pbytes;
+            const unsigned char* wsrc = Yw + y_off + (long long)i0 * pbytes;
+            const unsigned char* tsrc = mat_tc + t_off + (pair_start(i0, NP) + j0 - i0 - 1) * (long long)L.tile;
+            for (int jj = 0; run && jj < nj; jj++) {
+                const int n = min(rows, j0 + jj - i0);   // the column's blocks
+                const long long cw = cw0 + term * BR;
+                const unsigned char* ts = tsrc;
+                const unsigned char* ws = wsrc;
+                for (int ii = 0; ii < n; ii++, k++) {
+                    run = __all_sync(0xffffffffu, bar_wait(hd.empty + s, phase, stop));
+                    if (!run) break;
+                    if (elect_one()) {
+                        TcJob J;
+                        J.cw = cw;
+                        J.cu = cu;
+                        J.row = ii;
+                        J.rows = ii == n - 1 && jj == nj - 1 ? rows : 0;
+                        J.stride = stride;
+                        J.last = ii == n - 1;
+                        hd.jobs[k % kTcJobs] = J;
+                        bar_expect_tx(hd.full + s, L.stage);   // arrive (release): the job record goes with it
+                        unsigned char* dst = stages + (size_t)s * L.stage;
+                        bulk_copy_hint(dst, ts, L.tile, hd.full + s, pol);
 #pragma unroll
-                    for (int c = 0; c < 8; c++)   // (hi / lo, sign, U / W)
-                        bulk_copy(dst + L.tile + c * L.piece, ((c & 1) ? wsrc : usrc) + (c >> 1) * L.piece, L.piece,
-                                  hd.full + s);
+                        for (int q = 0; q < 8; q++)   // (hi / lo, sign, U / W)
+                            bulk_copy(dst + L.tile + q * L.piece, ((q & 1) ? ws : usrc) + (q >> 1) * L.piece, L.piece,
+                                      hd.full + s);
+                    }
+                    __syncwarp();
+                    ts += (long long)(NP - 2 - i0 - ii) * L.tile;   // (i + 1, j)
+                    ws += pbytes;
+                    if (++s == S) {
+                        s = 0;
+                        phase ^= 1u;
+                    }
                 }
-                __syncwarp();
                 tsrc += L.tile;
-                usrc += 4u * L.piece;
-                if (++s == S) {
-                    s = 0;
-                    phase ^= 1u;
-                }
+                usrc += pbytes;
+                term += (j0 + jj + I - 1) / I;   // column j has one per row group that starts above it
             }
         }
         if (!run && lane == 0) give_up();
@@ -455,14 +488,28 @@ k_pgemv_tc(const gb::SysDev* __restrict__ sys, const gb::Strip* __restrict__ str
         int at = 0;          // its 16-byte word in a term: column rho(m) of the other sign
         unsigned eneg = 0;
         if (row) {
-            const int info = __ldg(sys[strips[sbeg].sys].rowinfo + m);   // every cluster of the launch has block size B
+            const int info = __ldg(sys[units[ubeg].sys].rowinfo + m);   // every cluster of the launch has block size B
             at = (sig ^ 1) * H + (info & ((1 << 29) - 1));
             eneg = (info >> 29) & 1;
         }
         const unsigned taddr = tmem + ((unsigned)(warp * 32) << 16) + (unsigned)(sig * 4 * R);
-        float u[2 * R];
+        float u[gb::kTcRows][2 * R], w[2 * R];   // sums of the unit's rows, of the column
 #pragma unroll
-        for (int q = 0; q < 2 * R; q++) u[q] = 0.f;
+        for (int q = 0; q < 2 * R; q++) {
+            w[q] = 0.f;
+#pragma unroll
+            for (int t = 0; t < gb::kTcRows; t++) u[t][q] = 0.f;
+        }
+        auto put = [&](float2* to, float (&v)[2 * R]) {   // a partial out, its sums back to zero
+            float4* p = reinterpret_cast<float4*>(to) + at;
+#pragma unroll
+            for (int q = 0; q < 2 * R; q += 4) {
+                if (row)
+                    p[q / 4 * B] = make_float4(flipf(v[q], eneg), flipf(v[q + 1], eneg), flipf(v[q + 2], eneg),
+                                               flipf(v[q + 3], eneg));
+                v[q] = v[q + 1] = v[q + 2] = v[q + 3] = 0.f;
+            }
+        };
         for (long long e = 0;; e++) {
             const int x = (int)(e & 1);
             const unsigned phase = (unsigned)((e >> 1) & 1);
@@ -481,32 +528,26 @@ k_pgemv_tc(const gb::SysDev* __restrict__ sys, const gb::Strip* __restrict__ str
                 break;
             }
             tc_after_sync();
-            float h[4 * R], l[4 * R];   // of z_h and of z_l: U, then W
-            tmem_ld2<4 * R>(taddr + (unsigned)(x * N), taddr + (unsigned)(x * N + 8 * R), h, l);
+            float h[2 * R], l[2 * R];   // of z_h and of z_l
+            const unsigned ta = taddr + (unsigned)(x * N);
+            tmem_ld2<2 * R>(ta, ta + 8 * R, h, l);
+#pragma unroll
+            for (int t = 0; t < gb::kTcRows; t++)
+                if (J.row == t) {
+#pragma unroll
+                    for (int q = 0; q < 2 * R; q++) u[t][q] += h[q] + l[q];
+                }
+            tmem_ld2<2 * R>(ta + 2 * R, ta + 10 * R, h, l);
             tc_before_sync();
             __syncwarp();
             if (lane == 0) bar_arrive(hd.free + x);
-            if (row) {
-                float4* cwp = reinterpret_cast<float4*>(CW + J.cw) + at;
 #pragma unroll
-                for (int q = 0; q < 2 * R; q += 4) {
+            for (int q = 0; q < 2 * R; q++) w[q] += h[q] + l[q];
+            if (J.last) put(CW + J.cw, w);
+            if (J.rows) {
 #pragma unroll
-                    for (int c = q; c < q + 4; c++) u[c] += h[c] + l[c];
-                    const int w = 2 * R + q;
-                    cwp[q / 4 * B] = make_float4(flipf(h[w] + l[w], eneg), flipf(h[w + 1] + l[w + 1], eneg),
-                                                 flipf(h[w + 2] + l[w + 2], eneg), flipf(h[w + 3] + l[w + 3], eneg));
-                }
-            }
-            if (J.cu >= 0) {   // the strip's row partial
-                if (row) {
-                    float4* cup = reinterpret_cast<float4*>(CU + J.cu) + at;
-#pragma unroll
-                    for (int q = 0; q < 2 * R; q += 4)
-                        cup[q / 4 * B] = make_float4(flipf(u[q], eneg), flipf(u[q + 1], eneg), flipf(u[q + 2], eneg),
-                                                     flipf(u[q + 3], eneg));
-                }
-#pragma unroll
-                for (int q = 0; q < 2 * R; q++) u[q] = 0.f;
+                for (int t = 0; t < gb::kTcRows; t++)
+                    if (t < J.rows) put(CU + J.cu + (long long)t * J.stride, u[t]);
             }
         }
     }
@@ -525,10 +566,10 @@ k_pgemv_tc(const gb::SysDev* __restrict__ sys, const gb::Strip* __restrict__ str
 
 namespace gb {
 
-int launch_pgemv_tc(int R, const SysDev* sys, const Strip* strips, long long sbeg, long long send, const KState* st,
-                    int mask, const void* mat_tc, const void* Yu, const void* Yw, void* CU, void* CW,
-                    const SysPlan* plan, int B, int* err, cudaStream_t stream) {
-    if (send <= sbeg) return GB_OK;
+int launch_pgemv_tc(int R, const SysDev* sys, const TcUnit* units, long long ubeg, long long uend, int I,
+                    const KState* st, int mask, const void* mat_tc, const void* Yu, const void* Yw, void* CU, void* CW,
+                    const SysPlan* plan, const long long* tc_rows, int B, int* err, cudaStream_t stream) {
+    if (uend <= ubeg) return GB_OK;
     if (R != 4 && R != 8) return gb_set_error(GB_UNSUPPORTED, "tensor-core pass: R must be 4 or 8 (got %d)", R);
     if (B > 70) return gb_set_error(GB_UNSUPPORTED, "tensor-core pass: block size %d > 70 (lmax 5)", B);
     if ((reinterpret_cast<uintptr_t>(mat_tc) | reinterpret_cast<uintptr_t>(Yu) | reinterpret_cast<uintptr_t>(Yw)) & 15)
@@ -540,7 +581,7 @@ int launch_pgemv_tc(int R, const SysDev* sys, const Strip* strips, long long sbe
     const TcLayout L = tc_layout(B, R, S);
     const void* kfn = R == 4 ? reinterpret_cast<const void*>(k_pgemv_tc<4>) : reinterpret_cast<const void*>(k_pgemv_tc<8>);
     GB_CUDA_TRY(ensure_dynamic_smem(kfn, L.total));
-    const long long n = send - sbeg;
+    const long long n = uend - ubeg;
     const long long grid = n < 2LL * sm_count() ? n : 2LL * sm_count();
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[1];
@@ -559,11 +600,11 @@ int launch_pgemv_tc(int R, const SysDev* sys, const Strip* strips, long long sbe
     float2* cu = static_cast<float2*>(CU);
     float2* cw = static_cast<float2*>(CW);
     if (R == 4)
-        GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_pgemv_tc<4>, sys, strips, sbeg, send, st, mask, m, yu, yw, cu, cw, plan, B,
-                                       S, err));
+        GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_pgemv_tc<4>, sys, units, ubeg, uend, I, st, mask, m, yu, yw, cu, cw, plan,
+                                       tc_rows, B, S, err));
     else
-        GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_pgemv_tc<8>, sys, strips, sbeg, send, st, mask, m, yu, yw, cu, cw, plan, B,
-                                       S, err));
+        GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_pgemv_tc<8>, sys, units, ubeg, uend, I, st, mask, m, yu, yw, cu, cw, plan,
+                                       tc_rows, B, S, err));
     return GB_OK;
 }
 

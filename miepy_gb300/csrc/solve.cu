@@ -1383,7 +1383,11 @@ k_reduce_blk(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items,
     const gb::SysDev S = sys[I.sys];
     const SysPlan pl = plan[I.sys];
     const int k = I.r0 / S.B;   // particle (block row) of this item
-    const long long s0 = row_strip[pl.strip_row_base + k], s1 = row_strip[pl.strip_row_base + k + 1];
+    // its terms in CU and in CW: one per strip of row k and per block (i, k), i < k, or (pm 2)
+    // as the tensor-core pass's plan numbers them
+    const long long* tr = row_strip + (pm == 2 ? pl.tc_base : pl.strip_row_base);
+    const long long u0 = tr[k], nu = tr[k + 1] - u0;
+    const long long w0 = pm == 2 ? tr[S.N + 1 + k] : (long long)k * (k - 1) / 2, nterm_w = pm == 2 ? tr[S.N + 2 + k] - w0 : k;
     constexpr int E = PWord<OutT>::E;
     const int B = S.B, BR = B * R;
     // The combine's inputs (row map, x, aux, b, the identity's scale, the solver
@@ -1414,17 +1418,16 @@ k_reduce_blk(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items,
     __shared__ C partU[2 * kRBThreads], partW[2 * kRBThreads];
     __shared__ DotAcc<T> red[kRBThreads / 32][R][2];
     if (g < G) {
-        const long long ns = s1 - s0;
-        const OutT* cu = CU + pl.cu_off + (s0 - pl.strip_base) * (long long)BR + w * E;
-        const OutT* cw = CW + pl.cw_off + ((long long)k * (k - 1) / 2) * BR + w * E;
+        const OutT* cu = CU + (pm == 2 ? pl.tc_cu + u0 * BR : pl.cu_off + (u0 - pl.strip_base) * BR) + w * E;
+        const OutT* cw = CW + (pm == 2 ? pl.tc_cw : pl.cw_off) + w0 * BR + w * E;
         RAcc<OutT> au[E], aw[E];
 #pragma unroll
         for (int e = 0; e < E; e++) {
             au[e].zero();
             aw[e].zero();
         }
-        sum_terms<OutT, E>(cu, g, ns, G, BR, au);
-        sum_terms<OutT, E>(cw, g, k, G, BR, aw);
+        sum_terms<OutT, E>(cu, g, nu, G, BR, au);
+        sum_terms<OutT, E>(cw, g, nterm_w, G, BR, aw);
 #pragma unroll
         for (int e = 0; e < E; e++) {
             partU[g * BR + w * E + e] = au[e].template as<C>();
@@ -1840,6 +1843,12 @@ struct Plan {
     std::vector<Item> vitems, ritems;
     std::vector<SysPlan> sp;
     std::vector<long long> row_strip;
+    // the tensor-core pass's units (R = 4 or 8 in the FP32 and mixed methods)
+    int tc_I = 0;
+    std::vector<gb::TcUnit> tc_units;
+    std::vector<StripGroup> tc_groups;
+    std::vector<long long> tc_rows;
+    long long tc_cu_elems = 0, tc_cw_elems = 0;
 };
 
 void add_items(std::vector<Item>& v, int s, int D, int rows, int& beg, int& end) {
@@ -1848,7 +1857,65 @@ void add_items(std::vector<Item>& v, int s, int D, int rows, int& beg, int& end)
     end = (int)v.size();
 }
 
-int build_plan(int nsys, const gb_system* sys, int R, cudaStream_t stream, Plan& P) {
+// Units of the tensor-core pass: rectangles of I rows x J columns of blocks.  Large ones
+// have few partials (a block's column partial per I blocks, its row partial per J), small
+// ones spread evenly over the pass's CTAs; of I = 1, 2, 4 and J <= 16 the pair with the
+// least time, in blocks: the CTA with the most units, and each partial's 2 B R x 8 bytes
+// to and from HBM over all CTAs, 0.4 of a block at B = 48, R = 8.
+void tc_units(Plan& P, const std::vector<int>& order) {
+    const double ctas = 2.0 * gb::sm_count();
+    double best = 1e300;
+    int I = 1, J = 1;
+    for (int i = 1; i <= gb::kTcRows; i *= 2)
+        for (int j = 1; j <= 16; j++) {
+            double cost = 0, n = 0, terms = 0;
+            int B = 0;
+            for (size_t q = 0; q <= order.size(); q++) {
+                const gb::SysDev* d = q < order.size() ? &P.sd[order[q]] : nullptr;
+                if (!d || d->B != B) {   // a block size is a launch
+                    cost += std::ceil(n / ctas) * i * j + 0.4 * (B * P.R / 384.0) * terms / ctas;
+                    n = terms = 0;
+                }
+                if (!d) break;
+                B = d->B;
+                const double groups = double((d->N - 1 + i - 1) / i);
+                n += double(d->P) / (i * j) + 0.5 * groups;
+                terms += double(d->P) / i + i * (double(d->P) / (i * j) + 0.5 * groups);
+            }
+            if (cost < best * (1 - 1e-9)) { best = cost; I = i; J = j; }
+        }
+    P.tc_I = I;
+    for (int s : order) {
+        const gb::SysDev& d = P.sd[s];
+        SysPlan& pl = P.sp[s];
+        if (P.tc_groups.empty() || P.tc_groups.back().B != d.B)
+            P.tc_groups.push_back(StripGroup{d.B, (long long)P.tc_units.size(), (long long)P.tc_units.size()});
+        pl.tc_base = (long long)P.tc_rows.size();
+        pl.tc_cu = P.tc_cu_elems;
+        pl.tc_cw = P.tc_cw_elems;
+        long long u = 0, w = 0;
+        for (int i = 0; i < d.N; i++) {
+            const int i0 = i - i % I, C = (d.N - 1 - i0 + J - 1) / J;
+            P.tc_rows.push_back(u);
+            u += C;
+            for (int c = 0; i == i0 && c < C; c++) {
+                const int j0 = i0 + 1 + c * J;
+                P.tc_units.push_back(gb::TcUnit{s, i0, j0, std::min(J, d.N - j0), c, C});
+            }
+        }
+        P.tc_rows.push_back(u);
+        for (int j = 0; j < d.N; j++) {
+            P.tc_rows.push_back(w);
+            w += (j + I - 1) / I;
+        }
+        P.tc_rows.push_back(w);
+        P.tc_groups.back().end = (long long)P.tc_units.size();
+        P.tc_cu_elems += u * d.B * P.R;
+        P.tc_cw_elems += w * d.B * P.R;
+    }
+}
+
+int build_plan(int nsys, const gb_system* sys, int R, int prec, cudaStream_t stream, Plan& P) {
     P.nsys = nsys;
     P.R = R;
     int st = gb::make_sysdev(nsys, sys, stream, P.sd);
@@ -1905,6 +1972,7 @@ int build_plan(int nsys, const gb_system* sys, int R, cudaStream_t stream, Plan&
         P.total_ty = std::max<long long>(P.total_ty, d.ty_off + d.N * gb::tc_y_bytes(d.B, 1));
         P.max_B = std::max<long long>(P.max_B, d.B);
     }
+    if (R >= 4 && prec != GB_PREC_FP64) tc_units(P, order);
     P.nstrips = (long long)P.strips.size();
     P.nv = (int)P.vitems.size();
     P.nr = (int)P.ritems.size();
@@ -1948,8 +2016,10 @@ WS ws_layout(const Plan& P, int prec, bool dense) {
     w.off_ostate = take(sizeof(KState) * P.nsys * R);
     w.off_dots = take(sizeof(double2) * 2 * (size_t)std::max(std::max(P.nv, P.nr), 1) * R);
     if (!dense) {
-        w.off_cu = take(sizeof(double2) * (size_t)std::max<long long>(P.cu_elems, 1));
-        w.off_cw = take(sizeof(double2) * (size_t)std::max<long long>(P.cw_elems, 1));
+        w.off_cu = take(std::max(sizeof(double2) * (size_t)std::max<long long>(P.cu_elems, 1),
+                                 sizeof(float2) * (size_t)P.tc_cu_elems));
+        w.off_cw = take(std::max(sizeof(double2) * (size_t)std::max<long long>(P.cw_elems, 1),
+                                 sizeof(float2) * (size_t)P.tc_cw_elems));
         // (the tensor-core pass pads its operands' columns to 16)
         const size_t yb = std::max<size_t>(16 * (size_t)P.total_vec,
                                            R >= 4 && prec != GB_PREC_FP64 ? (size_t)P.total_ty * R : 0);
@@ -1967,7 +2037,8 @@ WS ws_layout(const Plan& P, int prec, bool dense) {
     w.off_d128 = take(prec == GB_PREC_MIXED ? sizeof(double2) * (size_t)P.total_vec : 0);
     w.off_tp = take(dense ? 0 : sizeof(double2) * (size_t)std::max<long long>(P.total_t, 1));   // t D (preconditioned)
     w.off_blob = take(sizeof(gb::SysDev) * P.nsys + sizeof(Strip) * P.nstrips + sizeof(Item) * (P.nv + P.nr) +
-                      sizeof(SysPlan) * P.nsys + sizeof(long long) * P.row_strip.size() + sizeof(int) * P.nsys + 256);
+                      sizeof(SysPlan) * P.nsys + sizeof(long long) * P.row_strip.size() + sizeof(int) * P.nsys + 256 +
+                      sizeof(gb::TcUnit) * P.tc_units.size() + sizeof(long long) * P.tc_rows.size());
     w.total = o;
     return w;
 }
@@ -1979,6 +2050,8 @@ struct DevPlan {
     const Item* ritems;
     const SysPlan* sp;
     const long long* row_strip;
+    const gb::TcUnit* tc_units;
+    const long long* tc_rows;
     int* err;   // set by a GEMV whose bounded wait on a copy expired
     int* cnt;   // [nsys] arrival counters of the fused scalar updates (zero between launches)
 };
@@ -1997,6 +2070,8 @@ int upload_plan(const Plan& P, unsigned char* base, const WS& w, cudaStream_t st
     size_t o_ri = put(P.ritems.data(), sizeof(Item) * P.nr);
     size_t o_sp = put(P.sp.data(), sizeof(SysPlan) * P.nsys);
     size_t o_rs = put(P.row_strip.data(), sizeof(long long) * P.row_strip.size());
+    size_t o_tu = put(P.tc_units.data(), sizeof(gb::TcUnit) * P.tc_units.size());
+    size_t o_tr = put(P.tc_rows.data(), sizeof(long long) * P.tc_rows.size());
     const int zeros[4] = {0, 0, 0, 0};
     size_t o_err = put(zeros, sizeof(zeros));
     const std::vector<int> counters(P.nsys, 0);
@@ -2015,6 +2090,8 @@ int upload_plan(const Plan& P, unsigned char* base, const WS& w, cudaStream_t st
     D.ritems = reinterpret_cast<const Item*>(dst + o_ri);
     D.sp = reinterpret_cast<const SysPlan*>(dst + o_sp);
     D.row_strip = reinterpret_cast<const long long*>(dst + o_rs);
+    D.tc_units = reinterpret_cast<const gb::TcUnit*>(dst + o_tu);
+    D.tc_rows = reinterpret_cast<const long long*>(dst + o_tr);
     D.err = reinterpret_cast<int*>(dst + o_err);
     D.cnt = reinterpret_cast<int*>(dst + o_cnt);
     return GB_OK;
@@ -2222,10 +2299,9 @@ int launch_df(const Plan& P, const DevPlan& D, const KState* st, int mask, const
 // Tensor-core pass (gemv_tc.cu): one launch per block-size group.
 int launch_pgemv_tcore(const Plan& P, const DevPlan& D, int R, const KState* st, int mask, const void* mat_tc,
                        const void* Yu, const void* Yw, void* CU, void* CW, cudaStream_t stream) {
-    for (const StripGroup& grp : P.groups) {
-        if (grp.end == grp.beg) continue;
-        const int e = gb::launch_pgemv_tc(R, D.sys, D.strips, grp.beg, grp.end, st, mask, mat_tc, Yu, Yw, CU, CW, D.sp,
-                                          grp.B, D.err, stream);
+    for (const StripGroup& grp : P.tc_groups) {
+        const int e = gb::launch_pgemv_tc(R, D.sys, D.tc_units, grp.beg, grp.end, P.tc_I, st, mask, mat_tc, Yu, Yw, CU, CW,
+                                          D.sp, D.tc_rows, grp.B, D.err, stream);
         if (e) return e;
     }
     return GB_OK;
@@ -2264,7 +2340,7 @@ int launch_apply(const Plan& P, const DevPlan& D, const WS& w, unsigned char* ba
         using OutT = decltype(out);
         gb::note_launch();
         GB_CUDA_TRY(launch_pdl(k_reduce_blk<OutT, VT, R>, dim3((unsigned)P.nr), dim3(kRBThreads), 0, stream, D.sys,
-                               D.ritems, P.nr, D.sp, D.row_strip, st, mask, reinterpret_cast<const OutT*>(CU),
+                               D.ritems, P.nr, D.sp, pm == 2 ? D.tc_rows : D.row_strip, st, mask, reinterpret_cast<const OutT*>(CU),
                                reinterpret_cast<const OutT*>(CW), xin, yout, mode, aux, b128, dots, fz, xscale, pm));
         return GB_OK;
     };
@@ -2354,11 +2430,12 @@ struct GraphUse {
 // FNV-1a over the block-size groups of a plan (each group is one GEMV launch in a graph)
 long long groups_hash(const Plan& P) {
     unsigned long long h = 1469598103934665603ull;
-    for (const StripGroup& g : P.groups) {
-        const long long v[3] = {g.B, g.beg, g.end};
-        const unsigned char* b = reinterpret_cast<const unsigned char*>(v);
-        for (size_t i = 0; i < sizeof(v); i++) h = (h ^ b[i]) * 1099511628211ull;
-    }
+    for (const std::vector<StripGroup>* gs : {&P.groups, &P.tc_groups})
+        for (const StripGroup& g : *gs) {
+            const long long v[3] = {g.B + ((long long)P.tc_I << 32), g.beg, g.end};
+            const unsigned char* b = reinterpret_cast<const unsigned char*>(v);
+            for (size_t i = 0; i < sizeof(v); i++) h = (h ^ b[i]) * 1099511628211ull;
+        }
     return (long long)h;
 }
 
@@ -2946,7 +3023,7 @@ int apply_entry(int nsys, const gb_system* sys, int R, int prec, const double* m
 #endif
     if (prec == GB_PREC_MIXED_FP64RES) prec = GB_PREC_FP64;
     Plan P;
-    int e = build_plan(nsys, sys, R, s, P);
+    int e = build_plan(nsys, sys, R, prec, s, P);
     if (e) return e;
     WS w = ws_layout(P, prec, false);
     if (ws_bytes < w.total) return gb_set_error(GB_OVER_BUDGET, "workspace %zu B < required %zu B", ws_bytes, w.total);
@@ -2978,7 +3055,7 @@ int solve_entry(int nsys, const gb_system* sys, int R, int prec, double tol, int
                                      mat_tc, pdiag, tvec, b, x, workspace, ws_bytes, status, iters, resid, s);
 #endif
     Plan P;
-    int e = build_plan(nsys, sys, R, s, P);
+    int e = build_plan(nsys, sys, R, prec, s, P);
     if (e) return e;
     WS w = ws_layout(P, prec, false);
     if (ws_bytes < w.total) return gb_set_error(GB_OVER_BUDGET, "workspace %zu B < required %zu B", ws_bytes, w.total);
@@ -3006,7 +3083,7 @@ extern "C" {
 
 size_t gb_solve_workspace_size(int nsys, const gb_system* sys, int R, int prec) {
     Plan P;
-    if (build_plan(nsys, sys, R, 0, P)) return 0;
+    if (build_plan(nsys, sys, R, prec, 0, P)) return 0;
     return ws_layout(P, prec, false).total;
 }
 
@@ -3041,7 +3118,7 @@ int gb_solve_batch_tmatrix(int nsys, const gb_system* sys, int R, int prec, doub
     if (!(tol > 0) || maxiter < 1) return gb_set_error(GB_BAD_ARG, "tol must be > 0 and maxiter >= 1");
     cudaStream_t s = (cudaStream_t)stream;
     Plan P;
-    int e = build_plan(nsys, sys, R, s, P);
+    int e = build_plan(nsys, sys, R, prec, s, P);
     if (e) return e;
     for (int q = 0; q < nsys; q++) {
         if (P.sd[q].B * R > kRBThreads) return gb_set_error(GB_UNSUPPORTED, "T-matrix clusters need lmax <= 8");
@@ -3075,7 +3152,7 @@ int gb_autotune_gemv(int nsys, const gb_system* sys, int R, int prec, const doub
     const int aprec = f64 ? GB_PREC_FP64 : GB_PREC_FP32;
     cudaStream_t s = (cudaStream_t)stream;
     Plan P;
-    int e = build_plan(nsys, sys, R, s, P);
+    int e = build_plan(nsys, sys, R, prec, s, P);
     if (e) return e;
     WS w = ws_layout(P, aprec, false);
     if (ws_bytes < w.total) return gb_set_error(GB_OVER_BUDGET, "workspace %zu B < required %zu B", ws_bytes, w.total);

@@ -16,6 +16,10 @@ struct Strip {          // GEMV work: blocks (i, j0 .. j0+nb-1) of cluster sys
 struct Item {           // rows [r0, r0+nr) of cluster sys
     int sys, r0, nr, pad;
 };
+struct TcUnit {         // tensor-core pass: the pairs (i, j) of cluster sys with i < j, i0 <= i <
+    int sys, i0, j0, nj;   // i0 + I (I of the plan), j0 <= j < j0 + nj; unit c of its rows
+    int c, C;              // among C: row i's partials of its C units are contiguous
+};
 struct SysPlan {
     long long strip_row_base;   // index into row_strip (first block row of this cluster)
     long long strip_base;       // global index of the first strip of this cluster
@@ -23,6 +27,9 @@ struct SysPlan {
     long long cu_off;           // element offset of this cluster's per-strip row partials
     int vbeg, vend;             // vector items
     int rbeg, rend;             // reduce items
+    // tensor-core pass: the cluster's N + 1 first terms of every row's partials in CU, then of
+    // every column's in CW, in tc_rows; its first elements there
+    long long tc_base, tc_cu, tc_cw;
 };
 
 struct KState {         // per (cluster, rhs) BiCGSTAB scalars
@@ -56,15 +63,15 @@ __device__ __forceinline__ unsigned bf2(float first, float second) {
 }
 __device__ __forceinline__ float bf_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
-// Tensor-core matrix pass (gemv_tc.cu) over strips [sbeg, send) of one block size
-// B: the same column partials (CW, per pair by destination block row) and row
-// partials (CU, per strip) as the CUDA-core pass with complex64 arithmetic, as
-// float2 [B][R] per term, from the bf16 hi/lo tiles of the matrix (mat_tc) and the
-// operands Yu, Yw of the particles (tc_y_bytes(B, R) each, k_yprep_tc), as +- column sums.
-// R is 4 or 8.
-int launch_pgemv_tc(int R, const SysDev* sys, const Strip* strips, long long sbeg, long long send, const KState* st,
-                    int mask, const void* mat_tc, const void* Yu, const void* Yw, void* CU, void* CW,
-                    const SysPlan* plan, int B, int* err, cudaStream_t stream);
+// Tensor-core matrix pass (gemv_tc.cu) over units [ubeg, uend) of rows groups of I and one
+// block size B: row partials per (row, unit) in CU and column partials per (row group,
+// column) in CW, float2 terms of B R elements as +- column sums, from the bf16 hi/lo tiles
+// of the matrix (mat_tc) and the operands Yu, Yw of the particles (tc_y_bytes(B, R) each,
+// k_yprep_tc).  R is 4 or 8.
+constexpr int kTcRows = 4;   // I at most
+int launch_pgemv_tc(int R, const SysDev* sys, const TcUnit* units, long long ubeg, long long uend, int I,
+                    const KState* st, int mask, const void* mat_tc, const void* Yu, const void* Yw, void* CU, void* CW,
+                    const SysPlan* plan, const long long* tc_rows, int B, int* err, cudaStream_t stream);
 
 // The R = 4 and 8 solves, applies and wait limit, compiled in their own unit
 // (solve_multi.cu, which includes solve.cu with GB_SOLVE_MULTI_RHS defined) so that
