@@ -694,13 +694,14 @@ struct GemvLayout {
 // producer runs S-1 chunks ahead of the consumer, so with cpb chunks per block the
 // y_u of at most 1 + ceil((S-1)/cpb) blocks are live: the first chunk of block
 // b + nys is issued only once every chunk of block b has been consumed.  (All
-// blocks of one launch have the block size Bmax; a pass reads Bmax / 2 rows of each.)
+// blocks of one launch have the block size Bmax; a pass reads Bmax / 2 rows of each, a
+// warp that shares its strip (split) some of them, in any number of chunks.)
 __host__ __device__ inline GemvLayout gemv_layout(int Bmax, int rows_per_chunk, int RR, int S, int mat_bytes, bool df,
-                                                  int y_bytes) {
+                                                  int y_bytes, bool split) {
     GemvLayout g;
     g.chunk_cap = ((rows_per_chunk * Bmax * mat_bytes) + 127) & ~127;
     g.y_bytes = (Bmax * RR * y_bytes + 127) & ~127;
-    const int cpb = (Bmax / 2 + rows_per_chunk - 1) / rows_per_chunk;
+    const int cpb = split ? 1 : (Bmax / 2 + rows_per_chunk - 1) / rows_per_chunk;
     const int live = 1 + (S - 1 + cpb - 1) / cpb;
     g.nys = live < S ? live : S;
     // + 256 B of padding (kGemvPad): lanes whose columns lie past the block's end
@@ -716,8 +717,13 @@ __host__ __device__ inline GemvLayout gemv_layout(int Bmax, int rows_per_chunk, 
 // Column sums of the RPW rows are combined by shuffles once per block.  A chunk
 // is G steps (G*RPW rows, the last chunk of a block may be shorter).
 // RR right-hand sides per launch (rr0 .. rr0+RR-1: plane rr0 / RR of the y vectors), RT
-// the row stride of the partials.
-template <class Pol, int RR, int RT, int LPR, int CPL, int G, int S>
+// the row stride of the partials.  SPLIT: a strip is a CTA's, each warp takes some of the
+// rows of its blocks (split_rows) and the warps' sums are added in shared memory.
+__host__ __device__ inline int split_rows(int H, int warps, int rpw) {   // rows per warp
+    const int r = (H + warps - 1) / warps;
+    return (r + rpw - 1) / rpw * rpw;
+}
+template <class Pol, int RR, int RT, int LPR, int CPL, int G, int S, bool SPLIT = false>
 __global__ void __launch_bounds__(kGemvThreads)
 k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, long long sbeg, long long send,
         const KState* __restrict__ st, int mask_mode, const void* __restrict__ mat_hi, const void* __restrict__ mat_lo,
@@ -737,7 +743,7 @@ k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, lo
     extern __shared__ __align__(128) unsigned char gemv_smem[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int ro = lane / LPR, cl = lane % LPR;
-    const GemvLayout lay = gemv_layout(Bmax, RC, RR, S, MB, DF, sizeof(YT));
+    const GemvLayout lay = gemv_layout(Bmax, RC, RR, S, MB, DF, sizeof(YT), SPLIT);
     const float sign = (cl & 1) ? -1.f : 1.f;
     unsigned char* wbase = gemv_smem + (size_t)wid * lay.warp_bytes;
     uint64_t* bars = reinterpret_cast<uint64_t*>(wbase);
@@ -754,8 +760,12 @@ k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, lo
     // ring position: chunk number gc of this warp lives in stage gc % S, phase gc / S
     unsigned cstage = 0, cphase = 0;      // consumer
     unsigned pstage = 0;                  // producer (lane 0)
-    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+    const long long warp = SPLIT ? blockIdx.x : ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long long nwarps = SPLIT ? gridDim.x : ((long long)gridDim.x * blockDim.x) >> 5;
+    const int nparts = SPLIT ? blockDim.x >> 5 : 1;
+    // the warps' sums: two buffers, so that one barrier per use is enough
+    OutT* exch = reinterpret_cast<OutT*>(gemv_smem + (size_t)nparts * lay.warp_bytes);
+    int ebuf = 0;
     bool failed = false;
     int in_flight = 0;                    // chunks issued and not yet consumed
     const uint64_t stream_pol = l2_evict_first_policy();
@@ -770,7 +780,10 @@ k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, lo
         for (int q = 0; q < RR; q++) act |= active_rhs<RT>(st, sp.sys, rr0 + q, mask_mode);
         if (!act) continue;
         const gb::SysDev& Sd = sys[sp.sys];
-        const int B = Sd.B, H = Sd.rmax;              // the pass reads rows 0 .. H - 1 of a block
+        const int B = Sd.B;
+        // the rows rb .. rb + H - 1 of a block that this warp reads (all warps: 0 .. rmax - 1)
+        const int rp = SPLIT ? split_rows(Sd.rmax, nparts, RPW) : Sd.rmax;
+        const int rb = SPLIT ? min(wid * rp, Sd.rmax) : 0, H = SPLIT ? min(rp, Sd.rmax - rb) : Sd.rmax;
         const long long vec_off = Sd.vec_off + (long long)rr0 * Sd.D;   // of the plane
         const SysPlan& pl = plan[sp.sys];
         const int cpb = (H + RC - 1) / RC;            // chunks per block
@@ -784,7 +797,7 @@ k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, lo
         // producer cursor: first row of the next chunk, its place in the strip, its block's
         // y vector and y slot
         int pr = 0, py = 0;
-        size_t psrc = 0;
+        size_t psrc = (size_t)rb * row_bytes;
         const YT* ysrc = Yu + vec_off + (long long)j0 * B * RR;
         auto issue = [&]() {                          // lane 0: next chunk (+ its block's y_u with the first)
             const unsigned bytes = (unsigned)min(RC, H - pr) * row_bytes;
@@ -801,7 +814,7 @@ k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, lo
             pstage = (pstage + 1 == S) ? 0 : pstage + 1;
             pr += RC;
             psrc += bytes;
-            if (pr >= H) {   // past the lower half, which is not read
+            if (pr >= H) {   // past the rows that are not read
                 pr = 0;
                 psrc += (size_t)(B - H) * row_bytes;
             }
@@ -822,6 +835,27 @@ k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, lo
             for (int t = 0; t < npre; t++) issue();
         in_flight = npre;
         int issued = npre, cy = 0;
+        // the CTA's sums of the warps' partials v (its lanes ro == 0 hold them), to out; false
+        // once any warp has failed
+        auto combine = [&](auto value, OutT* out) -> bool {
+            OutT* e = exch + (size_t)ebuf * nparts * B * RR;
+            ebuf ^= 1;
+#pragma unroll
+            for (int k = 0; k < CPL; k++)
+#pragma unroll
+                for (int q = 0; q < RR; q++) {
+                    const OutT v = value(k, q);
+                    const int col = cl + LPR * k;
+                    if (ro == 0 && col < B) e[(wid * B + col) * RR + q] = v;
+                }
+            if (__syncthreads_or(failed)) return false;
+            for (int t = threadIdx.x; t < B * RR; t += blockDim.x) {
+                OutT v = e[t];
+                for (int p = 1; p < nparts; p++) v = Pol::add(v, e[p * B * RR + t]);
+                out[t / RR * RT + rr0 + t % RR] = v;
+            }
+            return true;
+        };
         for (int b = 0; b < sp.nb && !failed; b++) {
 #pragma unroll
             for (int k = 0; k < CPL; k++)
@@ -870,7 +904,7 @@ k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, lo
                     const unsigned char* col = stg + (cl >> 1) * MB;
                     auto pm_step = [&](int lr) {
                         const unsigned char* row = col + lr * row_bytes;
-                        step(2 * (row0 + lr) + (cl & 1), [&](int k) {
+                        step(2 * (rb + row0 + lr) + (cl & 1), [&](int k) {
                             return Pol::load(row, row + lay.chunk_cap, LPR / 2 * k * MB, LPR / 2 * k * MB + qoff, sign);
                         });
                     };
@@ -913,35 +947,51 @@ k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, lo
                 cstage = (cstage + 1 == S) ? 0 : cstage + 1;
                 if (cstage == 0) cphase ^= 1u;
             }
-            if (failed) break;
+            if (!SPLIT && failed) break;
             // block done: column partial of block row j
             // column partials by destination: block row j's partials from i < j are
             // contiguous (index j(j-1)/2 + i), so the reduction streams them
             const long long jb = j0 + b;
             OutT* cwp = CW + pl.cw_off + (jb * (jb - 1) / 2 + sp.i) * (long long)B * RT;
+            auto wsum = [&](int k, int q) {
+                OutT v = Pol::out(cw[k][q]);
+#pragma unroll
+                for (int off = LPR; off < 32; off <<= 1) v = Pol::add(v, Pol::shfl(v, off));
+                return v;
+            };
+            if constexpr (SPLIT) {
+                if (!combine(wsum, cwp)) failed = true;
+            } else {
+#pragma unroll
+                for (int k = 0; k < CPL; k++)
+#pragma unroll
+                    for (int q = 0; q < RR; q++) {
+                        const OutT v = wsum(k, q);
+                        const int col = cl + LPR * k;
+                        if (ro == 0 && col < B) cwp[col * RT + rr0 + q] = v;
+                    }
+            }
+        }
+        if (failed) break;
+        OutT* cup = CU + pl.cu_off + (w - pl.strip_base) * (long long)B * RT;
+        auto usum = [&](int k, int q) {
+            OutT v = Pol::out(cu[k][q]);
+#pragma unroll
+            for (int off = LPR; off < 32; off <<= 1) v = Pol::add(v, Pol::shfl(v, off));
+            return v;
+        };
+        if constexpr (SPLIT) {
+            if (!combine(usum, cup)) failed = true;
+        } else {
 #pragma unroll
             for (int k = 0; k < CPL; k++)
 #pragma unroll
                 for (int q = 0; q < RR; q++) {
-                    OutT v = Pol::out(cw[k][q]);
-#pragma unroll
-                    for (int off = LPR; off < 32; off <<= 1) v = Pol::add(v, Pol::shfl(v, off));
+                    const OutT v = usum(k, q);
                     const int col = cl + LPR * k;
-                    if (ro == 0 && col < B) cwp[col * RT + rr0 + q] = v;
+                    if (ro == 0 && col < B) cup[col * RT + rr0 + q] = v;
                 }
         }
-        if (failed) break;
-        OutT* cup = CU + pl.cu_off + (w - pl.strip_base) * (long long)B * RT;
-#pragma unroll
-        for (int k = 0; k < CPL; k++)
-#pragma unroll
-            for (int q = 0; q < RR; q++) {
-                OutT v = Pol::out(cu[k][q]);
-#pragma unroll
-                for (int off = LPR; off < 32; off <<= 1) v = Pol::add(v, Pol::shfl(v, off));
-                const int col = cl + LPR * k;
-                if (ro == 0 && col < B) cup[col * RT + rr0 + q] = v;
-            }
     }
     if (failed) {   // drain: wait (bounded) for every copy this warp still has in flight
         for (int k = 0; k < in_flight; k++) {
@@ -2179,6 +2229,23 @@ constexpr int gemv_steps(int lpr, int cpl, int elem_bytes, int bytes = 6144) {
                                                                 : bytes / ((32 / lpr) * lpr * cpl * elem_bytes);
 }
 
+// Warps that share each of n strips of a complex128 pass, 1 to 4: the time is that of the
+// sub-partition with the most FP64 instructions, of its warps' steps over their rows of a
+// block (RPW rows each; 8 instructions per column and right-hand side, cols in all, and the
+// 2 of P + Q per column) and of the sums over the lanes and warps.
+int split_warps(long long n, int H, int rpw, int cols) {
+    int best = 1;
+    double tbest = 1e300;
+    for (int w = 1; w <= 4; w++) {
+        const int steps = split_rows(H, w, rpw) / rpw;
+        int levels = 0;
+        while ((1 << levels) < rpw) levels++;
+        const double t = std::ceil(double(n * w) / (4.0 * gb::sm_count())) * (steps * cols * 9.0 + cols * 4.0 * levels + 30.0);
+        if (t < 0.96 * tbest) { tbest = t; best = w; }
+    }
+    return best;
+}
+
 template <class Pol, int RR, int RT>
 int launch_pgemv_group(const Plan& P, const DevPlan& D, const StripGroup& grp, const KState* st, int mask,
                        const void* mat_hi, const void* mat_lo, const void* Yu, const void* Yw, void* CU, void* CW,
@@ -2197,23 +2264,32 @@ int launch_pgemv_group(const Plan& P, const DevPlan& D, const StripGroup& grp, c
     const int rpw = 32 / sh.lpr;
     const bool whole = sh.lpr * sh.cpl <= kWholeB + 2;
     const bool fine = Pol::ID == 1 && !whole && grp.end - grp.beg > 8LL * gb::sm_count();
-    const int G = gemv_steps(sh.lpr, sh.cpl, Pol::MB * (Pol::DF ? 2 : 1), fine ? 3072 : 6144);
-    const GemvLayout g = gemv_layout(Bmax, whole ? Bmax / 2 : G * rpw, RR, S, Pol::MB, Pol::DF, sizeof(YT));
     // complex128 passes of few strips per SM: one warp per CTA, so that the strips, all of
     // the time there, spread over the sub-partitions (N = 61, lmax 5: 120 us against 124,
-    // R = 2 205 against 216; no gain for the other passes)
-    const int warps = Pol::ID == 0 && grp.end - grp.beg <= 32LL * gb::sm_count() ? 1 : kGemvWarps, threads = 32 * warps;
-    const size_t smem = (size_t)warps * g.warp_bytes;
-    if (smem > 227 * 1024) return gb_set_error(GB_UNSUPPORTED, "GEMV needs %zu B of shared memory", smem);
+    // R = 2 205 against 216; no gain for the other passes), or, above kWholeB, a CTA's warps
+    // share a strip where that spreads them more evenly (N = 61, lmax 5: 119 -> 107 us, R = 2
+    // 205 -> 190; N = 42, lmax 6 105 -> 76; N = 25, lmax 8 149 -> 94; with 6 KB chunks for it,
+    // fewer CTAs per SM, 107, 197, 82 and 106)
     const long long n = grp.end - grp.beg;
-    // one strip per warp (no persistent loop): CTAs retire after their strips, so
+    const bool single = Pol::ID == 0 && n <= 32LL * gb::sm_count();
+    const int parts = single && !whole ? split_warps(n, Bmax / 2, rpw, sh.cpl * RR) : 1;
+    const int warps = single ? parts : kGemvWarps, threads = 32 * warps;
+    const int G = gemv_steps(sh.lpr, sh.cpl, Pol::MB * (Pol::DF ? 2 : 1), fine || parts > 1 ? 3072 : 6144);
+    const GemvLayout g = gemv_layout(Bmax, whole ? Bmax / 2 : G * rpw, RR, S, Pol::MB, Pol::DF, sizeof(YT), parts > 1);
+    const size_t smem = (size_t)warps * g.warp_bytes + (parts > 1 ? 2 * parts * (size_t)Bmax * RR * sizeof(OutT) : 0);
+    if (smem > 227 * 1024) return gb_set_error(GB_UNSUPPORTED, "GEMV needs %zu B of shared memory", smem);
+    // one strip per warp, or per CTA (no persistent loop): CTAs retire after their strips, so
     // kernels of higher-priority streams are dispatched between them
-    const long long grid = std::max<long long>(1, std::min<long long>((n + warps - 1) / warps, 0x7fffffffLL));
+    const int strips = parts > 1 ? 1 : warps;   // per CTA
+    const long long grid = std::max<long long>(1, std::min<long long>((n + strips - 1) / strips, 0x7fffffffLL));
 #define GB_PG(LPRV, CPLV)                                                                                        \
     if (sh.lpr == LPRV && sh.cpl == CPLV) {                                                                      \
         constexpr int EB = Pol::MB * (Pol::DF ? 2 : 1);                                                          \
-        constexpr int GV = gemv_steps(LPRV, CPLV, EB), GF = Pol::ID == 1 ? gemv_steps(LPRV, CPLV, EB, 3072) : GV; \
+        constexpr int GV = gemv_steps(LPRV, CPLV, EB), G3 = gemv_steps(LPRV, CPLV, EB, 3072);                   \
+        constexpr int GF = Pol::ID == 1 ? G3 : GV;                                                              \
         auto kfn = fine ? k_pgemv<Pol, RR, RT, LPRV, CPLV, GF, S> : k_pgemv<Pol, RR, RT, LPRV, CPLV, GV, S>;     \
+        if constexpr (Pol::ID == 0 && LPRV * CPLV > kWholeB + 2)                                                 \
+            if (parts > 1) kfn = k_pgemv<Pol, RR, RT, LPRV, CPLV, G3, S, true>;                                  \
         if (smem > 48 * 1024)                                                                                    \
             GB_CUDA_TRY(gb::ensure_dynamic_smem(reinterpret_cast<const void*>(kfn), smem));      \
         gb::note_launch();                                                                                       \
