@@ -723,8 +723,15 @@ __host__ __device__ inline int split_rows(int H, int warps, int rpw) {   // rows
     const int r = (H + warps - 1) / warps;
     return (r + rpw - 1) / rpw * rpw;
 }
+// Small blocks' complex64 pass, one right-hand side (small32): two stages and registers for
+// five CTAs per SM (four with three stages), as it waits for latencies rather than bytes
+// (14 warps per SM issued half the time): N = 401, lmax 3 67.9 -> 62.8 us, N = 800 240 ->
+// 229; six CTAs spill (69, 255).
+template <class Pol, int RR, int LPR, int CPL> constexpr bool small32() {
+    return Pol::ID == 1 && RR == 1 && LPR * CPL <= kWholeB + 2;
+}
 template <class Pol, int RR, int RT, int LPR, int CPL, int G, int S, bool SPLIT = false>
-__global__ void __launch_bounds__(kGemvThreads)
+__global__ void __launch_bounds__(kGemvThreads, small32<Pol, RR, LPR, CPL>() ? 5 : 1)
 k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, long long sbeg, long long send,
         const KState* __restrict__ st, int mask_mode, const void* __restrict__ mat_hi, const void* __restrict__ mat_lo,
         const typename Pol::YT* __restrict__ Yu, const typename Pol::YT* __restrict__ Yw,
@@ -2252,7 +2259,6 @@ int launch_pgemv_group(const Plan& P, const DevPlan& D, const StripGroup& grp, c
                        int rr0, int* err, cudaStream_t stream, const Shape* force = nullptr) {
     using YT = typename Pol::YT;
     using OutT = typename Pol::OutT;
-    constexpr int S = 3;   // stages per warp: one being read, two in flight
     const int Bmax = grp.B;
     // the double-float pass keeps the model's shape: launch_df splits the right-hand
     // sides by that shape's width
@@ -2263,6 +2269,7 @@ int launch_pgemv_group(const Plan& P, const DevPlan& D, const StripGroup& grp, c
                             Bmax);
     const int rpw = 32 / sh.lpr;
     const bool whole = sh.lpr * sh.cpl <= kWholeB + 2;
+    const int S = Pol::ID == 1 && RR == 1 && whole ? 2 : 3;   // stages per warp: one being read, the others in flight
     const bool fine = Pol::ID == 1 && !whole && grp.end - grp.beg > 8LL * gb::sm_count();
     // complex128 passes of few strips per SM: one warp per CTA, so that the strips, all of
     // the time there, spread over the sub-partitions (N = 61, lmax 5: 120 us against 124,
@@ -2286,10 +2293,10 @@ int launch_pgemv_group(const Plan& P, const DevPlan& D, const StripGroup& grp, c
     if (sh.lpr == LPRV && sh.cpl == CPLV) {                                                                      \
         constexpr int EB = Pol::MB * (Pol::DF ? 2 : 1);                                                          \
         constexpr int GV = gemv_steps(LPRV, CPLV, EB), G3 = gemv_steps(LPRV, CPLV, EB, 3072);                   \
-        constexpr int GF = Pol::ID == 1 ? G3 : GV;                                                              \
-        auto kfn = fine ? k_pgemv<Pol, RR, RT, LPRV, CPLV, GF, S> : k_pgemv<Pol, RR, RT, LPRV, CPLV, GV, S>;     \
+        constexpr int GF = Pol::ID == 1 ? G3 : GV, SV = small32<Pol, RR, LPRV, CPLV>() ? 2 : 3;                 \
+        auto kfn = fine ? k_pgemv<Pol, RR, RT, LPRV, CPLV, GF, SV> : k_pgemv<Pol, RR, RT, LPRV, CPLV, GV, SV>;     \
         if constexpr (Pol::ID == 0 && LPRV * CPLV > kWholeB + 2)                                                 \
-            if (parts > 1) kfn = k_pgemv<Pol, RR, RT, LPRV, CPLV, G3, S, true>;                                  \
+            if (parts > 1) kfn = k_pgemv<Pol, RR, RT, LPRV, CPLV, G3, SV, true>;                                  \
         if (smem > 48 * 1024)                                                                                    \
             GB_CUDA_TRY(gb::ensure_dynamic_smem(reinterpret_cast<const void*>(kfn), smem));      \
         gb::note_launch();                                                                                       \
