@@ -723,15 +723,19 @@ __host__ __device__ inline int split_rows(int H, int warps, int rpw) {   // rows
     const int r = (H + warps - 1) / warps;
     return (r + rpw - 1) / rpw * rpw;
 }
-// Small blocks' complex64 pass, one right-hand side (small32): two stages and registers for
-// five CTAs per SM (four with three stages), as it waits for latencies rather than bytes
-// (14 warps per SM issued half the time): N = 401, lmax 3 67.9 -> 62.8 us, N = 800 240 ->
-// 229; six CTAs spill (69, 255).
-template <class Pol, int RR, int LPR, int CPL> constexpr bool small32() {
-    return Pol::ID == 1 && RR == 1 && LPR * CPL <= kWholeB + 2;
+// CTAs per SM that the registers are held to, 0: the compiler's choice.  The complex64 pass
+// of small blocks, one right-hand side, and of shapes of 3 columns per lane waits for
+// latencies rather than bytes (small blocks: 14 warps per SM issued half the time); two
+// stages per warp there leave shared memory for these CTAs.  N = 401, lmax 3 67.9 -> 62.8
+// us, N = 800 240 -> 229 (six CTAs spill: 69, 255); N = 200, lmax 4, R = 2 38.3 -> 35.9,
+// R = 1 33.6 -> 33.6; N = 120, lmax 6, R = 2 52.5 -> 47.3, R = 1 45.0 both.
+template <class Pol, int RR, int LPR, int CPL> constexpr int more_ctas() {
+    return Pol::ID != 1 || CPL > 4 || (CPL > 3 && LPR * CPL > kWholeB + 2) ? 0
+           : LPR * CPL <= kWholeB + 2                                    ? (RR == 1 ? 5 : 0)
+                                                                         : (RR == 1 ? 5 : 4);
 }
 template <class Pol, int RR, int RT, int LPR, int CPL, int G, int S, bool SPLIT = false>
-__global__ void __launch_bounds__(kGemvThreads, small32<Pol, RR, LPR, CPL>() ? 5 : 1)
+__global__ void __launch_bounds__(kGemvThreads, S == 2 ? more_ctas<Pol, RR, LPR, CPL>() : 0)
 k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, long long sbeg, long long send,
         const KState* __restrict__ st, int mask_mode, const void* __restrict__ mat_hi, const void* __restrict__ mat_lo,
         const typename Pol::YT* __restrict__ Yu, const typename Pol::YT* __restrict__ Yw,
@@ -2269,8 +2273,10 @@ int launch_pgemv_group(const Plan& P, const DevPlan& D, const StripGroup& grp, c
                             Bmax);
     const int rpw = 32 / sh.lpr;
     const bool whole = sh.lpr * sh.cpl <= kWholeB + 2;
-    const int S = Pol::ID == 1 && RR == 1 && whole ? 2 : 3;   // stages per warp: one being read, the others in flight
     const bool fine = Pol::ID == 1 && !whole && grp.end - grp.beg > 8LL * gb::sm_count();
+    // stages per warp, one being read, the others in flight: two where more_ctas and there
+    // are strips for them
+    const int S = Pol::ID == 1 && (whole ? RR == 1 : fine && sh.cpl <= 3) ? 2 : 3;
     // complex128 passes of few strips per SM: one warp per CTA, so that the strips, all of
     // the time there, spread over the sub-partitions (N = 61, lmax 5: 120 us against 124,
     // R = 2 205 against 216; no gain for the other passes), or, above kWholeB, a CTA's warps
@@ -2293,8 +2299,9 @@ int launch_pgemv_group(const Plan& P, const DevPlan& D, const StripGroup& grp, c
     if (sh.lpr == LPRV && sh.cpl == CPLV) {                                                                      \
         constexpr int EB = Pol::MB * (Pol::DF ? 2 : 1);                                                          \
         constexpr int GV = gemv_steps(LPRV, CPLV, EB), G3 = gemv_steps(LPRV, CPLV, EB, 3072);                   \
-        constexpr int GF = Pol::ID == 1 ? G3 : GV, SV = small32<Pol, RR, LPRV, CPLV>() ? 2 : 3;                 \
-        auto kfn = fine ? k_pgemv<Pol, RR, RT, LPRV, CPLV, GF, SV> : k_pgemv<Pol, RR, RT, LPRV, CPLV, GV, SV>;     \
+        constexpr int GF = Pol::ID == 1 ? G3 : GV, SF = more_ctas<Pol, RR, LPRV, CPLV>() ? 2 : 3;               \
+        constexpr int SV = LPRV * CPLV <= kWholeB + 2 ? SF : 3;                                                  \
+        auto kfn = fine ? k_pgemv<Pol, RR, RT, LPRV, CPLV, GF, SF> : k_pgemv<Pol, RR, RT, LPRV, CPLV, GV, SV>;     \
         if constexpr (Pol::ID == 0 && LPRV * CPLV > kWholeB + 2)                                                 \
             if (parts > 1) kfn = k_pgemv<Pol, RR, RT, LPRV, CPLV, G3, SV, true>;                                  \
         if (smem > 48 * 1024)                                                                                    \
