@@ -42,8 +42,8 @@ WORKLOAD = "random cluster N=200 lmax=4 R=2 (D=9600), n=1.5+0.01i, vacuum, 600 n
 # DRAM bytes (read + write) of one k_pgemv<Pol32> launch on this workload, from one
 # ncu capture (dram__bytes_read.sum + dram__bytes_write.sum); summary and command in
 # profiles/k_pgemv_pol32_cluster_n200_lmax4.txt
-GEMV_TRAFFIC_BYTES = 375_720_448
-GEMV_TRAFFIC_SOURCE = "ncu: dram__bytes_read.sum 367.70 MB + dram__bytes_write.sum 8.02 MB per launch"
+GEMV_TRAFFIC_BYTES = 191_050_240
+GEMV_TRAFFIC_SOURCE = "ncu: dram__bytes_read.sum 184.29 MB + dram__bytes_write.sum 6.76 MB per launch"
 
 
 # ---------------------------------------------------------------- workload --
@@ -272,6 +272,8 @@ def run_gpu(args, rank, world):
     B = 2 * lmax * (lmax + 2)
     mat_bytes_64 = P * B * B * 8
     mat_bytes_128 = P * B * B * 16
+    # a matrix pass reads the upper half of every block
+    pass_bytes_64, pass_bytes_128 = mat_bytes_64 // 2, mat_bytes_128 // 2
     peak, peak_kind = peaks()
 
     # ---- end to end from host buffers through the public batch API
@@ -371,18 +373,18 @@ def run_gpu(args, rank, world):
                         p50_ms=float(np.percentile(per_c, 50)), p99_ms=float(np.percentile(per_c, 99)),
                         results_identical_across_streams=bool(conc_same), gpu_launches=int(launches_conc),
                         note="mixed solves of the same workload on concurrent streams, inputs resident"),
-        roofline=dict(bound="hbm", achieved=mat_bytes_64 / t_gemv64 / 1e9, peak=peak, unit="GB/s",
-                      frac=mat_bytes_64 / t_gemv64 / 1e9 / peak, traffic=GEMV_TRAFFIC_BYTES,
+        roofline=dict(bound="hbm", achieved=pass_bytes_64 / t_gemv64 / 1e9, peak=peak, unit="GB/s",
+                      frac=pass_bytes_64 / t_gemv64 / 1e9 / peak, traffic=GEMV_TRAFFIC_BYTES,
                       traffic_source=GEMV_TRAFFIC_SOURCE,
                       kernel="k_pgemv<Pol32> (packed complex64 matrix pass of the inner BiCGSTAB)",
-                      algorithmic_bytes_per_launch=int(mat_bytes_64),
+                      algorithmic_bytes_per_launch=int(pass_bytes_64),
                       peak_source=peak_kind + " (MEASURED_PEAKS.json hbm_gbs, copy burst)",
                       ms_per_launch=1e3 * t_gemv64),
         operators=dict(
-            c64_fp32=dict(ms=1e3 * t_apply64, matrix_gbs=mat_bytes_64 / t_apply64 / 1e9,
+            c64_fp32=dict(ms=1e3 * t_apply64, matrix_gbs=pass_bytes_64 / t_apply64 / 1e9,
                           gemv_ms=1e3 * t_gemv64),
-            double_float_hi_lo=dict(ms=1e3 * t_applydf, matrix_gbs=2 * mat_bytes_64 / t_applydf / 1e9),
-            c128_fp64=dict(ms=1e3 * t_apply128, matrix_gbs=mat_bytes_128 / t_apply128 / 1e9)),
+            double_float_hi_lo=dict(ms=1e3 * t_applydf, matrix_gbs=2 * pass_bytes_64 / t_applydf / 1e9),
+            c128_fp64=dict(ms=1e3 * t_apply128, matrix_gbs=pass_bytes_128 / t_apply128 / 1e9)),
         assembly=dict(
             kernel="k_assemble (packed pair blocks; mixed writes complex64 hi + lo, FP64 complex128)",
             mixed_ms=1e3 * t_asm["mixed"], fp64_ms=1e3 * t_asm["fp64"], bytes_written=int(mat_bytes_128),
@@ -497,8 +499,8 @@ def run_multi_rhs(args, W, dev, peak):
     err = lambda b: float(np.max(np.abs(cext(b) - c64) / np.abs(c64)))
     P = N * (N - 1) // 2
     B = 2 * lmax * (lmax + 2)
-    tile_bytes = P * 2 * (((B + 7) // 8) * 8) * (((2 * B + 15) // 16) * 16) * 2
-    mat64 = P * B * B * 8
+    tile_bytes = P * 4 * max(16, (B // 2 + 7) // 8 * 8) * ((B + 15) // 16 * 16) * 2
+    mat64 = P * B * B * 4   # the half of every block that a pass reads
     return dict(
         workload=f"{WORKLOAD.split(' R=2')[0]}, R=8 (x/y polarisation at 4 incidence directions)",
         tensor_core=dict(solves_per_s=1.0 / t_tc, source_solves_per_s=R / t_tc, ms_per_step=1e3 * t_tc,

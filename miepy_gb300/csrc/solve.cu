@@ -28,10 +28,11 @@
 // by the copies and the work per block rather than by the multiplications, and the sums
 // stay those of the block itself, to the last bit, so that quantities that cancel (the
 // torque on a lossless sphere) keep their residues.
-// Per pass, before and after: complex64 N = 200, lmax 4, R = 2 66 -> 51 us; N = 97, lmax 8
-// 131 -> 73 us; N = 2000, lmax 3 2.26 -> 1.86 ms; double-float N = 200, lmax 4, R = 2 292
-// -> 172 us, one pair of eight right-hand sides 404 -> 172 us (its own y plane: two CTAs
-// per SM instead of one); complex128 N = 61, lmax 5 155 -> 97 us.
+// Per pass, whole blocks before and now (launch shapes included): complex64 N = 200, lmax 4,
+// R = 2 66 -> 36 us; N = 97, lmax 8 131 -> 77 us; N = 401, lmax 3 79 -> 63 us;
+// double-float N = 200, lmax 4, R = 2 292 -> 167 us, one pair of eight right-hand sides 404
+// -> 190 us (its own y plane: two CTAs per SM instead of one); complex128 N = 61, lmax 5
+// 155 -> 107 us.
 //
 // Three arithmetic policies share the kernel:
 //   Pol64  complex128 matrix, FP64 FMAs (the plain method);
@@ -44,7 +45,7 @@
 //
 // K3a (k_pgemv): warp per strip of consecutive blocks (i, j0..j0+J-1) of one block
 //   row; c_u accumulates across the strip, c_w is written per block.
-// K3b (k_reduce): 8 warps x 32 rows; warps split the partial terms of a row, a
+// K3b (k_reduce_blk): a CTA per particle; groups of threads split the partial terms, a
 //   fixed-order shared-memory sum combines them (deterministic, no atomics),
 //   adds the identity term and emits per-item partial dot products.
 // K4: BiCGSTAB vector updates fused with the dot-product partials, and one-thread-
@@ -2227,8 +2228,8 @@ Shape tuned_shape(int B, int pol, int RR, int RT) {
     return f != g_tuned.end() ? f->second : pick_shape(B);
 }
 
-// Steps per chunk of bytes of matrix for a shape (LPR*CPL columns), with three stages and
-// two y slots per warp.  6 KB chunks (two 4-warp CTAs per SM) where the pass is
+// Steps per chunk of bytes of matrix for a shape (LPR*CPL columns), with three stages (the
+// figures below) and two y slots per warp.  6 KB chunks (two 4-warp CTAs per SM) where the pass is
 // compute-bound (double-float, complex128) or has no more strips than those CTAs have
 // warps, so that the bytes in flight per warp count; else 3 KB (three or four CTAs): the
 // complex64 pass of N = 200, lmax 4 takes 33.9 us against 41.7 (R = 1), 38.9 against 44.8

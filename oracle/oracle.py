@@ -2,7 +2,7 @@
 
 numpy-level access to ``oracle/src/oracle_miepy.cpp``, the C++17 restatement of
 the native module of johnaparker/miepy (``cpp/src/*.cpp``).  It is loaded only by
-the parity tests, by ``__graft_entry__.smoke()`` (as the checker) and by the
+the parity tests, by ``__graft_entry__.smoke()`` (for comparison) and by the
 CPU-baseline leg of ``bench.py``.  The product package ``miepy_gb300`` never
 imports it.
 
