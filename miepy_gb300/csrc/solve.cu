@@ -2868,7 +2868,7 @@ int solve_impl(const Plan& P, int prec, double tol, int maxiter, double inner_to
                            status, iters, resid, stream);
             const int e2 = gb::stage_release(slot, stream);   // the solve has synchronised (or failed)
             if (e2) return e2;
-            if (!mixed || e == GB_OK || e == GB_CUDA_ERROR || e == GB_TIMEOUT) return e;
+            if (e != GB_UNSUPPORTED && (!mixed || e == GB_OK || e == GB_CUDA_ERROR || e == GB_TIMEOUT)) return e;
         }
     }
     DevPlan D;
@@ -3377,9 +3377,11 @@ int gb_solve_dense(int D, int R, const double* T, const double* b, double* x, do
     if (ws_bytes < w.total) return gb_set_error(GB_OVER_BUDGET, "workspace %zu B < required %zu B", ws_bytes, w.total);
     unsigned char* base = static_cast<unsigned char*>(workspace);
     const gb::TeamPlan tp = gb::team_plan(1, D, R, false);
-    if (tp.ok)
-        return team_route(tp, P, nullptr, D, reinterpret_cast<const double2*>(T), nullptr, nullptr, nullptr, b, x, tol, 0.0,
-                          maxiter, base, w, status, iters, resid, s);
+    if (tp.ok) {
+        const int e = team_route(tp, P, nullptr, D, reinterpret_cast<const double2*>(T), nullptr, nullptr, nullptr, b, x,
+                                 tol, 0.0, maxiter, base, w, status, iters, resid, s);
+        if (e != GB_UNSUPPORTED) return e;   // (no room for the team on this device)
+    }
     DevPlan Dp;
     int e = upload_plan(P, base, w, s, Dp);
     if (e) return e;
@@ -3422,9 +3424,11 @@ int gb_solve_dense_noalloc(int D, int R, const double* T, const double* b, doubl
     int e = noalloc_scratch(&base);
     if (e) return e;
     const gb::TeamPlan tp = gb::team_plan(1, D, R, false);
-    if (tp.ok)
-        return team_route(tp, P, nullptr, D, reinterpret_cast<const double2*>(T), nullptr, nullptr, nullptr, b, x, tol, 0.0,
-                          maxiter, base, w, status, iters, resid, s);
+    if (tp.ok) {
+        const int e = team_route(tp, P, nullptr, D, reinterpret_cast<const double2*>(T), nullptr, nullptr, nullptr, b, x,
+                                 tol, 0.0, maxiter, base, w, status, iters, resid, s);
+        if (e != GB_UNSUPPORTED) return e;   // (no room for the team on this device)
+    }
     DevPlan Dp;
     e = upload_plan_pageable(P, base, w, s, Dp);
     if (e) return e;

@@ -480,8 +480,14 @@ int launch_team(const TeamArgs& a, int nsys, size_t smem, cudaStream_t stream) {
         at[0].id = cudaLaunchAttributeCooperative;
         at[0].val.cooperative = 1;
     }
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kfn, a);
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources || e == cudaErrorInvalidClusterSize ||
+        e == cudaErrorInvalidConfiguration) {   // no room for a team (part of a device): the caller's other path
+        (void)cudaGetLastError();
+        return gb_set_error(GB_UNSUPPORTED, "single-launch solve: %s", cudaGetErrorString(e));
+    }
+    GB_CUDA_TRY(e);
     gb::note_launch();
-    GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, kfn, a));
     return GB_OK;
 }
 
