@@ -1429,8 +1429,11 @@ __device__ __forceinline__ void sum_terms(const OutT* __restrict__ p, long long 
 // in order (deterministic),
 // then thread (row, rhs) recombines the +- columns (pm 1: of blocks above kWholeB, 2: in
 // the tensor-core pass's order), applies the sign/permutation of its row, adds the identity term, stores y and contributes to the CTA's partial dot products (modes as k_reduce).
+// R <= 2: registers for three CTAs per SM (two otherwise), so that batches and large clusters
+// take fewer waves: 24 clusters of 40 13.18 -> 13.0 ms, N = 2000 157.8 -> 156.2 ms whole
+// calls; four spill (N = 97, lmax 8 +1%), and R = 8 was 1% slower with three.
 template <typename OutT, typename VT, int R>
-__global__ void __launch_bounds__(kRBThreads)
+__global__ void __launch_bounds__(kRBThreads, R <= 2 ? 3 : 0)
 k_reduce_blk(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items, int nitems,
              const SysPlan* __restrict__ plan, const long long* __restrict__ row_strip, const KState* __restrict__ st,
              int mask_mode, const OutT* __restrict__ CU, const OutT* __restrict__ CW, const VT* __restrict__ x,
