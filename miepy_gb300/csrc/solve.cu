@@ -2818,21 +2818,18 @@ __global__ void k_scale_t(const double2* __restrict__ t, const double2* __restri
 // the error flag and barrier counters in the refinement states' place, the operand
 // vectors and partial dots in the vectors' place; one readback at the end.
 int team_route(const gb::TeamPlan& tp, const Plan& P, const gb::SysDev* dsys, int dense_D, const double2* mat,
-               const float* hi, const float* lo, const double2* tvec, const double* b, double* x, double tol, double verify,
-               int maxiter, unsigned char* base, const WS& w, int* status, int* iters, double* resid, cudaStream_t stream) {
+               const double2* tvec, const double* b, double* x, double tol, int maxiter, unsigned char* base, const WS& w,
+               int* status, int* iters, double* resid, cudaStream_t stream) {
     KState* st = reinterpret_cast<KState*>(base + w.off_state);
     DevPlan D{};
     D.err = reinterpret_cast<int*>(base + w.off_ostate);
-    int e = gb::team_solve(tp, P.nsys, dsys, dense_D, P.R, mat, reinterpret_cast<const float2*>(hi),
-                           reinterpret_cast<const float2*>(lo), tvec, reinterpret_cast<const double2*>(b),
+    int e = gb::team_solve(tp, P.nsys, dsys, dense_D, P.R, mat, tvec, reinterpret_cast<const double2*>(b),
                            reinterpret_cast<double2*>(x), st, D.err, reinterpret_cast<double2*>(base + w.off_vec),
-                           P.total_vec, tol, verify, maxiter, stream);
+                           P.total_vec, tol, maxiter, stream);
     if (e) return e;
     std::vector<KState> h;
     e = read_state(D, st, P.nsys * P.R, h, stream);
     if (e) return e;
-    if (verify > 0)
-        for (KState& k : h) k.iters = 1;   // refinement passes
     return finish_status(h.data(), P.nsys * P.R, status, iters, resid);
 }
 
@@ -2848,30 +2845,23 @@ int solve_impl(const Plan& P, int prec, double tol, int maxiter, double inner_to
                cudaStream_t stream, const void* mat_tc = nullptr, const double* pdiag = nullptr) {
     const int pol32 = mat_tc ? 3 : 1;
     const void* m32 = mat_tc ? mat_tc : static_cast<const void*>(mat64);
-    // small systems in one launch, in FP64.  The mixed method's too: it is all launches
-    // there, its matrix (hi + lo) serves FP64 as it is, and the solve goes on to 1e-3 tol,
-    // about as far below tol as the last FP32 correction ends, with the true residual held
-    // to tol; whatever does not end well takes the refinement below instead.  Solves to
-    // 1e-10: N = 5, lmax 2 505 -> 155 us, N = 26, lmax 3 610 -> 334, N = 14, lmax 6 (D =
-    // 1344, about the largest that fits the SMs) 897 -> 669, 150 clusters of N = 5 916 -> 495
-    if ((prec == GB_PREC_FP64 || prec == GB_PREC_MIXED) && !mat_tc && !pdiag && !P.tmat) {
+    // small FP64 systems in one launch (the mixed method's end where its refinement does: its
+    // results are its own, also where they cancel)
+    if (prec == GB_PREC_FP64 && !pdiag && !P.tmat) {
         int Dmax = 0;
         for (const gb::SysDev& d : P.sd) Dmax = std::max(Dmax, d.D);
         const gb::TeamPlan tp = gb::team_plan(P.nsys, Dmax, R, true);
-        const bool mixed = prec == GB_PREC_MIXED;
         if (tp.ok) {
             void* dsys = nullptr;
             int slot = 0;
             int e = gb::stage_acquire(P.sd.data(), sizeof(gb::SysDev) * P.nsys, stream, &dsys, &slot);
             if (e) return e;
-            e = team_route(tp, P, static_cast<const gb::SysDev*>(dsys), 0,
-                           mixed ? nullptr : reinterpret_cast<const double2*>(mat128), mat64, mat64lo,
-                           reinterpret_cast<const double2*>(tvec), b, x,
-                           mixed ? std::max(1e-3 * tol, std::min(tol, 1e-13)) : tol, mixed ? tol : 0.0, maxiter, base, w,
-                           status, iters, resid, stream);
+            const double2* t2 = reinterpret_cast<const double2*>(tvec);
+            e = team_route(tp, P, static_cast<const gb::SysDev*>(dsys), 0, reinterpret_cast<const double2*>(mat128), t2, b,
+                           x, tol, maxiter, base, w, status, iters, resid, stream);
             const int e2 = gb::stage_release(slot, stream);   // the solve has synchronised (or failed)
             if (e2) return e2;
-            if (e != GB_UNSUPPORTED && (!mixed || e == GB_OK || e == GB_CUDA_ERROR || e == GB_TIMEOUT)) return e;
+            if (e != GB_UNSUPPORTED) return e;   // (no room for the team on this device)
         }
     }
     DevPlan D;
@@ -3381,8 +3371,8 @@ int gb_solve_dense(int D, int R, const double* T, const double* b, double* x, do
     unsigned char* base = static_cast<unsigned char*>(workspace);
     const gb::TeamPlan tp = gb::team_plan(1, D, R, false);
     if (tp.ok) {
-        const int e = team_route(tp, P, nullptr, D, reinterpret_cast<const double2*>(T), nullptr, nullptr, nullptr, b, x,
-                                 tol, 0.0, maxiter, base, w, status, iters, resid, s);
+        const int e = team_route(tp, P, nullptr, D, reinterpret_cast<const double2*>(T), nullptr, b, x, tol, maxiter, base,
+                                 w, status, iters, resid, s);
         if (e != GB_UNSUPPORTED) return e;   // (no room for the team on this device)
     }
     DevPlan Dp;
@@ -3428,8 +3418,8 @@ int gb_solve_dense_noalloc(int D, int R, const double* T, const double* b, doubl
     if (e) return e;
     const gb::TeamPlan tp = gb::team_plan(1, D, R, false);
     if (tp.ok) {
-        const int e = team_route(tp, P, nullptr, D, reinterpret_cast<const double2*>(T), nullptr, nullptr, nullptr, b, x,
-                                 tol, 0.0, maxiter, base, w, status, iters, resid, s);
+        const int e = team_route(tp, P, nullptr, D, reinterpret_cast<const double2*>(T), nullptr, b, x, tol, maxiter, base,
+                                 w, status, iters, resid, s);
         if (e != GB_UNSUPPORTED) return e;   // (no room for the team on this device)
     }
     DevPlan Dp;

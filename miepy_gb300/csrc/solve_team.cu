@@ -59,7 +59,6 @@ constexpr int kTeamMaxD = 4000;
 struct TeamArgs {
     const gb::SysDev* sys;      // packed: [nsys]
     const double2* mat;         // packed blocks, or the dense matrix
-    const float2 *hi, *lo;      // packed blocks as hi + lo (mat null)
     const double2* tvec;        // packed: Mie factors
     const double2* b;
     double2* x;
@@ -69,7 +68,6 @@ struct TeamArgs {
     double2 *g1, *g2;           // operand vectors, at the clusters' vec offsets
     double* part;               // [nsys][2 buffers][3 R][G]
     double tol;
-    double verify;              // > 0: the true residual must meet this tolerance at the end
     int maxiter, D, G, resident, CP;   // D: the dense system; CP: column parts of a product
 };
 
@@ -103,14 +101,9 @@ enum { STATE_RUNNING = -1 };
 __device__ __forceinline__ bool finite1(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
 
 // Eigen's BiCGSTAB scalars, the phases of the launch-per-step solver.  Phase 0 starts
-// from |b|^2, phase 4 ends a restart (r0 = r = b - A x; the first one resets the count),
-// phase 5 holds a converged solution's true |r|^2 to tol: one thread per right-hand side.
+// from |b|^2, phase 4 ends a restart (r0 = r = b - A x; the first one resets the count):
+// one thread per right-hand side.
 __device__ void team_scalars_rare(KState& k, int phase, double d0, double tol, int maxiter) {
-    if (phase == 5) {
-        k.rsq = d0;
-        if (k.status == GB_OK && !(d0 <= tol * tol * k.bsq)) k.status = GB_NOT_CONVERGED;
-        return;
-    }
     if (phase == 0) {
         k.bsq = k.r0sq = k.rsq = d0;
         k.tol2 = tol * tol * d0;
@@ -235,13 +228,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team_bicgstab(const TeamArg
             double2 v = make_double2(0.0, 0.0);
             if (i != j) {   // T[i, j] = A_ij, T[j, i] = S A_ij S for i < j (times t_j, in the operand)
                 const long long lo = min(i, j), hi = max(i, j), p = pair_start(lo, N) + (hi - lo - 1);
-                const long long at = S.mat_off + p * (long long)B * B + (long long)r * B + cc;
-                if (a.mat) {
-                    v = __ldg(a.mat + at);
-                } else {
-                    const float2 h = __ldg(a.hi + at), l = __ldg(a.lo + at);
-                    v = make_double2((double)h.x + (double)l.x, (double)h.y + (double)l.y);
-                }
+                v = __ldg(a.mat + S.mat_off + p * (long long)B * B + (long long)r * B + cc);
                 if (i > j) {
                     const unsigned s = ((unsigned)(__ldg(S.rowinfo + r) ^ __ldg(S.rowinfo + cc)) >> 30) & 1u;
                     v = make_double2(flipd(v.x, s), flipd(v.y, s));
@@ -372,8 +359,8 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team_bicgstab(const TeamArg
             if (lane == 0) tot[wid] = s;
         }
         __syncthreads();
-        if (phase == 0 || phase >= 4) {
-            if (tid < R) team_scalars_rare(ks[tid], phase, tot[3 * tid], phase == 5 ? a.verify : a.tol, a.maxiter);
+        if (phase == 0 || phase == 4) {
+            if (tid < R) team_scalars_rare(ks[tid], phase, tot[3 * tid], a.tol, a.maxiter);
         } else if (wid == 0) {
             team_scalars<R>(ks, phase, tot, lane);
         }
@@ -445,13 +432,6 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team_bicgstab(const TeamArg
             }
         }
         if (!(ok = dots(true, true, r, rs, 3))) break;
-    }
-    if (ok && a.verify > 0.0) {
-        publish(g1, x);
-        if ((ok = team_barrier())) {
-            const double y = product(a.g1);
-            dots(true, false, bv - (x + y), 0.0, 5);
-        }
     }
     if (own && kind == 0) reinterpret_cast<double*>(a.x)[ge] = x;
     if (member == 0 && tid < R) a.st[sidx * R + tid] = ks[tid];
@@ -553,15 +533,12 @@ TeamPlan team_plan(int nsys, int Dmax, int R, bool packed) {
     return best;
 }
 
-int team_solve(const TeamPlan& t, int nsys, const SysDev* sys, int D, int R, const double2* mat, const float2* hi,
-               const float2* lo, const double2* tvec, const double2* b, double2* x, KState* st, int* err_cnt,
-               double2* vectors, long long total_vec, double tol, double verify, int maxiter, cudaStream_t stream) {
+int team_solve(const TeamPlan& t, int nsys, const SysDev* sys, int D, int R, const double2* mat, const double2* tvec,
+               const double2* b, double2* x, KState* st, int* err_cnt, double2* vectors, long long total_vec, double tol,
+               int maxiter, cudaStream_t stream) {
     TeamArgs a{};
     a.sys = sys;
     a.mat = mat;
-    a.hi = hi;
-    a.lo = lo;
-    a.verify = verify;
     a.tvec = tvec;
     a.b = b;
     a.x = x;

@@ -20,13 +20,11 @@ struct TeamPlan {
 
 TeamPlan team_plan(int nsys, int Dmax, int R, bool packed);
 
-// Solves nsys systems (sys: packed operator, its blocks in mat or as hi + lo; null: one
-// dense D x D matrix) from x = 0 to tol; verify > 0: the true residual is held to that
-// tolerance and reported.  err_cnt: nsys + 1 ints; vectors: at least 2 total_vec +
-// 3 nsys R G complex values; the states of every (system, right-hand side) go to st.
-// Asynchronous.
-int team_solve(const TeamPlan& t, int nsys, const SysDev* sys, int D, int R, const double2* mat, const float2* hi,
-               const float2* lo, const double2* tvec, const double2* b, double2* x, KState* st, int* err_cnt,
-               double2* vectors, long long total_vec, double tol, double verify, int maxiter, cudaStream_t stream);
+// Solves nsys systems (sys: packed operator; null: one dense D x D matrix) from x = 0.
+// err_cnt: nsys + 1 ints; vectors: at least 2 total_vec + 3 nsys R G complex values; the
+// states of every (system, right-hand side) go to st.  Asynchronous.
+int team_solve(const TeamPlan& t, int nsys, const SysDev* sys, int D, int R, const double2* mat, const double2* tvec,
+               const double2* b, double2* x, KState* st, int* err_cnt, double2* vectors, long long total_vec, double tol,
+               int maxiter, cudaStream_t stream);
 
 }   // namespace gb

@@ -108,8 +108,8 @@ def test_packed_ragged_batches(R):
 @pytest.mark.parametrize("shapes", [[(2, 1)], [(5, 2)], [(3, 7)], [(26, 3)], [(14, 6)], [(15, 6)], [(5, 2), (7, 1), (2, 4)],
                                     [(5, 2)] * 152, [(5, 2)] * 153])
 def test_small_mixed_solves(shapes, R):
-    """The mixed method's small systems and batches, at and past the limits of the
-    single-launch solve: the true residual (double-float product) meets the tolerance."""
+    """The mixed method's small systems and batches: the true residual (double-float
+    product) meets the tolerance."""
     from miepy_gb300.engine import ClusterBatch
     rng = np.random.default_rng(11)
     specs = []
