@@ -246,6 +246,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team_bicgstab(const TeamArg
     // bounded wait has expired.
     auto team_barrier = [&]() -> bool {
         if (CLUSTER) {
+            __syncwarp();   // the aligned barrier takes whole warps: callers come out of divergent stores
             asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
             return true;
         }

@@ -1,0 +1,66 @@
+"""Which solver ran: the single-launch BiCGSTAB is one launch, the launch-per-step one many.
+Both team forms at sizes whose last CTA and last warp are partly filled (stores by some of
+a warp's lanes directly before the team's barrier), and the limits of the plan."""
+
+import numpy as np
+import pytest
+
+from miepy_gb300 import _native as nat
+
+pytestmark = pytest.mark.gpu
+
+
+def _dense(D, R, seed=0):
+    import torch
+
+    from miepy_gb300.engine import current_stream
+    L, dev = nat.lib(), torch.device("cuda", 0)
+    g = torch.Generator(device="cuda").manual_seed(D * 2 + R + seed)
+    T = torch.randn(D, D, dtype=torch.complex128, device=dev, generator=g) * (0.4 / D ** 0.5)
+    b = torch.randn(D, R, dtype=torch.complex128, device=dev, generator=g)
+    x = torch.empty_like(b)
+    ws = torch.empty(L.gb_solve_dense_workspace_size(D, R), dtype=torch.uint8, device=dev)
+    st, it, rs = np.zeros(R, np.int32), np.zeros(R, np.int32), np.zeros(R)
+    n0 = L.gb_launch_count()
+    rc = L.gb_solve_dense(D, R, nat.ptr(T), nat.ptr(b), nat.ptr(x), 1e-12, 1000, nat.ptr(ws), ws.numel(), st.ctypes.data,
+                          it.ctypes.data, rs.ctypes.data, current_stream(dev))
+    n = L.gb_launch_count() - n0
+    assert rc == nat.GB_OK and np.all(st == 0)
+    res = ((b - x - T @ x).norm(dim=0) / b.norm(dim=0)).cpu().numpy()
+    assert np.all(res < 2e-12), res   # the recurrence's 1e-12 and the rounding of ~30 products
+    return n
+
+
+@pytest.mark.parametrize("R", [1, 2])
+@pytest.mark.parametrize("D", [1, 3, 7, 62, 130, 501, 999, 1301, 2999, 4000])
+def test_dense_systems_take_one_launch(D, R):
+    assert _dense(D, R) == 1
+
+
+def test_larger_dense_systems_take_the_launch_per_step_solver():
+    assert _dense(4001, 1) > 1
+
+
+@pytest.mark.parametrize("n,single", [(1, True), (19, True), (150, True), (152, True), (304, True), (305, False)])
+def test_fp64_batches(n, single):
+    """Batches of one-launch systems up to two CTAs per SM (152 SMs; N = 5, lmax 2: two CTAs
+    per system up to 152 of them) and beyond, against the packed operator's product."""
+    from miepy_gb300.engine import ClusterBatch
+    if nat.lib().gb_device_sm_count() != 152:
+        pytest.skip("batch limits of 152 SMs")
+    rng = np.random.default_rng(5)
+    N, L = (5, 2) if n <= 152 else (2, 1)
+    specs = []
+    for _ in range(n):
+        pos = np.array([(i % 2, i // 2 % 2, i // 4) for i in range(N)], float) * 3e-7 + rng.uniform(-2e-8, 2e-8, (N, 3))
+        mie = (rng.normal(size=(N, 2, L)) + 1j * rng.normal(size=(N, 2, L))) * 0.1 ** np.arange(1, L + 1)
+        p = rng.normal(size=(N, 2, L * (L + 2))) + 1j * rng.normal(size=(N, 2, L * (L + 2)))
+        specs.append(dict(position=pos, mie_scat=mie, k=1.05e7, p_src=p))
+    b = ClusterBatch(specs, R=1, precision="fp64").assemble()
+    n0 = nat.lib().gb_launch_count()
+    b.solve(tol=1e-11)
+    launches = nat.lib().gb_launch_count() - n0
+    assert (launches == 1) == single, launches
+    d = b.b - b.apply(b.x)
+    for s in range(n):
+        assert float(b.cluster_view(s, d).norm() / b.cluster_view(s, b.b).norm()) < 2e-11
