@@ -929,9 +929,13 @@ k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, lo
                             if (g * RPW + ro < nrows) pm_step(g * RPW + ro);
                     }
                 } else {   // the block's rows: the upper ones, then row r + rmax as row r with its halves exchanged
-                    constexpr int NS = (kWholeB / 2 + RPW - 1) / RPW;   // steps over the rows of one half
+                    // Straight-line steps, except in double-float: its eight steps of up to 16
+                    // products are more than the instruction cache holds (N = 600, lmax 3, R = 2
+                    // 1668 -> 1306 us a product with the loops kept, 1409 with whole blocks).
+                    constexpr int NS = (LPR * CPL / 2 + RPW - 1) / RPW;   // steps over the rows of one half
+                    constexpr int UNROLL = DF ? 1 : NS;
                     const unsigned char* col = stg + cl * MB;
-#pragma unroll
+#pragma unroll UNROLL
                     for (int g = 0; g < NS; g++) {
                         const int r = ro + g * RPW;
                         if (r < H) {
@@ -944,7 +948,7 @@ k_pgemv(const gb::SysDev* __restrict__ sys, const Strip* __restrict__ strips, lo
 #pragma unroll
                     for (int k = 0; k < CPL; k++)
                         swap[k] = LPR * k * MB + (cl + LPR * k < H ? (int)qoff : -(int)qoff);
-#pragma unroll
+#pragma unroll UNROLL
                     for (int g = 0; g < NS; g++) {
                         const int r = low + g * RPW;
                         if (r < H) {
@@ -2303,7 +2307,7 @@ int launch_pgemv_group(const Plan& P, const DevPlan& D, const StripGroup& grp, c
     if (sh.lpr == LPRV && sh.cpl == CPLV) {                                                                      \
         constexpr int EB = Pol::MB * (Pol::DF ? 2 : 1);                                                          \
         constexpr int GV = gemv_steps(LPRV, CPLV, EB), G3 = gemv_steps(LPRV, CPLV, EB, 3072);                   \
-        constexpr int GF = Pol::ID == 1 ? G3 : GV, SF = more_ctas<Pol, RR, LPRV, CPLV>() ? 2 : 3;               \
+        constexpr int GF = Pol::ID == 1 && LPRV * CPLV > kWholeB + 2 ? G3 : GV, SF = more_ctas<Pol, RR, LPRV, CPLV>() ? 2 : 3;               \
         constexpr int SV = LPRV * CPLV <= kWholeB + 2 ? SF : 3;                                                  \
         auto kfn = fine ? k_pgemv<Pol, RR, RT, LPRV, CPLV, GF, SF> : k_pgemv<Pol, RR, RT, LPRV, CPLV, GV, SV>;     \
         if constexpr (Pol::ID == 0 && LPRV * CPLV > kWholeB + 2)                                                 \
