@@ -2218,6 +2218,7 @@ Shape pick_shape(int Bmax) {
 // block by no more than that padding (the model's shapes overshoot by at most
 // 10 elements of 16 B).
 constexpr int kGemvPad = 256;
+constexpr size_t kSmemPerSM = 228 * 1024;   // of which every resident CTA takes 1 KB besides its own
 inline bool shape_fits(const Shape& c, int B, int elem_bytes) {
     // (small blocks and the others have shapes of their own)
     return c.lpr * c.cpl >= B && (c.lpr * c.cpl - B) * elem_bytes <= kGemvPad &&
@@ -2297,12 +2298,21 @@ int launch_pgemv_group(const Plan& P, const DevPlan& D, const StripGroup& grp, c
     const int warps = single ? parts : kGemvWarps, threads = 32 * warps;
     const int G = gemv_steps(sh.lpr, sh.cpl, Pol::MB * (Pol::DF ? 2 : 1), fine || parts > 1 ? 3072 : 6144);
     const GemvLayout g = gemv_layout(Bmax, whole ? Bmax / 2 : G * rpw, RR, S, Pol::MB, Pol::DF, sizeof(YT), parts > 1);
-    const size_t smem = (size_t)warps * g.warp_bytes + (parts > 1 ? 2 * parts * (size_t)Bmax * RR * sizeof(OutT) : 0);
+    size_t smem = (size_t)warps * g.warp_bytes + (parts > 1 ? 2 * parts * (size_t)Bmax * RR * sizeof(OutT) : 0);
     if (smem > 227 * 1024) return gb_set_error(GB_UNSUPPORTED, "GEMV needs %zu B of shared memory", smem);
     // one strip per warp, or per CTA (no persistent loop): CTAs retire after their strips, so
     // kernels of higher-priority streams are dispatched between them
     const int strips = parts > 1 ? 1 : warps;   // per CTA
     const long long grid = std::max<long long>(1, std::min<long long>((n + strips - 1) / strips, 0x7fffffffLL));
+    // ... and shared memory for no more CTAs per SM than an even spread of them needs: with room
+    // for more, the CTAs that start while the preceding kernel still runs pile up on some SMs,
+    // whose sub-partitions then have a strip more than the others (products of N = 30, lmax 3,
+    // R = 8 124 -> 102 us; N = 60, lmax 2, R = 2 31.3 -> 28.0; N = 25, lmax 8 115 -> 93)
+    if (Pol::ID == 0) {
+        const long long per = (grid + gb::sm_count() - 1) / gb::sm_count();
+        const size_t share = (kSmemPerSM / (size_t)(per + 1) - 1024) / 128 * 128 + 128;   // too much for per + 1
+        if (per <= 32 && share > smem && share <= 227 * 1024) smem = share;
+    }
 #define GB_PG(LPRV, CPLV)                                                                                        \
     if (sh.lpr == LPRV && sh.cpl == CPLV) {                                                                      \
         constexpr int EB = Pol::MB * (Pol::DF ? 2 : 1);                                                          \
