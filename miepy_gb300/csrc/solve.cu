@@ -1433,11 +1433,14 @@ __device__ __forceinline__ void sum_terms(const OutT* __restrict__ p, long long 
 // in order (deterministic),
 // then thread (row, rhs) recombines the +- columns (pm 1: of blocks above kWholeB, 2: in
 // the tensor-core pass's order), applies the sign/permutation of its row, adds the identity term, stores y and contributes to the CTA's partial dot products (modes as k_reduce).
-// R <= 2: registers for three CTAs per SM (two otherwise), so that batches and large clusters
-// take fewer waves: 24 clusters of 40 13.18 -> 13.0 ms, N = 2000 157.8 -> 156.2 ms whole
-// calls; four spill (N = 97, lmax 8 +1%), and R = 8 was 1% slower with three.
-template <typename OutT, typename VT, int R>
-__global__ void __launch_bounds__(kRBThreads, R <= 2 ? 3 : 0)
+// CTAS: registers for so many CTAs per SM (0: the compiler's choice, two).  Three where
+// there are more than two CTAs per SM and R <= 2, so that batches and large clusters take
+// fewer waves: 24 clusters of 40 13.18 -> 13.0 ms, N = 2000 157.8 -> 156.2 ms whole calls;
+// four spill (N = 97, lmax 8 +1%), and R = 8 was 1% slower with three.  Fewer CTAs are
+// quicker each with more loads in flight (products of N = 60, lmax 2, R = 2 in FP32 9.9 ->
+// 9.1 us, of N = 120, lmax 3 in FP64 130.2 -> 127.4).
+template <typename OutT, typename VT, int R, int CTAS>
+__global__ void __launch_bounds__(kRBThreads, CTAS)
 k_reduce_blk(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items, int nitems,
              const SysPlan* __restrict__ plan, const long long* __restrict__ row_strip, const KState* __restrict__ st,
              int mask_mode, const OutT* __restrict__ CU, const OutT* __restrict__ CW, const VT* __restrict__ x,
@@ -2447,7 +2450,10 @@ int launch_apply(const Plan& P, const DevPlan& D, const WS& w, unsigned char* ba
     auto reduce = [&](auto out, int pm) -> int {
         using OutT = decltype(out);
         gb::note_launch();
-        GB_CUDA_TRY(launch_pdl(k_reduce_blk<OutT, VT, R>, dim3((unsigned)P.nr), dim3(kRBThreads), 0, stream, D.sys,
+        auto kfn = k_reduce_blk<OutT, VT, R, 0>;
+        if constexpr (R <= 2)
+            if (P.nr > 2 * gb::sm_count()) kfn = k_reduce_blk<OutT, VT, R, 3>;
+        GB_CUDA_TRY(launch_pdl(kfn, dim3((unsigned)P.nr), dim3(kRBThreads), 0, stream, D.sys,
                                D.ritems, P.nr, D.sp, pm == 2 ? D.tc_rows : D.row_strip, st, mask, reinterpret_cast<const OutT*>(CU),
                                reinterpret_cast<const OutT*>(CW), xin, yout, mode, aux, b128, dots, fz, xscale, pm));
         return GB_OK;
