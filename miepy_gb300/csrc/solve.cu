@@ -437,10 +437,13 @@ __device__ __forceinline__ C updated_x(const YUpd<VT>& up, bool update, const KS
     return to_c<C>(q);
 }
 
-// One thread per (row of the first polarisation, rhs), for the rows of both; x is [D][R]
-// interleaved (element (row, rr) at vec_off + row*R + rr).  blockDim = kVRows / 2 * R.
+// One thread per (row of the first polarisation, rhs), for the rows of both; small blocks
+// with R <= 2, which combine no rows, one per (row, rhs) (half the chain of FP64 operations
+// per thread: products of N = 60, lmax 2 19.3 -> 18.2 us, R = 2 in FP32 9.1 -> 8.2); x is
+// [D][R] interleaved (element (row, rr) at vec_off + row*R + rr).
+__host__ __device__ constexpr int yprep_threads(int R) { return R <= 2 ? kVRows * R : kVRows / 2 * R; }
 template <int YK, typename VT, int R>
-__global__ void __launch_bounds__(kVRows / 2 * R)
+__global__ void __launch_bounds__(yprep_threads(R))
 k_yprep(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items, int nitems, const KState* __restrict__ st,
         int mask_mode, const double2* __restrict__ tvec, const VT* __restrict__ x, typename YType<YK>::t* __restrict__ Yu,
         typename YType<YK>::t* __restrict__ Yw, YUpd<VT> up, int pl) {
@@ -452,15 +455,35 @@ k_yprep(const gb::SysDev* __restrict__ sys, const Item* __restrict__ items, int 
     // prologue on plan data and the Mie vector (constant during a solve)
     const Item I = items[it];
     const gb::SysDev S = sys[I.sys];
+    using C = typename Arith<VT>::C;
+    using T = typename Arith<VT>::T;
     const int hr = threadIdx.x / R, rr = threadIdx.x - hr * R;
+    if constexpr (R <= 2) {
+        if (S.B <= kWholeB) {
+            const bool row_ok = hr < I.nr;
+            const int row = I.r0 + (row_ok ? hr : 0), part = row / S.B, r = row - part * S.B;
+            const int info = __ldg(S.rowinfo + r), rho = info & ((1 << 29) - 1);
+            const unsigned eneg = (info >> 29) & 1, sneg = (info >> 30) & 1;
+            const long long src = (long long)part * S.B + rho;
+            const C t = to_c<C>(tvec[S.t_off + src]);
+            pdl_wait();
+            pdl_trigger();
+            if (!row_ok || !any_active<R>(st, I.sys, mask_mode)) return;
+            const bool update = up.kind != 0 && active_rhs<R>(st, I.sys, rr, 0);
+            const long long es = S.vec_off + src * R + rr;
+            const C z = cflip(tmul(t, updated_x<C, T>(up, update, st, I.sys * R + rr, x, es)), eneg);
+            const long long o = S.vec_off + (long long)(rr / pl) * pl * S.D + (long long)row * pl + rr % pl;
+            Yu[o] = make_y<YK>(z);
+            Yw[o] = make_y<YK>(cflip(z, sneg));
+            return;
+        }
+    }
     const bool row_ok = 2 * hr < I.nr;
     const int h = I.r0 / 2 + (row_ok ? hr : 0);
     const int part = h / S.rmax, r = h - part * S.rmax;
     const int info = __ldg(S.rowinfo + r);   // of (0, r); the other polarisation's signs are opposite
     const int rho = info & ((1 << 29) - 1);
     const unsigned eneg = (info >> 29) & 1, sneg = (info >> 30) & 1;
-    using C = typename Arith<VT>::C;
-    using T = typename Arith<VT>::T;
     const long long src = (long long)part * S.B + rho;
     const C t0 = to_c<C>(tvec[S.t_off + src]), t1 = to_c<C>(tvec[S.t_off + src + S.rmax]);
     pdl_wait();
@@ -2443,7 +2466,7 @@ int launch_apply(const Plan& P, const DevPlan& D, const WS& w, unsigned char* ba
                                    reinterpret_cast<YT*>(Yw), up, pl));
             return GB_OK;
         }
-        GB_CUDA_TRY(launch_pdl(k_yprep<YK, VT, R>, dim3(vb), dim3(kVRows / 2 * R), 0, stream, D.sys, D.vitems, P.nv, st,
+        GB_CUDA_TRY(launch_pdl(k_yprep<YK, VT, R>, dim3(vb), dim3(yprep_threads(R)), 0, stream, D.sys, D.vitems, P.nv, st,
                                mask, tvec, xin, reinterpret_cast<YT*>(Yu), reinterpret_cast<YT*>(Yw), up, pl));
         return GB_OK;
     };
