@@ -292,7 +292,10 @@ int gb_apply_repeat_tc(int nsys, const gb_system* sys, int R, const void* mat_tc
  * makes every consumer wait expire at once (a test of that path); cycles < 0
  * restores the default (4e8 cycles, about 0.2 s).  The limit is per device (the
  * current one), read by every later launch, graph replays included.  previous, if
- * not null, receives the limit before the call. */
+ * not null, receives the limit before the call.
+ * The barriers of single-launch solves (small FP64 systems) wait ten times as long.
+ * One that expires, because other streams' kernels kept part of the launch waiting,
+ * is no error: the call solves the systems again with a launch per step. */
 int gb_set_gemv_wait_limit(long long cycles, long long* previous);
 
 /* -------------------------------------------------------------- epilogue --

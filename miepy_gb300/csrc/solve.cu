@@ -2859,7 +2859,9 @@ __global__ void k_scale_t(const double2* __restrict__ t, const double2* __restri
 
 // The single-launch solve (solve_team.cu) in the solver's workspace: states at off_state,
 // the error flag and barrier counters in the refinement states' place, the operand
-// vectors and partial dots in the vectors' place; one readback at the end.
+// vectors and partial dots in the vectors' place; one readback at the end.  GB_UNSUPPORTED
+// where the device has no room for the team or its barrier's wait ran out: the caller's
+// launch-per-step solver takes the systems then.
 int team_route(const gb::TeamPlan& tp, const Plan& P, const gb::SysDev* dsys, int dense_D, const double2* mat,
                const double2* tvec, const double* b, double* x, double tol, int maxiter, unsigned char* base, const WS& w,
                int* status, int* iters, double* resid, cudaStream_t stream) {
@@ -2872,6 +2874,8 @@ int team_route(const gb::TeamPlan& tp, const Plan& P, const gb::SysDev* dsys, in
     if (e) return e;
     std::vector<KState> h;
     e = read_state(D, st, P.nsys * P.R, h, stream);
+    if (e == GB_TIMEOUT)
+        return gb_set_error(GB_UNSUPPORTED, "single-launch solve: a team barrier did not complete within its wait limit");
     if (e) return e;
     return finish_status(h.data(), P.nsys * P.R, status, iters, resid);
 }
@@ -2904,7 +2908,7 @@ int solve_impl(const Plan& P, int prec, double tol, int maxiter, double inner_to
                            x, tol, maxiter, base, w, status, iters, resid, stream);
             const int e2 = gb::stage_release(slot, stream);   // the solve has synchronised (or failed)
             if (e2) return e2;
-            if (e != GB_UNSUPPORTED) return e;   // (no room for the team on this device)
+            if (e != GB_UNSUPPORTED) return e;
         }
     }
     DevPlan D;
@@ -3389,7 +3393,8 @@ int gb_set_gemv_wait_limit(long long cycles, long long* previous) {
     GB_CUDA_TRY(cudaMemcpyFromSymbol(&old, g_gemv_wait_cycles, sizeof(old)));
     const long long v = cycles < 0 ? kWaitCycles : cycles;
     GB_CUDA_TRY(cudaMemcpyToSymbol(g_gemv_wait_cycles, &v, sizeof(v)));
-    const int e = gb::set_wait_limit_multi(v);   // the copy of the R = 4 / 8 unit
+    int e = gb::set_wait_limit_multi(v);   // the copy of the R = 4 / 8 unit
+    if (!e) e = gb::set_team_wait_limit(cycles);
     if (e) return e;
     if (previous) *previous = old;
     return GB_OK;
@@ -3416,7 +3421,7 @@ int gb_solve_dense(int D, int R, const double* T, const double* b, double* x, do
     if (tp.ok) {
         const int e = team_route(tp, P, nullptr, D, reinterpret_cast<const double2*>(T), nullptr, b, x, tol, maxiter, base,
                                  w, status, iters, resid, s);
-        if (e != GB_UNSUPPORTED) return e;   // (no room for the team on this device)
+        if (e != GB_UNSUPPORTED) return e;
     }
     DevPlan Dp;
     int e = upload_plan(P, base, w, s, Dp);
@@ -3463,7 +3468,7 @@ int gb_solve_dense_noalloc(int D, int R, const double* T, const double* b, doubl
     if (tp.ok) {
         const int e = team_route(tp, P, nullptr, D, reinterpret_cast<const double2*>(T), nullptr, b, x, tol, maxiter, base,
                                  w, status, iters, resid, s);
-        if (e != GB_UNSUPPORTED) return e;   // (no room for the team on this device)
+        if (e != GB_UNSUPPORTED) return e;
     }
     DevPlan Dp;
     e = upload_plan_pageable(P, base, w, s, Dp);

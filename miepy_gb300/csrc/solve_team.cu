@@ -15,7 +15,9 @@
 //     <r, r> and <r0, r>.
 // Teams of up to kClusterG CTAs are thread-block clusters with the hardware barrier
 // (any number of systems per launch).  Larger systems take up to one CTA per SM in a
-// cooperative launch with a barrier through L2, whose waits are bounded.
+// cooperative launch with a barrier through L2, whose waits are bounded: where one runs out
+// (other streams' kernels kept part of the team off the SMs) the launch-per-step solver
+// takes the systems.
 //
 // FP64 issues one warp instruction per 64 cycles and SM sub-partition, whatever its lanes
 // do, so the iteration's small steps count instructions too: a warp holds eight vector
@@ -31,6 +33,7 @@
 // epilogue included): 440 -> 186 us.
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -50,7 +53,11 @@ constexpr int kClusterG = 16;        // CTAs of a cluster team
 constexpr int kElems = 8;            // vector elements per warp
 constexpr int kMaxElems = kElems * kTeamWarps;
 constexpr int kMaxRestarts = 8;      // as the launch-per-step solver
-constexpr long long kTeamWaitCycles = 4000000000LL;   // about 2 s: the team may wait for other streams' kernels
+// Cycles a cooperative team waits at a barrier (per device), ten times the matrix pass's
+// limit, about 2 s: its CTAs may have to wait for other streams' kernels to leave their SMs.
+constexpr int kDevices = 64;
+std::atomic<long long> g_team_wait[kDevices];   // 0: the default
+constexpr long long kTeamWaitCycles = 4000000000LL;
 constexpr size_t kTeamSmem = 222 * 1024;
 // beyond this the products are all of the time and the launch-per-step solver streams the
 // matrix with more warps
@@ -68,6 +75,7 @@ struct TeamArgs {
     double2 *g1, *g2;           // operand vectors, at the clusters' vec offsets
     double* part;               // [nsys][2 buffers][3 R][G]
     double tol;
+    long long wait;             // limit of a cooperative team's barrier, in cycles
     int maxiter, D, G, resident, CP;   // D: the dense system; CP: column parts of a product
 };
 
@@ -262,7 +270,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team_bicgstab(const TeamArg
                 int v;
                 asm volatile("ld.acquire.gpu.global.s32 %0, [%1];\n" : "=r"(v) : "l"(n) : "memory");
                 if (v >= target) break;
-                if (clock64() - t0 > kTeamWaitCycles) {
+                if (clock64() - t0 > a.wait) {
                     s_abort = 1;
                     atomicExch(a.err, 1);
                     break;
@@ -534,6 +542,15 @@ TeamPlan team_plan(int nsys, int Dmax, int R, bool packed) {
     return best;
 }
 
+int set_team_wait_limit(long long gemv_cycles) {
+    int dev = 0;
+    GB_CUDA_TRY(cudaGetDevice(&dev));
+    const long long most = 0x7fffffffffffffffLL;
+    const long long v = gemv_cycles < 0 ? 0 : gemv_cycles == 0 ? 1 : gemv_cycles > most / 10 ? most : 10 * gemv_cycles;
+    g_team_wait[dev % kDevices].store(v, std::memory_order_relaxed);
+    return GB_OK;
+}
+
 int team_solve(const TeamPlan& t, int nsys, const SysDev* sys, int D, int R, const double2* mat, const double2* tvec,
                const double2* b, double2* x, KState* st, int* err_cnt, double2* vectors, long long total_vec, double tol,
                int maxiter, cudaStream_t stream) {
@@ -555,6 +572,10 @@ int team_solve(const TeamPlan& t, int nsys, const SysDev* sys, int D, int R, con
     a.G = t.G;
     a.resident = t.resident;
     a.CP = t.cp;
+    int dev = 0;
+    GB_CUDA_TRY(cudaGetDevice(&dev));
+    const long long limit = g_team_wait[dev % kDevices].load(std::memory_order_relaxed);
+    a.wait = limit ? limit : kTeamWaitCycles;
     GB_CUDA_TRY(cudaMemsetAsync(err_cnt, 0, sizeof(int) * (size_t)(nsys + 1), stream));
     if (R == 1) return sys ? launch_any<1, true>(a, nsys, t, stream) : launch_any<1, false>(a, nsys, t, stream);
     return sys ? launch_any<2, true>(a, nsys, t, stream) : launch_any<2, false>(a, nsys, t, stream);

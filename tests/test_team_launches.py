@@ -64,3 +64,16 @@ def test_fp64_batches(n, single):
     d = b.b - b.apply(b.x)
     for s in range(n):
         assert float(b.cluster_view(s, d).norm() / b.cluster_view(s, b.b).norm()) < 2e-11
+
+
+@pytest.mark.parametrize("R", [1, 2])
+def test_expired_team_wait_falls_back(R):
+    """A cooperative team whose barrier runs out of its limit is no error: the
+    launch-per-step solver takes the system, and the next call is one launch again."""
+    L = nat.lib()
+    nat.check(L.gb_set_gemv_wait_limit(0, None))
+    try:
+        assert _dense(1301, R) > 1
+    finally:
+        nat.check(L.gb_set_gemv_wait_limit(-1, None))
+    assert _dense(1301, R) == 1
