@@ -27,8 +27,8 @@
 // sums reduce by halving exchanges (9 additions for four complex sums instead of 40), and
 // the tile and the column split are those of the fewest instructions per sub-partition.
 // Dense systems solved to 1e-12 with one right-hand side (20 iterations): D = 80 962 ->
-// 314 us, D = 224 1149 -> 411, D = 600 1383 -> 537, D = 1300 2052 -> 1105, D = 2880 4674
-// -> 3701 us.  At D = 5000 (10.1 ms either way, the products all of it) the launch-per-step
+// 314 us, D = 224 1149 -> 412, D = 600 1383 -> 538, D = 1300 2052 -> 1168, D = 2880 4674
+// -> 3752 us.  At D = 5000 (10.1 ms either way, the products all of it) the launch-per-step
 // solver takes over: kTeamMaxD.  A step of five spheres, lmax 2 (D = 80, assembly and
 // epilogue included): 440 -> 186 us.
 
@@ -58,7 +58,15 @@ constexpr int kMaxRestarts = 8;      // as the launch-per-step solver
 constexpr int kDevices = 64;
 std::atomic<long long> g_team_wait[kDevices];   // 0: the default
 constexpr long long kTeamWaitCycles = 4000000000LL;
-constexpr size_t kTeamSmem = 222 * 1024;
+// A team's CTA takes at most half of an SM's shared memory and registers (two CTAs per SM),
+// so that kernels of other streams run beside a solve, which lasts up to milliseconds: with
+// 222 KB and 208 registers a mixed solve of N = 12, lmax 3 took 46.8 ms beside dense solves
+// of D = 2880, and 0.71 ms with half (0.60 alone; 0.98 beside the launch-per-step solver).
+// Fewer registers cost 1 to 2 %; the operands beyond 110 KB, dense rows are streamed (D =
+// 1000, R = 1 620 -> 698 us) and larger packed systems (D above about 950) are left to the
+// launch-per-step solver (D = 960: 344 -> 611 us); batches share the SMs (19 systems of D =
+// 80 265 -> 186 us).
+constexpr size_t kTeamSmem = 110 * 1024;
 // beyond this the products are all of the time and the launch-per-step solver streams the
 // matrix with more warps
 constexpr int kTeamMaxD = 4000;
@@ -200,7 +208,7 @@ template <int R> __device__ __forceinline__ void team_scalars(KState* ks, int ph
 
 // TILE: rows per warp tile of a product.
 template <int R, bool PACKED, bool CLUSTER, int TILE>
-__global__ void __launch_bounds__(kTeamThreads, 1) k_team_bicgstab(const TeamArgs a) {
+__global__ void __launch_bounds__(kTeamThreads, 2) k_team_bicgstab(const TeamArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ KState ks[R];
     __shared__ double ysum[kTeamWarps][TILE * 2 * R];
