@@ -88,12 +88,16 @@ def _mode_constants(lmax):
     n, m = (np.array(v) for v in zip(*nm))
     neg = np.array([_neg_factor(*v) if v[1] < 0 else 1.0 for v in nm])
     emn = np.array([np.sqrt((2 * a + 1) * factorial(a - b) / (a * (a + 1) * factorial(a + b))) for a, b in nm])
-    return n, np.abs(m), m, neg, emn
+    tables = n, np.abs(m), m, neg, emn
+    for t in tables:   # shared by every caller
+        t.setflags(write=False)
+    return tables
 
 
 def pi_tau_emn(lmax, theta):
     """pi_func, tau_func and |Emn| of every mode (in mode order) at one angle, from one
-    Legendre table: the values of the functions above, in the same arithmetic."""
+    Legendre table: the values of the functions above, in the same arithmetic.  |Emn| is a
+    shared, read-only table."""
     n, am, m, neg, emn = _mode_constants(int(lmax))
     theta = float(theta)
     if theta == 0 or theta == np.pi:
