@@ -1923,6 +1923,8 @@ __global__ void k_cast_f(const gb::SysDev* __restrict__ sys, const Item* __restr
 }
 
 // ================================================================== host ==
+constexpr int kTcMaxB = 70;   // largest block of the tensor-core pass (gemv_tc.cu)
+
 struct StripGroup {     // strips [beg, end) of clusters with block size B (one GEMV launch each)
     int B;
     long long beg, end;
@@ -1938,7 +1940,8 @@ struct Plan {
     std::vector<Item> vitems, ritems;
     std::vector<SysPlan> sp;
     std::vector<long long> row_strip;
-    // the tensor-core pass's units (R = 4 or 8 in the FP32 and mixed methods)
+    // the tensor-core pass's units (R = 4 or 8 in the FP32 and mixed methods); rows of a unit,
+    // 0: no units
     int tc_I = 0;
     std::vector<gb::TcUnit> tc_units;
     std::vector<StripGroup> tc_groups;
@@ -2010,7 +2013,8 @@ void tc_units(Plan& P, const std::vector<int>& order) {
     }
 }
 
-int build_plan(int nsys, const gb_system* sys, int R, int prec, cudaStream_t stream, Plan& P) {
+// tiles: the plan may serve the tensor-core pass (its tiles are given, or a workspace is sized)
+int build_plan(int nsys, const gb_system* sys, int R, int prec, bool tiles, cudaStream_t stream, Plan& P) {
     P.nsys = nsys;
     P.R = R;
     int st = gb::make_sysdev(nsys, sys, stream, P.sd);
@@ -2067,7 +2071,7 @@ int build_plan(int nsys, const gb_system* sys, int R, int prec, cudaStream_t str
         P.total_ty = std::max<long long>(P.total_ty, d.ty_off + d.N * gb::tc_y_bytes(d.B, 1));
         P.max_B = std::max<long long>(P.max_B, d.B);
     }
-    if (R >= 4 && prec != GB_PREC_FP64) tc_units(P, order);
+    if (tiles && R >= 4 && prec != GB_PREC_FP64 && P.max_B <= kTcMaxB) tc_units(P, order);
     P.nstrips = (long long)P.strips.size();
     P.nv = (int)P.vitems.size();
     P.nr = (int)P.ritems.size();
@@ -2117,7 +2121,7 @@ WS ws_layout(const Plan& P, int prec, bool dense) {
                                  sizeof(float2) * (size_t)P.tc_cw_elems));
         // (the tensor-core pass pads its operands' columns to 16)
         const size_t yb = std::max<size_t>(16 * (size_t)P.total_vec,
-                                           R >= 4 && prec != GB_PREC_FP64 ? (size_t)P.total_ty * R : 0);
+                                           P.tc_I ? (size_t)P.total_ty * R : 0);
         w.off_yu = take(yb);
         w.off_yw = take(yb);
         w.off_tx = take(0);
@@ -2493,8 +2497,8 @@ int launch_apply(const Plan& P, const DevPlan& D, const WS& w, unsigned char* ba
     } else if (pol == 3) {   // tensor-core pass on the bf16 tiles (mat_hi): float2 partials
         if constexpr (R == 4 || R == 8) {
             if (P.tmat) return gb_set_error(GB_UNSUPPORTED, "the tensor-core pass serves sphere clusters");
-            if (P.max_B > 70)
-                return gb_set_error(GB_UNSUPPORTED, "tensor-core pass: block size %lld > 70 (lmax 5)", P.max_B);
+            if (P.max_B > kTcMaxB)
+                return gb_set_error(GB_UNSUPPORTED, "tensor-core pass: block size %lld > %d (lmax 5)", P.max_B, kTcMaxB);
             gb::note_launch();
             GB_CUDA_TRY(launch_pdl(k_yprep_tc<VT, R>, dim3((unsigned)P.nr), dim3(kTcYThreads), 0, stream, D.sys, D.ritems,
                                    st, mask, tvec, xin, static_cast<unsigned char*>(Yu), static_cast<unsigned char*>(Yw),
@@ -3154,7 +3158,7 @@ int apply_entry(int nsys, const gb_system* sys, int R, int prec, const double* m
 #endif
     if (prec == GB_PREC_MIXED_FP64RES) prec = GB_PREC_FP64;
     Plan P;
-    int e = build_plan(nsys, sys, R, prec, s, P);
+    int e = build_plan(nsys, sys, R, prec, mat_tc != nullptr, s, P);
     if (e) return e;
     WS w = ws_layout(P, prec, false);
     if (ws_bytes < w.total) return gb_set_error(GB_OVER_BUDGET, "workspace %zu B < required %zu B", ws_bytes, w.total);
@@ -3186,7 +3190,7 @@ int solve_entry(int nsys, const gb_system* sys, int R, int prec, double tol, int
                                      mat_tc, pdiag, tvec, b, x, workspace, ws_bytes, status, iters, resid, s);
 #endif
     Plan P;
-    int e = build_plan(nsys, sys, R, prec, s, P);
+    int e = build_plan(nsys, sys, R, prec, mat_tc != nullptr, s, P);
     if (e) return e;
     WS w = ws_layout(P, prec, false);
     if (ws_bytes < w.total) return gb_set_error(GB_OVER_BUDGET, "workspace %zu B < required %zu B", ws_bytes, w.total);
@@ -3214,7 +3218,7 @@ extern "C" {
 
 size_t gb_solve_workspace_size(int nsys, const gb_system* sys, int R, int prec) {
     Plan P;
-    if (build_plan(nsys, sys, R, prec, 0, P)) return 0;
+    if (build_plan(nsys, sys, R, prec, true, 0, P)) return 0;
     return ws_layout(P, prec, false).total;
 }
 
@@ -3249,7 +3253,7 @@ int gb_solve_batch_tmatrix(int nsys, const gb_system* sys, int R, int prec, doub
     if (!(tol > 0) || maxiter < 1) return gb_set_error(GB_BAD_ARG, "tol must be > 0 and maxiter >= 1");
     cudaStream_t s = (cudaStream_t)stream;
     Plan P;
-    int e = build_plan(nsys, sys, R, prec, s, P);
+    int e = build_plan(nsys, sys, R, prec, false, s, P);
     if (e) return e;
     for (int q = 0; q < nsys; q++) {
         if (P.sd[q].B * R > kRBThreads) return gb_set_error(GB_UNSUPPORTED, "T-matrix clusters need lmax <= 8");
@@ -3283,7 +3287,7 @@ int gb_autotune_gemv(int nsys, const gb_system* sys, int R, int prec, const doub
     const int aprec = f64 ? GB_PREC_FP64 : GB_PREC_FP32;
     cudaStream_t s = (cudaStream_t)stream;
     Plan P;
-    int e = build_plan(nsys, sys, R, prec, s, P);
+    int e = build_plan(nsys, sys, R, prec, false, s, P);
     if (e) return e;
     WS w = ws_layout(P, aprec, false);
     if (ws_bytes < w.total) return gb_set_error(GB_OVER_BUDGET, "workspace %zu B < required %zu B", ws_bytes, w.total);
