@@ -21,8 +21,10 @@
 // k_field32 (FP32 exterior sums for large maps: a 512 x 512 plane around thousands of
 // spheres is ~5e8 point-particle terms).  Bound by the FP32 pipe; a thread takes two
 // points in packed f32x2 arithmetic and reads every folded coefficient once for both
-// (16-byte broadcast loads of duplicated pairs).  Coordinates are split into two floats so
-// that separations keep FP32 accuracy without FP64 arithmetic; k r is reduced with a
+// (16-byte broadcast loads of duplicated pairs).  Coordinates, from the first particle's
+// position, are split into two floats so that separations keep FP32 accuracy without FP64
+// arithmetic (their error is 2^-48 of the extent of points and particles, wherever the
+// origin lies); k r is reduced with a
 // two-float k / pi, which the phase of distant spheres needs.  Points inside a sphere are
 // found by the FP32 distance, decided in FP64 and collected, so that their FP64 interior
 // expansions run on full warps.  512 x 512 points, 2000 spheres, lmax 3: 30.7 -> 7.6 ms
@@ -327,9 +329,10 @@ k_field32(const __grid_constant__ FieldArgs a, float kpi_h, float kpi_l, float i
     __shared__ int n_in, list[kPoints32];
     const int tid = threadIdx.x;
     const long long p0 = (long long)blockIdx.x * kPoints32 + tid, p1 = p0 + kThreads32;
+    const double o[3] = {a.pos[0], a.pos[1], a.pos[2]};
     float2 Xh[3], Xl[3];
     for (int c = 0; c < 3; c++) {
-        const double u = p0 < a.Npts ? a.pts[3 * p0 + c] : 0.0, v = p1 < a.Npts ? a.pts[3 * p1 + c] : 0.0;
+        const double u = p0 < a.Npts ? a.pts[3 * p0 + c] - o[c] : 0.0, v = p1 < a.Npts ? a.pts[3 * p1 + c] - o[c] : 0.0;
         Xh[c] = make_float2((float)u, (float)v);
         Xl[c] = make_float2((float)(u - (double)Xh[c].x), (float)(v - (double)Xh[c].y));
     }
@@ -343,7 +346,7 @@ k_field32(const __grid_constant__ FieldArgs a, float kpi_h, float kpi_l, float i
         for (int q = tid; q < cnt; q += kThreads32) {
             float h[3], l[3];
             for (int c = 0; c < 3; c++) {
-                const double v = a.pos[3LL * (t0 + q) + c];
+                const double v = a.pos[3LL * (t0 + q) + c] - o[c];
                 h[c] = (float)v;
                 l[c] = (float)(v - (double)h[c]);
             }
