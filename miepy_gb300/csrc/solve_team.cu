@@ -67,6 +67,8 @@ constexpr long long kTeamWaitCycles = 4000000000LL;
 // launch-per-step solver (D = 960: 344 -> 611 us); batches share the SMs (19 systems of D =
 // 80 265 -> 186 us).
 constexpr size_t kTeamSmem = 110 * 1024;
+// a dense matrix up to this size (of 129 MB of L2) stays there between products
+constexpr size_t kL2Matrix = 96 << 20;
 // beyond this the products are all of the time and the launch-per-step solver streams the
 // matrix with more warps
 constexpr int kTeamMaxD = 4000;
@@ -497,15 +499,22 @@ int launch_any(const TeamArgs& a, int nsys, const gb::TeamPlan& t, cudaStream_t 
 }
 
 // FP64 instructions per sub-partition (its share of the warps' units) of one product with
-// rows rows per CTA, for the best tile and column split.
-int product_cost(int rows, int D, int R, int* tile, int* cp) {
+// rows rows per CTA, for the best tile and column split.  Rows that come from HBM are bound
+// by the loads in flight: there a round of tiles costs what all of its warps would take,
+// idle ones included, and two or four warps share a tile (dense D = 3500, R = 1 3.73 -> 3.12
+// ms, 3.53 with a launch per step; D = 2900 2.44 -> 2.24; where the matrix stays in L2, D =
+// 2400, a warp per tile is as quick).
+int product_cost(int rows, int D, int R, bool from_hbm, int* tile, int* cp) {
     int best = 1 << 30;
     for (int T = 4; T >= 2; T -= 2)
-        for (int C = 1; C <= kTeamWarps; C *= 2) {
+        for (int C = from_hbm ? 2 : 1; C <= (from_hbm ? 4 : kTeamWarps); C *= 2) {
             const int tiles = (rows + T - 1) / T, per = kTeamWarps / C;   // tiles per round of the warps
             const int step = (D + 32 * C - 1) / (32 * C) * 4 * T * R + (T == 4 ? 9 : 6) * R;
             int cost = 0;
-            for (int t = 0; t < tiles; t += per) cost += (std::min(per, tiles - t) * C + 3) / 4 * step + C;
+            for (int t = 0; t < tiles; t += per) {
+                const int warps = from_hbm ? kTeamWarps : std::min(per, tiles - t) * C;
+                cost += (warps + 3) / 4 * step + C;
+            }
             if (cost < best) {
                 best = cost;
                 *tile = T;
@@ -542,8 +551,9 @@ TeamPlan team_plan(int nsys, int Dmax, int R, bool packed) {
         t.resident = vec + mat <= kTeamSmem;
         t.smem = vec + (t.resident ? mat : 0);
         if (t.smem > kTeamSmem || (packed && !t.resident)) continue;
+        const bool from_hbm = !t.resident && sizeof(double2) * (size_t)Dmax * Dmax > kL2Matrix;
         const long long waves = ((long long)nsys * t.G + sms - 1) / sms;
-        t.cycles = waves * (2LL * 64 * product_cost(rows, Dmax, R, &t.tile, &t.cp) + 5 * (t.cluster ? 1500 : 3300));
+        t.cycles = waves * (2LL * 64 * product_cost(rows, Dmax, R, from_hbm, &t.tile, &t.cp) + 5 * (t.cluster ? 1500 : 3300));
         t.ok = true;
         if (!best.ok || t.cycles < best.cycles) best = t;
     }

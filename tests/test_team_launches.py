@@ -42,7 +42,7 @@ def _dense(D, R):
     return n
 
 
-@pytest.mark.parametrize("D,R", [(D, R) for D in (1, 3, 7, 62, 130, 501, 999, 1301, 2999) for R in (1, 2)] + [(4000, 1)])
+@pytest.mark.parametrize("D,R", [(D, R) for D in (1, 3, 7, 62, 130, 501, 999, 1301, 2999, 3450) for R in (1, 2)] + [(4000, 1)])
 def test_dense_systems_take_one_launch(D, R):
     assert _dense(D, R) == 1
 
