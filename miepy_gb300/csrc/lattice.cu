@@ -18,7 +18,11 @@
 //     (-1)^mu (p-mu)!/(p+mu)! of negative orders multiply the sums once.
 // A pair's chunks put their tables into the pair's own block of the output, which the
 // assembler reads back (in order: the result does not depend on scheduling) and then
-// overwrites.  All pairs i = j share one sum.  5040 cells, the whole aggregate, against a
+// overwrites.  Small blocks have room for few tables (two at lmax 1), so where the pairs
+// are few as well a chunk's cells are shared by a cluster of up to eight CTAs, whose sums
+// the first one adds in order (whole aggregates of 5040 cells: N = 1, lmax 1 126 -> 29 us,
+// lmax 3 63 -> 35; N = 2, lmax 1 126 -> 29; N = 6, lmax 1 127 -> 75).  All pairs i = j share
+// one sum.  5040 cells, the whole aggregate, against a
 // thread per cell for the special functions, the table entries in passes over shared memory
 // and atomic adds of the blocks: N = 5, lmax 2 465 -> 84 us, N = 30, lmax 3 21.5 -> 2.9 ms
 // (74 % of the FP64 pipe's time for 300 instructions per cell), N = 30, lmax 4 39.3 -> 4.5 ms.
@@ -32,10 +36,12 @@
 namespace {
 
 constexpr int kLatThreads = 256;
+constexpr int kPortableCluster = 8;
 constexpr int kPM = 2 * GB_LMAX_MAX + 2;
 
 struct LatArgs {
     int N, ncell, nch, per;      // chunks per pair, cells per chunk (the origin is cell 0)
+    int split, sub;              // CTAs per chunk (a cluster, if several), cells of each
     const double* pos;
     const double* cells;
     double k, kx, ky, kz;
@@ -147,14 +153,30 @@ __device__ __forceinline__ void columns(int warp, const double* st, int n, doubl
     }
 }
 
-template <int L>
+// Every thread of the cluster arrives before any passes.
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::: "memory");
+}
+// *p of the cluster's CTA rank
+__device__ __forceinline__ double cluster_read(const double* p, unsigned rank) {
+    unsigned at;
+    double v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(at) : "memory");
+    return v;
+}
+
+// SPLIT: a.split CTAs per chunk (a kernel of its own, so that the other keeps its registers)
+template <int L, bool SPLIT>
 __global__ void __launch_bounds__(kLatThreads) k_lattice_sums(const __grid_constant__ LatArgs a) {
     constexpr int PM = 2 * L + 2, MM = 2 * L, SC = stage_cells<L>();
     extern __shared__ __align__(16) double st[];                // [2 PM + 3][SC]
     __shared__ double sums[MM + 1][4 * PM];
     const int tid = threadIdx.x, warp = tid >> 5;
     // pairs: (0, 0) for every i = j, then the ordered pairs i != j
-    const int pair = blockIdx.x / a.nch, chunk = blockIdx.x - pair * a.nch;
+    const unsigned unit = SPLIT ? blockIdx.x / a.split : blockIdx.x;
+    const int pair = unit / a.nch, chunk = unit - pair * a.nch;
+    const int rank = SPLIT ? blockIdx.x - unit * a.split : 0;
     int i = 0, j = 0;
     if (pair > 0) {
         i = (pair - 1) / (a.N - 1);
@@ -164,8 +186,12 @@ __global__ void __launch_bounds__(kLatThreads) k_lattice_sums(const __grid_const
     const double px = a.pos[3 * i] - a.pos[3 * j], py = a.pos[3 * i + 1] - a.pos[3 * j + 1],
                  pz = a.pos[3 * i + 2] - a.pos[3 * j + 2];
     for (int e = tid; e < (MM + 1) * 4 * PM; e += kLatThreads) (&sums[0][0])[e] = 0.0;
-    const int c1 = min((chunk + 1) * a.per, a.ncell + 1);
-    for (int c0 = chunk * a.per; c0 < c1; c0 += SC) {
+    int cb = chunk * a.per, c1 = min((chunk + 1) * a.per, a.ncell + 1);
+    if constexpr (SPLIT) {
+        cb += rank * a.sub;
+        c1 = min(c1, cb + a.sub);
+    }
+    for (int c0 = cb; c0 < c1; c0 += SC) {
         const int n = min(SC, c1 - c0);
         __syncthreads();
         // ---- A: one thread per cell
@@ -211,6 +237,18 @@ __global__ void __launch_bounds__(kLatThreads) k_lattice_sums(const __grid_const
         columns<L, 0>(warp, st, n, sums);
     }
     __syncthreads();
+    if constexpr (SPLIT) {   // the other CTAs' sums, in order
+        cluster_barrier();
+        if (rank == 0)
+            for (int e = tid; e < (MM + 1) * 4 * PM; e += kLatThreads) {
+                double* at = &sums[0][0] + e;
+                double v = *at;
+                for (int q = 1; q < a.split; q++) v += cluster_read(at, q);
+                *at = v;
+            }
+        cluster_barrier();   // (their shared memory lives until it is read)
+        if (rank) return;
+    }
     // the chunk's table, entries p^2 + p + mu, into the pair's block (all of i = j: the
     // one sum into every diagonal block)
     const int B = 2 * L * (L + 2), copies = pair == 0 ? a.N : 1;
@@ -235,14 +273,37 @@ __global__ void __launch_bounds__(kLatThreads) k_lattice_sums(const __grid_const
 }
 
 template <int L>
-int launch(const LatArgs& a, cudaStream_t stream) {
+int launch(LatArgs a, cudaStream_t stream) {
     const size_t smem = sizeof(double) * (2 * (2 * L + 2) + 3) * stage_cells<L>();
-    auto kfn = k_lattice_sums<L>;
+    auto kfn = a.split > 1 ? k_lattice_sums<L, true> : k_lattice_sums<L, false>;
     GB_CUDA_TRY(gb::ensure_dynamic_smem(reinterpret_cast<const void*>(kfn), smem));
     const long long pairs = 1 + (long long)a.N * (a.N - 1);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    cfg.blockDim = dim3(kLatThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    for (;; a.split = kPortableCluster) {
+        a.sub = (a.per + a.split - 1) / a.split;
+        cfg.gridDim = dim3((unsigned)(pairs * a.nch * a.split));
+        at[0].val.clusterDim.x = (unsigned)a.split;
+        cfg.numAttrs = a.split > 1 ? 1 : 0;
+        if (a.split > kPortableCluster)
+            GB_CUDA_TRY(cudaFuncSetAttribute(reinterpret_cast<const void*>(kfn),
+                                             cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, kfn, a);
+        if (a.split > kPortableCluster && (e == cudaErrorInvalidClusterSize || e == cudaErrorLaunchOutOfResources ||
+                                           e == cudaErrorInvalidConfiguration)) {   // (part of a device)
+            (void)cudaGetLastError();
+            continue;
+        }
+        GB_CUDA_TRY(e);
+        break;
+    }
     gb::note_launch();
-    kfn<<<(unsigned)(pairs * a.nch), kLatThreads, smem, stream>>>(a);
-    GB_CUDA_TRY(cudaGetLastError());
     return GB_OK;
 }
 
@@ -258,6 +319,16 @@ int lattice_chunks(int N, int lmax, int ncell) {
     return (int)std::max<long long>(1, std::min({room, want, (ncell + 128LL) / 128}));
 }
 
+// CTAs per chunk: where the chunks are fewer than the SMs, as many more as still have an SM
+// each and 16 cells, up to sixteen.  (Beyond one per SM the clusters queue: N = 2, lmax 5, 5040
+// cells 79 us with 102 CTAs, 112 with 408.)
+static int lattice_split(int N, int ncell, int nch) {
+    const long long units = (1 + (long long)N * (N - 1)) * nch;
+    int k = 1;
+    while (k < 16 && 2 * k * units <= sm_count() && 2LL * k * nch * 16 <= ncell + 1) k *= 2;
+    return k;
+}
+
 int launch_lattice_sums(int N, int lmax, const double* pos, double k, const double* cells, int ncell, double kx, double ky,
                         double kz, const double* neg_ratio, double2* out, long long ld, cudaStream_t stream) {
     LatArgs a{};
@@ -265,6 +336,7 @@ int launch_lattice_sums(int N, int lmax, const double* pos, double k, const doub
     a.ncell = ncell;
     a.nch = lattice_chunks(N, lmax, ncell);
     a.per = (ncell + 1 + a.nch - 1) / a.nch;
+    a.split = lattice_split(N, ncell, a.nch);
     a.pos = pos;
     a.cells = cells;
     a.k = k;
