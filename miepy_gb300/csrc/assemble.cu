@@ -1221,10 +1221,9 @@ int gb_aggregate_periodic_dense(int N, int lmax, const double* pos, const double
     cudaStream_t st = (cudaStream_t)stream;
     const long long D = 2LL * lmax_to_rmax(lmax) * N;
     gb_system s{N, lmax, k, 0, 0, 0, 0};
-    if (lmax > 9) {   // the lattice blocks' tuple values exceed a CTA's shared memory (as the assembler reports)
-        if (ncell > 0) return gb_set_error(GB_UNSUPPORTED, "lattice sums support lmax 1..9 (got %d)", lmax);
-        return gb_assemble_sphere_dense(N, lmax, pos, mie, k, out, stream);
-    }
+    if (ncell == 0) return gb_assemble_sphere_dense(N, lmax, pos, mie, k, out, stream);   // no sums to form
+    if (lmax > 9)   // the lattice blocks' tuple values exceed a CTA's shared memory (as the assembler reports)
+        return gb_set_error(GB_UNSUPPORTED, "lattice sums support lmax 1..9 (got %d)", lmax);
     const gb::Tables* T = nullptr;
     int e = gb::get_tables(lmax, st, &T);
     if (e) return e;

@@ -44,3 +44,25 @@ def test_periodic_aggregate(N, L, ncell):
     ref = O.sphere_aggregate_tmatrix_periodic(pos, mie.reshape(N, -1), k, cells.reshape(-1, 3), kh).reshape(D, D)
     err = np.max(np.abs(out.cpu().numpy() - ref)) / np.max(np.abs(ref))
     assert err < (1e-12 if L <= 8 else 1e-10)   # the aggregate's bars
+
+
+@pytest.mark.parametrize("N,L", [(1, 1), (1, 9), (7, 3)])
+def test_no_cells(N, L):
+    """Without cells the aggregate is the plain one: the same bits from the same launches."""
+    import torch
+
+    from miepy_gb300.engine import current_stream
+    lib = nat.lib()
+    rng = np.random.default_rng([N, L])
+    dev = torch.device("cuda", 0)
+    pos = torch.from_numpy(np.array([(i, i % 2, 0.3 * i) for i in range(N)], float) * 3e-7).to(dev)
+    mie = torch.from_numpy(rng.normal(size=(N, 2, L)) + 1j * rng.normal(size=(N, 2, L))).to(dev)
+    D = 2 * L * (L + 2) * N
+    out = [torch.full((D, D), complex(np.nan, np.nan), dtype=torch.complex128, device=dev) for _ in range(2)]
+    n0 = lib.gb_launch_count()
+    nat.check(lib.gb_assemble_sphere_dense(N, L, nat.ptr(pos), nat.ptr(mie), 1.05e7, nat.ptr(out[0]), current_stream(dev)))
+    n1 = lib.gb_launch_count()
+    nat.check(lib.gb_aggregate_periodic_dense(N, L, nat.ptr(pos), nat.ptr(mie), 1.05e7, None, 0, 0.0, 0.0, 1.0,
+                                              nat.ptr(out[1]), current_stream(dev)))
+    assert lib.gb_launch_count() - n1 == n1 - n0
+    assert torch.equal(out[0], out[1])
