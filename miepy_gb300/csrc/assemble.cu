@@ -908,8 +908,6 @@ int make_sysdev(int nsys, const gb_system* sys, cudaStream_t stream, std::vector
         d.mat_off = a.mat_off;
         d.vec_off = a.vec_off;
         d.t_off = a.t_off;
-        d.nmvu = T->nmvu;
-        d.qab = T->qab;
         d.cA = T->cA;
         d.cB = T->cB;
         d.cA2 = T->cA2;

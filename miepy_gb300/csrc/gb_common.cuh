@@ -20,7 +20,6 @@ __host__ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
 __host__ __device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
     return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
-// acc += a * b
 // a - b on packed f32x2 (sub.rn.f32x2): the packed add takes no negated operand,
 // so a - b written as a + (-b) costs a sign flip per component on the integer pipe
 __device__ __forceinline__ float2 fsub2(float2 a, float2 b) {
@@ -32,6 +31,7 @@ __device__ __forceinline__ float2 fsub2(float2 a, float2 b) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(rd));
     return d;
 }
+// acc += a * b
 __device__ __forceinline__ void cfma(double2& acc, double2 a, double2 b) {
     acc.x = fma(a.x, b.x, acc.x);
     acc.x = fma(-a.y, b.y, acc.x);
@@ -58,6 +58,26 @@ __device__ __forceinline__ double flipd(double v, unsigned neg) {
 }
 __device__ __forceinline__ float flipf(float v, unsigned neg) {
     return __int_as_float(__float_as_int(v) ^ (neg << 31));
+}
+
+// -------------------------------------------------------------- lane sums --
+// Sums V values (a power of two, at most 32) over the warp's lanes by halving exchanges: afterwards
+// lane l holds the sum of value l >> (5 - log2 V).
+template <int V> __device__ __forceinline__ double halving_sum(double (&a)[V]) {
+    const int lane = threadIdx.x & 31;
+    int off = 16;
+#pragma unroll
+    for (int n = V / 2; n >= 1; n >>= 1) {
+        const bool hi = lane & off;
+#pragma unroll
+        for (int q = 0; q < n; q++) {
+            const double send = hi ? a[q] : a[q + n], keep = hi ? a[q + n] : a[q];
+            a[q] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+        }
+        off >>= 1;
+    }
+    for (; off > 0; off >>= 1) a[0] += __shfl_xor_sync(0xffffffffu, a[0], off);
+    return a[0];
 }
 
 // --------------------------------------------------------------- indexing --

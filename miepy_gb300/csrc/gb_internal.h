@@ -66,8 +66,6 @@ struct SysDev {
     double k;
     long long pos_off, mat_off, vec_off, t_off;
     // table pointers for this lmax
-    const int4* nmvu;
-    const int2* qab;
     const double* cA;
     const double* cB;
     const float2* cA2;

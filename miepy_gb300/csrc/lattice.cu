@@ -53,25 +53,6 @@ struct LatArgs {
 
 template <int L> __host__ __device__ constexpr int stage_cells() { return L <= 4 ? 512 : L <= 7 ? 256 : 128; }
 
-// Sums V (a power of two, at most 32) values over the lanes: lane l holds the sum of value
-// l >> (5 - log2 V).
-template <int V> __device__ __forceinline__ double lane_sums(double (&a)[V]) {
-    const int lane = threadIdx.x & 31;
-    int off = 16;
-#pragma unroll
-    for (int n = V / 2; n >= 1; n >>= 1) {
-        const bool hi = lane & off;
-#pragma unroll
-        for (int q = 0; q < n; q++) {
-            const double send = hi ? a[q] : a[q + n], keep = hi ? a[q + n] : a[q];
-            a[q] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-        }
-        off >>= 1;
-    }
-    for (; off > 0; off >>= 1) a[0] += __shfl_xor_sync(0xffffffffu, a[0], off);
-    return a[0];
-}
-
 // Column MU over the staged cells, added to sums[4 (p - MU) ..] (re re, im im, re im, im re).
 template <int L, int MU>
 __device__ __forceinline__ void column(const double* __restrict__ st, int n, double* __restrict__ sums) {
@@ -127,14 +108,14 @@ __device__ __forceinline__ void column(const double* __restrict__ st, int n, dou
             double v[32];
 #pragma unroll
             for (int q = 0; q < 32; q++) v[q] = acc[q0 + q < NV ? q0 + q : 0];
-            const double s = lane_sums<32>(v);
+            const double s = halving_sum<32>(v);
             sums[q0 + lane] += s;
         } else {
             constexpr int V = LAST <= 8 ? 8 : LAST <= 16 ? 16 : 32, SH = V == 8 ? 2 : V == 16 ? 1 : 0;
             double v[V];
 #pragma unroll
             for (int q = 0; q < V; q++) v[q] = (q < LAST && q0 + q < NV) ? acc[q0 + q < NV ? q0 + q : 0] : 0.0;
-            const double s = lane_sums<V>(v);
+            const double s = halving_sum<V>(v);
             const int at = lane >> SH;
             if ((lane & ((1 << SH) - 1)) == 0 && at < LAST) sums[q0 + at] += s;
         }

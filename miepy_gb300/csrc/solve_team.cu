@@ -95,25 +95,6 @@ __device__ __forceinline__ double2 cquot(double2 a, double2 b) {
 }
 __device__ __forceinline__ bool finite2(double2 a) { return isfinite(a.x) && isfinite(a.y); }
 
-// Sums V values (a power of two) over the warp's lanes by halving exchanges: afterwards
-// lane l holds the sum of value l >> (5 - log2 V).
-template <int V> __device__ __forceinline__ double halving_sum(double (&a)[V]) {
-    const int lane = threadIdx.x & 31;
-    int off = 16;
-#pragma unroll
-    for (int n = V / 2; n >= 1; n >>= 1) {
-        const bool hi = lane & off;
-#pragma unroll
-        for (int q = 0; q < n; q++) {
-            const double send = hi ? a[q] : a[q + n], keep = hi ? a[q + n] : a[q];
-            a[q] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-        }
-        off >>= 1;
-    }
-    for (; off > 0; off >>= 1) a[0] += __shfl_xor_sync(0xffffffffu, a[0], off);
-    return a[0];
-}
-
 enum { STATE_RUNNING = -1 };
 
 __device__ __forceinline__ bool finite1(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
