@@ -25,7 +25,8 @@
  * aggregate matrix follows as  T[i,j] = A_ij diag(t_j)  and
  * T[j,i] = S A_ij S diag(t_i),  S = diag((-1)^(n+a)),  t_j = mie of particle j
  * expanded per row.  Half the storage of the dense matrix, no per-element Mie
- * product.
+ * product.  Over the two polarisations a block is [[P, Q], [Q, P]]; the matrix passes
+ * read its upper half, so a caller's own blocks have to have that form.
  */
 #ifndef MIEPY_GB300_H
 #define MIEPY_GB300_H

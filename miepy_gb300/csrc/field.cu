@@ -28,7 +28,7 @@
 // two-float k / pi, which the phase of distant spheres needs.  Points inside a sphere are
 // found by the FP32 distance, decided in FP64 and collected, so that their FP64 interior
 // expansions run on full warps.  512 x 512 points, 2000 spheres, lmax 3: 30.7 -> 7.6 ms
-// (526 instructions per 64 terms; with fewer than three warps per sub-partition, the
+// (535 warp instructions per particle and 64 points; with fewer than three warps per sub-partition, the
 // last of its 1.7 waves, the packed FMA pipe is 54 % busy).
 
 #include <algorithm>

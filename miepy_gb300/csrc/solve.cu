@@ -24,10 +24,11 @@
 // The products therefore read the upper half of every block and take half the
 // multiplications; a column index 2 s + (0: +, 1: -) has a fixed sign per lane.  Blocks of
 // up to kWholeB columns (lmax <= 3) read the upper half too, but run through all rows of
-// the block, taking the lower ones from the upper ones' other half: their passes are bound
-// by the copies and the work per block rather than by the multiplications, and the sums
-// stay those of the block itself, to the last bit, so that quantities that cancel (the
-// torque on a lossless sphere) keep their residues.
+// the block, taking the lower ones from the upper ones' other half, so that the sums are
+// those of the block itself, to the last bit.  complex64 passes of such blocks are bound by
+// the copies and the work per block, so half the multiplications would give them little;
+// complex128 and double-float passes are bound by the multiplications (N = 401, lmax 3 in
+// FP64 1.21 ms a product with whole and half blocks) and could gain from +- sums.
 // Per pass, whole blocks before and now (launch shapes included): complex64 N = 200, lmax 4,
 // R = 2 66 -> 36 us; N = 97, lmax 8 131 -> 77 us; N = 401, lmax 3 79 -> 63 us;
 // double-float N = 200, lmax 4, R = 2 292 -> 167 us, one pair of eight right-hand sides 404
@@ -751,8 +752,8 @@ __host__ __device__ inline int split_rows(int H, int warps, int rpw) {   // rows
 // of small blocks, one right-hand side, and of shapes of 3 columns per lane waits for
 // latencies rather than bytes (small blocks: 14 warps per SM issued half the time); two
 // stages per warp there leave shared memory for these CTAs.  N = 401, lmax 3 67.9 -> 62.8
-// us, N = 800 240 -> 229 (six CTAs spill: 69, 255); N = 200, lmax 4, R = 2 38.3 -> 35.9,
-// R = 1 33.6 -> 33.6; N = 120, lmax 6, R = 2 52.5 -> 47.3, R = 1 45.0 both.
+// us, N = 800 240 -> 229 (six CTAs spill: 69, 255); N = 200, lmax 4, R = 2 38.3 -> 35.9;
+// N = 120, lmax 6, R = 2 52.5 -> 47.3, R = 1 45.0 both.
 template <class Pol, int RR, int LPR, int CPL> constexpr int more_ctas() {
     return Pol::ID != 1 || CPL > 4 || (CPL > 3 && LPR * CPL > kWholeB + 2) ? 0
            : LPR * CPL <= kWholeB + 2                                    ? (RR == 1 ? 5 : 0)

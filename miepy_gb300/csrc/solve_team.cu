@@ -26,11 +26,11 @@
 // scalar step run in the lanes of one division; rows are tiled so that the lanes' partial
 // sums reduce by halving exchanges (9 additions for four complex sums instead of 40), and
 // the tile and the column split are those of the fewest instructions per sub-partition.
-// Dense systems solved to 1e-12 with one right-hand side (20 iterations): D = 80 962 ->
-// 314 us, D = 224 1149 -> 412, D = 600 1383 -> 538, D = 1300 2052 -> 1168, D = 2880 4674
-// -> 3752 us.  At D = 5000 (10.1 ms either way, the products all of it) the launch-per-step
-// solver takes over: kTeamMaxD.  A step of five spheres, lmax 2 (D = 80, assembly and
-// epilogue included): 440 -> 186 us.
+// Dense systems solved to 1e-10 with one right-hand side (14 iterations), a launch per step
+// and in one: D = 80 705 -> 202 us, D = 224 803 -> 288, D = 600 897 -> 358, D = 1300 1312 ->
+// 743, D = 2900 2842 -> 2247, D = 4000 4390 -> 3818.  Beyond that the products are all of
+// it (4.85 ms either way at D = 4500): kTeamMaxD.  A step of five spheres, lmax 2 (D = 80,
+// assembly and epilogue included): 440 -> 186 us.
 
 #include <algorithm>
 #include <atomic>
