@@ -62,11 +62,14 @@ constexpr long long kTeamWaitCycles = 4000000000LL;
 // so that kernels of other streams run beside a solve, which lasts up to milliseconds: with
 // 222 KB and 208 registers a mixed solve of N = 12, lmax 3 took 46.8 ms beside dense solves
 // of D = 2880, and 0.71 ms with half (0.60 alone; 0.98 beside the launch-per-step solver).
-// Fewer registers cost 1 to 2 %; the operands beyond 110 KB, dense rows are streamed (D =
-// 1000, R = 1 620 -> 698 us) and larger packed systems (D above about 950) are left to the
-// launch-per-step solver (D = 960: 344 -> 611 us); batches share the SMs (19 systems of D =
-// 80 265 -> 186 us).
-constexpr size_t kTeamSmem = 110 * 1024;
+// Fewer registers cost 1 to 2 %; dense rows beyond 110 KB are streamed (D = 1000, R = 1 620 ->
+// 698 us); batches share the SMs (19 systems of D = 80 265 -> 186 us).  Packed rows are not in
+// memory in that form: systems that half of every SM cannot hold (D above about 950) take
+// whole SMs and leave the others free, a quarter where the rows fit the rest, else a
+// sixteenth at least (D up to 1291, R = 2 1287).  D = 960 594 us with a launch per step, 402
+// so, 347 with every SM; D = 1200 773, 526, 438; the mixed solve beside a stream of D = 1200
+// solves 0.58 ms, 3.1 with every SM.
+constexpr size_t kTeamSmem = 110 * 1024, kWholeSmem = 222 * 1024;
 // a dense matrix up to this size (of 129 MB of L2) stays there between products
 constexpr size_t kL2Matrix = 96 << 20;
 // beyond this the products are all of the time and the launch-per-step solver streams the
@@ -537,6 +540,23 @@ TeamPlan team_plan(int nsys, int Dmax, int R, bool packed) {
         t.cycles = waves * (2LL * 64 * product_cost(rows, Dmax, R, from_hbm, &t.tile, &t.cp) + 5 * (t.cluster ? 1500 : 3300));
         t.ok = true;
         if (!best.ok || t.cycles < best.cycles) best = t;
+    }
+    if (packed && !best.ok) {   // whole SMs: as few as hold the rows, or up to three quarters of all where that is quicker
+        const size_t vec = sizeof(double2) * (size_t)Dmax * R, row = sizeof(double2) * (size_t)Dmax;
+        const int most = vec < kWholeSmem ? (int)std::min<size_t>((kWholeSmem - vec) / row, kMaxElems / R) : 0;
+        if (most < 1) return best;
+        const int least = (Dmax + most - 1) / most;
+        if ((long long)nsys * least > sms - sms / 16) return best;
+        for (int G = least; G == least || (long long)nsys * G <= sms * 3 / 4; G++) {
+            TeamPlan t;
+            t.G = G;
+            const int rows = (Dmax + G - 1) / G;
+            t.resident = true;
+            t.smem = vec + rows * row;
+            t.cycles = 2LL * 64 * product_cost(rows, Dmax, R, false, &t.tile, &t.cp) + 5 * 3300;
+            t.ok = true;
+            if (!best.ok || t.cycles < best.cycles) best = t;
+        }
     }
     return best;
 }

@@ -77,6 +77,28 @@ def test_fp64_batches(n, single):
         assert float(b.cluster_view(s, d).norm() / b.cluster_view(s, b.b).norm()) < 2e-11
 
 
+@pytest.mark.parametrize("N,L,R,single", [(31, 3, 1, True), (32, 3, 1, True), (25, 4, 1, True), (43, 3, 1, True),
+                                          (44, 3, 1, False), (30, 3, 2, True), (42, 3, 2, True), (43, 3, 2, False),
+                                          (200, 1, 1, True), (9, 7, 1, True)])
+def test_fp64_clusters_beyond_half_of_every_sm(N, L, R, single):
+    """Packed systems whose rows take whole SMs, up to the limits (152 SMs), against the
+    packed operator's product."""
+    from miepy_gb300.engine import ClusterBatch
+    if nat.lib().gb_device_sm_count() != 152:
+        pytest.skip("limits of 152 SMs")
+    rng = np.random.default_rng([N, L])
+    pos = np.array([(i % 6, i // 6 % 6, i // 36) for i in range(N)], float) * 4e-7 + rng.uniform(-2e-8, 2e-8, (N, 3))
+    mie = (rng.normal(size=(N, 2, L)) + 1j * rng.normal(size=(N, 2, L))) * 0.1 ** np.arange(1, L + 1)
+    p = rng.normal(size=(N, 2, L * (L + 2), R)) + 1j * rng.normal(size=(N, 2, L * (L + 2), R))
+    b = ClusterBatch([dict(position=pos, mie_scat=mie, k=1.05e7, p_src=p)], R=R, precision="fp64").assemble()
+    n0 = nat.lib().gb_launch_count()
+    b.solve(tol=1e-11)
+    launches = nat.lib().gb_launch_count() - n0
+    assert (launches == 1) == single, launches
+    d = (b.b - b.apply(b.x)).view(-1, R)
+    assert np.all((d.norm(dim=0) / b.b.view(-1, R).norm(dim=0)).cpu().numpy() < 2e-11)
+
+
 @pytest.mark.parametrize("R", [1, 2])
 def test_expired_team_wait_falls_back(R):
     """A cooperative team whose barrier runs out of its limit is no error: the
